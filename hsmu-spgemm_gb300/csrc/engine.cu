@@ -97,6 +97,10 @@ constexpr long long HOST_PANEL_BYTES = 32ll << 20;
 
 // entries of B from which its tile conversion runs on a second stream beside the bounds pass
 constexpr int TILES_ASIDE_MIN_NNZ = 1 << 19;
+// average entries of B's rows from which repeated rows are looked for: chains of shorter rows
+// are not taken (hsmu_products.cuh), and the chain kernel's registers cost rows without chains
+// (scalar 27-point rows: 296 us with it, 169 us without)
+constexpr int REPEAT_MIN_ROW = 36;
 constexpr long long HOST_MAX_PANELS = 8;
 constexpr double HOST_PANEL_GROWTH = 2.0;
 constexpr double HOST_PANEL_RATIO = 0.7;
@@ -255,6 +259,7 @@ struct PlainRun {
     bool tiles_aside = false;  // B's tiles are being built on the handle's conversion stream
     DevTiles Btd{};
     RowInfo ri{};
+    unsigned char *rep = nullptr;     // B rows that repeat the row before them
     long long *chunk_prod = nullptr;  // products per PROD_CHUNK rows (host-buffer entry)
     int *scan_tmp = nullptr;
     Window *win = nullptr;
@@ -333,6 +338,12 @@ struct PlainRun {
         }
         Btd = DevTiles{bt.tile_ptr, bt.tile_col, reinterpret_cast<const unsigned long long *>(bt.mask), bt.tile_off};
         if (ev_tiles) cudaEventRecord(ev_tiles, tiles_aside ? h->cs_tiles : st);
+        if (B->M > 0 && B->nnz >= (long long)REPEAT_MIN_ROW * B->M) {
+            CKR(palloc(&rep, (size_t)B->M, st));
+            launch_row_repeat(Bd, rep, grid_rows(h), st);
+            launches++;
+            ri.rep = rep;
+        }
         CKR(palloc(&ri.prod, (size_t)M, st));
         CKR(palloc(&ri.tmin, (size_t)M, st));
         CKR(palloc(&ri.tmax, (size_t)M, st));
@@ -490,6 +501,7 @@ struct PlainRun {
             pfree(bt.tile_off, st);
             own_tiles = false;
         }
+        pfree(rep, st);
         pfree(ri.prod, st);
         pfree(chunk_prod, st);
         pfree(ri.tmin, st);

@@ -48,6 +48,7 @@ struct RowInfo {
     signed char *cls;  // row class (RowBin) of every row, -1 for an empty row
     int *bin_cnt;      // [NBIN][ceil(M/32)] rows of each class per 32-row chunk, then
                        // its exclusive scan (bin_scratch_ints(M) entries)
+    const unsigned char *rep;  // B rows that repeat the row before them (nullable; launch_row_repeat)
     int store;         // 1: the tile store is in use -- the count pass sizes each large row's
                        // list, min(tile span, sum of its B rows' tile counts), and adds the
                        // sizes up in Ctl::store_tiles (the arena the next call wants)
@@ -88,6 +89,8 @@ size_t bin_scratch_ints(int M);
 void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int grid, cudaStream_t st);
 void launch_tiles_fill(const DevCSR &B, const int *tptr, int *tcol, unsigned long long *tmask, int *toff, Ctl *ctl,
                        int grid, cudaStream_t st);
+// rep[k]: row k of B has the columns of row k - 1 (B.M bytes)
+void launch_row_repeat(const DevCSR &B, unsigned char *rep, int grid, cudaStream_t st);
 void launch_validate(const DevCSR &A, Ctl *ctl, int grid, cudaStream_t st);
 
 // k_rows.cu

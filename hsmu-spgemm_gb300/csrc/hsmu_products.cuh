@@ -10,12 +10,25 @@
 //
 // The A entries are taken 32 at a time (one per lane); seg(p) gives the B
 // entry range [elo, ehi) that A entry p contributes to this accumulator.
-//   * long B segments (average >= LONG_SEG_MIN entries; callers may turn this
-//     path off): one segment at a time, in chunks of up to LU steps of 32
-//     entries.  Entries of one B row have distinct columns, so a chunk has no
-//     slot conflicts and only a change of segment needs a warp sync.  The
-//     next chunk's B loads are issued before the current chunk's
-//     multiply/lookup/add (software pipeline).
+//   * repeated rows (rep given): consecutive A entries whose B rows are
+//     consecutive and hold the same columns -- the rows of one finite-element
+//     node -- form chains of up to REP_MAX rows.  A lane takes one column of a
+//     chain: one look-up and one accumulator round trip for all its rows'
+//     products, added in row order.  The columns of successive chains are laid
+//     end to end over the lanes, which leaves none idle: the FP64 pipe, which
+//     binds these rows, takes as long for a step of 17 lanes as for one of 32.
+//     Two chains that share a step share no slot when the younger one's last
+//     column lies before the older one's first (stencil rows: always);
+//     otherwise they add one after the other.  27-point stencil, 40^3 grid x 3
+//     dofs: fused row kernel 5.68 -> 5.16 ms (FP64 pipe 78 % busy, no lane
+//     idle); holding the sums in registers over repeated rows without laying
+//     chains end to end left 16 % of the lanes idle and took 5.79 ms.
+//   * segments that fill steps of 32 well (callers may turn this path off): the
+//     segments one after another, 32 entries per step, the B loads of the next
+//     LU steps issued before the current ones are used.  Entries of one B row
+//     have distinct columns, so a step has no slot conflict and only a change
+//     of segment needs a warp sync.  Scalar 27-point rows (33^3 grid, fused
+//     multiply-add): 215 us on the flat path with its match per step, 169 us.
 //   * otherwise: the flat sequence of (A entry, B entry) items, 32 per step.
 //     The non-empty segments are packed into lanes; one OR-reduction per step
 //     marks the segment starts inside it, so every lane gets its segment from
@@ -51,29 +64,35 @@ __device__ __forceinline__ double add_term(double c, double a, double t) {
     return __dadd_rn(c, t);
 }
 
-// steps of 32 B entries per chunk of the long-segment path
+// steps of 32 B entries in flight on the segment path
 constexpr int LU = 3;
-// a group of A entries takes the long-segment path when its non-empty
-// segments average at least this many B entries (measured: the flat path
-// is as fast below it, e.g. on power-law rows)
-constexpr int LONG_SEG_MIN = 64;
+// groups of A entries take the segment path where one segment at a time keeps this share of
+// the lanes busy (27-point rows: 84 %); below it the flat path wins
+constexpr int WALK_LANES_PCT = 70;
+// most rows of a chain (4: the wider step's registers spill, 5.16 -> 5.99 ms), and the columns its leaders must average: shorter chains laid end to
+// end would often meet the same columns twice in a step
+constexpr int REP_MAX = 3;
+constexpr int CROSS_SEG_MIN = 36;
 
 // SegFn:    void(int p, int k, int &elo, int &ehi)  -- called for valid lanes
 // LookupFn: int(int j) -> slot in acc, or -1 if j is not in the accumulator
 // PG: load the next group of 32 A entries before processing the current one
 // (for rows with many A entries; costs registers in the short-row kernels)
+// REP: rep[k] is nonzero when B row k holds the same columns as row k - 1
+// (k_row_repeat); seg() must then give whole B rows.
 // TAG: `tag` is a byte per accumulator slot (any contents), used to find the
 // lanes of a step that share a slot; without it every multi-entry step runs
 // a full-warp match.
-// LONG: groups with long segments take the long-segment path (else every group
+// LONG: groups may take the segment path (else every group
 // runs flat, where a step inside one segment needs no conflict test either).
-template <int AR, bool NC = true, bool PG = false, bool TAG = false, bool LONG = true, class SegFn,
+template <int AR, bool NC = true, bool PG = false, bool TAG = false, bool LONG = true, bool REP = false,
+          class SegFn,
           class LookupFn>
 __device__ __forceinline__ void warp_accumulate(int a_lo, int a_hi, const int *__restrict__ acol,
                                                 const double *__restrict__ aval, const int *__restrict__ brp,
                                                 const int *__restrict__ bcol, const double *__restrict__ bval,
                                                 SegFn seg, LookupFn lookup, double *acc, bool &bad,
-                                                unsigned char *tag = nullptr) {
+                                                unsigned char *tag = nullptr, const unsigned char *rep = nullptr) {
     const int lane = lane_id();
     // A entries 32 at a time (PG: the next group's entries and segments are
     // loaded before the current group is processed)
@@ -84,8 +103,10 @@ __device__ __forceinline__ void warp_accumulate(int a_lo, int a_hi, const int *_
         seg(a_lo + lane, ldx<NC>(acol + a_lo + lane), n_elo, n_ehi);
     }
     for (int pb = a_lo; pb < a_hi; pb += WARP) {
-        int elo = 0, ehi = 0;
+        int elo = 0, ehi = 0, k = -1;
         double a = 0.0;
+        bool join = false;  // this entry's B row repeats the previous entry's
+        static_assert(!(PG && REP), "repeated rows are found in the group being processed");
         if (PG) {
             elo = n_elo;
             ehi = n_ehi;
@@ -99,85 +120,185 @@ __device__ __forceinline__ void warp_accumulate(int a_lo, int a_hi, const int *_
             }
         } else if (pb + lane < a_hi) {
             a = ldx<NC>(aval + pb + lane);
-            seg(pb + lane, ldx<NC>(acol + pb + lane), elo, ehi);
+            k = ldx<NC>(acol + pb + lane);
+            seg(pb + lane, k, elo, ehi);
+        }
+        if (REP) {
+            const int k_up = __shfl_up_sync(FULL, k, 1);
+            join = lane > 0 && k >= 0 && k == k_up + 1 && rep[k];
         }
         const int len = ehi - elo;
         const int incl = warp_incl_scan(len);
         const int total = __shfl_sync(FULL, incl, WARP - 1);
         if (total == 0) continue;
         const unsigned ne = __ballot_sync(FULL, len > 0);
-        unsigned todo = ne;
-        if (LONG && total >= LONG_SEG_MIN * __popc(todo)) {
-            // ---- long segments: one A entry at a time, its B entries in chunks of up
-            // to LU*32 (LU steps of 32); the next chunk's loads are issued before the
-            // current chunk is used.  Entries of one B row have distinct columns, so a
-            // chunk has no slot conflicts; a change of A entry needs a warp sync.
-            int sgi = __ffs(todo) - 1;
-            todo &= todo - 1;
-            int es = __shfl_sync(FULL, elo, sgi), ls = __shfl_sync(FULL, len, sgi);
-            double as = __shfl_sync(FULL, a, sgi);
-            int off = 0;
-            int jc[LU];
-            double bc[LU];
+        const int nseg = __popc(ne);
+        if (REP) {
+            // ---- repeated rows: the chains of each leader's columns, 32 per step
+            const unsigned jm = __ballot_sync(FULL, join);
+            const int pos = lane - (31 - __clz(~jm & lanemask_le()));  // place in the run of repeated rows
+            const unsigned behind = lane == 31 ? 0u : jm >> (lane + 1);
+            const int grp = min(REP_MAX, __ffs(~behind));            // rows of the chain a leader starts
+            unsigned todo = __ballot_sync(FULL, len > 0 && pos % REP_MAX == 0);
+            const int nlead = __popc(todo);
+            const int lead_len = ((todo >> lane) & 1u) ? len : 0;
+            const int items = (int)__reduce_add_sync(FULL, (unsigned)lead_len);
+            if (4 * nlead <= 3 * nseg && items >= CROSS_SEG_MIN * nlead) {
+                int es = 0, ls = 0, g = 0, l0 = 0, off = 0;  // current chain rows: first entry, length, rows, lane
+                auto next_seg = [&]() {
+                    l0 = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    es = __shfl_sync(FULL, elo, l0);
+                    ls = __shfl_sync(FULL, len, l0);
+                    g = __shfl_sync(FULL, grp, l0);
+                };
+                // one step: nv valid lanes, the first rm of them of the older leader (rm = 32: one
+                // leader); every lane's rows (gl), first lane (sl) and B entries (j, b)
+                auto fetch = [&](int &j, double *b, int &gl, int &sl, int &rm, int &nv) {
+                    nv = 0;
+                    if (off >= ls) {
+                        if (!todo) return;
+                        next_seg();
+                        off = 0;
+                    }
+                    int e = es + off + lane, l = ls;
+                    gl = g;
+                    sl = l0;
+                    rm = WARP;
+                    nv = min(WARP, ls - off);
+                    off += nv;
+                    if (nv < WARP && todo) {
+                        rm = nv;
+                        next_seg();
+                        off = min(WARP - rm, ls);
+                        nv = rm + off;
+                        if (lane >= rm) {
+                            e = es + lane - rm;
+                            l = ls;
+                            gl = g;
+                            sl = l0;
+                        }
+                    }
+                    j = 0;
+                    if (lane < nv) j = ldx<NC>(bcol + e);
+                    else gl = 0;
+#pragma unroll
+                    for (int m = 0; m < REP_MAX; m++) {
+                        b[m] = 0.0;
+                        if (m < gl) b[m] = ldx<NC>(bval + e + m * l);
+                    }
+                };
+                int jc = 0, gc = 0, lc = 0, rc = WARP, nc;
+                double bc[REP_MAX];
+                fetch(jc, bc, gc, lc, rc, nc);
+                while (nc > 0) {
+                    int jn = 0, gn = 0, ln = 0, rn = WARP, nn;
+                    double bn[REP_MAX];
+                    fetch(jn, bn, gn, ln, rn, nn);
+                    const int q = lookup(jc);
+                    const bool act = lane < nc && q >= 0;
+                    bad |= lane < nc && q < 0;
+                    double av[REP_MAX], pr[REP_MAX];
+                    const int gm = (int)__reduce_max_sync(FULL, (unsigned)gc);
+#pragma unroll
+                    for (int m = 0; m < REP_MAX; m++) {
+                        if (m < gm) {
+                            av[m] = __shfl_sync(FULL, a, lc + m);
+                            pr[m] = term<AR>(av[m], bc[m]);
+                        }
+                    }
+                    auto chain = [&]() {
+                        double v = acc[q];
+#pragma unroll
+                        for (int m = 0; m < REP_MAX; m++)
+                            if (m < gc) v = add_term<AR>(v, av[m], pr[m]);
+                        acc[q] = v;
+                    };
+                    // two leaders: their columns ascend, so when the younger one's last column
+                    // lies before the older one's first, no two lanes share a slot
+                    if (rc == WARP || __shfl_sync(FULL, jc, nc - 1) < __shfl_sync(FULL, jc, 0)) {
+                        if (act) chain();
+                    } else {
+                        if (act && lane < rc) chain();
+                        __syncwarp();
+                        if (act && lane >= rc) chain();
+                    }
+                    __syncwarp();
+                    jc = jn;
+                    gc = gn;
+                    lc = ln;
+                    rc = rn;
+                    nc = nn;
+#pragma unroll
+                    for (int m = 0; m < REP_MAX; m++) bc[m] = bn[m];
+                }
+                continue;
+            }
+        }
+        if (LONG && 32 * WALK_LANES_PCT * (int)__reduce_add_sync(FULL, (unsigned)(len + 31) >> 5) <= 100 * total) {
+            // ---- one segment after another, 32 entries per step
+            unsigned todo = ne;
+            int es = 0, ls = 0, off = 0;  // current segment: first entry, length, entries taken
+            double as = 0.0;
+            // one step: nv valid lanes (0: no step left), sy: the first of its segment
+            auto fetch = [&](int &j, double &b, double &av, int &nv, bool &sy) {
+                nv = 0;
+                sy = false;
+                if (off >= ls) {
+                    if (!todo) return;
+                    const int sgi = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    es = __shfl_sync(FULL, elo, sgi);
+                    ls = __shfl_sync(FULL, len, sgi);
+                    as = __shfl_sync(FULL, a, sgi);
+                    off = 0;
+                    sy = true;
+                }
+                nv = min(WARP, ls - off);
+                av = as;
+                if (lane < nv) {
+                    j = ldx<NC>(bcol + es + off + lane);
+                    b = ldx<NC>(bval + es + off + lane);
+                }
+                off += nv;
+            };
+            int jc[LU], nc[LU];
+            double bc[LU], ac[LU];
+            bool sc[LU];
 #pragma unroll
             for (int u = 0; u < LU; u++) {
-                const int e = u * WARP + lane;
                 jc[u] = 0;
-                bc[u] = 0.0;
-                if (e < ls) {
-                    jc[u] = ldx<NC>(bcol + es + e);
-                    bc[u] = ldx<NC>(bval + es + e);
-                }
+                bc[u] = ac[u] = 0.0;
+                fetch(jc[u], bc[u], ac[u], nc[u], sc[u]);
             }
-            while (true) {
-                int n_off = off + LU * WARP, n_es = es, n_ls = ls;
-                double n_as = as;
-                bool more = true, seg_change = false;
-                if (n_off >= ls) {
-                    if (!todo) {
-                        more = false;
-                    } else {
-                        const int n_sgi = __ffs(todo) - 1;
-                        todo &= todo - 1;
-                        n_es = __shfl_sync(FULL, elo, n_sgi);
-                        n_ls = __shfl_sync(FULL, len, n_sgi);
-                        n_as = __shfl_sync(FULL, a, n_sgi);
-                        n_off = 0;
-                        seg_change = true;
-                    }
-                }
-                int jn[LU];
-                double bn[LU];
+            while (nc[0] > 0) {
+                int jn[LU], nn[LU];
+                double bn[LU], an[LU];
+                bool sn[LU];
 #pragma unroll
                 for (int u = 0; u < LU; u++) {
-                    const int e = n_off + u * WARP + lane;
                     jn[u] = 0;
-                    bn[u] = 0.0;
-                    if (more && e < n_ls) {
-                        jn[u] = ldx<NC>(bcol + n_es + e);
-                        bn[u] = ldx<NC>(bval + n_es + e);
-                    }
+                    bn[u] = an[u] = 0.0;
+                    fetch(jn[u], bn[u], an[u], nn[u], sn[u]);
                 }
 #pragma unroll
                 for (int u = 0; u < LU; u++) {
-                    if (off + u * WARP >= ls) break;  // warp-uniform: the chunk is shorter
-                    if (off + u * WARP + lane < ls) {
-                        const double pr = term<AR>(as, bc[u]);
-                        const int q = lookup(jc[u]);
-                        if (q >= 0) acc[q] = add_term<AR>(acc[q], as, pr);
-                        else bad = true;
-                    }
+                    if (nc[u] == 0) break;
+                    if (sc[u]) __syncwarp();
+                    // every lane multiplies and looks up (invalid lanes: b = 0, result unused)
+                    const double pr = term<AR>(ac[u], bc[u]);
+                    const int q = lookup(jc[u]);
+                    const bool v = lane < nc[u];
+                    bad |= v && q < 0;
+                    if (v && q >= 0) acc[q] = add_term<AR>(acc[q], ac[u], pr);
                 }
-                if (!more) break;
-                if (seg_change) __syncwarp();
-                es = n_es;
-                ls = n_ls;
-                as = n_as;
-                off = n_off;
 #pragma unroll
                 for (int u = 0; u < LU; u++) {
                     jc[u] = jn[u];
                     bc[u] = bn[u];
+                    ac[u] = an[u];
+                    nc[u] = nn[u];
+                    sc[u] = sn[u];
                 }
             }
             __syncwarp();
@@ -189,7 +310,6 @@ __device__ __forceinline__ void warp_accumulate(int a_lo, int a_hi, const int *_
         // fall inside it into one 32-bit mask; the segment of a lane's item is
         // then the number of starts up to it (one popc), and a step with no
         // start after its first item holds one A entry (no slot conflicts).
-        const int nseg = __popc(ne);
         const int excl = incl - len;
         const int src = nth_set_bit(ne, min(lane, nseg - 1));
         const int st_src = __shfl_sync(FULL, excl, src);

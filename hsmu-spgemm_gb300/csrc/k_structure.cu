@@ -107,7 +107,8 @@ struct SdsSmem {
 };
 static_assert(SDS_WARPS * sizeof(SdsSmem) * SDS_CTAS_PER_SM <= 227 * 1024, "CTAs per SM fit in shared memory");
 
-template <int AR>
+// REP: ri.rep is given, and repeated B rows are taken as chains (hsmu_products.cuh)
+template <int AR, bool REP>
 __global__ void __launch_bounds__(SDS_WARPS * 32, SDS_CTAS_PER_SM)
     k_struct_ds(int M, const int *__restrict__ arp, const int *__restrict__ acol, const double *__restrict__ aval,
                 const int *__restrict__ brp, const int *__restrict__ bcol, const double *__restrict__ bval,
@@ -196,7 +197,8 @@ __global__ void __launch_bounds__(SDS_WARPS * 32, SDS_CTAS_PER_SM)
                 return tile_slot(S.msk[t], S.base[t], j);
             };
             bool vbad = false;
-            warp_accumulate<AR>(arp[i], arp[i + 1], acol, aval, brp, bcol, bval, seg, lookup, S.acc, vbad);
+            warp_accumulate<AR, true, false, false, true, REP>(arp[i], arp[i + 1], acol, aval, brp, bcol, bval, seg,
+                                                               lookup, S.acc, vbad, nullptr, ri.rep);
             __syncwarp();
             for (int q = lane; q < nnz; q += WARP) cval[rowbase + q] = S.acc[q];
             if (__any_sync(FULL, vbad) && lane == 0) set_err(&ctl->err, DERR_INTERNAL);
@@ -523,7 +525,10 @@ void launch_structure(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowI
         kt<<<nsm * 4, TINYF_THREADS, 0, st>>>(A.M, A.rp, A.col, A.val, B.rp, B.col, B.val, ri, out, ctl);
     }
     if (!class_rows || class_rows[BIN_DS] > 0) {
-        auto kds = arith == AR_IMUL ? k_struct_ds<AR_IMUL> : arith == AR_FMA ? k_struct_ds<AR_FMA> : k_struct_ds<AR_RN>;
+        const bool rep = ri.rep != nullptr;
+        auto kds = arith == AR_IMUL  ? (rep ? k_struct_ds<AR_IMUL, true> : k_struct_ds<AR_IMUL, false>)
+                   : arith == AR_FMA ? (rep ? k_struct_ds<AR_FMA, true> : k_struct_ds<AR_FMA, false>)
+                                     : (rep ? k_struct_ds<AR_RN, true> : k_struct_ds<AR_RN, false>);
         kds<<<nsm * SDS_CTAS_PER_SM, SDS_WARPS * 32, SDS_WARPS * sizeof(SdsSmem), st>>>(
             A.M, A.rp, A.col, A.val, B.rp, B.col, B.val, Bt.ptr, Bt.col, Bt.mask, ri, out, win, win_cap, ctl);
     }
@@ -539,7 +544,8 @@ void launch_structure(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowI
 }
 
 int configure_structure() {
-    for (auto k : {k_struct_ds<AR_RN>, k_struct_ds<AR_FMA>, k_struct_ds<AR_IMUL>}) {
+    for (auto k : {k_struct_ds<AR_RN, false>, k_struct_ds<AR_FMA, false>, k_struct_ds<AR_IMUL, false>,
+                   k_struct_ds<AR_RN, true>, k_struct_ds<AR_FMA, true>, k_struct_ds<AR_IMUL, true>}) {
         const int e = (int)cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 SDS_WARPS * (int)sizeof(SdsSmem));
         if (e) return e;

@@ -113,6 +113,29 @@ void launch_tiles_fill(const DevCSR &B, const int *tptr, int *tcol, unsigned lon
     k_tiles<true><<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, const_cast<int *>(tptr), tcol, tmask, toff, 0, ctl);
 }
 
+// rep[k] = 1 when row k of B holds the same columns as row k - 1 (the rows of one finite-element
+// node; the fused row kernel chains their products).  One warp per row, stopped at the first
+// difference.
+__global__ void __launch_bounds__(256) k_row_repeat(int K, const int *__restrict__ brp, const int *__restrict__ bcol,
+                                                    unsigned char *__restrict__ rep) {
+    const int lane = lane_id();
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    for (int k = gw; k < K; k += nw) {
+        const int s = brp[k], n = brp[k + 1] - s;
+        bool same = k > 0 && n > 0 && s - brp[k - 1] == n;
+        for (int base = 0; same && base < n; base += WARP) {
+            const int i = base + lane;
+            same = !__any_sync(FULL, i < n && __ldg(bcol + s + i) != __ldg(bcol + s - n + i));
+        }
+        if (lane == 0) rep[k] = same;
+    }
+}
+
+void launch_row_repeat(const DevCSR &B, unsigned char *rep, int grid, cudaStream_t st) {
+    k_row_repeat<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, rep);
+}
+
 // Validation of A: sorted, unique, in-range columns (one warp per row).
 __global__ void __launch_bounds__(256) k_validate(int M, const int *__restrict__ rp, const int *__restrict__ col,
                                                   int N, long long nnz, Ctl *ctl) {
