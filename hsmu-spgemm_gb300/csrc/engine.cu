@@ -449,6 +449,7 @@ struct PlainRun {
         CKR(palloc(&wc.scan_tmp, scan_tmp_ints((int)nwin), st));
         CKR(palloc(&wc.item_off, (size_t)nwin + 1, st));
         CKR(palloc(&wc.cur, (size_t)cap, st));
+        CKR(palloc(&wc.heavy, (size_t)nwin, st));
         return HSMU_OK;
     }
 
@@ -523,6 +524,7 @@ struct PlainRun {
         pfree(wc.scan_tmp, st);
         pfree(wc.item_off, st);
         pfree(wc.cur, st);
+        pfree(wc.heavy, st);
         pfree(crp, st);
         if (ext_col) {
             ccol = nullptr;
@@ -957,6 +959,7 @@ learned:
             CK(palloc(&wc.scan_tmp, scan_tmp_ints((int)win_cap), st));
             CK(palloc(&wc.item_off, (size_t)win_cap + 1, st));
             CK(palloc(&wc.cur, (size_t)cur_cap, st));
+            CK(palloc(&wc.heavy, (size_t)win_cap, st));
         }
         if (stats) cudaEventRecord(h->ev[3], st);
         // structure (+ values of warp-sized rows) into the slots; exact counts found here.
@@ -1066,6 +1069,7 @@ done:
     pfree(wc.scan_tmp, st);
     pfree(wc.item_off, st);
     pfree(wc.cur, st);
+    pfree(wc.heavy, st);
     pfree(crp, st);
     pfree(ccol, st);
     pfree(cval, st);

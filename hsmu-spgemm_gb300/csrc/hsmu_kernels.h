@@ -153,6 +153,7 @@ struct WinCursors {
     int *scan_tmp;
     int *item_off;  // the cursor pass's work items per window, scanned in place
     int *cur;
+    int *heavy;     // windows of rows with many A entries (win_cap entries)
     long long cap;
 };
 void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const int *crp, int *ccol, double *cval,

@@ -46,6 +46,16 @@ namespace hsmu {
 constexpr int NUM_WARPS = 3;
 constexpr int NUM_CTAS_PER_SM = 6;
 constexpr int GW = 2;  // consecutive windows per work item, handed out dynamically
+// A window is walked by one warp, 32 A entries at a time, so the windows of rows with thousands
+// of A entries take the longest: handed out in array order, the last ones of a launch (of a row
+// panel above all) run alone at its end.  They go first instead, one by one: rows of HEAVY_ROW
+// entries or more, then of LONG_ROW, then the others.  k_numeric: R-MAT scale 15 with its
+// transpose cropped to 30,011 vertices 1.49 -> 1.01 ms, scale 16 2.93 -> 2.27, scale 18
+// 19.00 -> 18.57, four row panels of a 49,999-vertex graph 2.75 -> 1.92 ms.  (One limit of 2,048
+// changed little, one of 512 gave 2.43 and one of 128 2.30 ms at scale 16; second limits of 64 and
+// first ones of 384 or 768 are within 3 % of these.)
+constexpr int HEAVY_ROW = 512;
+constexpr int LONG_ROW = 128;
 constexpr int STAGE_LIMIT = 1 << 20;  // polls of a column copy before the kernel reports a timeout
 
 // per warp; acc first: it also receives the window's columns by bulk copy
@@ -78,10 +88,12 @@ __device__ __forceinline__ bool cur_continues(const Window *win, int w, int row,
 // here: up to the next window's first slot when that window continues the
 // same row, else up to the row's end; and its tile count likewise, up to the
 // next window's first tile or the end of the row's list.
+// Windows of rows with at least HEAVY_ROW A entries are listed (in any order) from the front of
+// `heavy`, those of rows with at least LONG_ROW from its back: the value pass hands them out first.
 __global__ void __launch_bounds__(256) k_win_len(Window *__restrict__ win, int win_cap, int M, const int *__restrict__ arp,
                                                  const int *__restrict__ crp, const long long *__restrict__ ts_off,
                                                  const int *__restrict__ ts_cnt, Ctl *ctl, int *__restrict__ len,
-                                                 int *__restrict__ items) {
+                                                 int *__restrict__ items, int *__restrict__ heavy) {
     const int nwin = min(ctl->win_count, win_cap);
     for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < win_cap; w += gridDim.x * blockDim.x) {
         int n = 0, it = 0;
@@ -94,6 +106,8 @@ __global__ void __launch_bounds__(256) k_win_len(Window *__restrict__ win, int w
                 continue;
             }
             n = arp[row + 1] - arp[row];
+            if (n >= HEAVY_ROW) heavy[atomicAdd(&ctl->win_heavy, 1)] = w;
+            else if (n >= LONG_ROW) heavy[win_cap - 1 - atomicAdd(&ctl->win_long, 1)] = w;
             // a chunk of the cursor pass starts here: one work item per 32 A entries
             if (!cur_continues(win, w, row, win[w].t0)) it = (n + WARP - 1) / WARP;
             if (win[w].cnt == 0) {
@@ -207,7 +221,8 @@ __global__ void __launch_bounds__(NUM_WARPS * 32, NUM_CTAS_PER_SM) k_numeric(con
                                                             const long long *__restrict__ woff,
                                                             const int *__restrict__ wcur, int wait_polls, int M,
                                                             const int *__restrict__ ts_tcol,
-                                                            const TileEnt *__restrict__ ts_tent, Ctl *ctl) {
+                                                            const TileEnt *__restrict__ ts_tent,
+                                                            const int *__restrict__ heavy, Ctl *ctl) {
     extern __shared__ __align__(16) unsigned long long s_dyn[];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     NumSmem &S = reinterpret_cast<NumSmem *>(s_dyn)[w];
@@ -215,7 +230,8 @@ __global__ void __launch_bounds__(NUM_WARPS * 32, NUM_CTAS_PER_SM) k_numeric(con
     __syncwarp();
     unsigned phase = 0;
     const int nwin = min(ctl->win_count, win_cap);
-    const int ngroups = (nwin + GW - 1) / GW;
+    const int nheavy = ctl->win_heavy, nlisted = nheavy + ctl->win_long;
+    const int ngroups = nlisted + (nwin + GW - 1) / GW;
     bool bad = false;
     // window costs differ by orders of magnitude (rows with thousands of A entries):
     // warps take the next group of windows from a counter instead of a fixed stride
@@ -224,14 +240,17 @@ __global__ void __launch_bounds__(NUM_WARPS * 32, NUM_CTAS_PER_SM) k_numeric(con
         if (lane == 0) g = atomicAdd(&ctl->win_next, 1);
         g = __shfl_sync(FULL, g, 0);
         if (g >= ngroups) break;
-        const int wend = min(nwin, (g + 1) * GW);
-        for (int wi = g * GW; wi < wend; wi++) {
+        const bool listed = g < nlisted;  // one listed window, else GW windows less the listed ones
+        const int wbeg = !listed ? (g - nlisted) * GW : heavy[g < nheavy ? g : win_cap - 1 - (g - nheavy)];
+        const int wend = listed ? wbeg + 1 : min(nwin, wbeg + GW);
+        for (int wi = wbeg; wi < wend; wi++) {
             const Window W = win[wi];
             const int row = W.row, cnt = W.cnt, t0 = W.t0;
             if ((unsigned)row >= (unsigned)M) {  // reported by k_win_len
                 bad = true;
                 continue;
             }
+            if (!listed && arp[row + 1] - arp[row] >= LONG_ROW) continue;
             if (flag && flag[row] == ROW_OVERFLOW && !W.redo) continue;  // stale: the redo pass emitted fresh windows
             const int row_lo = crp[row], row_hi = crp[row + 1];
             const int s0 = row_lo + W.s0;  // windows carry row-relative offsets
@@ -452,9 +471,9 @@ void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const 
                     const long long *soff, const WinCursors &wc, Ctl *ctl, int arith, int nsm, cudaStream_t st,
                     int wait_polls, const TileStore *ts) {
     if (win_cap <= 0) return;
-    cudaMemsetAsync(&ctl->win_next, 0, sizeof(int), st);
+    cudaMemsetAsync(&ctl->win_next, 0, 3 * sizeof(int), st);  // and win_heavy, win_long
     k_win_len<<<nsm * 4, 256, 0, st>>>(const_cast<Window *>(win), (int)win_cap, A.M, A.rp, crp, ts ? ts->off : nullptr,
-                                       ts ? ts->cnt : nullptr, ctl, wc.len, wc.item_off);
+                                       ts ? ts->cnt : nullptr, ctl, wc.len, wc.item_off, wc.heavy);
     launch_scan64(wc.len, wc.off, (int)win_cap, wc.total, wc.scan_tmp, st);
     launch_scan(wc.item_off, wc.item_off, (int)win_cap, wc.total + 1, wc.scan_tmp, ctl, st);
     k_win_cursors<<<nsm * 16, 256, 0, st>>>(win, (int)win_cap, A.M, wc.off, wc.cap, A.rp, A.col, B.rp, Bt.ptr, Bt.col,
@@ -462,7 +481,7 @@ void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const 
     auto k = arith == AR_IMUL ? k_numeric<AR_IMUL> : arith == AR_FMA ? k_numeric<AR_FMA> : k_numeric<AR_RN>;
     k<<<nsm * NUM_CTAS_PER_SM, NUM_WARPS * 32, NUM_WARPS * sizeof(NumSmem), st>>>(
         A.rp, A.col, A.val, B.rp, B.col, B.val, crp, ccol, cval, win, (int)win_cap, flag, scol, soff, wc.off, wc.cur,
-        wait_polls, A.M, ts ? ts->tcol : nullptr, ts ? ts->tent : nullptr, ctl);
+        wait_polls, A.M, ts ? ts->tcol : nullptr, ts ? ts->tent : nullptr, wc.heavy, ctl);
 }
 
 int configure_numeric() {
