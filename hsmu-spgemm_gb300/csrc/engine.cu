@@ -41,6 +41,7 @@ int status_from_dev_err(int err) {
 }
 int configure_structure();
 int configure_numeric();
+int configure_scattered();
 }  // namespace hsmu
 
 using namespace hsmu;
@@ -406,7 +407,7 @@ struct PlainRun {
             launches += 3;
         }
         launch_scan(ri.cnnz, crp, M, &ctl->nnz, scan_tmp, ctl, st);
-        launches += 6;  // count 3, scan 3
+        launches += 6 + (Bd.N > SPAN_T * 64);  // count 3 (and the scattered rows'), scan 3
         CKR(cudaGetLastError());
         CKR(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
         if (host_rp) CKR(cudaMemcpyAsync(host_rp, crp, sizeof(int32_t) * ((size_t)M + 1), cudaMemcpyDeviceToHost, st));
@@ -973,8 +974,8 @@ learned:
         // without barriers.
         TileStore tsd{r.ts_off, r.ts_cnt, r.ts_nwin, r.ts_wbase, h->arena_col, h->arena_ent,
                       h->arena_cap, 0};
-        const int small_rows[NBIN] = {hc.bin_count[BIN_DS], 0, hc.bin_count[BIN_TINY]};
-        const int large_rows[NBIN] = {0, hc.bin_count[BIN_L], 0};
+        const int small_rows[NBIN] = {hc.bin_count[BIN_DS], 0, hc.bin_count[BIN_TINY], hc.bin_count[BIN_H]};
+        const int large_rows[NBIN] = {0, hc.bin_count[BIN_L], 0, 0};
         if (hc.bin_count[BIN_L] > 0 && r.have_store) {
             launch_spec_large(Ad, Btd, ri, tsd, spec, ctl, h->nsm, st);
             launch_scan(r.ts_nwin, r.ts_wbase, M, &ctl->win_listed, r.scan_tmp, ctl, st);
@@ -1267,6 +1268,7 @@ int hsmu_handle_create(hsmu_handle *out) {
     int e = configure_count();
     if (!e) e = configure_structure();
     if (!e) e = configure_numeric();
+    if (!e) e = configure_scattered();
     if (e) {
         hsmu_handle_destroy(h);
         return HSMU_ERR_CUDA;

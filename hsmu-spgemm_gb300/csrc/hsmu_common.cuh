@@ -42,8 +42,14 @@ enum RowBin : int {
     BIN_DS = 0,    // tile span <= SPAN_T : one warp, dense span table
     BIN_L = 1,     // wider rows          : one CTA, dense chunked table
     BIN_TINY = 2,  // <= TINY_MAX products: one thread, sorted insertion list
-    NBIN = 3
+    BIN_H = 3,     // wide span, <= H_MAX products: one warp, ranked tiles (k_scatter.cu)
+    NBIN = 4
 };
+// limits of the scattered class: a row's entries of A (a lane each), its products (16 per lane, in
+// registers) and its tile span (one bit per tile in shared memory: 1,048,576 columns)
+constexpr int H_ROW = 32;
+constexpr int H_MAX = 512;
+constexpr int H_SPAN = 16384;
 
 // device error bits (ctl->err)
 enum DevErr : int {

@@ -132,6 +132,11 @@ void launch_count_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const T
 void launch_spec_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const TileStore &ts, RowOut out, Ctl *ctl,
                        int nsm, cudaStream_t st);
 
+// k_scatter.cu: rows of the scattered class (exact count; columns and values)
+void launch_count_scattered(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int nsm, cudaStream_t st);
+void launch_fill_scattered(const DevCSR &A, const DevCSR &B, RowInfo ri, RowOut out, Ctl *ctl, int arith, int nsm,
+                           cudaStream_t st);
+
 // k_structure.cu
 // writes C's columns and numeric windows; rows that fit one warp also get their values
 // class_rows: rows per class (BIN_*) when known on the host; kernels of empty classes are skipped

@@ -156,6 +156,24 @@ __device__ bool chunk_to_list(const unsigned long long *msk, int len, int c0, in
     return fits;
 }
 
+// positions [b0, b1) of a bin (rows in ascending order) that hold the panel's rows lo <= i < hi
+__device__ __forceinline__ void bin_slice(const int *rows, int n, const RowOut &o, int M, int &b0, int &b1) {
+    b0 = o.lo > 0 ? lower_bound_i32(rows, 0, n, o.lo) : 0;
+    b1 = o.hi < M ? lower_bound_i32(rows, b0, n, o.hi) : n;
+}
+
+// rows outside the panel, and in REDO mode rows that fitted their slots, are left alone
+__device__ __forceinline__ bool skip_row(const RowOut &o, int i) {
+    return i < o.lo || i >= o.hi || (o.mode == OUT_REDO && o.flag[i] != ROW_OVERFLOW);
+}
+
+__device__ __forceinline__ long long out_base(const RowOut &o, int i) {
+    return o.mode == OUT_SPEC ? o.soff[i] : (long long)o.crp[i];
+}
+__device__ __forceinline__ int out_limit(const RowOut &o, int i) {
+    return o.mode == OUT_SPEC ? (int)(o.soff[i + 1] - o.soff[i]) : o.crp[i + 1] - o.crp[i];
+}
+
 // Columns of 32 consecutive tiles of a row's list, one per lane (t, m; lanes
 // past the list carry m = 0), whose first entry goes to out[0].  The tiles'
 // entries are consecutive in the row:

@@ -66,14 +66,15 @@ __global__ void __launch_bounds__(256) k_bounds(int M, const int *__restrict__ a
                 ri.cnnz[i] = 0;
             } else {
                 const int span = tmax - tmin + 1;
-                bin = prod <= TINY_MAX ? BIN_TINY : (span <= SPAN_T ? BIN_DS : BIN_L);
+                const bool scattered = prod <= H_MAX && span <= H_SPAN && arp[i + 1] - arp[i] <= H_ROW;
+                bin = prod <= TINY_MAX ? BIN_TINY : span <= SPAN_T ? BIN_DS : scattered ? BIN_H : BIN_L;
                 atomicAdd(&s_cnt[bin], 1);
                 my_prod += (unsigned long long)prod;
                 const long long cap = prod < (long long)N ? prod : (long long)N;
                 // windows per row <= slot cuts + tile-rank cuts + span cuts + 1
                 const long long tl = cap < (long long)span ? cap : (long long)span;
                 const unsigned long long wb = (unsigned long long)(cap / WIN_CUT + tl / WIN_TCAP + (span - 1) / WIN_SPAN + 1);
-                my_wb += wb;
+                if (bin == BIN_L || (bin == BIN_DS && prod > FUSE_CAP)) my_wb += wb;
                 // rows that can reach the window pass: the large class, and warp rows above FUSE_CAP
                 if (bin == BIN_L) {
                     my_cb += wb * (unsigned long long)(arp[i + 1] - arp[i]);

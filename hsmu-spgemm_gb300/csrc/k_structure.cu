@@ -75,24 +75,6 @@ __device__ __forceinline__ void emit_tiles(const unsigned long long *msk, const 
     }
 }
 
-// positions [b0, b1) of a bin (rows in ascending order) that hold the panel's rows lo <= i < hi
-__device__ __forceinline__ void bin_slice(const int *rows, int n, const RowOut &o, int M, int &b0, int &b1) {
-    b0 = o.lo > 0 ? lower_bound_i32(rows, 0, n, o.lo) : 0;
-    b1 = o.hi < M ? lower_bound_i32(rows, b0, n, o.hi) : n;
-}
-
-// rows outside the panel, and in REDO mode rows that fitted their slots, are left alone
-__device__ __forceinline__ bool skip_row(const RowOut &o, int i) {
-    return i < o.lo || i >= o.hi || (o.mode == OUT_REDO && o.flag[i] != ROW_OVERFLOW);
-}
-
-__device__ __forceinline__ long long out_base(const RowOut &o, int i) {
-    return o.mode == OUT_SPEC ? o.soff[i] : (long long)o.crp[i];
-}
-__device__ __forceinline__ int out_limit(const RowOut &o, int i) {
-    return o.mode == OUT_SPEC ? (int)(o.soff[i + 1] - o.soff[i]) : o.crp[i + 1] - o.crp[i];
-}
-
 constexpr int SDS_WARPS = 4;
 constexpr int SDS_CTAS_PER_SM = 6;
 constexpr int SDS_WL = 64;     // > max windows of one DS row (slot cuts + tile cuts + 1)
@@ -524,6 +506,8 @@ void launch_structure(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowI
         auto kt = arith == AR_IMUL ? k_fill_tiny<AR_IMUL> : arith == AR_FMA ? k_fill_tiny<AR_FMA> : k_fill_tiny<AR_RN>;
         kt<<<nsm * 4, TINYF_THREADS, 0, st>>>(A.M, A.rp, A.col, A.val, B.rp, B.col, B.val, ri, out, ctl);
     }
+    if (class_rows ? class_rows[BIN_H] > 0 : B.N > SPAN_T * 64)
+        launch_fill_scattered(A, B, ri, out, ctl, arith, nsm, st);
     if (!class_rows || class_rows[BIN_DS] > 0) {
         const bool rep = ri.rep != nullptr;
         auto kds = arith == AR_IMUL  ? (rep ? k_struct_ds<AR_IMUL, true> : k_struct_ds<AR_IMUL, false>)

@@ -214,6 +214,7 @@ __global__ void __launch_bounds__(TINY_THREADS) k_count_tiny(int M, const int *_
 void launch_count_small(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm,
                         cudaStream_t st) {
     k_count_tiny<<<nsm * 4, TINY_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, ri, ctl);
+    if (B.N > SPAN_T * 64) launch_count_scattered(A, B, ri, ctl, nsm, st);  // else no row's span is that wide
     k_count_ds<<<nsm * 6, DS_WARPS * 32, 0, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, ctl);
 }
 
