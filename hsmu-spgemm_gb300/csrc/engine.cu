@@ -46,8 +46,24 @@ int configure_scattered();
 
 using namespace hsmu;
 
+// Scratch of a handle's calls: one block, handed out from its start and taken back when the
+// call ends (every call waits for its work before it returns, so nothing still reads it then,
+// whatever stream the next call uses).  What does not fit comes from a memory pool of the
+// handle's own, and the block then grows to the call's need, up to SCRATCH_BLOCK_MAX.  C's arrays
+// stay in the device's default pool: with the scratch carved from the block a freed C had left
+// there, the pool re-mapped memory for every second C (1 ms for 2 GB, 7 ms for 15 GB).
+struct Scratch {
+    char *base = nullptr;
+    size_t cap = 0, used = 0;    // the block
+    size_t need = 0, peak = 0;   // bytes handed out, in the block or not; the most in a call
+    int depth = 0;               // nested scopes
+    cudaMemPool_t pool = nullptr;
+    std::vector<void *> extra;   // allocations outside the block
+};
+
 struct hsmu_handle_s {
     int device;
+    Scratch scratch;
     int nsm;
     Ctl *h_ctl;  // pinned host mirror of the control block
     cudaEvent_t ev[8];
@@ -165,6 +181,78 @@ void pfree(T *&p, cudaStream_t st) {
     p = nullptr;
 }
 
+// the block a handle keeps between calls, and what its pool may hold on to beyond it
+constexpr size_t SCRATCH_BLOCK_MAX = 1ull << 30;
+constexpr unsigned long long SCRATCH_POOL_KEEP = 8ull << 30;
+constexpr size_t SCRATCH_ALIGN = 256;
+
+// scratch of the current call (released with the ScratchScope around it)
+template <class T>
+cudaError_t salloc(hsmu_handle_s *h, T **p, size_t n, cudaStream_t st) {
+    Scratch &s = h->scratch;
+    *p = nullptr;
+    const size_t bytes = ((n ? n : 1) * sizeof(T) + SCRATCH_ALIGN - 1) & ~(SCRATCH_ALIGN - 1);
+    if (g_fail_alloc_countdown.load(std::memory_order_relaxed) > 0 &&
+        g_fail_alloc_countdown.fetch_sub(1, std::memory_order_relaxed) == 1)
+        return cudaErrorMemoryAllocation;
+    if (bytes <= s.cap - s.used) {
+        *p = reinterpret_cast<T *>(s.base + s.used);
+        s.used += bytes;
+    } else {
+        void *q = nullptr;
+        const cudaError_t e = cudaMallocFromPoolAsync(&q, bytes, s.pool, st);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            return e;
+        }
+        try {
+            s.extra.push_back(q);
+        } catch (const std::bad_alloc &) {
+            cudaFreeAsync(q, st);
+            return cudaErrorMemoryAllocation;
+        }
+        *p = reinterpret_cast<T *>(q);
+    }
+    s.need += bytes;
+    s.peak = std::max(s.peak, s.need);
+    return cudaSuccess;
+}
+
+// gives back, at its end, what was taken since its start; the outermost one (a public call's)
+// then sizes the block for what the call needed.  `st` has finished every use by then.
+struct ScratchScope {
+    hsmu_handle_s *h;
+    cudaStream_t st;
+    size_t used, need, extra;
+    ScratchScope(hsmu_handle_s *h_, cudaStream_t st_)
+        : h(h_), st(st_), used(h_->scratch.used), need(h_->scratch.need), extra(h_->scratch.extra.size()) {
+        if (h->scratch.depth++ == 0) h->scratch.peak = 0;
+    }
+    ScratchScope(const ScratchScope &) = delete;
+    ~ScratchScope() {
+        Scratch &s = h->scratch;
+        while (s.extra.size() > extra) {
+            cudaFreeAsync(s.extra.back(), st);
+            s.extra.pop_back();
+        }
+        s.used = used;
+        s.need = need;
+        if (--s.depth > 0 || s.peak <= s.cap || s.cap >= SCRATCH_BLOCK_MAX) return;
+        if (s.base) cudaFreeAsync(s.base, st);
+        s.base = nullptr;
+        s.cap = 0;
+        const size_t want = std::min(SCRATCH_BLOCK_MAX, s.peak + s.peak / 4 + (1 << 20));
+        void *q = nullptr;
+        // the block must be there for a later call on any stream
+        if (cudaMallocFromPoolAsync(&q, want, s.pool, st) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) {
+            s.base = static_cast<char *>(q);
+            s.cap = want;
+        } else {
+            (void)cudaGetLastError();
+        }
+    }
+};
+
 int grid_rows(const hsmu_handle_s *h) { return h->nsm * 8; }
 
 // arrays the library allocated from the stream-ordered pool and handed to the caller:
@@ -181,13 +269,12 @@ void free_owned(std::initializer_list<const void *> ptrs) {
     cudaStreamSynchronize(0);
 }
 
-// B -> tiles into caller-visible arrays (tile arrays sized by nnz(B) >= tiles)
-// B -> 64-column tiles.  Allocations on `st`; with `run` the kernels run on that
-// stream instead (after everything already queued on `st`), the scratch is
-// released there too, and ev_done marks the end: the caller makes `st` wait on
-// it before anything reads the tiles.
+// B -> 64-column tiles, in arrays sized by nnz(B) >= tiles: for the caller to keep
+// (keep: from the default pool), or scratch.  With `run` the kernels run on that
+// stream instead (after everything already queued on `st`), and ev_done marks the
+// end: the caller makes `st` wait on it before anything reads the tiles.
 int build_tiles(hsmu_handle_s *h, const hsmu_csr *B, hsmu_btiles *out, Ctl *ctl, int validate, cudaStream_t st,
-                bool read_count, cudaStream_t run = nullptr, cudaEvent_t ev_start = nullptr,
+                bool read_count, bool keep, cudaStream_t run = nullptr, cudaEvent_t ev_start = nullptr,
                 cudaEvent_t ev_done = nullptr) {
     int rc = HSMU_OK;
     cudaStream_t ks = st;
@@ -201,13 +288,20 @@ int build_tiles(hsmu_handle_s *h, const hsmu_csr *B, hsmu_btiles *out, Ctl *ctl,
     out->tile_col = nullptr;
     out->mask = nullptr;
     out->tile_off = nullptr;
-    CK(palloc(&out->tile_ptr, (size_t)B->M + 1, st));
-    CK(palloc(&out->tile_col, (size_t)B->nnz, st));
-    CK(palloc(&out->mask, (size_t)B->nnz, st));
-    CK(palloc(&out->tile_off, (size_t)B->nnz, st));
-    CK(palloc(&tcnt, (size_t)B->M + 1, st));
-    CK(palloc(&scan_tmp, scan_tmp_ints(B->M), st));
-    CK(palloc(&tot, 1, st));
+    if (keep) {
+        CK(palloc(&out->tile_ptr, (size_t)B->M + 1, st));
+        CK(palloc(&out->tile_col, (size_t)B->nnz, st));
+        CK(palloc(&out->mask, (size_t)B->nnz, st));
+        CK(palloc(&out->tile_off, (size_t)B->nnz, st));
+    } else {
+        CK(salloc(h, &out->tile_ptr, (size_t)B->M + 1, st));
+        CK(salloc(h, &out->tile_col, (size_t)B->nnz, st));
+        CK(salloc(h, &out->mask, (size_t)B->nnz, st));
+        CK(salloc(h, &out->tile_off, (size_t)B->nnz, st));
+    }
+    CK(salloc(h, &tcnt, (size_t)B->M + 1, st));
+    CK(salloc(h, &scan_tmp, scan_tmp_ints(B->M), st));
+    CK(salloc(h, &tot, 1, st));
     if (run && ev_start && ev_done) {
         CK(cudaEventRecord(ev_start, st));
         CK(cudaStreamWaitEvent(run, ev_start, 0));
@@ -221,12 +315,8 @@ int build_tiles(hsmu_handle_s *h, const hsmu_csr *B, hsmu_btiles *out, Ctl *ctl,
         CK(cudaMemcpyAsync(&ctl->ntiles, out->tile_ptr + B->M, sizeof(int), cudaMemcpyDeviceToDevice, ks));
     }
 done:
-    pfree(tcnt, ks);
-    pfree(scan_tmp, ks);
-    pfree(tot, ks);
     if (ks != st && ev_done) cudaEventRecord(ev_done, ks);
-    if (rc != HSMU_OK) {
-        // stream-ordered allocations go back the same way
+    if (rc != HSMU_OK && keep) {
         pfree(out->tile_ptr, st);
         pfree(out->tile_col, st);
         pfree(out->mask, st);
@@ -256,7 +346,6 @@ struct PlainRun {
     int M = 0;
     DevCSR Ad{}, Bd{};
     hsmu_btiles bt{};
-    bool own_tiles = false;
     bool tiles_aside = false;  // B's tiles are being built on the handle's conversion stream
     DevTiles Btd{};
     RowInfo ri{};
@@ -291,7 +380,7 @@ struct PlainRun {
         M = A->M;
         Ad = dev(A);
         Bd = dev(B);
-        CKR(palloc(&ctl, 1, st));
+        CKR(salloc(h, &ctl, 1, st));
         CKR(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
         if (o.validate) {
             // check both operands before any kernel indexes through them
@@ -327,41 +416,37 @@ struct PlainRun {
             // B's tiles on their own stream, beside the bounds pass (which reads B's columns);
             // a small B is converted in line (the hand-over would cost more than it overlaps)
             tiles_aside = B->nnz >= TILES_ASIDE_MIN_NNZ;
-            const int rc = tiles_aside ? build_tiles(h, B, &bt, ctl, 0, st, count_tiles, h->cs_tiles,
+            const int rc = tiles_aside ? build_tiles(h, B, &bt, ctl, 0, st, count_tiles, false, h->cs_tiles,
                                                      h->ev_tiles_start, h->ev_tiles_done)
-                                       : build_tiles(h, B, &bt, ctl, 0, st, count_tiles);
-            if (rc) {
-                if (tiles_aside) cudaStreamWaitEvent(st, h->ev_tiles_done, 0);
-                return rc;
-            }
-            own_tiles = true;
+                                       : build_tiles(h, B, &bt, ctl, 0, st, count_tiles, false);
+            if (rc) return rc;
             launches += 5;
         }
         Btd = DevTiles{bt.tile_ptr, bt.tile_col, reinterpret_cast<const unsigned long long *>(bt.mask), bt.tile_off};
         if (ev_tiles) cudaEventRecord(ev_tiles, tiles_aside ? h->cs_tiles : st);
         if (B->M > 0 && B->nnz >= (long long)REPEAT_MIN_ROW * B->M) {
-            CKR(palloc(&rep, (size_t)B->M, st));
+            CKR(salloc(h, &rep, (size_t)B->M, st));
             launch_row_repeat(Bd, rep, grid_rows(h), st);
             launches++;
             ri.rep = rep;
         }
-        CKR(palloc(&ri.prod, (size_t)M, st));
-        CKR(palloc(&ri.tmin, (size_t)M, st));
-        CKR(palloc(&ri.tmax, (size_t)M, st));
-        CKR(palloc(&ri.bins, (size_t)M * NBIN, st));
-        CKR(palloc(&ri.cls, (size_t)M, st));
-        CKR(palloc(&ri.bin_cnt, bin_scratch_ints(M), st));
-        CKR(palloc(&ri.cnnz, (size_t)M + 1, st));
-        CKR(palloc(&scan_tmp, scan_tmp_ints(M), st));
+        CKR(salloc(h, &ri.prod, (size_t)M, st));
+        CKR(salloc(h, &ri.tmin, (size_t)M, st));
+        CKR(salloc(h, &ri.tmax, (size_t)M, st));
+        CKR(salloc(h, &ri.bins, (size_t)M * NBIN, st));
+        CKR(salloc(h, &ri.cls, (size_t)M, st));
+        CKR(salloc(h, &ri.bin_cnt, bin_scratch_ints(M), st));
+        CKR(salloc(h, &ri.cnnz, (size_t)M + 1, st));
+        CKR(salloc(h, &scan_tmp, scan_tmp_ints(M), st));
         if (store) {
             CKR(grow_arena());
             ri.store = 1;
             if (h->arena_cap > 0) {
-                CKR(palloc(&ts_off, (size_t)M, st));
-                CKR(palloc(&ts_cnt, (size_t)M, st));
-                CKR(palloc(&ts_nwin, (size_t)M, st));
+                CKR(salloc(h, &ts_off, (size_t)M, st));
+                CKR(salloc(h, &ts_cnt, (size_t)M, st));
+                CKR(salloc(h, &ts_nwin, (size_t)M, st));
                 CKR(cudaMemsetAsync(ts_nwin, 0, sizeof(int) * (size_t)M, st));
-                if (reserve_windows) CKR(palloc(&ts_wbase, (size_t)M + 1, st));
+                if (reserve_windows) CKR(salloc(h, &ts_wbase, (size_t)M + 1, st));
                 have_store = true;
             }
         }
@@ -369,6 +454,7 @@ struct PlainRun {
         launches += 6;  // bounds + binning
         // everything after this reads B's tiles
         if (tiles_aside) CKR(cudaStreamWaitEvent(st, h->ev_tiles_done, 0));
+        tiles_aside = false;
         CKR(cudaGetLastError());
         return HSMU_OK;
     }
@@ -413,7 +499,7 @@ struct PlainRun {
         if (host_rp) CKR(cudaMemcpyAsync(host_rp, crp, sizeof(int32_t) * ((size_t)M + 1), cudaMemcpyDeviceToHost, st));
         if (host_prod && M > 0) {
             const size_t nch = ((size_t)M + PROD_CHUNK - 1) / PROD_CHUNK;
-            CKR(palloc(&chunk_prod, nch, st));
+            CKR(salloc(h, &chunk_prod, nch, st));
             launch_chunk_prod(M, ri.prod, chunk_prod, grid_rows(h), st);
             launches++;
             CKR(cudaMemcpyAsync(host_prod, chunk_prod, sizeof(long long) * nch, cudaMemcpyDeviceToHost, st));
@@ -436,7 +522,7 @@ struct PlainRun {
             CKR(palloc(&ccol, (size_t)hc.nnz + COL_PAD, st));
             CKR(palloc(&cval, (size_t)hc.nnz, st));
         }
-        CKR(palloc(&win, (size_t)win_cap, st));
+        CKR(salloc(h, &win, (size_t)win_cap, st));
         if (hc.bin_count[BIN_L] == 0 && hc.wide_rows == 0) return HSMU_OK;  // no windows
         return alloc_cursors(win_cap, (long long)hc.cur_bound);
     }
@@ -444,13 +530,13 @@ struct PlainRun {
     int alloc_cursors(long long nwin, long long cap) {
         if (nwin == 0) return HSMU_OK;
         wc.cap = cap;
-        CKR(palloc(&wc.len, (size_t)nwin, st));
-        CKR(palloc(&wc.off, (size_t)nwin + 1, st));
-        CKR(palloc(&wc.total, 2, st));
-        CKR(palloc(&wc.scan_tmp, scan_tmp_ints((int)nwin), st));
-        CKR(palloc(&wc.item_off, (size_t)nwin + 1, st));
-        CKR(palloc(&wc.cur, (size_t)cap, st));
-        CKR(palloc(&wc.heavy, (size_t)nwin, st));
+        CKR(salloc(h, &wc.len, (size_t)nwin, st));
+        CKR(salloc(h, &wc.off, (size_t)nwin + 1, st));
+        CKR(salloc(h, &wc.total, 2, st));
+        CKR(salloc(h, &wc.scan_tmp, scan_tmp_ints((int)nwin), st));
+        CKR(salloc(h, &wc.item_off, (size_t)nwin + 1, st));
+        CKR(salloc(h, &wc.cur, (size_t)cap, st));
+        CKR(salloc(h, &wc.heavy, (size_t)nwin, st));
         return HSMU_OK;
     }
 
@@ -494,38 +580,11 @@ struct PlainRun {
         return hc.err ? err_from_dev(hc.err) : HSMU_OK;
     }
 
+    // the outputs that were not handed on; the rest goes with `scope`, which outlives this
     void release() {
-        pfree(ctl, st);
-        if (own_tiles) {
-            pfree(bt.tile_ptr, st);
-            pfree(bt.tile_col, st);
-            pfree(bt.mask, st);
-            pfree(bt.tile_off, st);
-            own_tiles = false;
-        }
-        pfree(rep, st);
-        pfree(ri.prod, st);
-        pfree(chunk_prod, st);
-        pfree(ri.tmin, st);
-        pfree(ri.tmax, st);
-        pfree(ri.bins, st);
-        pfree(ri.cls, st);
-        pfree(ri.bin_cnt, st);
-        pfree(ri.cnnz, st);
-        pfree(ts_off, st);
-        pfree(ts_cnt, st);
-        pfree(ts_nwin, st);
-        pfree(ts_wbase, st);
-        have_store = false;
-        pfree(scan_tmp, st);
-        pfree(win, st);
-        pfree(wc.len, st);
-        pfree(wc.off, st);
-        pfree(wc.total, st);
-        pfree(wc.scan_tmp, st);
-        pfree(wc.item_off, st);
-        pfree(wc.cur, st);
-        pfree(wc.heavy, st);
+        // an early return may leave the conversion stream at work on the scratch
+        if (tiles_aside) cudaStreamWaitEvent(st, h->ev_tiles_done, 0);
+        tiles_aside = have_store = false;
         pfree(crp, st);
         if (ext_col) {
             ccol = nullptr;
@@ -570,6 +629,7 @@ int spgemm_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, const hs
         std::memset(stats, 0, sizeof(*stats));
         cudaEventRecord(h->ev[0], st);
     }
+    ScratchScope scope(h, st);
     PlainRun r(h, st, o);
     int rc = r.begin(A, B);
     if (!rc) rc = r.symbolic(B, Bt_in, stats != nullptr, nullptr, stats ? h->ev[1] : nullptr);
@@ -690,6 +750,7 @@ int spgemm_host_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsm
     const int M = A->M;
     int rc = HSMU_OK;
     hsmu_csr dA{}, dB{};
+    ScratchScope scope(h, st);
     PlainRun r(h, st, o);
     if (stats) {
         std::memset(stats, 0, sizeof(*stats));
@@ -701,9 +762,9 @@ int spgemm_host_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsm
         D->row_ptr = nullptr;
         D->col = nullptr;
         D->val = nullptr;
-        CKR(palloc(&D->row_ptr, (size_t)X->M + 1, st));
-        CKR(palloc(&D->col, (size_t)X->nnz, st));
-        CKR(palloc(&D->val, (size_t)X->nnz, st));
+        CKR(salloc(h, &D->row_ptr, (size_t)X->M + 1, st));
+        CKR(salloc(h, &D->col, (size_t)X->nnz, st));
+        CKR(salloc(h, &D->val, (size_t)X->nnz, st));
         // index arrays on st (the symbolic pass needs them first) ...
         CKR(cudaMemcpyAsync(D->row_ptr, X->row_ptr, sizeof(int32_t) * ((size_t)X->M + 1), cudaMemcpyHostToDevice, st));
         if (X->nnz) CKR(cudaMemcpyAsync(D->col, X->col, sizeof(int32_t) * (size_t)X->nnz, cudaMemcpyHostToDevice, st));
@@ -788,14 +849,6 @@ done:
     cudaStreamSynchronize(h->cs_in);
     cudaStreamSynchronize(h->cs_out);
     r.release();
-    if (dA.row_ptr && dA.row_ptr != dB.row_ptr) {
-        pfree(dA.row_ptr, st);
-        pfree(dA.col, st);
-        pfree(dA.val, st);
-    }
-    pfree(dB.row_ptr, st);
-    pfree(dB.col, st);
-    pfree(dB.val, st);
     if (rc != HSMU_OK) {
         cudaStreamSynchronize(st);
         return rc;
@@ -847,6 +900,7 @@ int spgemm_learned_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, 
         std::memset(stats, 0, sizeof(*stats));
         cudaEventRecord(h->ev[0], st);
     }
+    ScratchScope scope(h, st);
     PlainRun r(h, st, o);
     rc = r.begin(A, B);
     if (!rc) rc = r.tiles_bounds(B, nullptr, stats != nullptr, stats ? h->ev[1] : nullptr, o.no_tile_store == 0);
@@ -872,17 +926,17 @@ int spgemm_learned_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, 
             if (h->arena_want == 0) h->arena_want = hc.span_tiles;
             CK(r.grow_arena());
             if (h->arena_cap > 0 && !r.ts_off) {
-                CK(palloc(&r.ts_off, (size_t)M, st));
-                CK(palloc(&r.ts_cnt, (size_t)M, st));
-                CK(palloc(&r.ts_nwin, (size_t)M, st));
+                CK(salloc(h, &r.ts_off, (size_t)M, st));
+                CK(salloc(h, &r.ts_cnt, (size_t)M, st));
+                CK(salloc(h, &r.ts_nwin, (size_t)M, st));
                 CK(cudaMemsetAsync(r.ts_nwin, 0, sizeof(int) * (size_t)M, st));
-                CK(palloc(&r.ts_wbase, (size_t)M + 1, st));
+                CK(salloc(h, &r.ts_wbase, (size_t)M + 1, st));
             }
             r.have_store = h->arena_cap > 0;
         }
-        CK(palloc(&feat, (size_t)M, st));
-        CK(palloc(&cap, (size_t)M + 1, st));
-        CK(palloc(&soff, (size_t)M + 1, st));
+        CK(salloc(h, &feat, (size_t)M, st));
+        CK(salloc(h, &cap, (size_t)M + 1, st));
+        CK(salloc(h, &soff, (size_t)M + 1, st));
         launch_features(r.Ad, r.Bd, feat, nullptr, h->nsm, st);
         // large rows with a tile list need no slot (they are written at their place in C)
         launch_capacity(model->params, feat, r.ri.prod, r.ri.cls, M, B->N, model->margin, cap, h->nsm, st,
@@ -937,7 +991,7 @@ learned:
         const DevCSR &Ad = r.Ad, &Bd = r.Bd;
         const DevTiles &Btd = r.Btd;
         RowInfo &ri = r.ri;
-        CK(palloc(&flag, (size_t)M, st));
+        CK(salloc(h, &flag, (size_t)M, st));
         CK(cudaMemsetAsync(flag, 0, (size_t)M, st));
         if (stats) cudaEventRecord(h->ev[2], st);
         spec_total = hc.nnz;
@@ -946,21 +1000,21 @@ learned:
             rc = HSMU_ERR_OVERFLOW;
             goto done;
         }
-        CK(palloc(&scol, (size_t)spec_total + COL_PAD, st));
-        CK(palloc(&sval, (size_t)spec_total, st));
-        CK(palloc(&win, (size_t)win_cap, st));
+        CK(salloc(h, &scol, (size_t)spec_total + COL_PAD, st));
+        CK(salloc(h, &sval, (size_t)spec_total, st));
+        CK(salloc(h, &win, (size_t)win_cap, st));
         CK(palloc(&crp, (size_t)M + 1, st));
         // cursors of the windows of both passes (no exact count pass: every warp row above FUSE_CAP products)
         cur_cap = 2 * (long long)(hc.cur_bound + hc.cur_bound_ds);
         if (win_cap > 0) {
             wc.cap = cur_cap;
-            CK(palloc(&wc.len, (size_t)win_cap, st));
-            CK(palloc(&wc.off, (size_t)win_cap + 1, st));
-            CK(palloc(&wc.total, 2, st));
-            CK(palloc(&wc.scan_tmp, scan_tmp_ints((int)win_cap), st));
-            CK(palloc(&wc.item_off, (size_t)win_cap + 1, st));
-            CK(palloc(&wc.cur, (size_t)cur_cap, st));
-            CK(palloc(&wc.heavy, (size_t)win_cap, st));
+            CK(salloc(h, &wc.len, (size_t)win_cap, st));
+            CK(salloc(h, &wc.off, (size_t)win_cap + 1, st));
+            CK(salloc(h, &wc.total, 2, st));
+            CK(salloc(h, &wc.scan_tmp, scan_tmp_ints((int)win_cap), st));
+            CK(salloc(h, &wc.item_off, (size_t)win_cap + 1, st));
+            CK(salloc(h, &wc.cur, (size_t)cur_cap, st));
+            CK(salloc(h, &wc.heavy, (size_t)win_cap, st));
         }
         if (stats) cudaEventRecord(h->ev[3], st);
         // structure (+ values of warp-sized rows) into the slots; exact counts found here.
@@ -1057,20 +1111,6 @@ learned:
         stats->launches = (o.validate ? 2 : 0) + (win_cap > 0 ? 35 : 27);
     }
 done:
-    pfree(feat, st);
-    pfree(cap, st);
-    pfree(soff, st);
-    pfree(flag, st);
-    pfree(scol, st);
-    pfree(sval, st);
-    pfree(win, st);
-    pfree(wc.len, st);
-    pfree(wc.off, st);
-    pfree(wc.total, st);
-    pfree(wc.scan_tmp, st);
-    pfree(wc.item_off, st);
-    pfree(wc.cur, st);
-    pfree(wc.heavy, st);
     pfree(crp, st);
     pfree(ccol, st);
     pfree(cval, st);
@@ -1090,18 +1130,19 @@ int row_nnz_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, int32_t
     int *scan_tmp = nullptr;
     DevCSR Ad = dev(A), Bd = dev(B);
     DevTiles Btd{};
-    CK(palloc(&ctl, 1, st));
+    ScratchScope scope(h, st);
+    CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
-    rc = build_tiles(h, B, &bt, ctl, 0, st, false);
+    rc = build_tiles(h, B, &bt, ctl, 0, st, false, false);
     if (rc) goto done;
     Btd = DevTiles{bt.tile_ptr, bt.tile_col, reinterpret_cast<const unsigned long long *>(bt.mask), bt.tile_off};
-    CK(palloc(&ri.prod, (size_t)M, st));
-    CK(palloc(&ri.tmin, (size_t)M, st));
-    CK(palloc(&ri.tmax, (size_t)M, st));
-    CK(palloc(&ri.bins, (size_t)M * NBIN, st));
-    CK(palloc(&ri.cls, (size_t)M, st));
-    CK(palloc(&ri.bin_cnt, bin_scratch_ints(M), st));
-    CK(palloc(&scan_tmp, scan_tmp_ints(M), st));
+    CK(salloc(h, &ri.prod, (size_t)M, st));
+    CK(salloc(h, &ri.tmin, (size_t)M, st));
+    CK(salloc(h, &ri.tmax, (size_t)M, st));
+    CK(salloc(h, &ri.bins, (size_t)M * NBIN, st));
+    CK(salloc(h, &ri.cls, (size_t)M, st));
+    CK(salloc(h, &ri.bin_cnt, bin_scratch_ints(M), st));
+    CK(salloc(h, &scan_tmp, scan_tmp_ints(M), st));
     ri.cnnz = nnz_out;
     launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), scan_tmp, st);
     launch_count(Ad, Bd, Btd, ri, ctl, h->nsm, st);
@@ -1110,18 +1151,6 @@ int row_nnz_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, int32_t
     CK(cudaStreamSynchronize(st));
     if (h->h_ctl->err) rc = err_from_dev(h->h_ctl->err);
 done:
-    pfree(ctl, st);
-    pfree(bt.tile_ptr, st);
-    pfree(bt.tile_col, st);
-    pfree(bt.mask, st);
-    pfree(bt.tile_off, st);
-    pfree(ri.prod, st);
-    pfree(ri.tmin, st);
-    pfree(ri.tmax, st);
-    pfree(ri.bins, st);
-    pfree(ri.cls, st);
-    pfree(ri.bin_cnt, st);
-    pfree(scan_tmp, st);
     if (rc != HSMU_OK) cudaStreamSynchronize(st);
     return rc;
 }
@@ -1145,20 +1174,22 @@ int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_c
     Ctl *ctl = nullptr;
     hsmu_btiles bt{};
     std::vector<long long> hrp;
+    ScratchScope scope(h, st);
     hsmu_opts po = o;
     po.validate = 0;  // the panels are views into A: the operands are checked once, here
     if (o.validate) {
+        ScratchScope checked(h, st);
         PlainRun v(h, st, o);
         rc = v.begin(A, B);
         v.release();
         if (rc) goto done;
     }
-    CK(palloc(&cnt, (size_t)M + 1, st));
+    CK(salloc(h, &cnt, (size_t)M + 1, st));
     rc = row_nnz_impl(h, A, B, cnt, st);
     if (rc) goto done;
     CK(palloc(&rp, (size_t)M + 1, st));
-    CK(palloc(&tot, 1, st));
-    CK(palloc(&scan_tmp, scan_tmp_ints(M), st));
+    CK(salloc(h, &tot, 1, st));
+    CK(salloc(h, &scan_tmp, scan_tmp_ints(M), st));
     launch_scan64(cnt, rp, M, tot, scan_tmp, st);
     CK(cudaGetLastError());
     hrp.resize((size_t)M + 1);
@@ -1166,9 +1197,9 @@ int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_c
     CK(cudaStreamSynchronize(st));
     CK(palloc(&col, (size_t)hrp[M] + COL_PAD, st));
     CK(palloc(&val, (size_t)hrp[M], st));
-    CK(palloc(&ctl, 1, st));
+    CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
-    rc = build_tiles(h, B, &bt, ctl, 0, st, true);
+    rc = build_tiles(h, B, &bt, ctl, 0, st, true, false);
     if (rc) goto done;
     for (int r0 = 0; r0 < M;) {
         // rows r0 .. r1-1: as many as keep the panel within the cap, at least one
@@ -1177,6 +1208,7 @@ int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_c
         hsmu_csr Ap = *A;
         Ap.M = r1 - r0;
         Ap.row_ptr = A->row_ptr + r0;
+        ScratchScope panel(h, st);
         PlainRun r(h, st, po);
         r.ext_col = col + hrp[r0];
         r.ext_val = val + hrp[r0];
@@ -1204,14 +1236,6 @@ int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_c
     col = nullptr;
     val = nullptr;
 done:
-    pfree(cnt, st);
-    pfree(scan_tmp, st);
-    pfree(tot, st);
-    pfree(ctl, st);
-    pfree(bt.tile_ptr, st);
-    pfree(bt.tile_col, st);
-    pfree(bt.mask, st);
-    pfree(bt.tile_off, st);
     pfree(rp, st);
     pfree(col, st);
     pfree(val, st);
@@ -1259,6 +1283,18 @@ int hsmu_handle_create(hsmu_handle *out) {
         hsmu_handle_destroy(h);
         return HSMU_ERR_CUDA;
     }
+    {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        unsigned long long keep = SCRATCH_POOL_KEEP;
+        if (cudaMemPoolCreate(&h->scratch.pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(h->scratch.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            hsmu_handle_destroy(h);
+            return HSMU_ERR_CUDA;
+        }
+    }
     // keep freed pool memory cached between calls (no re-mapping of large outputs)
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
@@ -1291,6 +1327,11 @@ int hsmu_handle_destroy(hsmu_handle h) {
     }
     for (cudaStream_t s : {h->cs_in, h->cs_out, h->cs_tiles})
         if (s) cudaStreamDestroy(s);
+    if (h->scratch.base) {
+        cudaFreeAsync(h->scratch.base, 0);  // every call of the handle has finished
+        cudaStreamSynchronize(0);
+    }
+    if (h->scratch.pool) cudaMemPoolDestroy(h->scratch.pool);
     if (h->h_ctl) cudaFreeHost(h->h_ctl);
     if (h->h_prod) cudaFreeHost(h->h_prod);
     delete h;
@@ -1341,7 +1382,8 @@ int hsmu_btiles_build(hsmu_handle h, const hsmu_csr *B, hsmu_btiles *out, void *
     Ctl *ctl = nullptr;
     Ctl hc{};
     std::memset(out, 0, sizeof(*out));
-    CK(palloc(&ctl, 1, st));
+    ScratchScope scope(h, st);
+    CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     launch_validate(dev(B), ctl, grid_rows(h), st);
     CK(cudaGetLastError());
@@ -1351,7 +1393,7 @@ int hsmu_btiles_build(hsmu_handle h, const hsmu_csr *B, hsmu_btiles *out, void *
         rc = err_from_dev(h->h_ctl->err);
         goto done;
     }
-    rc = build_tiles(h, B, out, ctl, 0, st, true);
+    rc = build_tiles(h, B, out, ctl, 0, st, true, true);
     if (rc) goto done;
     CK(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -1363,7 +1405,7 @@ int hsmu_btiles_build(hsmu_handle h, const hsmu_csr *B, hsmu_btiles *out, void *
     }
     out->ntiles = hc.ntiles;
 done:
-    pfree(ctl, st);
+    if (rc != HSMU_OK) cudaStreamSynchronize(st);
     return rc;
 }
 
@@ -1385,15 +1427,16 @@ int hsmu_csr_transpose(hsmu_handle h, const hsmu_csr *A, hsmu_csr *At, void *str
     long long *tot = nullptr;
     Ctl *ctl = nullptr;
     const long long ntiles_scan = (long long)transpose_hist_ints(n) / 2;
+    ScratchScope scope(h, st);
     CK(palloc(&trp, (size_t)A->N + 1, st));
     CK(palloc(&tcol, (size_t)n, st));
     CK(palloc(&tval, (size_t)n, st));
-    CK(palloc(&si, transpose_scratch_ints(n), st));
-    CK(palloc(&sd, transpose_scratch_doubles(n), st));
-    CK(palloc(&hist, transpose_hist_ints(n), st));
-    CK(palloc(&scan_tmp, scan_tmp_ints((int)ntiles_scan), st));
-    CK(palloc(&tot, 1, st));
-    CK(palloc(&ctl, 1, st));
+    CK(salloc(h, &si, transpose_scratch_ints(n), st));
+    CK(salloc(h, &sd, transpose_scratch_doubles(n), st));
+    CK(salloc(h, &hist, transpose_hist_ints(n), st));
+    CK(salloc(h, &scan_tmp, scan_tmp_ints((int)ntiles_scan), st));
+    CK(salloc(h, &tot, 1, st));
+    CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     CK((cudaError_t)launch_transpose(dev(A), trp, tcol, tval, si, sd, hist, scan_tmp, tot, ctl, h->nsm, st));
     CK(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
@@ -1415,12 +1458,6 @@ done:
     pfree(trp, st);
     pfree(tcol, st);
     pfree(tval, st);
-    pfree(si, st);
-    pfree(sd, st);
-    pfree(hist, st);
-    pfree(scan_tmp, st);
-    pfree(tot, st);
-    pfree(ctl, st);
     if (rc != HSMU_OK) cudaStreamSynchronize(st);
     return rc;
 }
