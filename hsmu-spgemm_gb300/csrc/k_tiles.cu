@@ -16,7 +16,8 @@
 
 namespace hsmu {
 
-template <bool FILL>
+// TILE_U: steps of 32 entries whose loads are in flight (launch_tiles_*)
+template <bool FILL, int TILE_U>
 __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ brp, const int *__restrict__ bcol,
                                                int N, int *__restrict__ tcnt_or_ptr, int *__restrict__ tcol,
                                                unsigned long long *__restrict__ tmask, int *__restrict__ toff,
@@ -32,63 +33,74 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
         unsigned long long pend_m = 0;
         int prev_col = -1;
         bool bad = false;
-        for (int base = s; base < e; base += WARP) {
-            const int idx = base + lane;
-            const bool valid = idx < e;
-            const int c = valid ? __ldg(bcol + idx) : 0;
-            if (validate) {
-                int cp = __shfl_up_sync(FULL, c, 1);
-                if (lane == 0) cp = prev_col;
-                if (valid && (c <= cp || c < 0 || c >= N)) bad = true;
-                prev_col = __shfl_sync(FULL, c, WARP - 1);
-            }
-            const int t = c >> 6;
-            int tp = __shfl_up_sync(FULL, t, 1);
-            if (lane == 0) tp = have_pend ? pend_t : -1;
-            const bool head = valid && (t != tp);
-            const unsigned heads = __ballot_sync(FULL, head);
-            const int nvalid = min(WARP, e - base);
-            if (!FILL) {
-                run += __popc(heads);
-                pend_t = __shfl_sync(FULL, t, nvalid - 1);  // tile open at the end of this chunk
-                have_pend = true;
-                continue;
-            }
-            unsigned above = heads & ~((2u << lane) - 1u);
-            if (lane == 31) above = 0;
-            const int seg_end = above ? (__ffs(above) - 2) : (nvalid - 1);
-            unsigned long long v = valid ? (1ull << (c & 63)) : 0ull;
+        for (int base0 = s; base0 < e; base0 += WARP * TILE_U) {
+            int cu[TILE_U];
 #pragma unroll
-            for (int d = 1; d < WARP; d <<= 1) {
-                unsigned long long o = __shfl_down_sync(FULL, v, d);
-                if (lane + d <= seg_end) v |= o;
+            for (int u = 0; u < TILE_U; u++) {
+                const int idx = base0 + u * WARP + lane;
+                cu[u] = idx < e ? __ldg(bcol + idx) : 0;
             }
-            const unsigned long long lane0_or = __shfl_sync(FULL, v, 0);
-            if (have_pend) {
-                if (!(heads & 1u)) pend_m |= lane0_or;  // lane 0 continues the pending tile
-                if (heads) {
-                    if (lane == 0) {
-                        tcol[run] = pend_t;
-                        tmask[run] = pend_m;
-                        toff[run] = pend_off;
+#pragma unroll
+            for (int u = 0; u < TILE_U; u++) {
+                const int base = base0 + u * WARP;
+                if (base >= e) break;
+                const int idx = base + lane;
+                const bool valid = idx < e;
+                const int c = cu[u];
+                if (validate) {
+                    int cp = __shfl_up_sync(FULL, c, 1);
+                    if (lane == 0) cp = prev_col;
+                    if (valid && (c <= cp || c < 0 || c >= N)) bad = true;
+                    prev_col = __shfl_sync(FULL, c, WARP - 1);
+                }
+                const int t = c >> 6;
+                int tp = __shfl_up_sync(FULL, t, 1);
+                if (lane == 0) tp = have_pend ? pend_t : -1;
+                const bool head = valid && (t != tp);
+                const unsigned heads = __ballot_sync(FULL, head);
+                const int nvalid = min(WARP, e - base);
+                if (!FILL) {
+                    run += __popc(heads);
+                    pend_t = __shfl_sync(FULL, t, nvalid - 1);  // tile open at the end of this chunk
+                    have_pend = true;
+                    continue;
+                }
+                unsigned above = heads & ~((2u << lane) - 1u);
+                if (lane == 31) above = 0;
+                const int seg_end = above ? (__ffs(above) - 2) : (nvalid - 1);
+                unsigned long long v = valid ? (1ull << (c & 63)) : 0ull;
+#pragma unroll
+                for (int d = 1; d < WARP; d <<= 1) {
+                    unsigned long long o = __shfl_down_sync(FULL, v, d);
+                    if (lane + d <= seg_end) v |= o;
+                }
+                const unsigned long long lane0_or = __shfl_sync(FULL, v, 0);
+                if (have_pend) {
+                    if (!(heads & 1u)) pend_m |= lane0_or;  // lane 0 continues the pending tile
+                    if (heads) {
+                        if (lane == 0) {
+                            tcol[run] = pend_t;
+                            tmask[run] = pend_m;
+                            toff[run] = pend_off;
+                        }
+                        run++;
+                        have_pend = false;
                     }
-                    run++;
-                    have_pend = false;
                 }
-            }
-            if (heads) {
-                const int last = 31 - __clz(heads);
-                if (head && lane != last) {
-                    const int pos = run + __popc(heads & lanemask_lt());
-                    tcol[pos] = t;
-                    tmask[pos] = v;
-                    toff[pos] = idx;
+                if (heads) {
+                    const int last = 31 - __clz(heads);
+                    if (head && lane != last) {
+                        const int pos = run + __popc(heads & lanemask_lt());
+                        tcol[pos] = t;
+                        tmask[pos] = v;
+                        toff[pos] = idx;
+                    }
+                    run += __popc(heads) - 1;
+                    pend_t = __shfl_sync(FULL, t, last);
+                    pend_m = __shfl_sync(FULL, v, last);
+                    pend_off = base + last;
+                    have_pend = true;
                 }
-                run += __popc(heads) - 1;
-                pend_t = __shfl_sync(FULL, t, last);
-                pend_m = __shfl_sync(FULL, v, last);
-                pend_off = base + last;
-                have_pend = true;
             }
         }
         if (FILL) {
@@ -104,13 +116,19 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
     }
 }
 
+// A hub row of a power-law graph is a chain of hundreds of steps, and with one step's load in flight
+// it was the pass's tail: R-MAT scale 18 count 207 -> 120 us, fill 385 -> 310 us, scale 15 30 -> 16 and
+// 71 -> 56 us with four.  Rows that fit one step only pay for the wider loop (5-point Laplacian of
+// 65,536 rows: 5.7 -> 8.2 and 13.7 -> 15.7 us).
+static bool tiles_short(const DevCSR &B) { return B.nnz <= 8ll * B.M; }
+
 void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int grid, cudaStream_t st) {
-    k_tiles<false><<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, tcnt, nullptr, nullptr, nullptr, validate, ctl);
+    (tiles_short(B) ? k_tiles<false, 1> : k_tiles<false, 4>)<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, tcnt, nullptr, nullptr, nullptr, validate, ctl);
 }
 
 void launch_tiles_fill(const DevCSR &B, const int *tptr, int *tcol, unsigned long long *tmask, int *toff, Ctl *ctl,
                        int grid, cudaStream_t st) {
-    k_tiles<true><<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, const_cast<int *>(tptr), tcol, tmask, toff, 0, ctl);
+    (tiles_short(B) ? k_tiles<true, 1> : k_tiles<true, 4>)<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, const_cast<int *>(tptr), tcol, tmask, toff, 0, ctl);
 }
 
 // rep[k] = 1 when row k of B holds the same columns as row k - 1 (the rows of one finite-element
