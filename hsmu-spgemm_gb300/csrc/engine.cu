@@ -451,7 +451,7 @@ struct PlainRun {
             }
         }
         launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), scan_tmp, st);
-        launches += 6;  // bounds + binning
+        launches += 6 + long_rows_apart(Ad);  // bounds + binning
         // everything after this reads B's tiles
         if (tiles_aside) CKR(cudaStreamWaitEvent(st, h->ev_tiles_done, 0));
         tiles_aside = false;
@@ -937,7 +937,7 @@ int spgemm_learned_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, 
         CK(salloc(h, &feat, (size_t)M, st));
         CK(salloc(h, &cap, (size_t)M + 1, st));
         CK(salloc(h, &soff, (size_t)M + 1, st));
-        launch_features(r.Ad, r.Bd, feat, nullptr, h->nsm, st);
+        launch_features(r.Ad, r.Bd, feat, nullptr, h->nsm, st, cap);  // cap is written after
         // large rows with a tile list need no slot (they are written at their place in C)
         launch_capacity(model->params, feat, r.ri.prod, r.ri.cls, M, B->N, model->margin, cap, h->nsm, st,
                         &r.ctl->pred_wide_prod, r.have_store);
@@ -1049,6 +1049,7 @@ learned:
             rc = err_from_dev(hc.err);
             goto done;
         }
+        tsd.all_stored = hc.store_used <= tsd.cap;
         if (r.ri.store && hc.store_tiles > h->arena_want) h->arena_want = hc.store_tiles;  // for the next call
         if (hc.nnz > INT_MAX) {
             rc = HSMU_ERR_OVERFLOW;

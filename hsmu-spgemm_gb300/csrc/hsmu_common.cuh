@@ -22,6 +22,13 @@ constexpr unsigned FULL = 0xffffffffu;
 // A C row whose tile span is at most SPAN_T tiles is handled by one warp
 // with a dense per-tile table in shared memory (symbolic / structure).
 constexpr int SPAN_T = 512;
+// ... unless it has more products than this: then a CTA takes it (BIN_L), with a tile list.  One warp
+// took 1 ms over a hub row of a power-law graph within 512 tiles, in the count pass and again in the
+// structure pass: A*A^T of 30,011 vertices 4.18 ms without the limit, 2.99 at 65,536 products, 2.71 at
+// 32,768, 2.50 at 16,384, 2.42 at 8,192.  The line is kept where the learned scheduler still has its
+// saving, the warp class's count pass (R-MAT scale 15: 2.35 ms against 2.39 at 32,768; below, its own
+// passes cost more than that).
+constexpr long long DS_PROD = 32768;
 // Numeric windows: consecutive tiles of one C row with
 //   < WIN_CAP slots (cut where the tile's first slot crosses a multiple of WIN_CUT),
 //   <= WIN_TCAP tiles (cut where the tile's rank in the row crosses a multiple of WIN_TCAP),
@@ -110,6 +117,7 @@ struct Ctl {
     unsigned long long pred_wide_prod;  // learned path: products of warp-class rows predicted
                                      // above FUSE_CAP entries
     long long win_listed;            // windows of the rows with a tile list (scan total)
+    int long_rows;                   // rows listed by the bounds pass for its second launch
     RowCounter rows[3];              // row hand-out of the kernels that give a CTA one row at a time
 };
 

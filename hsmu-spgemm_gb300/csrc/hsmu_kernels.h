@@ -95,6 +95,12 @@ void launch_validate(const DevCSR &A, Ctl *ctl, int grid, cudaStream_t st);
 
 // k_rows.cu
 void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, int *scan_tmp, cudaStream_t st);
+// whether rows of many entries are taken in a launch of their own (hsmu_rowsums.cuh): it costs about
+// 3 us where there are none (a 5-point Laplacian of 65,536 rows: 9 + 3 us) and takes 30 us off a
+// power-law graph of 430,000 entries, so small or short-rowed matrices go without
+inline bool long_rows_apart(const DevCSR &A) {
+    return A.nnz >= (1 << 20) || (A.nnz >= (1 << 16) && A.nnz > 6ll * A.M);
+}
 // out[c] = products of rows c*PROD_CHUNK .. (c+1)*PROD_CHUNK-1 (ceil(M / PROD_CHUNK) entries)
 constexpr int PROD_CHUNK = 64;
 void launch_chunk_prod(int M, const long long *prod, long long *out, int grid, cudaStream_t st);
@@ -107,7 +113,9 @@ void launch_scan(const int *in, int *out, int n, long long *total64, int *tmp, C
 void launch_scan64(const int *in, long long *out, int n, long long *total64, int *tmp, cudaStream_t st);
 
 // learned.cu
-void launch_features(const DevCSR &A, const DevCSR &B, float4 *feat, long long *prod_out, int nsm, cudaStream_t st);
+// long_list (nullable): scratch of M + 1 ints
+void launch_features(const DevCSR &A, const DevCSR &B, float4 *feat, long long *prod_out, int nsm, cudaStream_t st,
+                     int *long_list = nullptr);
 // wide_prod (nullable): incremented by the products of every warp-class row predicted clearly
 // above FUSE_CAP entries; large_no_slot: rows of the large class get no slot (the caller keeps
 // their tile lists)

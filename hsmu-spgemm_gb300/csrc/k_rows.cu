@@ -22,88 +22,129 @@
 #include "hsmu_common.cuh"
 #include "hsmu_kernels.h"
 #include "hsmu_rowops.cuh"
+#include "hsmu_rowsums.cuh"
 
 namespace hsmu {
 
-template <int G>
-__global__ void __launch_bounds__(256) k_bounds(int M, const int *__restrict__ arp, const int *__restrict__ acol,
-                                                const int *__restrict__ brp, const int *__restrict__ bcol, int N,
-                                                RowInfo ri, Ctl *ctl) {
-    constexpr int RPB = 256 / G;  // rows per block iteration
-    __shared__ int s_cnt[NBIN];
-    const int sub = threadIdx.x & (G - 1);
-    const int rloc = threadIdx.x / G;
-    unsigned long long my_prod = 0, my_wb = 0, my_cb = 0, my_cbd = 0, my_wdp = 0, my_span = 0;
-    if (threadIdx.x < NBIN) s_cnt[threadIdx.x] = 0;
-    __syncthreads();
-    for (int rb = blockIdx.x * RPB; rb < M; rb += gridDim.x * RPB) {
-        const int i = rb + rloc;
-        long long prod = 0;
-        int tmin = INT_MAX, tmax = -1;
-        if (i < M) {
-            for (int p = arp[i] + sub; p < arp[i + 1]; p += G) {
-                const int k = __ldg(acol + p);
-                const int bs = __ldg(brp + k), be = __ldg(brp + k + 1);
-                prod += be - bs;
-                if (be > bs) {
-                    tmin = min(tmin, __ldg(bcol + bs) >> 6);
-                    tmax = max(tmax, __ldg(bcol + be - 1) >> 6);
-                }
+// What a block adds up over its rows for the control block: one thread per sum sends it there.
+enum BoundsSum { BS_PROD, BS_WB, BS_CB, BS_CBD, BS_WDP, BS_SPAN, BS_BIN, BS_N = BS_BIN + NBIN };
+struct BoundsSmem {
+    unsigned long long sum[BS_N];
+};
+
+// a thread's part of them
+struct BoundsSums {
+    unsigned long long t_prod = 0, t_wb = 0, t_cb = 0, t_cbd = 0, t_wdp = 0, t_span = 0;
+    int cnt[NBIN] = {};
+
+    // one row's products, tile span and class
+    __device__ __forceinline__ void row(int i, int len, const RowSums &sums, int N, const RowInfo &ri) {
+        const long long prod = sums.prod;
+        const int tmin = sums.cmin == INT_MAX ? INT_MAX : sums.cmin >> 6, tmax = sums.cmax >> 6;
+        ri.prod[i] = prod;
+        ri.tmin[i] = tmin;
+        ri.tmax[i] = tmax;
+        int bin = -1;
+        if (prod == 0) {
+            ri.cnnz[i] = 0;
+        } else {
+            const int span = tmax - tmin + 1;
+            const bool scattered = prod <= H_MAX && span <= H_SPAN && len <= H_ROW;
+            bin = prod <= TINY_MAX ? BIN_TINY : span <= SPAN_T && prod <= DS_PROD ? BIN_DS : scattered ? BIN_H : BIN_L;
+            t_prod += (unsigned long long)prod;
+            const long long cap = prod < (long long)N ? prod : (long long)N;
+            // windows per row <= slot cuts + tile-rank cuts + span cuts + 1
+            const long long tl = cap < (long long)span ? cap : (long long)span;
+            const unsigned long long wb = (unsigned long long)(cap / WIN_CUT + tl / WIN_TCAP + (span - 1) / WIN_SPAN + 1);
+            // rows that can reach the window pass: the large class, and warp rows above FUSE_CAP
+            if (bin == BIN_L) {
+                t_wb += wb;
+                t_cb += wb * (unsigned long long)len;
+                t_span += (unsigned long long)span;
+            }
+            if (bin == BIN_DS && prod > FUSE_CAP) {
+                t_wb += wb;
+                t_cbd += wb * (unsigned long long)len;
+                t_wdp += (unsigned long long)prod;
             }
         }
+        ri.cls[i] = (signed char)bin;
 #pragma unroll
-        for (int d = G / 2; d > 0; d >>= 1) {
-            prod += __shfl_xor_sync(FULL, prod, d, G);
-            tmin = min(tmin, __shfl_xor_sync(FULL, tmin, d, G));
-            tmax = max(tmax, __shfl_xor_sync(FULL, tmax, d, G));
+        for (int k = 0; k < NBIN; k++) cnt[k] += bin == k;
+    }
+
+    // every thread of the block
+    __device__ __forceinline__ void flush(BoundsSmem &S, Ctl *ctl) {
+        if (threadIdx.x < BS_N) S.sum[threadIdx.x] = 0;
+        __syncthreads();
+        auto add = [&](int k, unsigned long long v) {
+            v = warp_sum(v);
+            if (lane_id() == 0 && v) atomicAdd(&S.sum[k], v);
+        };
+        add(BS_PROD, t_prod);
+        add(BS_WB, t_wb);
+        add(BS_CB, t_cb);
+        add(BS_CBD, t_cbd);
+        add(BS_WDP, t_wdp);
+        add(BS_SPAN, t_span);
+#pragma unroll
+        for (int k = 0; k < NBIN; k++) add(BS_BIN + k, (unsigned long long)cnt[k]);
+        __syncthreads();
+        const unsigned long long v = threadIdx.x < BS_N ? S.sum[threadIdx.x] : 0ull;
+        if (!v) return;
+        switch (threadIdx.x) {
+        case BS_PROD: atomicAdd(&ctl->products, v); break;
+        case BS_WB: atomicAdd(&ctl->win_bound, v); break;
+        case BS_CB: atomicAdd(&ctl->cur_bound, v); break;
+        case BS_CBD: atomicAdd(&ctl->cur_bound_ds, v); break;
+        case BS_WDP: atomicAdd(&ctl->wide_ds_prod, v); break;
+        case BS_SPAN: atomicAdd(reinterpret_cast<unsigned long long *>(&ctl->span_tiles), v); break;
+        default: atomicAdd(&ctl->bin_count[threadIdx.x - BS_BIN], (int)v);
         }
+    }
+};
+
+// long_list: rows of more than SUM_LONG entries are listed there (ctl->long_rows of them) for
+// k_bounds_long; nullptr: every row is taken here
+template <int G>
+__global__ void __launch_bounds__(SUM_THREADS) k_bounds(int M, const int *__restrict__ arp,
+                                                        const int *__restrict__ acol, const int *__restrict__ brp,
+                                                        const int *__restrict__ bcol, int N, RowInfo ri,
+                                                        int *__restrict__ long_list, Ctl *ctl) {
+    constexpr int RPB = SUM_THREADS / G;  // rows per block iteration
+    __shared__ BoundsSmem s_tot;
+    const int sub = threadIdx.x & (G - 1);
+    BoundsSums mine;
+    for (int rb = blockIdx.x * RPB; rb < M; rb += gridDim.x * RPB) {
+        const int i = rb + (int)threadIdx.x / G;
+        const int lo = i < M ? arp[i] : 0, hi = i < M ? arp[i + 1] : 0;
+        const bool listed = long_list && hi - lo > SUM_LONG;
+        RowSums r;
+        r.walk(lo + sub, listed ? lo : hi, G, acol, brp, bcol);
+        r.reduce<G>();
         if (i < M && sub == 0) {
-            ri.prod[i] = prod;
-            ri.tmin[i] = tmin;
-            ri.tmax[i] = tmax;
-            int bin = -1;
-            if (prod == 0) {
-                ri.cnnz[i] = 0;
-            } else {
-                const int span = tmax - tmin + 1;
-                const bool scattered = prod <= H_MAX && span <= H_SPAN && arp[i + 1] - arp[i] <= H_ROW;
-                bin = prod <= TINY_MAX ? BIN_TINY : span <= SPAN_T ? BIN_DS : scattered ? BIN_H : BIN_L;
-                atomicAdd(&s_cnt[bin], 1);
-                my_prod += (unsigned long long)prod;
-                const long long cap = prod < (long long)N ? prod : (long long)N;
-                // windows per row <= slot cuts + tile-rank cuts + span cuts + 1
-                const long long tl = cap < (long long)span ? cap : (long long)span;
-                const unsigned long long wb = (unsigned long long)(cap / WIN_CUT + tl / WIN_TCAP + (span - 1) / WIN_SPAN + 1);
-                if (bin == BIN_L || (bin == BIN_DS && prod > FUSE_CAP)) my_wb += wb;
-                // rows that can reach the window pass: the large class, and warp rows above FUSE_CAP
-                if (bin == BIN_L) {
-                    my_cb += wb * (unsigned long long)(arp[i + 1] - arp[i]);
-                    my_span += (unsigned long long)span;
-                }
-                if (bin == BIN_DS && prod > FUSE_CAP) {
-                    my_cbd += wb * (unsigned long long)(arp[i + 1] - arp[i]);
-                    my_wdp += (unsigned long long)prod;
-                }
-            }
-            ri.cls[i] = (signed char)bin;
+            if (listed) long_list[atomicAdd(&ctl->long_rows, 1)] = i;
+            else mine.row(i, hi - lo, r, N, ri);
         }
     }
-    __syncthreads();
-    if (threadIdx.x < NBIN && s_cnt[threadIdx.x]) atomicAdd(&ctl->bin_count[threadIdx.x], s_cnt[threadIdx.x]);
-    my_prod = warp_sum(my_prod);
-    my_wb = warp_sum(my_wb);
-    my_cb = warp_sum(my_cb);
-    my_cbd = warp_sum(my_cbd);
-    my_wdp = warp_sum(my_wdp);
-    my_span = warp_sum(my_span);
-    if (lane_id() == 0) {
-        if (my_wdp) atomicAdd(&ctl->wide_ds_prod, my_wdp);
-        if (my_span) atomicAdd(reinterpret_cast<unsigned long long *>(&ctl->span_tiles), my_span);
-        if (my_prod) atomicAdd(&ctl->products, my_prod);
-        if (my_wb) atomicAdd(&ctl->win_bound, my_wb);
-        if (my_cb) atomicAdd(&ctl->cur_bound, my_cb);
-        if (my_cbd) atomicAdd(&ctl->cur_bound_ds, my_cbd);
+    mine.flush(s_tot, ctl);
+}
+
+__global__ void __launch_bounds__(SUM_THREADS) k_bounds_long(const int *__restrict__ arp, const int *__restrict__ acol,
+                                                             const int *__restrict__ brp, const int *__restrict__ bcol,
+                                                             int N, RowInfo ri, const int *__restrict__ long_list,
+                                                             Ctl *ctl) {
+    __shared__ SumSmem s_sum;
+    __shared__ BoundsSmem s_tot;
+    BoundsSums mine;
+    const int n = ctl->long_rows;
+    for (int e = blockIdx.x; e < n; e += gridDim.x) {
+        const int i = long_list[e];
+        const int lo = arp[i], hi = arp[i + 1];
+        const RowSums r = block_row_sums(lo, hi, acol, brp, bcol, s_sum);
+        if (threadIdx.x == 0) mine.row(i, hi - lo, r, N, ri);
     }
+    mine.flush(s_tot, ctl);
 }
 
 // stable binning: rows of each class per 32-row chunk (warp per chunk) ...
@@ -141,14 +182,11 @@ size_t bin_scratch_ints(int M) { return (size_t)NBIN * ((M + WARP - 1) / WARP) *
 
 void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, int *scan_tmp, cudaStream_t st) {
     const double avg = A.M ? (double)A.nnz / A.M : 0.0;
-    if (avg <= 6)
-        k_bounds<4><<<grid, 256, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, ctl);
-    else if (avg <= 12)
-        k_bounds<8><<<grid, 256, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, ctl);
-    else if (avg <= 24)
-        k_bounds<16><<<grid, 256, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, ctl);
-    else
-        k_bounds<32><<<grid, 256, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, ctl);
+    // the bins are written after this pass: until then their space holds the long rows
+    int *list = long_rows_apart(A) ? ri.bins : nullptr;
+    auto k = avg <= 6 ? k_bounds<4> : avg <= 12 ? k_bounds<8> : avg <= 24 ? k_bounds<16> : k_bounds<32>;
+    k<<<grid, SUM_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
+    if (list) k_bounds_long<<<grid / 2, SUM_THREADS, 0, st>>>(A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
     const int nch = (A.M + WARP - 1) / WARP;
     int *cnt = ri.bin_cnt, *off = ri.bin_cnt + (size_t)NBIN * nch + 1;
     k_bin_count<<<grid, 256, 0, st>>>(A.M, ri.cls, cnt);

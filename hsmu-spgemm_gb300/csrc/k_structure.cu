@@ -227,7 +227,10 @@ __global__ void __launch_bounds__(SDS_WARPS * 32, SDS_CTAS_PER_SM)
                 win[wbase + j] = Window{i, s0, e - s0, t0 + S.wt[j], out.mode == OUT_REDO, -1, 0};
             }
         }
-        emit_tiles(S.msk, S.base, lo, hi, t0 << 6, ccol + rowbase);
+        for (int tb = 0; tb < span; tb += WARP) {
+            const int t = tb + lane;
+            warp_emit_list(t0 + t, t < span ? S.msk[t] : 0ull, ccol + rowbase + S.base[tb]);
+        }
         __syncwarp();
     }
 }
@@ -251,7 +254,7 @@ struct SlSmem {
     int wt[SL_WL];
 };
 
-// stored: nullable per-row tile-list counts of the tile store; rows that have a
+// stored: nullable per-row tile-list counts of the tile store (arena: its entries); rows that have a
 // list (>= 0) are built by k_struct_ls (or, learned path, by the count kernel)
 // and skipped here
 __global__ void __launch_bounds__(SL_THREADS, 3) k_struct_l(int M, const int *__restrict__ arp,
@@ -260,7 +263,8 @@ __global__ void __launch_bounds__(SL_THREADS, 3) k_struct_l(int M, const int *__
                                                          const int *__restrict__ tcol,
                                                          const unsigned long long *__restrict__ tmask, RowInfo ri,
                                                          RowOut out, Window *__restrict__ win, long long win_cap,
-                                                         const int *__restrict__ stored, Ctl *ctl) {
+                                                         const int *__restrict__ stored, long long arena,
+                                                         Ctl *ctl) {
     extern __shared__ unsigned long long s_dyn[];
     SlSmem &S = *reinterpret_cast<SlSmem *>(s_dyn);
     // warp totals of the three block scans of a chunk (one array each: one barrier per scan)
@@ -272,6 +276,7 @@ __global__ void __launch_bounds__(SL_THREADS, 3) k_struct_l(int M, const int *__
     const int *rows = ri.bins + (size_t)BIN_L * M;
     int b0, b1;
     bin_slice(rows, ctl->bin_count[BIN_L], out, M, b0, b1);
+    if (stored && ctl->store_used <= arena) b1 = b0;  // every large row has a list
     int *__restrict__ ccol = out.ccol;
     // one row at a time from a counter (RowCounter)
     for (int r = b0 + blockIdx.x; r < b1; r = next_row_sync(&ctl->rows[ROWS_STRUCT_L], b0, &s_next)) {
@@ -523,7 +528,8 @@ void launch_structure(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowI
         if (list && out.mode != OUT_SPEC) k_struct_ls<<<nsm * 6, SLS_THREADS, 0, st>>>(A.M, ri, *ts, out, win, win_cap, ctl);
         if (!list || !ts->all_stored)
             k_struct_l<<<nsm * 3, SL_THREADS, sizeof(SlSmem), st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, out,
-                                                                    win, win_cap, list ? ts->cnt : nullptr, ctl);
+                                                                    win, win_cap, list ? ts->cnt : nullptr,
+                                                                    list ? ts->cap : 0, ctl);
     }
 }
 

@@ -35,6 +35,7 @@
 #include "hsmu_gb.h"
 #include "hsmu_kernels.h"
 #include "hsmu_rowops.cuh"
+#include "hsmu_rowsums.cuh"
 
 namespace hsmu {
 
@@ -47,53 +48,62 @@ constexpr int OFF_MU = MLP_NPARAM, OFF_SD = OFF_MU + NF, OFF_YMU = OFF_SD + NF, 
 static_assert(MLP_NTOTAL == HSMU_MLP_FLOATS, "parameter layout and the C ABI disagree");
 
 // ---------------------------------------------------------------- features
+__device__ __forceinline__ void store_features(int i, int len, const RowSums &r, float4 *__restrict__ feat,
+                                               long long *__restrict__ prod_out) {
+    const float span = r.cmax >= r.cmin ? (float)(r.cmax - r.cmin) : 0.f;
+    feat[i] = make_float4(log2f(1.f + (float)len), log2f(1.f + (float)r.prod), log2f(1.f + (float)r.longest),
+                          log2f(1.f + span));
+    if (prod_out) prod_out[i] = r.prod;
+}
+
+// long_list (nullable): as in the bounds pass, with its counter in front of the list
 template <int G>
-__global__ void __launch_bounds__(256) k_features(int M, const int *__restrict__ arp, const int *__restrict__ acol,
-                                                  const int *__restrict__ brp, const int *__restrict__ bcol,
-                                                  float4 *__restrict__ feat, long long *__restrict__ prod_out) {
-    constexpr int RPW = WARP / G;  // rows per warp per step
-    const int sub = threadIdx.x & (G - 1);
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int rb = gw * RPW; rb < M; rb += nw * RPW) {  // uniform across the warp
-        const int i = rb + (lane_id() / G);
-        long long prod = 0;
-        int mx = 0, cmin = INT_MAX, cmax = -1;
-        if (i < M) {
-            for (int p = arp[i] + sub; p < arp[i + 1]; p += G) {
-                const int k = __ldg(acol + p);
-                const int s = __ldg(brp + k), e = __ldg(brp + k + 1);
-                prod += e - s;
-                mx = max(mx, e - s);
-                if (e > s) {
-                    cmin = min(cmin, __ldg(bcol + s));
-                    cmax = max(cmax, __ldg(bcol + e - 1));
-                }
-            }
-        }
-#pragma unroll
-        for (int d = G / 2; d > 0; d >>= 1) {
-            prod += __shfl_xor_sync(FULL, prod, d, G);
-            mx = max(mx, __shfl_xor_sync(FULL, mx, d, G));
-            cmin = min(cmin, __shfl_xor_sync(FULL, cmin, d, G));
-            cmax = max(cmax, __shfl_xor_sync(FULL, cmax, d, G));
-        }
+__global__ void __launch_bounds__(SUM_THREADS) k_features(int M, const int *__restrict__ arp,
+                                                          const int *__restrict__ acol, const int *__restrict__ brp,
+                                                          const int *__restrict__ bcol, float4 *__restrict__ feat,
+                                                          long long *__restrict__ prod_out, int *long_list) {
+    constexpr int RPB = SUM_THREADS / G;
+    for (int rb = blockIdx.x * RPB; rb < M; rb += gridDim.x * RPB) {
+        const int i = rb + (int)threadIdx.x / G, sub = threadIdx.x & (G - 1);
+        const int lo = i < M ? arp[i] : 0, hi = i < M ? arp[i + 1] : 0;
+        const bool listed = long_list && hi - lo > SUM_LONG;
+        RowSums r;
+        r.walk(lo + sub, listed ? lo : hi, G, acol, brp, bcol);
+        r.reduce<G>();
         if (i < M && sub == 0) {
-            const int na = arp[i + 1] - arp[i];
-            const float span = cmax >= cmin ? (float)(cmax - cmin) : 0.f;
-            feat[i] = make_float4(log2f(1.f + (float)na), log2f(1.f + (float)prod), log2f(1.f + (float)mx),
-                                  log2f(1.f + span));
-            if (prod_out) prod_out[i] = prod;
+            if (listed) long_list[1 + atomicAdd(long_list, 1)] = i;
+            else store_features(i, hi - lo, r, feat, prod_out);
         }
     }
 }
 
-void launch_features(const DevCSR &A, const DevCSR &B, float4 *feat, long long *prod_out, int nsm, cudaStream_t st) {
+__global__ void __launch_bounds__(SUM_THREADS) k_features_long(const int *__restrict__ arp,
+                                                               const int *__restrict__ acol,
+                                                               const int *__restrict__ brp,
+                                                               const int *__restrict__ bcol,
+                                                               float4 *__restrict__ feat,
+                                                               long long *__restrict__ prod_out,
+                                                               const int *__restrict__ long_list) {
+    __shared__ SumSmem s_sum;
+    const int n = long_list[0];
+    for (int e = blockIdx.x; e < n; e += gridDim.x) {
+        const int i = long_list[1 + e];
+        const int lo = arp[i], hi = arp[i + 1];
+        const RowSums r = block_row_sums(lo, hi, acol, brp, bcol, s_sum);
+        if (threadIdx.x == 0) store_features(i, hi - lo, r, feat, prod_out);
+    }
+}
+
+void launch_features(const DevCSR &A, const DevCSR &B, float4 *feat, long long *prod_out, int nsm, cudaStream_t st,
+                     int *long_list) {
     const double avg = A.M ? (double)A.nnz / A.M : 0.0;
     const int grid = nsm * 8;
-    if (avg <= 6) k_features<4><<<grid, 256, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, feat, prod_out);
-    else if (avg <= 24) k_features<16><<<grid, 256, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, feat, prod_out);
-    else k_features<32><<<grid, 256, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, feat, prod_out);
+    auto k = avg <= 6 ? k_features<4> : avg <= 24 ? k_features<16> : k_features<32>;
+    if (!long_rows_apart(A)) long_list = nullptr;
+    if (long_list) cudaMemsetAsync(long_list, 0, sizeof(int), st);
+    k<<<grid, SUM_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, feat, prod_out, long_list);
+    if (long_list)
+        k_features_long<<<grid / 2, SUM_THREADS, 0, st>>>(A.rp, A.col, B.rp, B.col, feat, prod_out, long_list);
 }
 
 // ---------------------------------------------------------------- MLP
@@ -246,7 +256,8 @@ __global__ void __launch_bounds__(256) k_capacity(const float *__restrict__ para
                                                   const long long *__restrict__ prod, int M, int N, float margin,
                                                   int *__restrict__ cap, unsigned long long *wide_prod,
                                                   const signed char *__restrict__ cls, bool large_no_slot) {
-    __shared__ float P[MLP_NTOTAL];
+    __shared__ __align__(16) float P[MLP_NTOTAL];  // read as 128-bit words
+
     __shared__ unsigned long long s_wide;
     for (int q = threadIdx.x; q < MLP_NTOTAL; q += blockDim.x) P[q] = params[q];
     if (threadIdx.x == 0) s_wide = 0;
@@ -284,12 +295,29 @@ __global__ void __launch_bounds__(256) k_compact(int M, const long long *__restr
     const int lane = lane_id();
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
     for (int i = gw; i < M; i += nw) {
-        if (flag[i] != ROW_VALUES) continue;
+        // loaded together, not one after the other
+        const unsigned char f = flag[i];
         const long long src = soff[i];
         const int dst = crp[i], n = crp[i + 1] - dst;
-        for (int q = lane; q < n; q += WARP) {
-            ccol[dst + q] = scol[src + q];
-            cval[dst + q] = sval[src + q];
+        if (f != ROW_VALUES) continue;
+        constexpr int U = 4;  // steps in flight
+        for (int q0 = lane; q0 < n; q0 += U * WARP) {
+            int c[U];
+            double v[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int q = q0 + u * WARP;
+                c[u] = q < n ? scol[src + q] : 0;
+                v[u] = q < n ? sval[src + q] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int q = q0 + u * WARP;
+                if (q < n) {
+                    ccol[dst + q] = c[u];
+                    cval[dst + q] = v[u];
+                }
+            }
         }
     }
 }
