@@ -78,6 +78,8 @@ struct hsmu_handle_s {
     cudaEvent_t ev_in, ev_panel, ev_out;
     long long *h_prod;
     size_t h_prod_cap;
+    // look-back state of the scans on the caller's stream, and of those on cs_tiles
+    ScanState scan, scan_tiles;
     // B's tile conversion runs on its own stream beside the bounds pass
     cudaStream_t cs_tiles;
     cudaEvent_t ev_tiles_start, ev_tiles_done;
@@ -278,7 +280,7 @@ int build_tiles(hsmu_handle_s *h, const hsmu_csr *B, hsmu_btiles *out, Ctl *ctl,
                 cudaEvent_t ev_done = nullptr) {
     int rc = HSMU_OK;
     cudaStream_t ks = st;
-    int *tcnt = nullptr, *scan_tmp = nullptr;
+    int *tcnt = nullptr;
     long long *tot = nullptr;
     DevCSR Bd = dev(B);
     out->M = B->M;
@@ -300,7 +302,6 @@ int build_tiles(hsmu_handle_s *h, const hsmu_csr *B, hsmu_btiles *out, Ctl *ctl,
         CK(salloc(h, &out->tile_off, (size_t)B->nnz, st));
     }
     CK(salloc(h, &tcnt, (size_t)B->M + 1, st));
-    CK(salloc(h, &scan_tmp, scan_tmp_ints(B->M), st));
     CK(salloc(h, &tot, 1, st));
     if (run && ev_start && ev_done) {
         CK(cudaEventRecord(ev_start, st));
@@ -308,7 +309,7 @@ int build_tiles(hsmu_handle_s *h, const hsmu_csr *B, hsmu_btiles *out, Ctl *ctl,
         ks = run;
     }
     launch_tiles_count(Bd, tcnt, validate, ctl, grid_rows(h), ks);
-    launch_scan(tcnt, out->tile_ptr, B->M, tot, scan_tmp, ctl, ks);
+    launch_scan(tcnt, out->tile_ptr, B->M, tot, ks == st ? h->scan : h->scan_tiles, ctl, ks);
     launch_tiles_fill(Bd, out->tile_ptr, out->tile_col, reinterpret_cast<unsigned long long *>(out->mask), out->tile_off, ctl, grid_rows(h), ks);
     CK(cudaGetLastError());
     if (read_count) {
@@ -351,7 +352,6 @@ struct PlainRun {
     RowInfo ri{};
     unsigned char *rep = nullptr;     // B rows that repeat the row before them
     long long *chunk_prod = nullptr;  // products per PROD_CHUNK rows (host-buffer entry)
-    int *scan_tmp = nullptr;
     Window *win = nullptr;
     long long win_cap = 0;
     WinCursors wc{};
@@ -420,7 +420,7 @@ struct PlainRun {
                                                      h->ev_tiles_start, h->ev_tiles_done)
                                        : build_tiles(h, B, &bt, ctl, 0, st, count_tiles, false);
             if (rc) return rc;
-            launches += 5;
+            launches += 3;
         }
         Btd = DevTiles{bt.tile_ptr, bt.tile_col, reinterpret_cast<const unsigned long long *>(bt.mask), bt.tile_off};
         if (ev_tiles) cudaEventRecord(ev_tiles, tiles_aside ? h->cs_tiles : st);
@@ -435,9 +435,7 @@ struct PlainRun {
         CKR(salloc(h, &ri.tmax, (size_t)M, st));
         CKR(salloc(h, &ri.bins, (size_t)M * NBIN, st));
         CKR(salloc(h, &ri.cls, (size_t)M, st));
-        CKR(salloc(h, &ri.bin_cnt, bin_scratch_ints(M), st));
         CKR(salloc(h, &ri.cnnz, (size_t)M + 1, st));
-        CKR(salloc(h, &scan_tmp, scan_tmp_ints(M), st));
         if (store) {
             CKR(grow_arena());
             ri.store = 1;
@@ -450,8 +448,8 @@ struct PlainRun {
                 have_store = true;
             }
         }
-        launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), scan_tmp, st);
-        launches += 6 + long_rows_apart(Ad);  // bounds + binning
+        launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), h->scan, st);
+        launches += 2 + long_rows_apart(Ad);  // bounds + binning
         // everything after this reads B's tiles
         if (tiles_aside) CKR(cudaStreamWaitEvent(st, h->ev_tiles_done, 0));
         tiles_aside = false;
@@ -488,12 +486,12 @@ struct PlainRun {
         if (have_store && ts_wbase) {
             // the listed rows' windows in row order, ahead of every other window: the value
             // pass hands windows out in array order, and R-MAT's heaviest rows come first
-            launch_scan(ts_nwin, ts_wbase, M, &ctl->win_listed, scan_tmp, ctl, st);
+            launch_scan(ts_nwin, ts_wbase, M, &ctl->win_listed, h->scan, ctl, st);
             CKR(cudaMemcpyAsync(&ctl->win_count, ts_wbase + M, sizeof(int), cudaMemcpyDeviceToDevice, st));
-            launches += 3;
+            launches++;
         }
-        launch_scan(ri.cnnz, crp, M, &ctl->nnz, scan_tmp, ctl, st);
-        launches += 6 + (Bd.N > SPAN_T * 64);  // count 3 (and the scattered rows'), scan 3
+        launch_scan(ri.cnnz, crp, M, &ctl->nnz, h->scan, ctl, st);
+        launches += 4 + (Bd.N > SPAN_T * 64);  // count 3 (and the scattered rows'), scan
         CKR(cudaGetLastError());
         CKR(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
         if (host_rp) CKR(cudaMemcpyAsync(host_rp, crp, sizeof(int32_t) * ((size_t)M + 1), cudaMemcpyDeviceToHost, st));
@@ -533,7 +531,6 @@ struct PlainRun {
         CKR(salloc(h, &wc.len, (size_t)nwin, st));
         CKR(salloc(h, &wc.off, (size_t)nwin + 1, st));
         CKR(salloc(h, &wc.total, 2, st));
-        CKR(salloc(h, &wc.scan_tmp, scan_tmp_ints((int)nwin), st));
         CKR(salloc(h, &wc.item_off, (size_t)nwin + 1, st));
         CKR(salloc(h, &wc.cur, (size_t)cap, st));
         CKR(salloc(h, &wc.heavy, (size_t)nwin, st));
@@ -561,8 +558,8 @@ struct PlainRun {
         if (hc.nnz == 0 || win_cap == 0 || (hc.bin_count[BIN_L] == 0 && hc.wide_rows == 0)) return;
         const TileStore tsd = store_view();
         launch_numeric(Ad, Bd, Btd, crp, ccol, cval, win, win_cap, nullptr, nullptr, nullptr, wc, ctl, o.arith, h->nsm,
-                       st, o.wait_polls, have_store ? &tsd : nullptr);
-        launches += 9;  // window lengths, two scans of 3, cursors, values
+                       st, h->scan, o.wait_polls, have_store ? &tsd : nullptr);
+        launches += 5;  // window lengths, two scans, cursors, values
     }
 
     // start a new panel: its windows reuse the window buffer from slot 0
@@ -941,7 +938,7 @@ int spgemm_learned_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, 
         // large rows with a tile list need no slot (they are written at their place in C)
         launch_capacity(model->params, feat, r.ri.prod, r.ri.cls, M, B->N, model->margin, cap, h->nsm, st,
                         &r.ctl->pred_wide_prod, r.have_store);
-        launch_scan64(cap, soff, M, &r.ctl->nnz, r.scan_tmp, st);  // nnz field holds the slot total for now
+        launch_scan64(cap, soff, M, &r.ctl->nnz, h->scan, r.ctl, st);  // nnz field holds the slot total for now
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(h->h_ctl, r.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -1011,7 +1008,6 @@ learned:
             CK(salloc(h, &wc.len, (size_t)win_cap, st));
             CK(salloc(h, &wc.off, (size_t)win_cap + 1, st));
             CK(salloc(h, &wc.total, 2, st));
-            CK(salloc(h, &wc.scan_tmp, scan_tmp_ints((int)win_cap), st));
             CK(salloc(h, &wc.item_off, (size_t)win_cap + 1, st));
             CK(salloc(h, &wc.cur, (size_t)cur_cap, st));
             CK(salloc(h, &wc.heavy, (size_t)win_cap, st));
@@ -1032,14 +1028,14 @@ learned:
         const int large_rows[NBIN] = {0, hc.bin_count[BIN_L], 0, 0};
         if (hc.bin_count[BIN_L] > 0 && r.have_store) {
             launch_spec_large(Ad, Btd, ri, tsd, spec, ctl, h->nsm, st);
-            launch_scan(r.ts_nwin, r.ts_wbase, M, &ctl->win_listed, r.scan_tmp, ctl, st);
+            launch_scan(r.ts_nwin, r.ts_wbase, M, &ctl->win_listed, h->scan, ctl, st);
             CK(cudaMemcpyAsync(&ctl->win_count, r.ts_wbase + M, sizeof(int), cudaMemcpyDeviceToDevice, st));
         }
         launch_structure(Ad, Bd, Btd, ri, spec, win, win_cap, ctl, o.arith, h->nsm, st, small_rows);
         if (hc.bin_count[BIN_L] > 0)
             launch_structure(Ad, Bd, Btd, ri, spec, win, win_cap, ctl, o.arith, h->nsm, st, large_rows,
                              r.have_store ? &tsd : nullptr);
-        launch_scan(ri.cnnz, crp, M, &ctl->nnz, r.scan_tmp, ctl, st);
+        launch_scan(ri.cnnz, crp, M, &ctl->nnz, h->scan, ctl, st);
         // exact nnz(C): rows that overflowed their slot can make it larger than the slot total
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
@@ -1062,7 +1058,7 @@ learned:
                          win_cap, ctl, o.arith, h->nsm, st, nullptr, r.have_store ? &tsd : nullptr);
         if (stats) cudaEventRecord(h->ev[4], st);
         launch_numeric(Ad, Bd, Btd, crp, ccol, cval, win, win_cap, flag, scol, soff, wc, ctl, o.arith, h->nsm, st,
-                       o.wait_polls, r.have_store ? &tsd : nullptr);
+                       h->scan, o.wait_polls, r.have_store ? &tsd : nullptr);
         CK(cudaGetLastError());
         if (stats) cudaEventRecord(h->ev[5], st);
         CK(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
@@ -1107,9 +1103,9 @@ learned:
         stats->ms_numeric = t;
         cudaEventElapsedTime(&t, h->ev[0], h->ev[5]);
         stats->ms_total = t;
-        // tiles 5, bounds + binning 6, features 1, capacity 1, scan 3, structure 3, scan 3, compact 1, redo 3,
-        // window lengths 1, their two scans 6, cursors 1, numeric 1
-        stats->launches = (o.validate ? 2 : 0) + (win_cap > 0 ? 35 : 27);
+        // tiles 3, bounds + binning 2, features 1, capacity 1, scan 1, structure 3, scan 1, compact 1, redo 3,
+        // window lengths 1, their two scans 2, cursors 1, numeric 1
+        stats->launches = (o.validate ? 2 : 0) + (win_cap > 0 ? 21 : 16);
     }
 done:
     pfree(crp, st);
@@ -1128,7 +1124,6 @@ int row_nnz_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, int32_t
     Ctl *ctl = nullptr;
     hsmu_btiles bt{};
     RowInfo ri{};
-    int *scan_tmp = nullptr;
     DevCSR Ad = dev(A), Bd = dev(B);
     DevTiles Btd{};
     ScratchScope scope(h, st);
@@ -1142,10 +1137,8 @@ int row_nnz_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, int32_t
     CK(salloc(h, &ri.tmax, (size_t)M, st));
     CK(salloc(h, &ri.bins, (size_t)M * NBIN, st));
     CK(salloc(h, &ri.cls, (size_t)M, st));
-    CK(salloc(h, &ri.bin_cnt, bin_scratch_ints(M), st));
-    CK(salloc(h, &scan_tmp, scan_tmp_ints(M), st));
     ri.cnnz = nnz_out;
-    launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), scan_tmp, st);
+    launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), h->scan, st);
     launch_count(Ad, Bd, Btd, ri, ctl, h->nsm, st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
@@ -1169,7 +1162,7 @@ int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_c
     const long long cap = (max_panel == 0 || max_panel > INT_MAX) ? INT_MAX : max_panel;
     const int M = A->M;
     int rc = HSMU_OK;
-    int *cnt = nullptr, *scan_tmp = nullptr, *col = nullptr;
+    int *cnt = nullptr, *col = nullptr;
     long long *rp = nullptr, *tot = nullptr;
     double *val = nullptr;
     Ctl *ctl = nullptr;
@@ -1190,16 +1183,15 @@ int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_c
     if (rc) goto done;
     CK(palloc(&rp, (size_t)M + 1, st));
     CK(salloc(h, &tot, 1, st));
-    CK(salloc(h, &scan_tmp, scan_tmp_ints(M), st));
-    launch_scan64(cnt, rp, M, tot, scan_tmp, st);
+    CK(salloc(h, &ctl, 1, st));
+    CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
+    launch_scan64(cnt, rp, M, tot, h->scan, ctl, st);
     CK(cudaGetLastError());
     hrp.resize((size_t)M + 1);
     CK(cudaMemcpyAsync(hrp.data(), rp, sizeof(long long) * ((size_t)M + 1), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     CK(palloc(&col, (size_t)hrp[M] + COL_PAD, st));
     CK(palloc(&val, (size_t)hrp[M], st));
-    CK(salloc(h, &ctl, 1, st));
-    CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     rc = build_tiles(h, B, &bt, ctl, 0, st, true, false);
     if (rc) goto done;
     for (int r0 = 0; r0 < M;) {
@@ -1296,6 +1288,12 @@ int hsmu_handle_create(hsmu_handle *out) {
             return HSMU_ERR_CUDA;
         }
     }
+    for (ScanState *s : {&h->scan, &h->scan_tiles})
+        if (cudaMalloc(&s->word, scan_state_bytes()) != cudaSuccess ||
+            cudaMemset(s->word, 0, scan_state_bytes()) != cudaSuccess) {
+            hsmu_handle_destroy(h);
+            return HSMU_ERR_ALLOC;
+        }
     // keep freed pool memory cached between calls (no re-mapping of large outputs)
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
@@ -1332,6 +1330,8 @@ int hsmu_handle_destroy(hsmu_handle h) {
         cudaFreeAsync(h->scratch.base, 0);  // every call of the handle has finished
         cudaStreamSynchronize(0);
     }
+    for (const ScanState *s : {&h->scan, &h->scan_tiles})
+        if (s->word) cudaFree(s->word);
     if (h->scratch.pool) cudaMemPoolDestroy(h->scratch.pool);
     if (h->h_ctl) cudaFreeHost(h->h_ctl);
     if (h->h_prod) cudaFreeHost(h->h_prod);
@@ -1423,11 +1423,10 @@ int hsmu_csr_transpose(hsmu_handle h, const hsmu_csr *A, hsmu_csr *At, void *str
     std::memset(At, 0, sizeof(*At));
     int rc = HSMU_OK;
     const long long n = A->nnz;
-    int *trp = nullptr, *tcol = nullptr, *si = nullptr, *hist = nullptr, *scan_tmp = nullptr;
+    int *trp = nullptr, *tcol = nullptr, *si = nullptr, *hist = nullptr;
     double *tval = nullptr, *sd = nullptr;
     long long *tot = nullptr;
     Ctl *ctl = nullptr;
-    const long long ntiles_scan = (long long)transpose_hist_ints(n) / 2;
     ScratchScope scope(h, st);
     CK(palloc(&trp, (size_t)A->N + 1, st));
     CK(palloc(&tcol, (size_t)n, st));
@@ -1435,11 +1434,10 @@ int hsmu_csr_transpose(hsmu_handle h, const hsmu_csr *A, hsmu_csr *At, void *str
     CK(salloc(h, &si, transpose_scratch_ints(n), st));
     CK(salloc(h, &sd, transpose_scratch_doubles(n), st));
     CK(salloc(h, &hist, transpose_hist_ints(n), st));
-    CK(salloc(h, &scan_tmp, scan_tmp_ints((int)ntiles_scan), st));
     CK(salloc(h, &tot, 1, st));
     CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
-    CK((cudaError_t)launch_transpose(dev(A), trp, tcol, tval, si, sd, hist, scan_tmp, tot, ctl, h->nsm, st));
+    CK((cudaError_t)launch_transpose(dev(A), trp, tcol, tval, si, sd, hist, h->scan, tot, ctl, h->nsm, st));
     CK(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (h->h_ctl->err) {

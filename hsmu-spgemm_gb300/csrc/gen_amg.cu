@@ -90,7 +90,7 @@ int scan_lengths(int *rp, int n, cudaStream_t st) {
         rc = HSMU_ERR_ALLOC;
     } else {
         cudaMemsetAsync(ctl, 0, sizeof(Ctl), st);
-        launch_scan(rp, rp, n, tot, tmp, ctl, st);
+        launch_scan3(rp, rp, n, tot, tmp, ctl, st);
         if (cudaGetLastError() != cudaSuccess) rc = HSMU_ERR_CUDA;
     }
     if (tmp) cudaFreeAsync(tmp, st);

@@ -46,8 +46,6 @@ struct RowInfo {
     int *bins;         // NBIN slabs of M row ids, each in ascending row order
     int *cnnz;         // exact nnz per row (count pass)
     signed char *cls;  // row class (RowBin) of every row, -1 for an empty row
-    int *bin_cnt;      // [NBIN][ceil(M/32)] rows of each class per 32-row chunk, then
-                       // its exclusive scan (bin_scratch_ints(M) entries)
     const unsigned char *rep;  // B rows that repeat the row before them (nullable; launch_row_repeat)
     int store;         // 1: the tile store is in use -- the count pass sizes each large row's
                        // list, min(tile span, sum of its B rows' tile counts), and adds the
@@ -82,8 +80,20 @@ struct TileStore {
     int all_stored;             // host: every large row got a list (no OR-walk rows left)
 };
 
-// scratch ints of RowInfo::bin_cnt for M rows
-size_t bin_scratch_ints(int M);
+// Look-back state of the single-pass scans (k_rows.cu): one per stream that scans, its words zeroed
+// once (scan_state_bytes())
+constexpr int LB_TILES = 4096;  // most tiles of a launch
+constexpr int LB_STREAMS = 4;   // sums looked back over at once
+struct ScanState {
+    void *word;
+    unsigned epoch;
+};
+struct LookBack {
+    unsigned *ctr;             // tickets handed out, blocks done
+    unsigned long long *word;  // [LB_STREAMS][LB_TILES]
+    unsigned epoch;
+};
+size_t scan_state_bytes();
 
 // k_tiles.cu
 void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int grid, cudaStream_t st);
@@ -94,7 +104,7 @@ void launch_row_repeat(const DevCSR &B, unsigned char *rep, int grid, cudaStream
 void launch_validate(const DevCSR &A, Ctl *ctl, int grid, cudaStream_t st);
 
 // k_rows.cu
-void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, int *scan_tmp, cudaStream_t st);
+void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, ScanState &scan, cudaStream_t st);
 // whether rows of many entries are taken in a launch of their own (hsmu_rowsums.cuh): it costs about
 // 3 us where there are none (a 5-point Laplacian of 65,536 rows: 9 + 3 us) and takes 30 us off a
 // power-law graph of 430,000 entries, so small or short-rowed matrices go without
@@ -105,12 +115,15 @@ inline bool long_rows_apart(const DevCSR &A) {
 constexpr int PROD_CHUNK = 64;
 void launch_chunk_prod(int M, const long long *prod, long long *out, int grid, cudaStream_t st);
 // exclusive scan of int counts (n entries) into out[0..n]; total (int64) into *total64;
-// sets DERR_OVERFLOW if the total exceeds INT32_MAX.  tmp must hold scan_tmp_ints(n) ints.
+// sets DERR_OVERFLOW if the total exceeds INT32_MAX.
 // in == out (an in-place scan) is allowed.
-size_t scan_tmp_ints(int n);
-void launch_scan(const int *in, int *out, int n, long long *total64, int *tmp, Ctl *ctl, cudaStream_t st);
+void launch_scan(const int *in, int *out, int n, long long *total64, ScanState &scan, Ctl *ctl, cudaStream_t st);
 // same with int64 output (no overflow limit)
-void launch_scan64(const int *in, long long *out, int n, long long *total64, int *tmp, cudaStream_t st);
+void launch_scan64(const int *in, long long *out, int n, long long *total64, ScanState &scan, Ctl *ctl,
+                   cudaStream_t st);
+// the int scan without a state: three launches, tmp holds scan_tmp_ints(n) ints
+size_t scan_tmp_ints(int n);
+void launch_scan3(const int *in, int *out, int n, long long *total64, int *tmp, Ctl *ctl, cudaStream_t st);
 
 // learned.cu
 // long_list (nullable): scratch of M + 1 ints
@@ -157,13 +170,12 @@ void launch_structure(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowI
 // flag (nullable): speculative-pass windows of rows flagged ROW_OVERFLOW are skipped;
 // scol/soff (nullable): speculative slots holding the columns of speculative-pass
 // windows, which the kernel copies to ccol
-// per-window cursors into the B rows (k_win_cursors): len/off/item_off/scan_tmp sized
+// per-window cursors into the B rows (k_win_cursors): len/off/item_off sized
 // for win_cap windows (+1), total for 2 entries, cur for cap entries (Ctl::cur_bound)
 struct WinCursors {
     int *len;
     long long *off;
     long long *total;
-    int *scan_tmp;
     int *item_off;  // the cursor pass's work items per window, scanned in place
     int *cur;
     int *heavy;     // windows of rows with many A entries (win_cap entries)
@@ -172,7 +184,7 @@ struct WinCursors {
 void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const int *crp, int *ccol, double *cval,
                     const Window *win, long long win_cap, const unsigned char *flag, const int *scol,
                     const long long *soff, const WinCursors &wc, Ctl *ctl, int arith, int nsm, cudaStream_t st,
-                    int wait_polls = 0, const TileStore *ts = nullptr);
+                    ScanState &scan, int wait_polls = 0, const TileStore *ts = nullptr);
 
 int run_dmul_selftest(unsigned long long n, unsigned long long seed, unsigned long long *out, cudaStream_t st);
 // FP64 lane operations per second of a full-grid chain probe
@@ -186,7 +198,7 @@ int configure_kernels();
 
 // k_transpose.cu: B = A^T (rows of B in ascending column order), scratch sized by the helpers
 int launch_transpose(const DevCSR &A, int *trp, int *tcol, double *tval, int *scratch_i, double *scratch_d,
-                     int *hist, int *scan_tmp, long long *total64, Ctl *ctl, int nsm, cudaStream_t st);
+                     int *hist, ScanState &scan, long long *total64, Ctl *ctl, int nsm, cudaStream_t st);
 size_t transpose_scratch_ints(long long nnz);
 size_t transpose_scratch_doubles(long long nnz);
 size_t transpose_hist_ints(long long nnz);

@@ -469,13 +469,13 @@ __global__ void __launch_bounds__(NUM_WARPS * 32, NUM_CTAS_PER_SM) k_numeric(con
 void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const int *crp, int *ccol, double *cval,
                     const Window *win, long long win_cap, const unsigned char *flag, const int *scol,
                     const long long *soff, const WinCursors &wc, Ctl *ctl, int arith, int nsm, cudaStream_t st,
-                    int wait_polls, const TileStore *ts) {
+                    ScanState &scan, int wait_polls, const TileStore *ts) {
     if (win_cap <= 0) return;
     cudaMemsetAsync(&ctl->win_next, 0, 3 * sizeof(int), st);  // and win_heavy, win_long
     k_win_len<<<nsm * 4, 256, 0, st>>>(const_cast<Window *>(win), (int)win_cap, A.M, A.rp, crp, ts ? ts->off : nullptr,
                                        ts ? ts->cnt : nullptr, ctl, wc.len, wc.item_off, wc.heavy);
-    launch_scan64(wc.len, wc.off, (int)win_cap, wc.total, wc.scan_tmp, st);
-    launch_scan(wc.item_off, wc.item_off, (int)win_cap, wc.total + 1, wc.scan_tmp, ctl, st);
+    launch_scan64(wc.len, wc.off, (int)win_cap, wc.total, scan, ctl, st);
+    launch_scan(wc.item_off, wc.item_off, (int)win_cap, wc.total + 1, scan, ctl, st);
     k_win_cursors<<<nsm * 16, 256, 0, st>>>(win, (int)win_cap, A.M, wc.off, wc.cap, A.rp, A.col, B.rp, Bt.ptr, Bt.col,
                                             Bt.off, wc.item_off, wc.cur, ctl);
     auto k = arith == AR_IMUL ? k_numeric<AR_IMUL> : arith == AR_FMA ? k_numeric<AR_FMA> : k_numeric<AR_RN>;

@@ -9,14 +9,13 @@
 // runs beside their construction).  The tile span decides the row class
 // (one warp with a dense span table, or one CTA with a chunked table), which
 // replaces the reference's host-round-trip binning (src/bining.cuh:1-207):
-// rows are binned on the device by a stable compaction (count per 32-row
-// chunk, scan, emit), so every bin lists its rows in ascending order and the
-// rows of a row panel are one contiguous slice of each bin.
+// rows are binned on the device by a stable single-pass compaction, so every bin
+// lists its rows in ascending order and the rows of a row panel are one
+// contiguous slice of each bin.
 //
-// Scan: three launches (block sums, scan of block sums, block scans), 64-bit
-// running totals, int32 output; replaces cub::DeviceScan::ExclusiveSum plus
-// the full-array D2H copies of the reference
-// (src/compressed/compressed_tileOR.cuh:620-622).
+// Scan: one launch with a look-back over the earlier tiles' sums, 64-bit running
+// totals; replaces cub::DeviceScan::ExclusiveSum plus the full-array D2H copies
+// of the reference (src/compressed/compressed_tileOR.cuh:620-622).
 #include <climits>
 
 #include "hsmu_common.cuh"
@@ -147,73 +146,7 @@ __global__ void __launch_bounds__(SUM_THREADS) k_bounds_long(const int *__restri
     mine.flush(s_tot, ctl);
 }
 
-// stable binning: rows of each class per 32-row chunk (warp per chunk) ...
-__global__ void __launch_bounds__(256) k_bin_count(int M, const signed char *__restrict__ cls, int *__restrict__ cnt) {
-    const int nch = (M + WARP - 1) / WARP;
-    const int lane = lane_id();
-    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) / WARP; c < nch; c += gridDim.x * blockDim.x / WARP) {
-        const int i = c * WARP + lane;
-        const int b = i < M ? cls[i] : -1;
-#pragma unroll
-        for (int k = 0; k < NBIN; k++) {
-            const int n = __popc(__ballot_sync(FULL, b == k));
-            if (lane == k) cnt[k * nch + c] = n;
-        }
-    }
-}
-
-// ... then, after the scan of those counts, every row at its place in its bin
-__global__ void __launch_bounds__(256) k_bin_emit(int M, const signed char *__restrict__ cls,
-                                                  const int *__restrict__ off, int *__restrict__ bins) {
-    const int nch = (M + WARP - 1) / WARP;
-    const int lane = lane_id();
-    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) / WARP; c < nch; c += gridDim.x * blockDim.x / WARP) {
-        const int i = c * WARP + lane;
-        const int b = i < M ? cls[i] : -1;
-#pragma unroll
-        for (int k = 0; k < NBIN; k++) {
-            const unsigned m = __ballot_sync(FULL, b == k);
-            if (b == k) bins[(size_t)k * M + (off[k * nch + c] - off[k * nch]) + __popc(m & lanemask_lt())] = i;
-        }
-    }
-}
-
-size_t bin_scratch_ints(int M) { return (size_t)NBIN * ((M + WARP - 1) / WARP) * 2 + 2; }
-
-void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, int *scan_tmp, cudaStream_t st) {
-    const double avg = A.M ? (double)A.nnz / A.M : 0.0;
-    // the bins are written after this pass: until then their space holds the long rows
-    int *list = long_rows_apart(A) ? ri.bins : nullptr;
-    auto k = avg <= 6 ? k_bounds<4> : avg <= 12 ? k_bounds<8> : avg <= 24 ? k_bounds<16> : k_bounds<32>;
-    k<<<grid, SUM_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
-    if (list) k_bounds_long<<<grid / 2, SUM_THREADS, 0, st>>>(A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
-    const int nch = (A.M + WARP - 1) / WARP;
-    int *cnt = ri.bin_cnt, *off = ri.bin_cnt + (size_t)NBIN * nch + 1;
-    k_bin_count<<<grid, 256, 0, st>>>(A.M, ri.cls, cnt);
-    launch_scan(cnt, off, NBIN * nch, &ctl->binned, scan_tmp, ctl, st);
-    k_bin_emit<<<grid, 256, 0, st>>>(A.M, ri.cls, off, ri.bins);
-}
-
-// products of every PROD_CHUNK consecutive rows: one warp per chunk (the host
-// orders its row panels by them)
-__global__ void __launch_bounds__(256) k_chunk_prod(int M, const long long *__restrict__ prod,
-                                                    long long *__restrict__ out) {
-    static_assert(PROD_CHUNK == 2 * WARP, "two rows per lane");
-    const int nch = (M + PROD_CHUNK - 1) / PROD_CHUNK;
-    const int lane = lane_id();
-    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nch; c += (gridDim.x * blockDim.x) >> 5) {
-        const int r0 = c * PROD_CHUNK + lane, r1 = r0 + WARP;
-        long long v = (r0 < M ? prod[r0] : 0ll) + (r1 < M ? prod[r1] : 0ll);
-        v = warp_sum(v);
-        if (lane == 0) out[c] = v;
-    }
-}
-
-void launch_chunk_prod(int M, const long long *prod, long long *out, int grid, cudaStream_t st) {
-    if (M > 0) k_chunk_prod<<<grid, 256, 0, st>>>(M, prod, out);
-}
-
-// ---------------------------------------------------------------- scan
+// ---------------------------------------------------------------- block scan
 constexpr int SCAN_T = 256;
 constexpr int SCAN_IPT = 8;
 constexpr int SCAN_ITEMS = SCAN_T * SCAN_IPT;
@@ -237,6 +170,270 @@ __device__ __forceinline__ long long block_excl_scan(long long v, long long *s_w
     return r;
 }
 
+// ---------------------------------------------------------------- single-pass scans
+// One launch instead of three: a block takes the next tile of the input (a
+// ticket, so every earlier tile has been started), publishes the tile's sum,
+// and looks back over its predecessors' words until one holds a prefix.  A word
+// is flag | epoch | value, so one 64-bit store publishes it; words of earlier
+// launches carry another epoch and need no clearing.  The ticket counter resets
+// itself when the last block is done.  The look-back's polls are bounded: a
+// block that gives up sets DERR_TIMEOUT and goes on with what it has.
+//
+// Small calls are launch-bound: with three launches per scan and two more for the
+// binning a Laplacian product had 18, now 10 (64^2 grid 163 -> 130 us, 256^2 210 ->
+// 177 us).  Two million items take 36 us (three launches: 32), 65,536 take 4.7 (9).
+constexpr int LB_EPOCH_BITS = 18;
+constexpr int LB_VALUE_BITS = 44;  // sums saturate there (1.7e13 entries are beyond any memory)
+constexpr unsigned long long LB_MAX = (1ull << LB_VALUE_BITS) - 1;
+constexpr unsigned long long LB_SUM = 1ull << 62, LB_PREFIX = 2ull << 62;
+constexpr int LB_POLLS = 1 << 20;
+
+__device__ __forceinline__ unsigned long long lb_word(unsigned long long flag, unsigned epoch, unsigned long long v) {
+    return flag | ((unsigned long long)epoch << LB_VALUE_BITS) | (v < LB_MAX ? v : LB_MAX);
+}
+
+// thread 0 of the block: the tile to take
+__device__ __forceinline__ int lb_ticket(LookBack lb) { return (int)atomicAdd(&lb.ctr[0], 1u); }
+// thread 0, once per block after its ticket and before it ends
+__device__ __forceinline__ void lb_done(LookBack lb, int ntiles) {
+    if (atomicAdd(&lb.ctr[1], 1u) == (unsigned)ntiles - 1u) {
+        lb.ctr[0] = 0;
+        lb.ctr[1] = 0;
+    }
+}
+
+// one whole warp: the sum of `stream`'s tiles before `tile`, whose own sum is `mine`
+__device__ __forceinline__ unsigned long long lb_prefix(LookBack lb, int stream, int tile, unsigned long long mine,
+                                                        Ctl *ctl) {
+    const int lane = lane_id();
+    volatile unsigned long long *w = lb.word + (size_t)stream * LB_TILES;
+    if (tile == 0) {
+        if (lane == 0) w[0] = lb_word(LB_PREFIX, lb.epoch, mine);
+        return 0;
+    }
+    if (lane == 0) w[tile] = lb_word(LB_SUM, lb.epoch, mine);
+    unsigned long long sum = 0;
+    for (int at = tile - 1; at >= 0; at -= WARP) {  // 32 predecessors, the nearest on lane 0
+        const int t = at - lane;
+        unsigned long long x = 0;
+        bool ready = false;
+        for (int poll = 0; poll < LB_POLLS; poll++) {
+            if (t >= 0 && !ready) {
+                x = w[t];
+                ready = (x >> 62) != 0 && (unsigned)((x >> LB_VALUE_BITS) & ((1u << LB_EPOCH_BITS) - 1u)) == lb.epoch;
+            }
+            if (__all_sync(FULL, t < 0 || ready)) break;
+        }
+        if (!__all_sync(FULL, t < 0 || ready)) {
+            if (lane == 0) set_err(&ctl->err, DERR_TIMEOUT);
+            if (!ready) x = 0;
+        }
+        // lanes up to the nearest prefix count
+        const unsigned pre = __ballot_sync(FULL, ready && (x >> 62) == 2);
+        const int last = pre ? __ffs(pre) - 1 : WARP - 1;
+        sum += warp_sum(t >= 0 && lane <= last ? x & LB_MAX : 0ull);
+        if (pre) break;
+    }
+    if (lane == 0) w[tile] = lb_word(LB_PREFIX, lb.epoch, sum + mine);
+    return sum;
+}
+
+// exclusive scan of n ints, `chunks` of SCAN_ITEMS per tile; in and out may be the same array (a
+// block reads each of its chunks before it writes it).  int output saturates, and a total beyond
+// INT_MAX sets DERR_OVERFLOW.
+template <class T>
+__global__ void __launch_bounds__(SCAN_T) k_scan_lb(const int *in, T *out, int n, int chunks, int ntiles,
+                                                    long long *total64, LookBack lb, Ctl *ctl) {
+    __shared__ long long s_warp[SCAN_T / 32 + 1];
+    __shared__ long long s_prefix;
+    __shared__ int s_tile;
+    if (threadIdx.x == 0) s_tile = lb_ticket(lb);
+    __syncthreads();
+    const int tile = s_tile;
+    const long long lo = (long long)tile * chunks * SCAN_ITEMS + (long long)threadIdx.x * SCAN_IPT;
+    int vals[SCAN_IPT];
+    long long v = 0;
+    for (int c = 0; c < chunks; c++) {
+        const long long base = lo + (long long)c * SCAN_ITEMS;
+#pragma unroll
+        for (int j = 0; j < SCAN_IPT; j++) {
+            vals[j] = base + j < n ? in[base + j] : 0;
+            v += vals[j];
+        }
+    }
+    long long sum;
+    const long long ex0 = block_excl_scan(v, s_warp, sum);
+    if (threadIdx.x < WARP) {
+        const unsigned long long p = lb_prefix(lb, 0, tile, (unsigned long long)sum, ctl);
+        if (threadIdx.x == 0) {
+            s_prefix = (long long)p;
+            lb_done(lb, ntiles);
+        }
+    }
+    __syncthreads();
+    long long run = s_prefix;
+    auto put = [&](long long at, long long x) {
+        if (sizeof(T) == 4) out[at] = (T)(x < (long long)INT_MAX ? x : (long long)INT_MAX);
+        else out[at] = (T)x;
+    };
+    if (tile == ntiles - 1 && threadIdx.x == 0) {
+        const long long total = run + sum;
+        *total64 = total;
+        put(n, total);
+        if (sizeof(T) == 4 && total > (long long)INT_MAX) set_err(&ctl->err, DERR_OVERFLOW);
+    }
+    for (int c = 0; c < chunks; c++) {
+        const long long base = lo + (long long)c * SCAN_ITEMS;
+        long long ex = ex0, tot = sum;
+        if (chunks > 1) {
+            v = 0;
+#pragma unroll
+            for (int j = 0; j < SCAN_IPT; j++) {
+                vals[j] = base + j < n ? in[base + j] : 0;
+                v += vals[j];
+            }
+            ex = block_excl_scan(v, s_warp, tot);
+        }
+        ex += run;
+#pragma unroll
+        for (int j = 0; j < SCAN_IPT; j++) {
+            if (base + j < n) put(base + j, ex);
+            ex += vals[j];
+        }
+        run += tot;
+    }
+}
+
+// tiles of a single-pass launch over n items: at most LB_TILES, of `chunks` pieces each
+static int lb_tiles(long long n, int piece, int &chunks) {
+    const long long pieces = n > 0 ? (n + piece - 1) / piece : 1;
+    chunks = (int)((pieces + LB_TILES - 1) / LB_TILES);
+    return (int)((pieces + chunks - 1) / chunks);
+}
+
+static LookBack next_epoch(ScanState &s, cudaStream_t st) {
+    if (++s.epoch >> LB_EPOCH_BITS) {  // the words of the launches before must not match again
+        cudaMemsetAsync(s.word, 0, scan_state_bytes(), st);
+        s.epoch = 1;
+    }
+    unsigned long long *w = reinterpret_cast<unsigned long long *>(s.word);
+    return LookBack{reinterpret_cast<unsigned *>(w + (size_t)LB_STREAMS * LB_TILES), w, s.epoch};
+}
+
+size_t scan_state_bytes() { return sizeof(unsigned long long) * ((size_t)LB_STREAMS * LB_TILES + 1); }
+
+void launch_scan(const int *in, int *out, int n, long long *total64, ScanState &scan, Ctl *ctl, cudaStream_t st) {
+    int chunks;
+    const int nt = lb_tiles(n, SCAN_ITEMS, chunks);
+    k_scan_lb<int><<<nt, SCAN_T, 0, st>>>(in, out, n, chunks, nt, total64, next_epoch(scan, st), ctl);
+}
+
+void launch_scan64(const int *in, long long *out, int n, long long *total64, ScanState &scan, Ctl *ctl,
+                   cudaStream_t st) {
+    int chunks;
+    const int nt = lb_tiles(n, SCAN_ITEMS, chunks);
+    k_scan_lb<long long><<<nt, SCAN_T, 0, st>>>(in, out, n, chunks, nt, total64, next_epoch(scan, st), ctl);
+}
+
+// Stable binning in one pass: every row at its place in its class's bin, rows in ascending order
+// (row panels are slices of the bins).  A tile counts its rows of each class, one warp per class
+// looks back, and the rows are then placed 256 at a time.
+constexpr int BIN_T = 256;
+constexpr int BIN_ROWS = 4 * BIN_T;
+static_assert(NBIN <= LB_STREAMS && NBIN <= BIN_T / WARP, "a look-back stream and a warp per class");
+
+__global__ void __launch_bounds__(BIN_T) k_bins(int M, const signed char *__restrict__ cls, int rows, int ntiles,
+                                                int *__restrict__ bins, LookBack lb, Ctl *ctl) {
+    constexpr int NW = BIN_T / WARP;
+    __shared__ int s_cnt[NBIN], s_warp[NBIN][NW];
+    __shared__ int s_tile;
+    const int lane = lane_id(), w = threadIdx.x >> 5;
+    if (threadIdx.x == 0) s_tile = lb_ticket(lb);
+    if (threadIdx.x < NBIN) s_cnt[threadIdx.x] = 0;
+    __syncthreads();
+    const int tile = s_tile;
+    const long long lo = (long long)tile * rows;
+    const int r0 = (int)lo, r1 = (int)min(lo + rows, (long long)M);
+    int cnt[NBIN] = {};
+    for (int i = r0 + (int)threadIdx.x; i < r1; i += BIN_T) {
+        const int b = cls[i];
+#pragma unroll
+        for (int k = 0; k < NBIN; k++) cnt[k] += b == k;
+    }
+#pragma unroll
+    for (int k = 0; k < NBIN; k++) {
+        const int c = warp_sum(cnt[k]);
+        if (lane == 0 && c) atomicAdd(&s_cnt[k], c);
+    }
+    __syncthreads();
+    if (w < NBIN) {
+        const unsigned long long p = lb_prefix(lb, w, tile, (unsigned long long)s_cnt[w], ctl);
+        __syncwarp();
+        if (lane == 0) s_cnt[w] = (int)p;  // from here: where the tile's next row of the class goes
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) lb_done(lb, ntiles);
+    for (int c0 = r0; c0 < r1; c0 += BIN_T) {
+        const int i = c0 + (int)threadIdx.x;
+        const int b = i < r1 ? cls[i] : -1;
+        unsigned mine = 0;
+#pragma unroll
+        for (int k = 0; k < NBIN; k++) {
+            const unsigned m = __ballot_sync(FULL, b == k);
+            if (b == k) mine = m;
+            if (lane == k) s_warp[k][w] = __popc(m);
+        }
+        __syncthreads();
+        if (b >= 0) {
+            int at = s_cnt[b] + __popc(mine & lanemask_lt());
+            for (int j = 0; j < w; j++) at += s_warp[b][j];
+            bins[(size_t)b * M + at] = i;
+        }
+        __syncthreads();
+        if (threadIdx.x < NBIN)
+            for (int j = 0; j < NW; j++) s_cnt[threadIdx.x] += s_warp[threadIdx.x][j];
+        __syncthreads();
+    }
+}
+
+static void launch_bins(int M, const RowInfo &ri, ScanState &scan, Ctl *ctl, cudaStream_t st) {
+    if (M <= 0) return;
+    int chunks;
+    const int nt = lb_tiles(M, BIN_ROWS, chunks);
+    k_bins<<<nt, BIN_T, 0, st>>>(M, ri.cls, chunks * BIN_ROWS, nt, ri.bins, next_epoch(scan, st), ctl);
+}
+
+void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, ScanState &scan, cudaStream_t st) {
+    const double avg = A.M ? (double)A.nnz / A.M : 0.0;
+    // the bins are written after this pass: until then their space holds the long rows
+    int *list = long_rows_apart(A) ? ri.bins : nullptr;
+    auto k = avg <= 6 ? k_bounds<4> : avg <= 12 ? k_bounds<8> : avg <= 24 ? k_bounds<16> : k_bounds<32>;
+    k<<<grid, SUM_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
+    if (list) k_bounds_long<<<grid / 2, SUM_THREADS, 0, st>>>(A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
+    launch_bins(A.M, ri, scan, ctl, st);
+}
+
+// products of every PROD_CHUNK consecutive rows: one warp per chunk (the host
+// orders its row panels by them)
+__global__ void __launch_bounds__(256) k_chunk_prod(int M, const long long *__restrict__ prod,
+                                                    long long *__restrict__ out) {
+    static_assert(PROD_CHUNK == 2 * WARP, "two rows per lane");
+    const int nch = (M + PROD_CHUNK - 1) / PROD_CHUNK;
+    const int lane = lane_id();
+    for (int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < nch; c += (gridDim.x * blockDim.x) >> 5) {
+        const int r0 = c * PROD_CHUNK + lane, r1 = r0 + WARP;
+        long long v = (r0 < M ? prod[r0] : 0ll) + (r1 < M ? prod[r1] : 0ll);
+        v = warp_sum(v);
+        if (lane == 0) out[c] = v;
+    }
+}
+
+void launch_chunk_prod(int M, const long long *prod, long long *out, int grid, cudaStream_t st) {
+    if (M > 0) k_chunk_prod<<<grid, 256, 0, st>>>(M, prod, out);
+}
+
+// ---------------------------------------------------------------- scan in three launches
+// for callers without a handle (the allocation-free tile conversion, the AMG generators)
 __global__ void __launch_bounds__(SCAN_T) k_scan_sums(const int *__restrict__ in, int n, long long *bsum) {
     __shared__ long long s_warp[SCAN_T / 32 + 1];
     const long long base = (long long)blockIdx.x * SCAN_ITEMS + threadIdx.x * SCAN_IPT;
@@ -293,42 +490,12 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_out(const int *in, int *out, in
     }
 }
 
-__global__ void __launch_bounds__(SCAN_T) k_scan_out64(const int *__restrict__ in, long long *__restrict__ out, int n,
-                                                       const long long *__restrict__ boff,
-                                                       const long long *total64) {
-    __shared__ long long s_warp[SCAN_T / 32 + 1];
-    const long long base = (long long)blockIdx.x * SCAN_ITEMS + threadIdx.x * SCAN_IPT;
-    int vals[SCAN_IPT];
-    long long v = 0;
-#pragma unroll
-    for (int j = 0; j < SCAN_IPT; j++) {
-        vals[j] = base + j < n ? in[base + j] : 0;
-        v += vals[j];
-    }
-    long long tot;
-    long long ex = block_excl_scan(v, s_warp, tot) + boff[blockIdx.x];
-#pragma unroll
-    for (int j = 0; j < SCAN_IPT; j++) {
-        if (base + j < n) out[base + j] = ex;
-        ex += vals[j];
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = *total64;
-}
-
-void launch_scan64(const int *in, long long *out, int n, long long *total64, int *tmp, cudaStream_t st) {
-    const int nb = n > 0 ? (n + SCAN_ITEMS - 1) / SCAN_ITEMS : 1;
-    long long *bsum = reinterpret_cast<long long *>(tmp);
-    k_scan_sums<<<nb, SCAN_T, 0, st>>>(in, n, bsum);
-    k_scan_top<<<1, SCAN_T, 0, st>>>(bsum, nb, total64);
-    k_scan_out64<<<nb, SCAN_T, 0, st>>>(in, out, n, bsum, total64);
-}
-
 size_t scan_tmp_ints(int n) {
     const int nb = (n + SCAN_ITEMS - 1) / SCAN_ITEMS;
     return (size_t)(nb > 0 ? nb : 1) * 2 + 2;
 }
 
-void launch_scan(const int *in, int *out, int n, long long *total64, int *tmp, Ctl *ctl, cudaStream_t st) {
+void launch_scan3(const int *in, int *out, int n, long long *total64, int *tmp, Ctl *ctl, cudaStream_t st) {
     const int nb = n > 0 ? (n + SCAN_ITEMS - 1) / SCAN_ITEMS : 1;
     long long *bsum = reinterpret_cast<long long *>(tmp);
     k_scan_sums<<<nb, SCAN_T, 0, st>>>(in, n, bsum);

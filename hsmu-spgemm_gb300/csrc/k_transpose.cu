@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256) k_tr_rowptr(const int *__restrict__ key, 
 }
 
 int launch_transpose(const DevCSR &A, int *trp, int *tcol, double *tval, int *scratch_i, double *scratch_d,
-                     int *hist, int *scan_tmp, long long *total64, Ctl *ctl, int nsm, cudaStream_t st) {
+                     int *hist, ScanState &scan, long long *total64, Ctl *ctl, int nsm, cudaStream_t st) {
     const int n = (int)A.nnz;
     if (n == 0) {
         return (int)cudaMemsetAsync(trp, 0, sizeof(int) * ((size_t)A.N + 1), st);
@@ -111,8 +111,7 @@ int launch_transpose(const DevCSR &A, int *trp, int *tcol, double *tval, int *sc
         int *drow = last ? tcol : ((p % 2 == 0) ? row1 : row0);
         double *dval = last ? tval : ((p % 2 == 0) ? val1 : val0);
         k_tr_hist<<<blocks, TR_WARPS * 32, 0, st>>>(skey, n, 8 * p, ntiles, hist);
-        launch_scan(hist, hist + (size_t)TR_RADIX * ntiles + 1, TR_RADIX * ntiles, total64, scan_tmp, ctl, st);
-        // (scan_tmp holds scan_tmp_ints(TR_RADIX * ntiles) ints)
+        launch_scan(hist, hist + (size_t)TR_RADIX * ntiles + 1, TR_RADIX * ntiles, total64, scan, ctl, st);
         k_tr_scatter<<<blocks, TR_WARPS * 32, 0, st>>>(skey, srow, sval, n, 8 * p, ntiles,
                                                       hist + (size_t)TR_RADIX * ntiles + 1, dkey, drow, dval);
         skey = dkey;

@@ -98,7 +98,7 @@ extern "C" int hsmu_btiles_build_noalloc(const hsmu_csr *B, int32_t *tile_ptr, i
     if (err) return status_from_dev_err(err);
     // counts into tile_ptr[0..M), in-place exclusive scan (tile_ptr[M] = total), then the fill
     launch_tiles_count(Bd, tile_ptr, 0, ctl, nsm * 8, st);
-    launch_scan(tile_ptr, tile_ptr, B->M, total, scan_tmp, ctl, st);
+    launch_scan3(tile_ptr, tile_ptr, B->M, total, scan_tmp, ctl, st);
     launch_tiles_fill(Bd, tile_ptr, tile_col, reinterpret_cast<unsigned long long *>(mask), tile_off, ctl, nsm * 8, st);
     if (cudaGetLastError() != cudaSuccess) return HSMU_ERR_CUDA;
     if (cudaMemcpyAsync(&err, &ctl->err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) return HSMU_ERR_CUDA;
