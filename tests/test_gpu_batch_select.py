@@ -1,0 +1,81 @@
+"""Selecting tiles of the batched engine: left rows around the limit of eight entries, right rows with
+no, one and two entries (the last send the rest of the product to the insertion lists), products that
+change kind from one to the next, partial tiles, every arithmetic, against the oracle."""
+import numpy as np
+import pytest
+
+import oracle
+from hsmu_gb import gen
+
+pytestmark = pytest.mark.gpu
+
+
+def rows_of(lengths, k, seed):
+    rng = np.random.default_rng(seed)
+    cols = [np.sort(rng.choice(k, size=min(int(n), k), replace=False)) for n in lengths]
+    rp = np.concatenate(([0], np.cumsum([c.size for c in cols]))).astype(np.int32)
+    col = np.concatenate(cols).astype(np.int32) if rp[-1] else np.zeros(0, np.int32)
+    return gen.CSR(len(lengths), k, rp, col, rng.uniform(-1, 1, col.size))
+
+
+def selector(k, n, seed, empty=0.0, two=()):
+    rng = np.random.default_rng(seed)
+    lens = np.where(rng.random(k) < empty, 0, 1)
+    for i in two:
+        lens[i] = 2
+    return rows_of(lens, n, seed + 1)
+
+
+def products():
+    rng = np.random.default_rng(5)
+    out = []
+    # rows of 0..8 entries, few right columns (runs of up to eight equal ones) and many
+    for M, n in ((1, 1), (31, 3), (32, 5), (33, 400), (1000, 7), (3001, 2000)):
+        out.append((rows_of(rng.integers(0, 9, M), 300, M), selector(300, n, M + 50, empty=0.2)))
+    # a row of nine entries in some tile; a right row of two entries met late; a plain product between
+    lens = np.full(500, 7)
+    lens[321] = 9
+    out.append((rows_of(lens, 200, 7), selector(200, 40, 8)))
+    out.append((rows_of(np.full(700, 6), 900, 9), selector(900, 50, 10, two=(899,))))
+    out.append((gen.laplacian2d(20, seed=1), gen.laplacian2d(20, seed=2)))
+    out.append((rows_of(np.full(257, 8), 64, 11), selector(64, 64, 12)))
+    return out
+
+
+@pytest.mark.parametrize("grid", [0, 1])  # every tile to another warp; all tiles of a warp's in turn
+@pytest.mark.parametrize("arith", [0, 1, 2])
+def test_selecting_products(engine, arith, grid):
+    import hsmu_gb
+
+    prods = products()
+    A = [hsmu_gb.DeviceCSR.from_host(a) for a, _ in prods]
+    B = [hsmu_gb.DeviceCSR.from_host(b) for _, b in prods]
+    batch = hsmu_gb.Batch(engine, hsmu_gb.BATCH_PRODUCT, A, B, arith=arith)
+    for tiny in (32, 8, 7):
+        batch.set_params(tiny, grid)
+        batch.execute()
+        batch.status()
+        for p, (a, b) in enumerate(prods):
+            C = batch.result(p).to_host()
+            rp, col, val = oracle.spgemm(a, b, fma=arith == 1)
+            np.testing.assert_array_equal(C.row_ptr.astype(np.int64), rp)
+            np.testing.assert_array_equal(C.col, col)
+            assert np.array_equal(C.val.view(np.int64), val.view(np.int64)), (tiny, p)
+    batch.close()
+
+
+def test_negative_zero_and_cancellation(engine):
+    # a lone product -0.0 becomes 0.0 + -0.0 = 0.0; products that cancel leave their entry
+    import hsmu_gb
+
+    A = gen.CSR(2, 4, np.array([0, 1, 4], np.int32), np.array([0, 1, 2, 3], np.int32), np.array([-0.0, 1.0, -1.0, 2.0]))
+    B = gen.CSR(4, 3, np.array([0, 1, 2, 3, 4], np.int32), np.array([2, 1, 1, 0], np.int32), np.ones(4))
+    batch = hsmu_gb.Batch(engine, hsmu_gb.BATCH_PRODUCT, [hsmu_gb.DeviceCSR.from_host(A)],
+                          [hsmu_gb.DeviceCSR.from_host(B)])
+    batch.execute()
+    batch.status()
+    C = batch.result(0).to_host()
+    rp, col, val = oracle.spgemm(A, B)
+    np.testing.assert_array_equal(C.col, col)
+    assert np.array_equal(C.val.view(np.int64), val.view(np.int64))
+    batch.close()
