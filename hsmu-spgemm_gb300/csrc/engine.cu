@@ -80,9 +80,9 @@ struct hsmu_handle_s {
     size_t h_prod_cap;
     // look-back state of the scans on the caller's stream, and of those on cs_tiles
     ScanState scan, scan_tiles;
-    // B's tile conversion runs on its own stream beside the bounds pass
+    // side stream: B's tile conversion beside the bounds pass, light row classes beside the others
     cudaStream_t cs_tiles;
-    cudaEvent_t ev_tiles_start, ev_tiles_done;
+    cudaEvent_t ev_side_start, ev_side_done;
 };
 
 namespace {
@@ -116,6 +116,8 @@ constexpr long long HOST_PANEL_BYTES = 32ll << 20;
 
 // entries of B from which its tile conversion runs on a second stream beside the bounds pass
 constexpr int TILES_ASIDE_MIN_NNZ = 1 << 19;
+// entries of A from which the count pass takes the side stream too
+constexpr int SIDE_MIN_NNZ = 1 << 16;
 // average entries of B's rows from which repeated rows are looked for: chains of shorter rows
 // are not taken (hsmu_products.cuh), and the chain kernel's registers cost rows without chains
 // (scalar 27-point rows: 296 us with it, 169 us without)
@@ -274,9 +276,10 @@ void free_owned(std::initializer_list<const void *> ptrs) {
 // B -> 64-column tiles, in arrays sized by nnz(B) >= tiles: for the caller to keep
 // (keep: from the default pool), or scratch.  With `run` the kernels run on that
 // stream instead (after everything already queued on `st`), and ev_done marks the
-// end: the caller makes `st` wait on it before anything reads the tiles.
+// end: the caller makes `st` wait on it before anything reads the tiles.  gated: after
+// the bounds pass, nothing is built when no row of A needs tiles.
 int build_tiles(hsmu_handle_s *h, const hsmu_csr *B, hsmu_btiles *out, Ctl *ctl, int validate, cudaStream_t st,
-                bool read_count, bool keep, cudaStream_t run = nullptr, cudaEvent_t ev_start = nullptr,
+                bool read_count, bool keep, bool gated = false, cudaStream_t run = nullptr, cudaEvent_t ev_start = nullptr,
                 cudaEvent_t ev_done = nullptr) {
     int rc = HSMU_OK;
     cudaStream_t ks = st;
@@ -308,9 +311,9 @@ int build_tiles(hsmu_handle_s *h, const hsmu_csr *B, hsmu_btiles *out, Ctl *ctl,
         CK(cudaStreamWaitEvent(run, ev_start, 0));
         ks = run;
     }
-    launch_tiles_count(Bd, tcnt, validate, ctl, grid_rows(h), ks);
-    launch_scan(tcnt, out->tile_ptr, B->M, tot, ks == st ? h->scan : h->scan_tiles, ctl, ks);
-    launch_tiles_fill(Bd, out->tile_ptr, out->tile_col, reinterpret_cast<unsigned long long *>(out->mask), out->tile_off, ctl, grid_rows(h), ks);
+    launch_tiles_count(Bd, tcnt, validate, ctl, grid_rows(h), ks, gated);
+    launch_scan(tcnt, out->tile_ptr, B->M, tot, ks == st ? h->scan : h->scan_tiles, ctl, ks, gated);
+    launch_tiles_fill(Bd, out->tile_ptr, out->tile_col, reinterpret_cast<unsigned long long *>(out->mask), out->tile_off, ctl, grid_rows(h), ks, gated);
     CK(cudaGetLastError());
     if (read_count) {
         CK(cudaMemcpyAsync(&ctl->ntiles, out->tile_ptr + B->M, sizeof(int), cudaMemcpyDeviceToDevice, ks));
@@ -325,6 +328,12 @@ done:
     }
     return rc;
 }
+
+#define CKQ(x)                    \
+    do {                          \
+        const int _rc = (x);      \
+        if (_rc) return _rc;      \
+    } while (0)
 
 #define CKR(x)                              \
     do {                                    \
@@ -347,7 +356,7 @@ struct PlainRun {
     int M = 0;
     DevCSR Ad{}, Bd{};
     hsmu_btiles bt{};
-    bool tiles_aside = false;  // B's tiles are being built on the handle's conversion stream
+    bool side_busy = false;  // the handle's side stream has work that `st` does not wait for yet
     DevTiles Btd{};
     RowInfo ri{};
     unsigned char *rep = nullptr;     // B rows that repeat the row before them
@@ -412,18 +421,17 @@ struct PlainRun {
                      bool store) {
         if (Bt_in) {
             bt = *Bt_in;
-        } else {
+        } else if (B->nnz >= TILES_ASIDE_MIN_NNZ) {
             // B's tiles on their own stream, beside the bounds pass (which reads B's columns);
-            // a small B is converted in line (the hand-over would cost more than it overlaps)
-            tiles_aside = B->nnz >= TILES_ASIDE_MIN_NNZ;
-            const int rc = tiles_aside ? build_tiles(h, B, &bt, ctl, 0, st, count_tiles, false, h->cs_tiles,
-                                                     h->ev_tiles_start, h->ev_tiles_done)
-                                       : build_tiles(h, B, &bt, ctl, 0, st, count_tiles, false);
-            if (rc) return rc;
+            // a small B is converted in line (the hand-over would cost more than it overlaps),
+            // after the bounds pass, which may find that no row needs its tiles
+            side_busy = true;
+            CKQ(build_tiles(h, B, &bt, ctl, 0, st, count_tiles, false, false, h->cs_tiles, h->ev_side_start,
+                            h->ev_side_done));
             launches += 3;
         }
-        Btd = DevTiles{bt.tile_ptr, bt.tile_col, reinterpret_cast<const unsigned long long *>(bt.mask), bt.tile_off};
-        if (ev_tiles) cudaEventRecord(ev_tiles, tiles_aside ? h->cs_tiles : st);
+        const bool in_line = !Bt_in && !side_busy;
+        if (ev_tiles && !in_line) cudaEventRecord(ev_tiles, side_busy ? h->cs_tiles : st);
         if (B->M > 0 && B->nnz >= (long long)REPEAT_MIN_ROW * B->M) {
             CKR(salloc(h, &rep, (size_t)B->M, st));
             launch_row_repeat(Bd, rep, grid_rows(h), st);
@@ -450,10 +458,32 @@ struct PlainRun {
         }
         launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), h->scan, st);
         launches += 2 + long_rows_apart(Ad);  // bounds + binning
+        if (in_line) {
+            CKQ(build_tiles(h, B, &bt, ctl, 0, st, count_tiles, false, !count_tiles));
+            launches += 3;
+            if (ev_tiles) cudaEventRecord(ev_tiles, st);
+        }
+        Btd = DevTiles{bt.tile_ptr, bt.tile_col, reinterpret_cast<const unsigned long long *>(bt.mask), bt.tile_off};
         // everything after this reads B's tiles
-        if (tiles_aside) CKR(cudaStreamWaitEvent(st, h->ev_tiles_done, 0));
-        tiles_aside = false;
+        if (side_busy) CKR(cudaStreamWaitEvent(st, h->ev_side_done, 0));
+        side_busy = false;
         CKR(cudaGetLastError());
+        return HSMU_OK;
+    }
+
+    // The handle's side stream for kernels that need nothing of what runs on `st` until join():
+    // rows of few products are latency-bound tails (50-80 us for a few thousand tiny rows) that
+    // hide behind the other classes.
+    int fork() {
+        CKR(cudaEventRecord(h->ev_side_start, st));
+        CKR(cudaStreamWaitEvent(h->cs_tiles, h->ev_side_start, 0));
+        side_busy = true;
+        return HSMU_OK;
+    }
+    int join() {
+        CKR(cudaEventRecord(h->ev_side_done, h->cs_tiles));
+        CKR(cudaStreamWaitEvent(st, h->ev_side_done, 0));
+        side_busy = false;
         return HSMU_OK;
     }
 
@@ -480,7 +510,12 @@ struct PlainRun {
     // scan into C's row pointers and nnz(C), one host read
     int count_scan(int32_t *host_rp, long long *host_prod = nullptr) {
         CKR(palloc(&crp, (size_t)M + 1, st));
-        launch_count_small(Ad, Bd, Btd, ri, ctl, h->nsm, st);
+        // the classes are not known here yet: short rows (a 5-point stencil: all tiny) and long ones
+        // (27 points and more: all of the warp class) gain nothing from a second stream
+        const bool apart = Ad.nnz >= SIDE_MIN_NNZ && Ad.nnz > 6ll * M && Ad.nnz <= 24ll * M;
+        if (apart) CKQ(fork());
+        launch_count_light(Ad, Bd, ri, ctl, h->nsm, apart ? h->cs_tiles : st);
+        launch_count_warp(Ad, Btd, ri, ctl, h->nsm, st);
         const TileStore tsd = store_view();
         launch_count_large(Ad, Btd, ri, have_store ? &tsd : nullptr, ctl, h->nsm, st);
         if (have_store && ts_wbase) {
@@ -490,6 +525,7 @@ struct PlainRun {
             CKR(cudaMemcpyAsync(&ctl->win_count, ts_wbase + M, sizeof(int), cudaMemcpyDeviceToDevice, st));
             launches++;
         }
+        if (apart) CKQ(join());
         launch_scan(ri.cnnz, crp, M, &ctl->nnz, h->scan, ctl, st);
         launches += 4 + (Bd.N > SPAN_T * 64);  // count 3 (and the scattered rows'), scan
         CKR(cudaGetLastError());
@@ -544,12 +580,28 @@ struct PlainRun {
     }
 
     // sorted columns of rows lo..hi-1, values of warp-sized rows, numeric windows of the others
-    void structure(int lo, int hi) {
-        if (hc.nnz == 0) return;
+    int structure(int lo, int hi) {
+        if (hc.nnz == 0) return HSMU_OK;
         const TileStore tsd = store_view();
-        launch_structure(Ad, Bd, Btd, ri, RowOut{OUT_PLAIN, crp, nullptr, ccol, cval, nullptr, nullptr, lo, hi}, win,
-                         win_cap, ctl, o.arith, h->nsm, st, hc.bin_count, have_store ? &tsd : nullptr);
-        for (int b = 0; b < NBIN; b++) launches += hc.bin_count[b] > 0;
+        const RowOut out{OUT_PLAIN, crp, nullptr, ccol, cval, nullptr, nullptr, lo, hi};
+        int rows[NBIN];
+        for (int b = 0; b < NBIN; b++) {
+            rows[b] = hc.bin_count[b];
+            launches += rows[b] > 0;
+        }
+        // tiny and scattered rows beside the warp and large classes, or beside each other
+        const bool heavy = rows[BIN_DS] > 0 || rows[BIN_L] > 0;
+        const bool apart = rows[BIN_TINY] > 0 ? heavy || rows[BIN_H] > 0 : heavy && rows[BIN_H] > 0;
+        if (apart) {
+            CKQ(fork());
+            int side[NBIN] = {0, 0, rows[BIN_TINY], heavy ? rows[BIN_H] : 0};
+            launch_structure_light(Ad, Bd, ri, out, ctl, o.arith, h->nsm, h->cs_tiles, side);
+            rows[BIN_TINY] = 0;
+            if (heavy) rows[BIN_H] = 0;
+        }
+        launch_structure(Ad, Bd, Btd, ri, out, win, win_cap, ctl, o.arith, h->nsm, st, rows,
+                         have_store ? &tsd : nullptr);
+        return apart ? join() : HSMU_OK;
     }
 
     // values of the windows made by the preceding structure() call (none unless a row
@@ -579,9 +631,9 @@ struct PlainRun {
 
     // the outputs that were not handed on; the rest goes with `scope`, which outlives this
     void release() {
-        // an early return may leave the conversion stream at work on the scratch
-        if (tiles_aside) cudaStreamWaitEvent(st, h->ev_tiles_done, 0);
-        tiles_aside = have_store = false;
+        // an early return may leave the side stream at work on the scratch
+        if (side_busy) cudaStreamSynchronize(h->cs_tiles);
+        side_busy = have_store = false;
         pfree(crp, st);
         if (ext_col) {
             ccol = nullptr;
@@ -634,11 +686,11 @@ int spgemm_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, const hs
     if (!rc) rc = r.alloc_output();
     if (!rc) {
         if (stats) cudaEventRecord(h->ev[3], st);
-        r.structure(0, A->M);
+        rc = r.structure(0, A->M);
         if (stats) cudaEventRecord(h->ev[4], st);
-        r.values();
+        if (!rc) r.values();
         if (stats) cudaEventRecord(h->ev[5], st);
-        rc = r.finish();
+        if (!rc) rc = r.finish();
     }
     if (rc != HSMU_OK) {
         r.release();
@@ -821,7 +873,8 @@ int spgemm_host_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsm
             const long long e0 = C->row_ptr[lo], e1 = C->row_ptr[hi];
             // the columns are final after the structure pass: their copy starts while the
             // value pass runs
-            r.structure(lo, hi);
+            rc = r.structure(lo, hi);
+            if (rc) break;
             if (e1 > e0) {
                 CK(cudaEventRecord(h->ev_panel, st));
                 CK(cudaStreamWaitEvent(h->cs_out, h->ev_panel, 0));
@@ -890,6 +943,7 @@ int spgemm_learned_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, 
     double *cval = nullptr, *sval = nullptr;
     Window *win = nullptr;
     long long win_cap = 0, spec_total = 0, cur_cap = 0;
+    bool listed = false;
     WinCursors wc{};
     Ctl hc{};
     std::memset(C, 0, sizeof(*C));
@@ -934,20 +988,45 @@ int spgemm_learned_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, 
         CK(salloc(h, &feat, (size_t)M, st));
         CK(salloc(h, &cap, (size_t)M + 1, st));
         CK(salloc(h, &soff, (size_t)M + 1, st));
-        launch_features(r.Ad, r.Bd, feat, nullptr, h->nsm, st, cap);  // cap is written after
+        CK(salloc(h, &flag, (size_t)M, st));
+        CK(cudaMemsetAsync(flag, 0, (size_t)M, st));
+        // The listed large rows are counted, and their windows placed (first, in row order: the value
+        // pass hands windows out in array order, and R-MAT's heaviest rows come first), whatever is
+        // predicted for the others: that runs beside the prediction (R-MAT scale 15: 240 us against
+        // 45 us and a host read).
+        listed = r.have_store && hc.bin_count[BIN_L] > 0;
+        cudaStream_t ps = listed ? h->cs_tiles : st;
+        if (listed) {
+            rc = r.fork();
+            if (rc) goto done;
+            launch_spec_large(r.Ad, r.Btd, r.ri, r.store_view(), RowOut{OUT_SPEC, nullptr, nullptr, nullptr, nullptr,
+                                                                        r.ri.cnnz, flag, 0, M},
+                              r.ctl, h->nsm, st);
+            launch_scan(r.ts_nwin, r.ts_wbase, M, &r.ctl->win_listed, h->scan, r.ctl, st);
+            CK(cudaMemcpyAsync(&r.ctl->win_count, r.ts_wbase + M, sizeof(int), cudaMemcpyDeviceToDevice, st));
+        }
+        launch_features(r.Ad, r.Bd, feat, nullptr, h->nsm, ps, cap);  // cap is written after
         // large rows with a tile list need no slot (they are written at their place in C)
-        launch_capacity(model->params, feat, r.ri.prod, r.ri.cls, M, B->N, model->margin, cap, h->nsm, st,
+        launch_capacity(model->params, feat, r.ri.prod, r.ri.cls, M, B->N, model->margin, cap, h->nsm, ps,
                         &r.ctl->pred_wide_prod, r.have_store);
-        launch_scan64(cap, soff, M, &r.ctl->nnz, h->scan, r.ctl, st);  // nnz field holds the slot total for now
+        // the nnz field holds the slot total for now
+        launch_scan64(cap, soff, M, &r.ctl->nnz, listed ? h->scan_tiles : h->scan, r.ctl, ps);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(h->h_ctl, r.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+        CK(cudaMemcpyAsync(h->h_ctl, r.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, ps));
+        CK(cudaStreamSynchronize(ps));
+        r.side_busy = false;
         hc = *h->h_ctl;
         if (hc.err) {
             rc = err_from_dev(hc.err);
             goto done;
         }
-        if (!o.learned_always && (double)hc.pred_wide_prod < LEARNED_MIN_SHARE * (double)hc.products) goto plain;
+        if (!o.learned_always && (double)hc.pred_wide_prod < LEARNED_MIN_SHARE * (double)hc.products) {
+            if (listed) {  // the plain path counts (and lists) the large rows itself
+                CK(cudaMemsetAsync(&r.ctl->store_tiles, 0, sizeof(long long), st));
+                CK(cudaMemsetAsync(&r.ctl->store_used, 0, sizeof(long long), st));
+            }
+            goto plain;
+        }
         goto learned;
     }
 plain:
@@ -959,11 +1038,11 @@ plain:
         if (!rc) rc = r.alloc_output();
         if (!rc) {
             if (stats) cudaEventRecord(h->ev[3], st);
-            r.structure(0, M);
+            rc = r.structure(0, M);
             if (stats) cudaEventRecord(h->ev[4], st);
-            r.values();
+            if (!rc) r.values();
             if (stats) cudaEventRecord(h->ev[5], st);
-            rc = r.finish();
+            if (!rc) rc = r.finish();
         }
         if (rc) goto done;
         C->M = M;
@@ -988,8 +1067,6 @@ learned:
         const DevCSR &Ad = r.Ad, &Bd = r.Bd;
         const DevTiles &Btd = r.Btd;
         RowInfo &ri = r.ri;
-        CK(salloc(h, &flag, (size_t)M, st));
-        CK(cudaMemsetAsync(flag, 0, (size_t)M, st));
         if (stats) cudaEventRecord(h->ev[2], st);
         spec_total = hc.nnz;
         win_cap = 2 * (long long)hc.win_bound;  // speculative pass + redo of overflowing rows
@@ -1018,23 +1095,26 @@ learned:
         // C by the redo pass (the prediction has nothing to skip for them: their count pass
         // builds the list the structure pass streams).
         const RowOut spec{OUT_SPEC, nullptr, soff, scol, sval, ri.cnnz, flag, 0, M};
-        // The listed large rows' windows are placed first, in row order (scan of their
-        // counts), before any warp row's window: the value pass hands windows out in array
-        // order, and R-MAT's heaviest rows come first.  The redo pass then streams those rows
-        // without barriers.
-        TileStore tsd{r.ts_off, r.ts_cnt, r.ts_nwin, r.ts_wbase, h->arena_col, h->arena_ent,
-                      h->arena_cap, 0};
-        const int small_rows[NBIN] = {hc.bin_count[BIN_DS], 0, hc.bin_count[BIN_TINY], hc.bin_count[BIN_H]};
+        TileStore tsd = r.store_view();
+        tsd.all_stored = 0;
+        // rows that need no tiles beside the others, as in PlainRun::structure
+        const bool apart = hc.bin_count[BIN_DS] > 0 && (hc.bin_count[BIN_TINY] > 0 || hc.bin_count[BIN_H] > 0);
+        const int light_rows[NBIN] = {0, 0, hc.bin_count[BIN_TINY], hc.bin_count[BIN_H]};
+        const int warp_rows[NBIN] = {hc.bin_count[BIN_DS], 0, 0, 0};
         const int large_rows[NBIN] = {0, hc.bin_count[BIN_L], 0, 0};
-        if (hc.bin_count[BIN_L] > 0 && r.have_store) {
-            launch_spec_large(Ad, Btd, ri, tsd, spec, ctl, h->nsm, st);
-            launch_scan(r.ts_nwin, r.ts_wbase, M, &ctl->win_listed, h->scan, ctl, st);
-            CK(cudaMemcpyAsync(&ctl->win_count, r.ts_wbase + M, sizeof(int), cudaMemcpyDeviceToDevice, st));
+        if (apart) {
+            rc = r.fork();
+            if (rc) goto done;
         }
-        launch_structure(Ad, Bd, Btd, ri, spec, win, win_cap, ctl, o.arith, h->nsm, st, small_rows);
+        launch_structure_light(Ad, Bd, ri, spec, ctl, o.arith, h->nsm, apart ? h->cs_tiles : st, light_rows);
+        launch_structure(Ad, Bd, Btd, ri, spec, win, win_cap, ctl, o.arith, h->nsm, st, warp_rows);
         if (hc.bin_count[BIN_L] > 0)
             launch_structure(Ad, Bd, Btd, ri, spec, win, win_cap, ctl, o.arith, h->nsm, st, large_rows,
                              r.have_store ? &tsd : nullptr);
+        if (apart) {
+            rc = r.join();
+            if (rc) goto done;
+        }
         launch_scan(ri.cnnz, crp, M, &ctl->nnz, h->scan, ctl, st);
         // exact nnz(C): rows that overflowed their slot can make it larger than the slot total
         CK(cudaGetLastError());
@@ -1210,9 +1290,9 @@ int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_c
         if (!rc && r.hc.nnz != hrp[r1] - hrp[r0]) rc = HSMU_ERR_INTERNAL;
         if (!rc) rc = r.alloc_output();
         if (!rc) {
-            r.structure(0, Ap.M);
-            r.values();
-            rc = r.finish();
+            rc = r.structure(0, Ap.M);
+            if (!rc) r.values();
+            if (!rc) rc = r.finish();
         }
         r.release();
         if (rc) goto done;
@@ -1271,8 +1351,8 @@ int hsmu_handle_create(hsmu_handle *out) {
         cudaEventCreateWithFlags(&h->ev_panel, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&h->ev_out, cudaEventDisableTiming) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->cs_tiles, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->ev_tiles_start, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->ev_tiles_done, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&h->ev_side_start, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&h->ev_side_done, cudaEventDisableTiming) != cudaSuccess) {
         hsmu_handle_destroy(h);
         return HSMU_ERR_CUDA;
     }
@@ -1316,7 +1396,7 @@ int hsmu_handle_destroy(hsmu_handle h) {
     if (!h) return HSMU_OK;
     for (auto &e : h->ev)
         if (e) cudaEventDestroy(e);
-    for (cudaEvent_t e : {h->ev_in, h->ev_panel, h->ev_out, h->ev_tiles_start, h->ev_tiles_done})
+    for (cudaEvent_t e : {h->ev_in, h->ev_panel, h->ev_out, h->ev_side_start, h->ev_side_done})
         if (e) cudaEventDestroy(e);
     if (h->arena_col || h->arena_ent) {
         cudaDeviceSynchronize();  // no call of this handle still reads the arena

@@ -24,11 +24,11 @@ constexpr unsigned FULL = 0xffffffffu;
 constexpr int SPAN_T = 512;
 // ... unless it has more products than this: then a CTA takes it (BIN_L), with a tile list.  One warp
 // took 1 ms over a hub row of a power-law graph within 512 tiles, in the count pass and again in the
-// structure pass: A*A^T of 30,011 vertices 4.18 ms without the limit, 2.99 at 65,536 products, 2.71 at
-// 32,768, 2.50 at 16,384, 2.42 at 8,192.  The line is kept where the learned scheduler still has its
-// saving, the warp class's count pass (R-MAT scale 15: 2.35 ms against 2.39 at 32,768; below, its own
-// passes cost more than that).
-constexpr long long DS_PROD = 32768;
+// structure pass: A*A^T of 30,011 vertices 4.18 ms without the limit, 2.44 at 32,768 products, 2.37 at
+// 24,576, 2.29 at 16,384, 2.25 at 12,288.  The line is kept where the learned scheduler still has its
+// saving, the warp class's count pass (R-MAT scale 15: 2.13 ms against 2.18 at 24,576; at 16,384 the
+// two are within 1.3 %).
+constexpr long long DS_PROD = 24576;
 // Numeric windows: consecutive tiles of one C row with
 //   < WIN_CAP slots (cut where the tile's first slot crosses a multiple of WIN_CUT),
 //   <= WIN_TCAP tiles (cut where the tile's rank in the row crosses a multiple of WIN_TCAP),
@@ -119,6 +119,9 @@ struct Ctl {
     int long_rows;                   // rows listed by the bounds pass for its second launch
     RowCounter rows[3];              // row hand-out of the kernels that give a CTA one row at a time
 };
+
+// whether any row of A reads B's tiles (after the bounds pass)
+__device__ __forceinline__ bool tiles_read(const Ctl *ctl) { return ctl->bin_count[BIN_DS] || ctl->bin_count[BIN_L]; }
 
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;

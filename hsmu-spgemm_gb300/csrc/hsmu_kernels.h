@@ -95,10 +95,19 @@ struct LookBack {
 };
 size_t scan_state_bytes();
 
+// blocks of a grid-stride launch: `most`, or fewer when `per_block` items each are enough (a small
+// call's launches otherwise spend their time on a thousand empty blocks)
+inline int grid_for(int most, long long items, int per_block) {
+    const long long need = (items + per_block - 1) / per_block;
+    return need < 1 ? 1 : (need < most ? (int)need : most);
+}
+
 // k_tiles.cu
-void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int grid, cudaStream_t st);
+// gated: nothing is done when no row of A reads B's tiles (Ctl::bin_count, after the bounds pass)
+void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int grid, cudaStream_t st,
+                        bool gated = false);
 void launch_tiles_fill(const DevCSR &B, const int *tptr, int *tcol, unsigned long long *tmask, int *toff, Ctl *ctl,
-                       int grid, cudaStream_t st);
+                       int grid, cudaStream_t st, bool gated = false);
 // rep[k]: row k of B has the columns of row k - 1 (B.M bytes)
 void launch_row_repeat(const DevCSR &B, unsigned char *rep, int grid, cudaStream_t st);
 void launch_validate(const DevCSR &A, Ctl *ctl, int grid, cudaStream_t st);
@@ -117,7 +126,9 @@ void launch_chunk_prod(int M, const long long *prod, long long *out, int grid, c
 // exclusive scan of int counts (n entries) into out[0..n]; total (int64) into *total64;
 // sets DERR_OVERFLOW if the total exceeds INT32_MAX.
 // in == out (an in-place scan) is allowed.
-void launch_scan(const int *in, int *out, int n, long long *total64, ScanState &scan, Ctl *ctl, cudaStream_t st);
+// gated: as launch_tiles_count (out and *total64 are then left alone)
+void launch_scan(const int *in, int *out, int n, long long *total64, ScanState &scan, Ctl *ctl, cudaStream_t st,
+                 bool gated = false);
 // same with int64 output (no overflow limit)
 void launch_scan64(const int *in, long long *out, int n, long long *total64, ScanState &scan, Ctl *ctl,
                    cudaStream_t st);
@@ -141,10 +152,10 @@ void launch_compact(int M, const long long *soff, const int *crp, const unsigned
 // k_symbolic.cu
 void launch_count(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm,
                   cudaStream_t st);
-// the same in two launches: rows of the tiny and warp classes, then the large class
+// the same by class: rows that need no tiles (tiny, scattered), warp rows, the large class
 // (ts: nullable; when given, the large rows' C tiles are stored while the arena lasts)
-void launch_count_small(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm,
-                        cudaStream_t st);
+void launch_count_light(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int nsm, cudaStream_t st);
+void launch_count_warp(const DevCSR &A, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm, cudaStream_t st);
 void launch_count_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const TileStore *ts, Ctl *ctl, int nsm,
                         cudaStream_t st);
 // learned path, large rows: exact count and tile list in its speculative pass;
@@ -165,6 +176,10 @@ void launch_fill_scattered(const DevCSR &A, const DevCSR &B, RowInfo ri, RowOut 
 void launch_structure(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, RowOut out, Window *win,
                       long long win_cap, Ctl *ctl, int arith, int nsm, cudaStream_t st,
                       const int *class_rows = nullptr, const TileStore *ts = nullptr);
+// the classes that need no tiles, alone (launch_structure launches them too unless class_rows says
+// that there are none)
+void launch_structure_light(const DevCSR &A, const DevCSR &B, RowInfo ri, RowOut out, Ctl *ctl, int arith, int nsm,
+                            cudaStream_t st, const int *class_rows);
 
 // k_numeric.cu
 // flag (nullable): speculative-pass windows of rows flagged ROW_OVERFLOW are skipped;

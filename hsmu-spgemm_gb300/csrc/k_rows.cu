@@ -243,7 +243,8 @@ __device__ __forceinline__ unsigned long long lb_prefix(LookBack lb, int stream,
 // INT_MAX sets DERR_OVERFLOW.
 template <class T>
 __global__ void __launch_bounds__(SCAN_T) k_scan_lb(const int *in, T *out, int n, int chunks, int ntiles,
-                                                    long long *total64, LookBack lb, Ctl *ctl) {
+                                                    long long *total64, LookBack lb, Ctl *ctl, bool gated) {
+    if (gated && !tiles_read(ctl)) return;  // every block: no ticket is taken
     __shared__ long long s_warp[SCAN_T / 32 + 1];
     __shared__ long long s_prefix;
     __shared__ int s_tile;
@@ -322,17 +323,18 @@ static LookBack next_epoch(ScanState &s, cudaStream_t st) {
 
 size_t scan_state_bytes() { return sizeof(unsigned long long) * ((size_t)LB_STREAMS * LB_TILES + 1); }
 
-void launch_scan(const int *in, int *out, int n, long long *total64, ScanState &scan, Ctl *ctl, cudaStream_t st) {
+void launch_scan(const int *in, int *out, int n, long long *total64, ScanState &scan, Ctl *ctl, cudaStream_t st,
+                 bool gated) {
     int chunks;
     const int nt = lb_tiles(n, SCAN_ITEMS, chunks);
-    k_scan_lb<int><<<nt, SCAN_T, 0, st>>>(in, out, n, chunks, nt, total64, next_epoch(scan, st), ctl);
+    k_scan_lb<int><<<nt, SCAN_T, 0, st>>>(in, out, n, chunks, nt, total64, next_epoch(scan, st), ctl, gated);
 }
 
 void launch_scan64(const int *in, long long *out, int n, long long *total64, ScanState &scan, Ctl *ctl,
                    cudaStream_t st) {
     int chunks;
     const int nt = lb_tiles(n, SCAN_ITEMS, chunks);
-    k_scan_lb<long long><<<nt, SCAN_T, 0, st>>>(in, out, n, chunks, nt, total64, next_epoch(scan, st), ctl);
+    k_scan_lb<long long><<<nt, SCAN_T, 0, st>>>(in, out, n, chunks, nt, total64, next_epoch(scan, st), ctl, false);
 }
 
 // Stable binning in one pass: every row at its place in its class's bin, rows in ascending order
@@ -407,8 +409,10 @@ void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int g
     const double avg = A.M ? (double)A.nnz / A.M : 0.0;
     // the bins are written after this pass: until then their space holds the long rows
     int *list = long_rows_apart(A) ? ri.bins : nullptr;
+    const int lanes = avg <= 6 ? 4 : avg <= 12 ? 8 : avg <= 24 ? 16 : 32;
     auto k = avg <= 6 ? k_bounds<4> : avg <= 12 ? k_bounds<8> : avg <= 24 ? k_bounds<16> : k_bounds<32>;
-    k<<<grid, SUM_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
+    k<<<grid_for(grid, A.M, SUM_THREADS / lanes), SUM_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, list,
+                                                                        ctl);
     if (list) k_bounds_long<<<grid / 2, SUM_THREADS, 0, st>>>(A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
     launch_bins(A.M, ri, scan, ctl, st);
 }

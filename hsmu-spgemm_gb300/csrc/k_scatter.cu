@@ -302,14 +302,14 @@ __global__ void __launch_bounds__(HF_WARPS * 32, hf_ctas<AR>())
 }
 
 void launch_count_scattered(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int nsm, cudaStream_t st) {
-    k_count_h<<<nsm * HC_CTAS_PER_SM, HC_WARPS * 32, HC_WARPS * sizeof(HSmem), st>>>(A.M, A.rp, A.col, B.rp, B.col, ri,
+    k_count_h<<<grid_for(nsm * HC_CTAS_PER_SM, A.M, HC_WARPS), HC_WARPS * 32, HC_WARPS * sizeof(HSmem), st>>>(A.M, A.rp, A.col, B.rp, B.col, ri,
                                                                                      ctl);
 }
 
 template <int AR>
 static void fill_scattered(const DevCSR &A, const DevCSR &B, RowInfo ri, RowOut out, Ctl *ctl, int nsm,
                            cudaStream_t st) {
-    k_fill_h<AR><<<nsm * hf_ctas<AR>(), HF_WARPS * 32, HF_WARPS * sizeof(HSmem), st>>>(A.M, A.rp, A.col, A.val, B.rp,
+    k_fill_h<AR><<<grid_for(nsm * hf_ctas<AR>(), A.M, HF_WARPS), HF_WARPS * 32, HF_WARPS * sizeof(HSmem), st>>>(A.M, A.rp, A.col, A.val, B.rp,
                                                                                        B.col, B.val, ri, out, ctl);
 }
 

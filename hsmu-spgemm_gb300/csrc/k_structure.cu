@@ -504,30 +504,38 @@ __global__ void __launch_bounds__(TINYF_THREADS) k_fill_tiny(int M, const int *_
     if (bad) set_err(&ctl->err, DERR_INTERNAL);
 }
 
-void launch_structure(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, RowOut out, Window *win,
-                      long long win_cap, Ctl *ctl, int arith, int nsm, cudaStream_t st, const int *class_rows,
-                      const TileStore *ts) {
+void launch_structure_light(const DevCSR &A, const DevCSR &B, RowInfo ri, RowOut out, Ctl *ctl, int arith, int nsm,
+                            cudaStream_t st, const int *class_rows) {
     if (!class_rows || class_rows[BIN_TINY] > 0) {
         auto kt = arith == AR_IMUL ? k_fill_tiny<AR_IMUL> : arith == AR_FMA ? k_fill_tiny<AR_FMA> : k_fill_tiny<AR_RN>;
-        kt<<<nsm * 4, TINYF_THREADS, 0, st>>>(A.M, A.rp, A.col, A.val, B.rp, B.col, B.val, ri, out, ctl);
+        kt<<<grid_for(nsm * 4, class_rows ? class_rows[BIN_TINY] : A.M, TINYF_THREADS), TINYF_THREADS, 0, st>>>(
+            A.M, A.rp, A.col, A.val, B.rp, B.col, B.val, ri, out, ctl);
     }
     if (class_rows ? class_rows[BIN_H] > 0 : B.N > SPAN_T * 64)
         launch_fill_scattered(A, B, ri, out, ctl, arith, nsm, st);
+}
+
+void launch_structure(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, RowOut out, Window *win,
+                      long long win_cap, Ctl *ctl, int arith, int nsm, cudaStream_t st, const int *class_rows,
+                      const TileStore *ts) {
+    launch_structure_light(A, B, ri, out, ctl, arith, nsm, st, class_rows);
     if (!class_rows || class_rows[BIN_DS] > 0) {
         const bool rep = ri.rep != nullptr;
         auto kds = arith == AR_IMUL  ? (rep ? k_struct_ds<AR_IMUL, true> : k_struct_ds<AR_IMUL, false>)
                    : arith == AR_FMA ? (rep ? k_struct_ds<AR_FMA, true> : k_struct_ds<AR_FMA, false>)
                                      : (rep ? k_struct_ds<AR_RN, true> : k_struct_ds<AR_RN, false>);
-        kds<<<nsm * SDS_CTAS_PER_SM, SDS_WARPS * 32, SDS_WARPS * sizeof(SdsSmem), st>>>(
+        kds<<<grid_for(nsm * SDS_CTAS_PER_SM, class_rows ? class_rows[BIN_DS] : A.M, SDS_WARPS), SDS_WARPS * 32, SDS_WARPS * sizeof(SdsSmem), st>>>(
             A.M, A.rp, A.col, A.val, B.rp, B.col, B.val, Bt.ptr, Bt.col, Bt.mask, ri, out, win, win_cap, ctl);
     }
     if (!class_rows || class_rows[BIN_L] > 0) {
         // rows with a stored tile list are streamed by k_struct_ls (PLAIN, REDO; in SPEC
         // mode the count kernel already wrote them), the others take the OR walk
         const bool list = ts && ts->cnt;
-        if (list && out.mode != OUT_SPEC) k_struct_ls<<<nsm * 6, SLS_THREADS, 0, st>>>(A.M, ri, *ts, out, win, win_cap, ctl);
+        const int rows_l = class_rows ? class_rows[BIN_L] : A.M;
+        if (list && out.mode != OUT_SPEC) 
+            k_struct_ls<<<grid_for(nsm * 6, rows_l, 1), SLS_THREADS, 0, st>>>(A.M, ri, *ts, out, win, win_cap, ctl);
         if (!list || !ts->all_stored)
-            k_struct_l<<<nsm * 3, SL_THREADS, sizeof(SlSmem), st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, out,
+            k_struct_l<<<grid_for(nsm * 3, rows_l, 1), SL_THREADS, sizeof(SlSmem), st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, out,
                                                                     win, win_cap, list ? ts->cnt : nullptr,
                                                                     list ? ts->cap : 0, ctl);
     }

@@ -211,33 +211,36 @@ __global__ void __launch_bounds__(TINY_THREADS) k_count_tiny(int M, const int *_
     if (bad) set_err(&ctl->err, DERR_INTERNAL);
 }
 
-void launch_count_small(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm,
-                        cudaStream_t st) {
-    k_count_tiny<<<nsm * 4, TINY_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, ri, ctl);
+void launch_count_light(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int nsm, cudaStream_t st) {
+    k_count_tiny<<<grid_for(nsm * 4, A.M, TINY_THREADS), TINY_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, ri, ctl);
     if (B.N > SPAN_T * 64) launch_count_scattered(A, B, ri, ctl, nsm, st);  // else no row's span is that wide
-    k_count_ds<<<nsm * 6, DS_WARPS * 32, 0, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, ctl);
+}
+
+void launch_count_warp(const DevCSR &A, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm, cudaStream_t st) {
+    k_count_ds<<<grid_for(nsm * 6, A.M, DS_WARPS), DS_WARPS * 32, 0, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, ctl);
 }
 
 void launch_count_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const TileStore *ts, Ctl *ctl, int nsm,
                         cudaStream_t st) {
     const size_t smem = DCH_COUNT * sizeof(unsigned long long);
     if (ts && ts->tcol && ts->tent && ts->cap > 0 && ri.store)
-        k_count_l<LM_STORE><<<nsm * 6, L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, *ts,
+        k_count_l<LM_STORE><<<grid_for(nsm * 6, A.M, 1), L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, *ts,
                                                                RowOut{}, ctl);
     else
-        k_count_l<LM_COUNT><<<nsm * 6, L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri,
+        k_count_l<LM_COUNT><<<grid_for(nsm * 6, A.M, 1), L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri,
                                                                TileStore{}, RowOut{}, ctl);
 }
 
 void launch_spec_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const TileStore &ts, RowOut out, Ctl *ctl,
                        int nsm, cudaStream_t st) {
     const size_t smem = DCH_COUNT * sizeof(unsigned long long);
-    k_count_l<LM_SPEC><<<nsm * 6, L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, ts, out, ctl);
+    k_count_l<LM_SPEC><<<grid_for(nsm * 6, A.M, 1), L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, ts, out, ctl);
 }
 
 void launch_count(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm,
                   cudaStream_t st) {
-    launch_count_small(A, B, Bt, ri, ctl, nsm, st);
+    launch_count_light(A, B, ri, ctl, nsm, st);
+    launch_count_warp(A, Bt, ri, ctl, nsm, st);
     launch_count_large(A, Bt, ri, nullptr, ctl, nsm, st);
 }
 

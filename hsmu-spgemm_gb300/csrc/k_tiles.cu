@@ -21,7 +21,8 @@ template <bool FILL, int TILE_U>
 __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ brp, const int *__restrict__ bcol,
                                                int N, int *__restrict__ tcnt_or_ptr, int *__restrict__ tcol,
                                                unsigned long long *__restrict__ tmask, int *__restrict__ toff,
-                                               int validate, Ctl *ctl) {
+                                               int validate, Ctl *ctl, bool gated) {
+    if (gated && !tiles_read(ctl)) return;
     const int lane = lane_id();
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
@@ -122,13 +123,15 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
 // 65,536 rows: 5.7 -> 8.2 and 13.7 -> 15.7 us).
 static bool tiles_short(const DevCSR &B) { return B.nnz <= 8ll * B.M; }
 
-void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int grid, cudaStream_t st) {
-    (tiles_short(B) ? k_tiles<false, 1> : k_tiles<false, 4>)<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, tcnt, nullptr, nullptr, nullptr, validate, ctl);
+void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int grid, cudaStream_t st, bool gated) {
+    grid = grid_for(grid, B.M, 256 / WARP);
+    (tiles_short(B) ? k_tiles<false, 1> : k_tiles<false, 4>)<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, tcnt, nullptr, nullptr, nullptr, validate, ctl, gated);
 }
 
 void launch_tiles_fill(const DevCSR &B, const int *tptr, int *tcol, unsigned long long *tmask, int *toff, Ctl *ctl,
-                       int grid, cudaStream_t st) {
-    (tiles_short(B) ? k_tiles<true, 1> : k_tiles<true, 4>)<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, const_cast<int *>(tptr), tcol, tmask, toff, 0, ctl);
+                       int grid, cudaStream_t st, bool gated) {
+    grid = grid_for(grid, B.M, 256 / WARP);
+    (tiles_short(B) ? k_tiles<true, 1> : k_tiles<true, 4>)<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, const_cast<int *>(tptr), tcol, tmask, toff, 0, ctl, gated);
 }
 
 // rep[k] = 1 when row k of B holds the same columns as row k - 1 (the rows of one finite-element
@@ -151,7 +154,7 @@ __global__ void __launch_bounds__(256) k_row_repeat(int K, const int *__restrict
 }
 
 void launch_row_repeat(const DevCSR &B, unsigned char *rep, int grid, cudaStream_t st) {
-    k_row_repeat<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, rep);
+    k_row_repeat<<<grid_for(grid, B.M, 256 / WARP), 256, 0, st>>>(B.M, B.rp, B.col, rep);
 }
 
 // Validation of A: sorted, unique, in-range columns (one warp per row).
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(256) k_validate(int M, const int *__restrict__
 }
 
 void launch_validate(const DevCSR &A, Ctl *ctl, int grid, cudaStream_t st) {
-    k_validate<<<grid, 256, 0, st>>>(A.M, A.rp, A.col, A.N, A.nnz, ctl);
+    k_validate<<<grid_for(grid, A.M, 256 / WARP), 256, 0, st>>>(A.M, A.rp, A.col, A.N, A.nnz, ctl);
 }
 
 }  // namespace hsmu

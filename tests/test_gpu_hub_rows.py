@@ -1,5 +1,5 @@
 """Rows of many entries: both sides of the length from which the bounds and feature passes take a row
-with a block (256), of the products from which a narrow row leaves the warp class (32,768), and B rows
+with a block (256), of the products from which a narrow row leaves the warp class (24,576), and B rows
 around the steps of the tile pass (multiples of 32 and 128), against the oracle."""
 import numpy as np
 import pytest
@@ -18,8 +18,8 @@ def rows_of(lengths, k, seed):
 
 
 def operands(span):
-    # B rows of 128 columns: 256 entries of A are 32,768 products, 257 are 32,896
-    lengths = [255, 256, 257, 1, 0, 700, 1900, 300, 31, 2] * 20 + [256, 257]
+    # B rows of 128 columns: 192 entries of A are 24,576 products, 193 are 24,704
+    lengths = [255, 256, 257, 192, 193, 1, 0, 700, 1900, 300, 31, 2] * 20 + [256, 257]
     A = rows_of(lengths, 2000, seed=1)
     B = rows_of([128] * 2000, span, seed=2)
     assert A.nnz >= 1 << 16 and A.nnz > 6 * A.M
