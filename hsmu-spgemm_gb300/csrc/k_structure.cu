@@ -115,7 +115,8 @@ __global__ void __launch_bounds__(SDS_WARPS * 32, SDS_CTAS_PER_SM)
         for (int t = lane; t < span; t += WARP) S.msk[t] = 0ull;
         __syncwarp();
         bool bad = false;
-        warp_or_tiles<false>(arp[i], arp[i + 1], 0, WARP, acol, tptr, tcol, tmask, t0, span, S.msk, bad);
+        warp_or_tiles<false>(arp[i], arp[i + 1], 0, WARP, acol, tptr, tcol, tmask, t0, span, S.msk, bad,
+                             REP ? ri.rep : nullptr);
         if (__any_sync(FULL, bad)) {
             if (lane == 0) {
                 set_err(&ctl->err, DERR_INTERNAL);

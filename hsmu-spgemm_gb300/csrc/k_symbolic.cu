@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(DS_WARPS * 32) k_count_ds(int M, const int *__
         for (int t = lane; t < span; t += WARP) msk[t] = 0ull;
         __syncwarp();
         bool bad = false;
-        warp_or_tiles<false>(arp[i], arp[i + 1], 0, WARP, acol, tptr, tcol, tmask, t0, span, msk, bad);
+        warp_or_tiles<false>(arp[i], arp[i + 1], 0, WARP, acol, tptr, tcol, tmask, t0, span, msk, bad, ri.rep);
         if (bad) set_err(&ctl->err, DERR_INTERNAL);
         __syncwarp();
         int cnt = 0;
