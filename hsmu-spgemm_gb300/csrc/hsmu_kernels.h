@@ -122,6 +122,8 @@ inline bool long_rows_apart(const DevCSR &A) {
 }
 // out[c] = products of rows c*PROD_CHUNK .. (c+1)*PROD_CHUNK-1 (ceil(M / PROD_CHUNK) entries)
 constexpr int PROD_CHUNK = 64;
+// crp[r0..r1] = rp[r0..r1] - rp[r0]
+void launch_panel_ptr(const long long *rp, int r0, int r1, int *crp, int grid, cudaStream_t st);
 void launch_chunk_prod(int M, const long long *prod, long long *out, int grid, cudaStream_t st);
 // exclusive scan of int counts (n entries) into out[0..n]; total (int64) into *total64;
 // sets DERR_OVERFLOW if the total exceeds INT32_MAX.

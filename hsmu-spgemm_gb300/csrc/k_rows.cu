@@ -432,6 +432,19 @@ __global__ void __launch_bounds__(256) k_chunk_prod(int M, const long long *__re
     }
 }
 
+// row pointers of rows r0..r1-1 as a panel of its own: crp[r0] = 0
+__global__ void __launch_bounds__(256) k_panel_ptr(const long long *__restrict__ rp, int r0, int r1,
+                                                   int *__restrict__ crp) {
+    const long long first = rp[r0];
+    for (long long i = r0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; i <= r1;
+         i += (long long)gridDim.x * blockDim.x)
+        crp[i] = (int)(rp[i] - first);
+}
+
+void launch_panel_ptr(const long long *rp, int r0, int r1, int *crp, int grid, cudaStream_t st) {
+    k_panel_ptr<<<grid_for(grid, (long long)r1 - r0 + 1, 256), 256, 0, st>>>(rp, r0, r1, crp);
+}
+
 void launch_chunk_prod(int M, const long long *prod, long long *out, int grid, cudaStream_t st) {
     if (M > 0) k_chunk_prod<<<grid, 256, 0, st>>>(M, prod, out);
 }
