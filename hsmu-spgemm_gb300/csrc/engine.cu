@@ -558,7 +558,7 @@ struct PlainRun {
         launch_count_light(Ad, Bd, ri, ctl, h->nsm, apart ? h->cs_tiles : st);
         launch_count_warp(Ad, Btd, ri, ctl, h->nsm, st);
         const TileStore tsd = store_view();
-        launch_count_large(Ad, Btd, ri, have_store ? &tsd : nullptr, ctl, h->nsm, st);
+        launch_count_large(Ad, Btd, Bd.N, ri, have_store ? &tsd : nullptr, ctl, h->nsm, st);
         if (have_store && ts_wbase) {
             // the listed rows' windows in row order, ahead of every other window: the value
             // pass hands windows out in array order, and R-MAT's heaviest rows come first
@@ -1021,7 +1021,7 @@ int spgemm_learned_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, 
         if (listed) {
             rc = r.fork();
             if (rc) goto done;
-            launch_spec_large(r.Ad, r.Btd, r.ri, r.store_view(), RowOut{OUT_SPEC, nullptr, nullptr, nullptr, nullptr,
+            launch_spec_large(r.Ad, r.Btd, r.Bd.N, r.ri, r.store_view(), RowOut{OUT_SPEC, nullptr, nullptr, nullptr, nullptr,
                                                                         r.ri.cnnz, flag, 0, M},
                               r.ctl, h->nsm, st);
             launch_scan(r.ts_nwin, r.ts_wbase, M, &r.ctl->win_listed, h->scan, r.ctl, st);

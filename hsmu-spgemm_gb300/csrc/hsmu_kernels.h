@@ -158,12 +158,13 @@ void launch_count(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo 
 // (ts: nullable; when given, the large rows' C tiles are stored while the arena lasts)
 void launch_count_light(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int nsm, cudaStream_t st);
 void launch_count_warp(const DevCSR &A, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm, cudaStream_t st);
-void launch_count_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const TileStore *ts, Ctl *ctl, int nsm,
+// N: columns of B
+void launch_count_large(const DevCSR &A, const DevTiles &Bt, int N, RowInfo ri, const TileStore *ts, Ctl *ctl, int nsm,
                         cudaStream_t st);
 // learned path, large rows: exact count and tile list in its speculative pass;
 // every listed row is flagged ROW_OVERFLOW (out.flag) so that the pass after the
 // exact scan writes it at its place in C (k_symbolic.cu)
-void launch_spec_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const TileStore &ts, RowOut out, Ctl *ctl,
+void launch_spec_large(const DevCSR &A, const DevTiles &Bt, int N, RowInfo ri, const TileStore &ts, RowOut out, Ctl *ctl,
                        int nsm, cudaStream_t st);
 
 // k_scatter.cu: rows of the scattered class (exact count; columns and values)

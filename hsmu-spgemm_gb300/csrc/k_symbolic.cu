@@ -64,7 +64,12 @@ __global__ void __launch_bounds__(DS_WARPS * 32) k_count_ds(int M, const int *__
     }
 }
 
-constexpr int L_THREADS = 256;
+// threads of a block, and of an SM's blocks together.  Where no row spans more than SPAN_T tiles the
+// large class holds only rows of many products, the heaviest of which is the pass's tail: 16 warps each
+// (A*A^T of 30,011 vertices: 257 us with 8, 187 with 16).  Wider rows are mostly lighter, and the
+// barriers between their phases cost more in larger blocks (R-MAT scale 18: 5.35 ms with 8, 6.17 with 16).
+constexpr int L_WIDE = 256, L_NARROW = 512;
+constexpr int L_BLOCK_THREADS = 1536;
 
 // Large rows, one CTA per row: the OR of B's tile masks per chunk of the row's
 // tile span, then
@@ -82,8 +87,8 @@ constexpr int L_THREADS = 256;
 // the OR-walk structure kernel.
 enum LMode { LM_COUNT = 0, LM_STORE = 1, LM_SPEC = 2 };
 
-template <int MODE>
-__global__ void __launch_bounds__(L_THREADS, 6) k_count_l(int M, const int *__restrict__ arp,
+template <int MODE, int L_THREADS>
+__global__ void __launch_bounds__(L_THREADS, L_BLOCK_THREADS / L_THREADS) k_count_l(int M, const int *__restrict__ arp,
                                                        const int *__restrict__ acol,
                                                        const int *__restrict__ tptr,
                                                        const int *__restrict__ tcol,
@@ -220,32 +225,39 @@ void launch_count_warp(const DevCSR &A, const DevTiles &Bt, RowInfo ri, Ctl *ctl
     k_count_ds<<<grid_for(nsm * 6, A.M, DS_WARPS), DS_WARPS * 32, 0, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, ctl);
 }
 
-void launch_count_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const TileStore *ts, Ctl *ctl, int nsm,
-                        cudaStream_t st) {
+template <int MODE, int NT>
+static void count_large(const DevCSR &A, const DevTiles &Bt, const RowInfo &ri, const TileStore &ts, const RowOut &out,
+                        Ctl *ctl, int nsm, cudaStream_t st) {
     const size_t smem = DCH_COUNT * sizeof(unsigned long long);
-    if (ts && ts->tcol && ts->tent && ts->cap > 0 && ri.store)
-        k_count_l<LM_STORE><<<grid_for(nsm * 6, A.M, 1), L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, *ts,
-                                                               RowOut{}, ctl);
-    else
-        k_count_l<LM_COUNT><<<grid_for(nsm * 6, A.M, 1), L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri,
-                                                               TileStore{}, RowOut{}, ctl);
+    k_count_l<MODE, NT><<<grid_for(nsm * (L_BLOCK_THREADS / NT), A.M, 1), NT, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col,
+                                                                                     Bt.mask, ri, ts, out, ctl);
 }
 
-void launch_spec_large(const DevCSR &A, const DevTiles &Bt, RowInfo ri, const TileStore &ts, RowOut out, Ctl *ctl,
+void launch_count_large(const DevCSR &A, const DevTiles &Bt, int N, RowInfo ri, const TileStore *ts, Ctl *ctl, int nsm,
+                        cudaStream_t st) {
+    const bool store = ts && ts->tcol && ts->tent && ts->cap > 0 && ri.store, narrow = N <= SPAN_T * 64;
+    if (store && narrow) count_large<LM_STORE, L_NARROW>(A, Bt, ri, *ts, RowOut{}, ctl, nsm, st);
+    else if (store) count_large<LM_STORE, L_WIDE>(A, Bt, ri, *ts, RowOut{}, ctl, nsm, st);
+    else if (narrow) count_large<LM_COUNT, L_NARROW>(A, Bt, ri, TileStore{}, RowOut{}, ctl, nsm, st);
+    else count_large<LM_COUNT, L_WIDE>(A, Bt, ri, TileStore{}, RowOut{}, ctl, nsm, st);
+}
+
+void launch_spec_large(const DevCSR &A, const DevTiles &Bt, int N, RowInfo ri, const TileStore &ts, RowOut out, Ctl *ctl,
                        int nsm, cudaStream_t st) {
-    const size_t smem = DCH_COUNT * sizeof(unsigned long long);
-    k_count_l<LM_SPEC><<<grid_for(nsm * 6, A.M, 1), L_THREADS, smem, st>>>(A.M, A.rp, A.col, Bt.ptr, Bt.col, Bt.mask, ri, ts, out, ctl);
+    if (N <= SPAN_T * 64) count_large<LM_SPEC, L_NARROW>(A, Bt, ri, ts, out, ctl, nsm, st);
+    else count_large<LM_SPEC, L_WIDE>(A, Bt, ri, ts, out, ctl, nsm, st);
 }
 
 void launch_count(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, RowInfo ri, Ctl *ctl, int nsm,
                   cudaStream_t st) {
     launch_count_light(A, B, ri, ctl, nsm, st);
     launch_count_warp(A, Bt, ri, ctl, nsm, st);
-    launch_count_large(A, Bt, ri, nullptr, ctl, nsm, st);
+    launch_count_large(A, Bt, B.N, ri, nullptr, ctl, nsm, st);
 }
 
 int configure_count() {
-    for (auto k : {k_count_l<LM_COUNT>, k_count_l<LM_STORE>, k_count_l<LM_SPEC>}) {
+    for (auto k : {k_count_l<LM_COUNT, L_WIDE>, k_count_l<LM_STORE, L_WIDE>, k_count_l<LM_SPEC, L_WIDE>,
+                   k_count_l<LM_COUNT, L_NARROW>, k_count_l<LM_STORE, L_NARROW>, k_count_l<LM_SPEC, L_NARROW>}) {
         const int e = (int)cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 DCH_COUNT * (int)sizeof(unsigned long long));
         if (e) return e;
