@@ -361,7 +361,7 @@ struct PlainRun {
     bool side_busy = false;  // the handle's side stream has work that `st` does not wait for yet
     DevTiles Btd{};
     RowInfo ri{};
-    unsigned char *rep = nullptr;     // B rows that repeat the row before them
+    unsigned char *rep = nullptr, *rep_a = nullptr;  // rows of B and of A that repeat the row before them
     long long *chunk_prod = nullptr;  // products per PROD_CHUNK rows (host-buffer entry)
     Window *win = nullptr;
     long long win_cap = 0;
@@ -439,6 +439,15 @@ struct PlainRun {
             launch_row_repeat(Bd, rep, grid_rows(h), st);
             launches++;
             ri.rep = rep;
+            const bool same = Ad.rp == Bd.rp && Ad.col == Bd.col && M == B->M;
+            if (same) {
+                ri.rep_a = rep;
+            } else if (Ad.nnz >= (long long)REPEAT_MIN_ROW * M && M > 0) {
+                CKR(salloc(h, &rep_a, (size_t)M, st));
+                launch_row_repeat(Ad, rep_a, grid_rows(h), st);
+                launches++;
+                ri.rep_a = rep_a;
+            }
         }
         CKR(salloc(h, &ri.prod, (size_t)M, st));
         CKR(salloc(h, &ri.tmin, (size_t)M, st));

@@ -47,6 +47,7 @@ struct RowInfo {
     int *cnnz;         // exact nnz per row (count pass)
     signed char *cls;  // row class (RowBin) of every row, -1 for an empty row
     const unsigned char *rep;  // B rows that repeat the row before them (nullable; launch_row_repeat)
+    const unsigned char *rep_a;  // the same of A (nullable): such a row's C row has the structure of the one before
     int store;         // 1: the tile store is in use -- the count pass sizes each large row's
                        // list, min(tile span, sum of its B rows' tile counts), and adds the
                        // sizes up in Ctl::store_tiles (the arena the next call wants)

@@ -81,3 +81,30 @@ def test_stencil_blocks(engine, dof):
         np.testing.assert_array_equal(X.row_ptr.astype(np.int64), rp)
         np.testing.assert_array_equal(X.col, col)
         assert np.array_equal(X.val.view(np.int64), val.view(np.int64))
+
+
+@pytest.mark.parametrize("run", [1, 2, 3, 4, 5, 8, 31, 32, 33, 40])
+def test_repeated_rows_of_a(engine, run):
+    # A's rows repeat in runs around the group of four and the 32 rows a run's place is told from; B is
+    # another matrix, with rows long enough to look for repeats, and outputs with and without windows
+    import hsmu_gb
+
+    rng = np.random.default_rng(run)
+    base = [np.sort(rng.choice(500, size=int(rng.integers(36, 60)), replace=False)) for _ in range(200 // run + 2)]
+    cols = [c for c in base for _ in range(run)]
+    rp = np.concatenate(([0], np.cumsum([c.size for c in cols]))).astype(np.int32)
+    col = np.concatenate(cols).astype(np.int32)
+    A = gen.CSR(len(cols), 500, rp, col, rng.uniform(-1, 1, col.size))
+    for ncols in (300, 9000):
+        B = repeated_rows((1, 3), ncols, 40, 60, seed=run)
+        B = gen.CSR(500, ncols, B.row_ptr[:501], B.col[:B.row_ptr[500]], B.val[:B.row_ptr[500]])
+        dA, dB = hsmu_gb.DeviceCSR.from_host(A), hsmu_gb.DeviceCSR.from_host(B)
+        want = oracle.spgemm(A, B)
+        np.testing.assert_array_equal(engine.row_nnz(dA, dB).cpu().numpy(), np.diff(want[0]))
+        C = engine.spgemm(dA, dB).to_host()
+        rp64, col64, val64 = engine.spgemm64(dA, dB, max_panel_nnz=5000).to_host()
+        np.testing.assert_array_equal(C.row_ptr.astype(np.int64), want[0])
+        np.testing.assert_array_equal(rp64, want[0])
+        for c, v in ((C.col, C.val), (col64, val64)):
+            np.testing.assert_array_equal(c, want[1])
+            assert np.array_equal(v.view(np.int64), want[2].view(np.int64))
