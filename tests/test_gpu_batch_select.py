@@ -79,3 +79,71 @@ def test_negative_zero_and_cancellation(engine):
     np.testing.assert_array_equal(C.col, col)
     assert np.array_equal(C.val.view(np.int64), val.view(np.int64))
     batch.close()
+
+
+def short_products():
+    rng = np.random.default_rng(15)
+    out = []
+    # rows of 0..8 entries against rows of 0..4: few columns (long runs) and many
+    for M, n in ((1, 1), (31, 4), (32, 6), (33, 5000), (2000, 9), (1501, 300)):
+        out.append((rows_of(rng.integers(0, 9, M), 250, M), rows_of(rng.integers(0, 5, 250), n, M + 70)))
+    out.append((rows_of(np.full(400, 8), 100, 16), rows_of(np.full(100, 4), 7, 17)))  # 32 products, 7 columns
+    out.append((rows_of(np.full(400, 8), 100, 18), rows_of(np.full(100, 4), 4000, 19)))  # 32 products, mostly distinct
+    lens = np.full(300, 4)
+    lens[257] = 5  # a right row of five entries met late: the lists from there
+    out.append((rows_of(np.full(900, 5), 300, 20), rows_of(lens, 60, 21)))
+    lens = np.full(500, 8)
+    lens[340] = 9
+    out.append((rows_of(lens, 200, 22), rows_of(np.full(200, 3), 90, 23)))
+    return out
+
+
+@pytest.mark.parametrize("grid", [0, 1])
+@pytest.mark.parametrize("arith", [0, 1, 2])
+def test_short_products(engine, arith, grid):
+    import hsmu_gb
+
+    prods = short_products()
+    A = [hsmu_gb.DeviceCSR.from_host(a) for a, _ in prods]
+    B = [hsmu_gb.DeviceCSR.from_host(b) for _, b in prods]
+    batch = hsmu_gb.Batch(engine, hsmu_gb.BATCH_PRODUCT, A, B, arith=arith)
+    for tiny in (32, 31):
+        batch.set_params(tiny, grid)
+        batch.execute()
+        batch.status()
+        for p, (a, b) in enumerate(prods):
+            C = batch.result(p).to_host()
+            rp, col, val = oracle.spgemm(a, b, fma=arith == 1)
+            np.testing.assert_array_equal(C.row_ptr.astype(np.int64), rp)
+            np.testing.assert_array_equal(C.col, col)
+            assert np.array_equal(C.val.view(np.int64), val.view(np.int64)), (tiny, p)
+    batch.close()
+
+
+def test_short_second_product(engine):
+    # Galerkin batches whose second product is short for some grids and not for others
+    import hsmu_gb
+
+    sides = [16, 5, 9, 33, 2, 1]
+    A, P, Pt = [], [], []
+    for k, s in enumerate(sides):
+        A.append(gen.poisson7(s, seed=k))
+        p = gen.aggregation_prolongator(s)
+        if k == 2:  # aggregates of random size: rows of P^T beyond eight entries
+            rng = np.random.default_rng(3)
+            p = gen.CSR(p.M, 11, p.row_ptr, rng.integers(0, 11, p.M).astype(np.int32), p.val)
+        P.append(p)
+        Pt.append(gen.transpose(p))
+    dev = lambda ms: [hsmu_gb.DeviceCSR.from_host(m) for m in ms]
+    batch = hsmu_gb.Batch(engine, hsmu_gb.BATCH_GALERKIN, dev(A), dev(P), dev(Pt))
+    batch.execute()
+    batch.status()
+    for p in range(len(sides)):
+        rp, col, val = oracle.spgemm(A[p], P[p])
+        AP = gen.CSR(A[p].M, P[p].N, rp.astype(np.int32), col, val)
+        rp, col, val = oracle.spgemm(Pt[p], AP)
+        C = batch.result(p).to_host()
+        np.testing.assert_array_equal(C.row_ptr.astype(np.int64), rp)
+        np.testing.assert_array_equal(C.col, col)
+        assert np.array_equal(C.val.view(np.int64), val.view(np.int64)), p
+    batch.close()
