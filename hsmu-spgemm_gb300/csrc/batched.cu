@@ -16,6 +16,10 @@
 //     sized by the products' nnz bounds when the batch is made), and the rows
 //     are written there, compact, with no count pass and no wait on any other
 //     tile.
+// Products whose right rows hold one entry (a piecewise-constant prolongator)
+// have their first round's tiles done by a launch of its own ahead of that
+// kernel, which such batches alone pay for (k_batch_select).
+//
 // The intermediate A*P of a Galerkin product is read in that form (every row
 // has a start and an end); the second product (Pt * (AP)) runs the same way
 // after one grid barrier.  The last product is put in row order at the end:
@@ -107,6 +111,8 @@ struct BParams {
     GridBar *bar;
     int *err;
     int arith;             // hsmu_opts.arith of the batch
+    const unsigned char *sel_done;  // first round: tiles that k_batch_select has finished (nullable)
+    const int *sel_left;            // the number it has not
     unsigned long long spin_limit;  // polls of a grid barrier before it gives up
 };
 
@@ -279,136 +285,232 @@ __device__ bool wide_row_fill(int a_lo, int a_hi, const BOp &A, const BOp &B, BW
     return done == nnz;
 }
 
+// A tile's block of its product's region: agg entries from the offset that take_block gives lane 0 (one
+// atomic, whose answer is waited for where place_tile uses it), and the row's place in it: cnt entries
+// after `before` of the tile's.  ro: the product's rows in the pools; li: the lane's row in the product.
+// The whole warp calls both; place_tile gives false (an error is set) when the region is full.
+__device__ __forceinline__ unsigned long long take_block(const BRound &R, int p, int agg) {
+    return lane_id() == 0 && agg ? atomicAdd(R.alloc + p, (unsigned long long)agg) : 0;
+}
+__device__ __forceinline__ bool place_tile(const BRound &R, int *err, unsigned long long tb, long long ro, long long region,
+                                           long long t, int li, bool valid, int cnt, int before, int agg, int &off) {
+    const int lane = lane_id();
+    tb = __shfl_sync(FULL, tb, 0);
+    if ((long long)tb + agg > region) {
+        if (lane == 0) atomicOr(err, BERR_CAPACITY);
+        return false;
+    }
+    off = (int)tb + before;  // within the region
+    if (R.last) {
+        if (valid) R.rp_pool[ro + li] = cnt;
+        if (lane == 0) {
+            R.tbase[t] = (int)tb;
+            R.tcnt[t] = agg;
+        }
+    } else if (valid) {
+        R.rs[ro + li] = off;
+        R.re[ro + li] = off + cnt;
+    }
+    return true;
+}
+
 // Selecting tiles: rows of at most SEL_MAX entries of A whose B rows hold at most one entry each (a
 // piecewise-constant prolongator): every entry of A is at most one product, so a row's products are
 // sorted by column in a thread's registers -- a network over column << 3 | entry, stable by the entry
 // number -- and summed run by run, one multiply and one add per product.  The tile's block is taken as
 // soon as the distinct columns are counted, and the rows leave through shared memory, 32 consecutive
-// entries per store.  The next tile's entries of A are copied to shared memory meanwhile (in registers
-// they spill).  Latency-bound at 16 warps per SM, as the lists are, with half their instructions and
-// two fewer waits per tile: 20 Galerkin products of sides 16..96, launch 1.045 -> 0.864 ms (0.936
-// without the copies ahead).  A product whose tile turns out otherwise goes on with the lists.
+// entries per store.  The tile's entries of A, one stretch of the CSR arrays, are copied to shared memory
+// while the tile before is computed (in registers they spill).
+// They have a launch of their own ahead of the persistent one, at 24 warps per SM where its registers
+// allow 16.  That alone gave nothing: the L1 pipe was 61 % busy, with each lane copying its own row and
+// the operands' descriptions read for every tile.  With one stretch per tile, the descriptions held until
+// the product changes and staging that skips a slot in 16 (strides of 2^k entries meet in few banks
+// otherwise) it took 355 us instead of 457 (20 Galerkin products of sides 16..96, 1.13 GB of DRAM
+// traffic), a contiguous range of tiles per warp 397 (neighbouring tiles share lines of B).  The whole
+// batch: 1.045 ms with these tiles on the lists, 0.743 within the persistent launch, 0.673 so, 0.662 with
+// the block asked for before the sums; 0.78 at 16 warps per SM, 0.70 at 20.
 constexpr int SEL_MAX = 8;
 constexpr int SEL_COLS = 1 << 28;  // B columns a key can hold
+constexpr int SEL_TILE = SEL_MAX * WARP;
 
+__device__ __forceinline__ int skew8(int i) { return i + (i >> 4); }  // of 8-byte entries
+__device__ __forceinline__ int skew4(int i) { return i + (i >> 5); }  // of 4-byte entries
+
+template <int AR>
 struct SelSmem {
     double t[SEL_MAX][WARP];   // add_term's term of every product
-    double a[SEL_MAX][WARP];   // and its A value (fused multiply-add)
-    double val[SEL_MAX * WARP];  // the tile's entries
-    int col[SEL_MAX * WARP];
-    double na[SEL_MAX][WARP];    // entries of A, copied here while the tile before is computed
-    int nk[SEL_MAX][WARP];
+    double a[AR == AR_FMA ? SEL_MAX : 1][WARP];  // and its A value
+    double val[SEL_TILE + SEL_TILE / 16];  // the tile's entries
+    double na[SEL_TILE + SEL_TILE / 16];   // entries of A, copied here while the tile before is computed
+    int col[SEL_TILE + SEL_TILE / 32];
+    int nk[SEL_TILE + SEL_TILE / 32];
 };
-static_assert(sizeof(SelSmem) <= sizeof(BWarpSmem), "selecting tiles use the warp's shared memory");
-
 __device__ __forceinline__ void key_order(unsigned &x, unsigned &y) {
     const unsigned lo = min(x, y), hi = max(x, y);
     x = lo;
     y = hi;
 }
 
-// a lane's row of a tile; ahead: the copy of its entries has been started
-struct SelRow {
-    int lo, hi;
-    bool ahead;
-};
-
-// start the copy of a row's first entries (a lane reads back only what it copied itself)
-__device__ __forceinline__ void sel_copy(const SelRow &row, const BOp &A, SelSmem &S) {
-    const int lane = lane_id();
+// start the copy of a tile's entries of A, [first, end) (at most SEL_TILE)
+template <int AR>
+__device__ __forceinline__ void sel_copy(int first, int end, const BOp &A, SelSmem<AR> &S) {
 #pragma unroll
     for (int u = 0; u < SEL_MAX; u++) {
-        if (u < row.hi - row.lo) {
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&S.nk[u][lane])), "l"(A.col + row.lo + u)
+        const int i = u * WARP + lane_id();
+        if (i < end - first) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(&S.nk[skew4(i)])), "l"(A.col + first + i)
                          : "memory");
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(&S.na[u][lane])), "l"(A.val + row.lo + u)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(&S.na[skew8(i)])), "l"(A.val + first + i)
                          : "memory");
         }
     }
 }
-__device__ __forceinline__ void sel_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// One tile, a row per lane (empty for lanes without one).  Returns -1, with nothing done, if the tile
-// is not a selecting one; else the lane's entries, after `take` (called by the whole warp with the
-// lane's offset in the tile and the tile's entries) has given the tile its place: a pointer pair, null
-// columns to write nothing.  next_rows / next_entries load the warp's next tile while this one waits.
-template <int AR, class Take, class Rows, class Entries>
-__device__ __forceinline__ int select_tile(SelRow &row, const BOp &A, const BOp &B, SelSmem &S, Take take,
-                                           Rows next_rows, Entries next_entries) {
-    const int lane = lane_id(), len = row.hi - row.lo;
-    if (!__all_sync(FULL, len <= SEL_MAX)) return -1;
-    unsigned key[SEL_MAX];
-    double b[SEL_MAX];
-    int s[SEL_MAX], e[SEL_MAX];
-    if (!row.ahead) sel_copy(row, A, S);
-    sel_wait();
-#pragma unroll
-    for (int u = 0; u < SEL_MAX; u++) {
-        s[u] = e[u] = 0;
-        if (u < len) {
-            const int k = S.nk[u][lane];
-            s[u] = __ldg(B.rp + k);
-            e[u] = __ldg(B.re + k);
+constexpr int SELK_WARPS = 4, SELK_CTAS_PER_SM = 6;
+static_assert(SELK_CTAS_PER_SM * (SELK_WARPS * sizeof(SelSmem<AR_RN>) + 1024) <= 228 * 1024, "CTAs per SM");
+
+// The selecting tiles of the first round (sel_prod: products that can have them), tile t by global warp
+// t mod (warps in the grid).  done[t]: whether the tile is finished; *nleft: tiles that are not (the
+// persistent launch does those).
+template <int AR>
+__global__ void __launch_bounds__(SELK_WARPS * 32, AR == AR_FMA ? 4 : SELK_CTAS_PER_SM)
+    k_batch_select(BRound R, const unsigned char *__restrict__ sel_prod, unsigned char *__restrict__ done, int *nleft,
+                   int *err) {
+    extern __shared__ unsigned long long s_dyn[];
+    SelSmem<AR> &S = reinterpret_cast<SelSmem<AR> *>(s_dyn)[threadIdx.x >> 5];
+    const int lane = lane_id();
+    const long long nw = (long long)gridDim.x * SELK_WARPS;
+    // the product of the tile in hand: held until a tile of another one
+    int p = 0;
+    long long p_t0 = 0, p_t1 = 0, reg0 = 0, rpo = 0;  // its tiles, its place in the pools
+    int region = 0;
+    bool psel = false;
+    BOp A{}, B{};
+    auto product_of = [&](long long t) {
+        if (t < p_t1) return;
+        while (__ldg(R.tile0 + p + 1) <= t) p++;
+        p_t0 = __ldg(R.tile0 + p);
+        p_t1 = __ldg(R.tile0 + p + 1);
+        reg0 = __ldg(R.reg + p);
+        region = (int)min((long long)INT_MAX, __ldg(R.reg + p + 1) - reg0);
+        rpo = __ldg(R.rpo + p);
+        psel = sel_prod[p];
+        A = R.A[p];
+        B = R.B[p];
+    };
+    long long t = (long long)blockIdx.x * SELK_WARPS + (threadIdx.x >> 5);
+    int left = 0, lo = 0, hi = 0;
+    bool ahead = false;  // lo, hi and the copy belong to tile t
+    if (t < R.T) p = find_prod(R.tile0, R.nprod, t);
+    for (; t < R.T; t += nw) {
+        product_of(t);
+        if (!psel) {
+            if (lane == 0) done[t] = 0;
+            left++;
+            continue;
         }
-    }
-    next_rows();
-    bool one = true;
-#pragma unroll
-    for (int u = 0; u < SEL_MAX; u++) one = one && e[u] - s[u] <= 1;
-    if (!__all_sync(FULL, one)) return -1;
-    __syncwarp();
-#pragma unroll
-    for (int u = 0; u < SEL_MAX; u++) {
-        key[u] = ~0u;
-        b[u] = 0.0;
-        if (e[u] > s[u]) {
-            key[u] = ((unsigned)__ldg(B.col + s[u]) << 3) | (unsigned)u;
-            b[u] = __ldg(B.val + s[u]);
+        const int li = (int)(t - p_t0) * TILE_ROWS + lane;
+        if (!ahead) {
+            lo = __ldg(A.rp + min(li, A.M));
+            hi = __ldg(A.rp + min(li + 1, A.M));
         }
-    }
+        const int first = __shfl_sync(FULL, lo, 0), len = hi - lo;
+        const bool rows_ok = __all_sync(FULL, len <= SEL_MAX);
+        if (!ahead && rows_ok) sel_copy(first, __shfl_sync(FULL, hi, WARP - 1), A, S);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        ahead = false;
+        unsigned key[SEL_MAX];
+        double b[SEL_MAX];
+        int s[SEL_MAX], e[SEL_MAX];
+        bool one = rows_ok;
+        if (rows_ok) {
 #pragma unroll
-    for (int u = 0; u < SEL_MAX; u++) {
-        const double a = u < len ? S.na[u][lane] : 0.0;
-        S.t[u][lane] = term<AR>(a, b[u]);
-        if (AR == AR_FMA) S.a[u][lane] = a;
-    }
-    next_entries();
-    // Batcher's odd-even merge sort of eight keys
-    constexpr int NET[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6}, {5, 7}, {1, 2}, {5, 6},
-                                {0, 4}, {1, 5}, {2, 6}, {3, 7}, {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
+            for (int u = 0; u < SEL_MAX; u++) {
+                s[u] = e[u] = 0;
+                if (u < len) {
+                    const int k = S.nk[skew4(lo - first + u)];
+                    s[u] = __ldg(B.rp + k);
+                    e[u] = __ldg(B.re + k);
+                }
+            }
 #pragma unroll
-    for (int c = 0; c < 19; c++) key_order(key[NET[c][0]], key[NET[c][1]]);
-    int n = 0;
+            for (int u = 0; u < SEL_MAX; u++) one = one && e[u] - s[u] <= 1;
+            one = __all_sync(FULL, one);
+        }
+        if (!one) {
+            if (lane == 0) done[t] = 0;
+            left++;
+            continue;
+        }
 #pragma unroll
-    for (int u = 0; u < SEL_MAX; u++) n += key[u] != ~0u && (u == 0 || key[u] >> 3 != key[u - 1] >> 3);
-    const int incl = warp_incl_scan(n);
-    const int agg = __shfl_sync(FULL, incl, WARP - 1);
-    int *ocol;
-    double *oval;
-    take(incl - n, n, agg, ocol, oval);
-    int at = incl - n - 1;
-    double acc = 0.0;
-#pragma unroll
-    for (int u = 0; u < SEL_MAX; u++) {
-        if (key[u] != ~0u) {
-            const bool head = u == 0 || key[u] >> 3 != key[u - 1] >> 3;
-            const int o = (int)(key[u] & 7u);
-            at += head;
-            acc = add_term<AR>(head ? 0.0 : acc, AR == AR_FMA ? S.a[o][lane] : 0.0, S.t[o][lane]);
-            if (u == SEL_MAX - 1 || key[u + 1] >> 3 != key[u] >> 3) {  // the run's last product
-                S.col[at] = (int)(key[u] >> 3);
-                S.val[at] = acc;
+        for (int u = 0; u < SEL_MAX; u++) {
+            key[u] = ~0u;
+            b[u] = 0.0;
+            if (e[u] > s[u]) {
+                key[u] = ((unsigned)__ldg(B.col + s[u]) << 3) | (unsigned)u;
+                b[u] = __ldg(B.val + s[u]);
             }
         }
-    }
-    __syncwarp();
-    if (ocol)
-        for (int q = lane; q < agg; q += WARP) {
-            ocol[q] = S.col[q];
-            oval[q] = S.val[q];
+        // the next tile's rows, if it is one of this product's
+        int nlo = 0, nhi = 0;
+        if (t + nw < p_t1) {
+            nlo = __ldg(A.rp + min(li + (int)nw * TILE_ROWS, A.M));
+            nhi = __ldg(A.rp + min(li + (int)nw * TILE_ROWS + 1, A.M));
         }
-    __syncwarp();
-    return n;
+#pragma unroll
+        for (int u = 0; u < SEL_MAX; u++) {
+            const double a = u < len ? S.na[skew8(lo - first + u)] : 0.0;
+            S.t[u][lane] = term<AR>(a, b[u]);
+            if (AR == AR_FMA) S.a[u][lane] = a;
+        }
+        __syncwarp();
+        if (t + nw < p_t1 && __all_sync(FULL, nhi - nlo <= SEL_MAX)) {
+            sel_copy(__shfl_sync(FULL, nlo, 0), __shfl_sync(FULL, nhi, WARP - 1), A, S);
+            ahead = true;
+        }
+        // Batcher's odd-even merge sort of eight keys
+        constexpr int NET[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6}, {5, 7}, {1, 2}, {5, 6},
+                                    {0, 4}, {1, 5}, {2, 6}, {3, 7}, {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
+#pragma unroll
+        for (int c = 0; c < 19; c++) key_order(key[NET[c][0]], key[NET[c][1]]);
+        int n = 0;
+#pragma unroll
+        for (int u = 0; u < SEL_MAX; u++) n += key[u] != ~0u && (u == 0 || key[u] >> 3 != key[u - 1] >> 3);
+        const int incl = warp_incl_scan(n), before = incl - n;
+        const int agg = __shfl_sync(FULL, incl, WARP - 1);
+        const unsigned long long tb = take_block(R, p, agg);
+        int at = before - 1;
+        double acc = 0.0;
+#pragma unroll
+        for (int u = 0; u < SEL_MAX; u++) {
+            if (key[u] != ~0u) {
+                const bool head = u == 0 || key[u] >> 3 != key[u - 1] >> 3;
+                const int o = (int)(key[u] & 7u);
+                at += head;
+                acc = add_term<AR>(head ? 0.0 : acc, AR == AR_FMA ? S.a[o][lane] : 0.0, S.t[o][lane]);
+                if (u == SEL_MAX - 1 || key[u + 1] >> 3 != key[u] >> 3) {  // the run's last product
+                    S.col[skew4(at)] = (int)(key[u] >> 3);
+                    S.val[skew8(at)] = acc;
+                }
+            }
+        }
+        __syncwarp();
+        int off = 0;
+        if (place_tile(R, err, tb, rpo, region, t, li, li < A.M, n, before, agg, off)) {
+            int *oc = R.col_pool + reg0 + (off - before);
+            double *ov = R.val_pool + reg0 + (off - before);
+            for (int q = lane; q < agg; q += WARP) {
+                oc[q] = S.col[skew4(q)];
+                ov[q] = S.val[skew8(q)];
+            }
+        }
+        if (lane == 0) done[t] = 1;
+        lo = nlo;
+        hi = nhi;
+        __syncwarp();
+    }
+    if (lane == 0 && left) atomicAdd(nleft, left);
 }
 
 // Short tiles: rows of at most SHORT_A entries of A whose B rows hold at most SHORT_B entries each (the
@@ -528,12 +630,12 @@ __device__ void phase_tiles(const BParams &P, int r, BWarpSmem &S) {
     const long long nw = (long long)gridDim.x * BW;
     const long long gw = (long long)blockIdx.x * BW + (threadIdx.x >> 5);
     int p = gw < R.T ? find_prod(R.tile0, R.nprod, gw) : 0;
-    int no_select = -1, no_short = -1;  // the product whose tiles turned out not to be selecting / short ones
-    int pn = p;          // the next tile's product
-    SelRow row{0, 0, false};
-    bool have_row = false;  // row holds this tile's ranges
+    int no_short = -1;  // the product whose tiles turned out not to be short ones
+    // tiles finished by k_batch_select
+    const unsigned char *done = r == 0 ? P.sel_done : nullptr;
+    if (done && *(volatile int *)P.sel_left == 0) return;
     for (long long t = gw; t < R.T; t += nw) {
-        p = pn;
+        if (done && done[t]) continue;
         while (__ldg(R.tile0 + p + 1) <= t) p++;
         const long long tfirst = __ldg(R.tile0 + p), prow0 = __ldg(R.row0 + p);
         const int M = (int)(__ldg(R.row0 + p + 1) - prow0);
@@ -541,70 +643,14 @@ __device__ void phase_tiles(const BParams &P, int r, BWarpSmem &S) {
         const bool valid = li < M;
         const BOp A = R.A[p];
         const BOp B = b_operand(P, r, p);
-        if (!have_row) {
-            row.lo = valid ? ldx<true>(A.rp + li) : 0;
-            row.hi = valid ? ldx<true>(A.rp + li + 1) : 0;
-            row.ahead = false;
-        }
-        have_row = false;
-        const int a_lo = row.lo, a_hi = row.hi;
-        const long long region = __ldg(R.reg + p + 1) - __ldg(R.reg + p);
-        const long long ro = __ldg(R.rpo + p);
-        const long long base = __ldg(R.reg + p);
-        // the tile's block of the product's region and the row's place in it; false: it does not fit
-        auto place = [&](int cnt, int before, int agg, int &off) -> bool {
-            unsigned long long tb = 0;
-            if (lane == 0 && agg) tb = atomicAdd(R.alloc + p, (unsigned long long)agg);
-            tb = __shfl_sync(FULL, tb, 0);
-            if ((long long)tb + agg > region) {
-                if (lane == 0) atomicOr(P.err, BERR_CAPACITY);
-                return false;
-            }
-            off = (int)tb + before;  // within the region
-            if (R.last) {
-                if (valid) R.rp_pool[ro + li] = cnt;
-                if (lane == 0) {
-                    R.tbase[t] = (int)tb;
-                    R.tcnt[t] = agg;
-                }
-            } else if (valid) {
-                R.rs[ro + li] = off;
-                R.re[ro + li] = off + cnt;
-            }
-            return true;
-        };
+        const int a_lo = valid ? ldx<true>(A.rp + li) : 0, a_hi = valid ? ldx<true>(A.rp + li + 1) : 0;
+        const long long base = __ldg(R.reg + p), region = __ldg(R.reg + p + 1) - base, ro = __ldg(R.rpo + p);
         auto take = [&](int before, int cnt, int agg, int *&oc, double *&ov) {
             int off = 0;
-            const bool fits = place(cnt, before, agg, off);
+            const bool fits = place_tile(R, P.err, take_block(R, p, agg), ro, region, t, li, valid, cnt, before, agg, off);
             oc = fits ? R.col_pool + base + (off - before) : nullptr;
             ov = R.val_pool + base + (off - before);
         };
-        if (NC && P.tiny >= SEL_MAX && p != no_select && B.N <= SEL_COLS) {
-            SelRow nrow{0, 0, true};
-            pn = p;
-            const int n = select_tile<AR>(
-                row, A, B, reinterpret_cast<SelSmem &>(S), take,
-                [&]() {
-                    const long long tn = t + nw;
-                    if (tn >= R.T) return;
-                    while (__ldg(R.tile0 + pn + 1) <= tn) pn++;
-                    const int ln = (int)(tn - __ldg(R.tile0 + pn)) * TILE_ROWS + lane;
-                    if (ln < (int)(__ldg(R.row0 + pn + 1) - __ldg(R.row0 + pn))) {
-                        const int *rp = R.A[pn].rp + ln;
-                        nrow.lo = __ldg(rp);
-                        nrow.hi = __ldg(rp + 1);
-                    }
-                },
-                [&]() { sel_copy(nrow, R.A[pn], reinterpret_cast<SelSmem &>(S)); });
-            if (n >= 0) {
-                row = nrow;
-                have_row = true;
-                continue;
-            }
-            no_select = p;  // (no copy has been started for the tile after)
-        }
-        if (row.ahead) sel_wait();  // copied for a tile that does not select: the lists use the same memory
-        __syncwarp();
         if (P.tiny >= SHORT_P && p != no_short && B.N <= SHORT_COLS) {
             if (short_tile<AR, NC>(a_lo, a_hi, A, B, reinterpret_cast<ShortSmem &>(S), take) >= 0) continue;
             no_short = p;
@@ -633,7 +679,7 @@ __device__ void phase_tiles(const BParams &P, int r, BWarpSmem &S) {
         const int incl = warp_incl_scan(cnt);
         const int agg = __shfl_sync(FULL, incl, WARP - 1);
         int off = 0;
-        if (!place(cnt, incl - cnt, agg, off)) continue;
+        if (!place_tile(R, P.err, take_block(R, p, agg), ro, region, t, li, valid, cnt, incl - cnt, agg, off)) continue;
         int *ocol = R.col_pool + base;
         double *oval = R.val_pool + base;
         if (!had_big) {
@@ -898,6 +944,8 @@ struct hsmu_batch_s {
     int kind, nprod;
     int nsm, grid, threads, tiny, arith;
     size_t smem;
+    unsigned char *sel_prod, *sel_done;  // products that can have selecting tiles (null: none has), tiles
+    int *sel_left;
     BParams P;
     std::vector<void *> allocs;
     std::vector<long long> row0[2], rpo[2], reg[2];
@@ -925,9 +973,27 @@ cudaError_t bupload(hsmu_batch_s *b, T **p, const std::vector<T> &h) {
     return e;
 }
 
+template <int AR>
+int launch_select(hsmu_batch_s *b, cudaStream_t st) {
+    const int per_sm = AR == AR_FMA ? 4 : SELK_CTAS_PER_SM;
+    const BRound &R = b->P.rnd[0];
+    k_batch_select<AR><<<grid_for(b->nsm * per_sm, R.T, SELK_WARPS), SELK_WARPS * 32, SELK_WARPS * sizeof(SelSmem<AR>), st>>>(
+        R, b->sel_prod, b->sel_done, b->sel_left, b->P.err);
+    return cudaGetLastError() == cudaSuccess ? HSMU_OK : HSMU_ERR_CUDA;
+}
+
 int launch_batch(hsmu_batch_s *b, cudaStream_t st) {
     if (cudaMemsetAsync(b->reset, 0, b->reset_bytes, st) != cudaSuccess) return HSMU_ERR_CUDA;
     b->P.tiny = b->tiny;
+    const bool sel = b->sel_prod && b->tiny >= SEL_MAX;
+    b->P.sel_done = sel ? b->sel_done : nullptr;
+    b->P.sel_left = b->sel_left;
+    if (sel) {
+        const int rc = b->arith == AR_IMUL  ? launch_select<AR_IMUL>(b, st)
+                       : b->arith == AR_FMA ? launch_select<AR_FMA>(b, st)
+                                            : launch_select<AR_RN>(b, st);
+        if (rc) return rc;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(b->grid);
     cfg.blockDim = dim3(b->threads);
@@ -950,6 +1016,13 @@ int configure_batch(hsmu_batch_s *b, int dev) {
     for (auto k : {k_batch<AR_RN>, k_batch<AR_FMA>, k_batch<AR_IMUL>})
         if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->smem) != cudaSuccess)
             return HSMU_ERR_CUDA;
+    if (cudaFuncSetAttribute(k_batch_select<AR_RN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SELK_WARPS * (int)sizeof(SelSmem<AR_RN>)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_batch_select<AR_FMA>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SELK_WARPS * (int)sizeof(SelSmem<AR_FMA>)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_batch_select<AR_IMUL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             SELK_WARPS * (int)sizeof(SelSmem<AR_IMUL>)) != cudaSuccess)
+        return HSMU_ERR_CUDA;
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch<AR_RN>, b->threads, b->smem) != cudaSuccess ||
         per_sm < 1)
@@ -1033,6 +1106,20 @@ int hsmu_batch_create(hsmu_handle h, int kind, int n, const hsmu_csr *A, const h
         R.R = b->row0[r][n];
         R.T = tiles[r][n];
     }
+    // products that can have selecting tiles: single-entry right rows, short left rows, columns that a
+    // sort key holds
+    {
+        std::vector<unsigned char> sel((size_t)n, 0);
+        bool any = false;
+        for (int p = 0; p < n; p++) {
+            sel[(size_t)p] = B[p].nnz <= B[p].M && A[p].nnz <= (long long)SEL_MAX * A[p].M && B[p].N <= SEL_COLS;
+            any |= sel[(size_t)p] != 0;
+        }
+        if (any && (bupload(b, &b->sel_prod, sel) || balloc(b, &b->sel_done, (size_t)b->P.rnd[0].T))) {
+            rc = HSMU_ERR_ALLOC;
+            goto fail;
+        }
+    }
     // nnz bound of every product (one sizing pass and one host read): min(products, N) per row of
     // the first product; for Galerkin, per row of the second the sum of its A*P rows' bounds
     if (balloc(b, &dpb, (size_t)n * nr) || (nr == 2 && balloc(b, &rowbound, (size_t)b->P.rnd[0].R))) {
@@ -1113,6 +1200,8 @@ int hsmu_batch_create(hsmu_handle h, int kind, int n, const hsmu_csr *A, const h
         o += sizeof(int);
         const size_t o_nwide = o;
         o += 2 * sizeof(int);
+        const size_t o_left = o;
+        o += sizeof(int);
         o = (o + 15) & ~size_t(15);
         size_t o_alloc[2] = {0, 0};
         for (int r = 0; r < nr; r++) {
@@ -1128,6 +1217,7 @@ int hsmu_batch_create(hsmu_handle h, int kind, int n, const hsmu_csr *A, const h
         b->reset_bytes = o;
         b->P.bar = reinterpret_cast<GridBar *>(rb + o_bar);
         b->P.err = reinterpret_cast<int *>(rb + o_err);
+        b->sel_left = reinterpret_cast<int *>(rb + o_left);
         for (int r = 0; r < nr; r++) {
             b->P.rnd[r].nwide = reinterpret_cast<int *>(rb + o_nwide) + r;
             b->P.rnd[r].alloc = reinterpret_cast<unsigned long long *>(rb + o_alloc[r]);

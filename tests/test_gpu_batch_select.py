@@ -81,6 +81,38 @@ def test_negative_zero_and_cancellation(engine):
     batch.close()
 
 
+def test_selecting_tiles_in_turn(engine):
+    # more tiles than the launch has warps, so that a warp meets tiles ahead of it: within a product, across
+    # a product that cannot have selecting tiles, and after a tile that is not one
+    import hsmu_gb
+
+    lens = np.full(200_001, 7)
+    lens[[40_000, 199_999]] = 9
+    prods = [(rows_of(np.arange(130_000) % 9, 500, 20), selector(500, 80, 21, empty=0.1)),
+             (gen.laplacian2d(30, seed=3), gen.laplacian2d(30, seed=4)),
+             (rows_of(lens, 300, 22), selector(300, 90, 23)),
+             (rows_of(np.full(120_000, 8), 64, 24), selector(64, 50, 25, two=(63,)))]
+    prods[3] = (prods[3][0], gen.CSR(64, 50, *trim(prods[3][1])))
+    batch = hsmu_gb.Batch(engine, hsmu_gb.BATCH_PRODUCT, [hsmu_gb.DeviceCSR.from_host(a) for a, _ in prods],
+                          [hsmu_gb.DeviceCSR.from_host(b) for _, b in prods])
+    for _ in range(2):
+        batch.execute()
+        batch.status()
+        for p, (a, b) in enumerate(prods):
+            C = batch.result(p).to_host()
+            rp, col, val = oracle.spgemm(a, b)
+            np.testing.assert_array_equal(C.row_ptr.astype(np.int64), rp)
+            np.testing.assert_array_equal(C.col, col)
+            assert np.array_equal(C.val.view(np.int64), val.view(np.int64)), p
+    batch.close()
+
+
+def trim(b):
+    """b without its first entry: row 63 keeps two, and there are no more entries than rows."""
+    rp = np.maximum(np.asarray(b.row_ptr) - 1, 0).astype(np.int32)
+    return rp, b.col[1:], b.val[1:]
+
+
 def short_products():
     rng = np.random.default_rng(15)
     out = []
