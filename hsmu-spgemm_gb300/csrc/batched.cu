@@ -519,7 +519,7 @@ __global__ void __launch_bounds__(SELK_WARPS * 32, AR == AR_FMA ? 4 : SELK_CTAS_
 // the insertion lists every entry of a B row after the first was a memory round trip of its own
 // (36 us per tile); 20 Galerkin products of sides 16..96: launch 0.864 -> 0.807 ms.
 constexpr int SHORT_A = 8, SHORT_B = 4, SHORT_P = SHORT_A * SHORT_B;
-constexpr int SHORT_COLS = 1 << 27;
+constexpr int SHORT_COLS = (1 << 27) - 1;  // column << 5 | product stays below the empty key
 
 struct ShortSmem {
     double t[SHORT_P][WARP];  // add_term's term of every product

@@ -107,6 +107,25 @@ def test_selecting_tiles_in_turn(engine):
     batch.close()
 
 
+def test_last_column_of_the_widest_keys(engine):
+    # column 2^27 - 1 as the 32nd product of a row: its sort key must not be the empty one
+    import hsmu_gb
+
+    n = 1 << 27
+    col = np.tile(np.array([0, 1, 2, 3]), 8)
+    col[-1] = n - 1
+    A = gen.CSR(1, 8, np.array([0, 8], np.int32), np.arange(8, dtype=np.int32), np.arange(1.0, 9.0))
+    B = gen.CSR(8, n, np.arange(0, 33, 4, dtype=np.int32), col.astype(np.int32), np.ones(32))
+    batch = hsmu_gb.Batch(engine, hsmu_gb.BATCH_PRODUCT, [hsmu_gb.DeviceCSR.from_host(A)],
+                          [hsmu_gb.DeviceCSR.from_host(B)])
+    batch.execute()
+    batch.status()
+    C = batch.result(0).to_host()
+    np.testing.assert_array_equal(C.col, [0, 1, 2, 3, n - 1])
+    np.testing.assert_array_equal(C.val, [36.0, 36.0, 36.0, 28.0, 8.0])
+    batch.close()
+
+
 def trim(b):
     """b without its first entry: row 63 keeps two, and there are no more entries than rows."""
     rp = np.maximum(np.asarray(b.row_ptr) - 1, 0).astype(np.int32)
