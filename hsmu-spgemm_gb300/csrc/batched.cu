@@ -345,12 +345,6 @@ struct SelSmem {
     int col[SEL_TILE + SEL_TILE / 32];
     int nk[SEL_TILE + SEL_TILE / 32];
 };
-__device__ __forceinline__ void key_order(unsigned &x, unsigned &y) {
-    const unsigned lo = min(x, y), hi = max(x, y);
-    x = lo;
-    y = hi;
-}
-
 // start the copy of a tile's entries of A, [first, end) (at most SEL_TILE)
 template <int AR>
 __device__ __forceinline__ void sel_copy(int first, int end, const BOp &A, SelSmem<AR> &S) {
@@ -469,11 +463,7 @@ __global__ void __launch_bounds__(SELK_WARPS * 32, AR == AR_FMA ? 4 : SELK_CTAS_
             sel_copy(__shfl_sync(FULL, nlo, 0), __shfl_sync(FULL, nhi, WARP - 1), A, S);
             ahead = true;
         }
-        // Batcher's odd-even merge sort of eight keys
-        constexpr int NET[19][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3}, {4, 6}, {5, 7}, {1, 2}, {5, 6},
-                                    {0, 4}, {1, 5}, {2, 6}, {3, 7}, {2, 4}, {3, 5}, {1, 2}, {3, 4}, {5, 6}};
-#pragma unroll
-        for (int c = 0; c < 19; c++) key_order(key[NET[c][0]], key[NET[c][1]]);
+        sort_keys<SEL_MAX>(key);
         int n = 0;
 #pragma unroll
         for (int u = 0; u < SEL_MAX; u++) n += key[u] != ~0u && (u == 0 || key[u] >> 3 != key[u - 1] >> 3);
@@ -527,24 +517,6 @@ struct ShortSmem {
 };
 static_assert(sizeof(ShortSmem) <= sizeof(BWarpSmem), "short tiles use the warp's shared memory");
 
-// Batcher's odd-even merge sort of SHORT_P keys
-struct ShortNet {
-    int n = 0, x[256] = {}, y[256] = {};
-    constexpr ShortNet() {
-        for (int p = 1; p < SHORT_P; p *= 2)
-            for (int k = p; k >= 1; k /= 2)
-                for (int j = k % p; j + k < SHORT_P; j += 2 * k)
-                    for (int i = 0; i < k && i + j + k < SHORT_P; i++)
-                        if ((i + j) / (2 * p) == (i + j + k) / (2 * p)) {
-                            x[n] = i + j;
-                            y[n] = i + j + k;
-                            n++;
-                        }
-    }
-};
-constexpr int SHORT_NET_SIZE = 191;
-static_assert(ShortNet().n == SHORT_NET_SIZE, "comparators of the network");
-
 // One tile, a row per lane; as select_tile, but each lane writes its own row (take gives the pointers of
 // the tile's block).
 template <int AR, bool NC, class Take>
@@ -588,9 +560,7 @@ __device__ __forceinline__ int short_tile(int a_lo, int a_hi, const BOp &A, cons
         for (int i = 0; i < SHORT_B; i++) S.t[u * SHORT_B + i][lane] = term<AR>(a[u], b[i]);
         if (AR == AR_FMA) S.a[u][lane] = a[u];
     }
-    constexpr ShortNet NET{};
-#pragma unroll
-    for (int c = 0; c < SHORT_NET_SIZE; c++) key_order(key[NET.x[c]], key[NET.y[c]]);
+    sort_keys<SHORT_P>(key);
     int n = 0;
 #pragma unroll
     for (int q = 0; q < SHORT_P; q++) n += key[q] != ~0u && (q == 0 || key[q] >> 5 != key[q - 1] >> 5);

@@ -48,7 +48,7 @@ constexpr int DCH_STRUCT = 4096;  // structure pass: 12 B per tile -> 48 KB (4 C
 enum RowBin : int {
     BIN_DS = 0,    // tile span <= SPAN_T : one warp, dense span table
     BIN_L = 1,     // wider rows          : one CTA, dense chunked table
-    BIN_TINY = 2,  // <= TINY_MAX products: one thread, sorted insertion list
+    BIN_TINY = 2,  // <= TINY_MAX products: one thread, sorted in registers
     BIN_H = 3,     // wide span, <= H_MAX products: one warp, ranked tiles (k_scatter.cu)
     NBIN = 4
 };

@@ -3,13 +3,13 @@
 //
 // The AMG Galerkin operands (A*P: <= 7 products per row, P^T*(AP): <= 32)
 // and the 2-D Laplacian (<= 25) consist of such rows only; a warp per row
-// would leave most lanes idle.  A thread walks its row's products in the
-// oracle's order (A entry, then B entry), keeping the distinct columns in a
-// small sorted list (insertion), so the count pass and the fill pass need no
-// B tiles and no sorting afterwards.  In the fill pass every product is added
-// to its column's accumulator in that same order: 0.0 + p_1 + p_2 + ...
-// (arithmetic per step as in hsmu_products.cuh), bit-identical to the host
-// oracle.
+// would leave most lanes idle.  The count pass and the fill pass need no B
+// tiles: a thread lists its row's products in the oracle's order (A entry,
+// then B entry) and sorts them by column in registers, stable by product.
+// Every product is added to its column's sum in that order: 0.0 + p_1 + p_2
+// + ... (arithmetic per step as in hsmu_products.cuh), bit-identical to the
+// host oracle.  The batched engine's general rows, and matrices of more
+// columns than a sort key holds, keep sorted insertion lists instead.
 //
 // The per-thread lists live in shared memory laid out element-major
 // ([TINY_MAX][threads]) so that neighbouring threads hit neighbouring banks.
@@ -22,6 +22,34 @@
 namespace hsmu {
 
 constexpr int TINY_MAX = 32;
+
+// Batcher's odd-even merge sort of N keys in registers: the pairs that are compared
+template <int N>
+struct SortNet {
+    int n = 0, x[8 * N] = {}, y[8 * N] = {};
+    constexpr SortNet() {
+        for (int p = 1; p < N; p *= 2)
+            for (int k = p; k >= 1; k /= 2)
+                for (int j = k % p; j + k < N; j += 2 * k)
+                    for (int i = 0; i < k && i + j + k < N; i++)
+                        if ((i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+                            x[n] = i + j;
+                            y[n] = i + j + k;
+                            n++;
+                        }
+    }
+};
+template <int N>
+__device__ __forceinline__ void sort_keys(unsigned (&key)[N]) {
+    constexpr SortNet<N> NET{};
+    constexpr int SIZE = NET.n;
+#pragma unroll
+    for (int c = 0; c < SIZE; c++) {
+        const unsigned lo = min(key[NET.x[c]], key[NET.y[c]]), hi = max(key[NET.x[c]], key[NET.y[c]]);
+        key[NET.x[c]] = lo;
+        key[NET.y[c]] = hi;
+    }
+}
 
 // A entries of a tiny row handled per batch: their column ids, B row bounds
 // and first B entries are fetched in three rounds of independent loads
@@ -64,31 +92,113 @@ struct TinyFetch {
     }
 };
 
-// number of distinct columns of row (a_lo..a_hi) of A*B; -1 if the row has
-// more than TINY_MAX products (caller classified it wrongly).
-template <bool NC = true>
-__device__ __forceinline__ int tiny_row_count(int a_lo, int a_hi, const int *__restrict__ acol,
-                                              const int *__restrict__ brp, const int *__restrict__ bre,
-                                              const int *__restrict__ bcol, int *cols, int stride) {
-    int n = 0, seen = 0;
-    for (int p0 = a_lo; p0 < a_hi; p0 += TINY_BATCH) {
-        TinyFetch<NC, false> F;
-        F.load(p0, a_hi, acol, nullptr, brp, bre, bcol, nullptr);
+// A warp's rows as flat product lists, one row per lane (element-major, as above): tiny_list writes every
+// product's place in B and the A value, then all products are loaded at once and their columns sorted by a
+// network of the size that the warp's longest row needs.  An insertion list costs a chain of shared-memory
+// steps per product, and every entry of a B row after the first is a memory round trip of its own
+// (150,001 random rows of 12 entries on average: fill 83 -> 26 us, count 45 -> 6.5; 2-D Laplacian of side 256,
+// 25 products per row: 21.5 -> 18.0 and 7.9 -> 5.7: the fill there is FP64 issue, 6 us, and
+// each lane's stores to its own row).
+template <int AR>
+struct TinySmem {
+    double t[TINY_MAX][WARP];  // the A value, then add_term's term, of every product
+    double a[AR == AR_FMA ? TINY_MAX : 1][WARP];  // its A value (fused multiply-add)
+    int q[TINY_MAX][WARP];     // its entry of B
+};
+// sort keys are column << 5 | product, below the empty key
+constexpr int TINY_KEY_COLS = (1 << 27) - 1;
+
+// the number of products of the lane's row, listed; more than TINY_MAX if there are more
+template <bool VALS>
+__device__ __forceinline__ int tiny_list(int a_lo, int a_hi, const int *__restrict__ acol,
+                                         const double *__restrict__ aval, const int *__restrict__ brp,
+                                         int (*qs)[WARP], double (*t)[WARP]) {
+    const int lane = lane_id();
+    int n = 0;
+    for (int p0 = a_lo; p0 < a_hi && n <= TINY_MAX; p0 += TINY_BATCH) {
+        int s[TINY_BATCH], e[TINY_BATCH];
+        double a[TINY_BATCH];
 #pragma unroll
         for (int u = 0; u < TINY_BATCH; u++) {
-            for (int q = F.qs[u]; q < F.qe[u]; q++) {
-                if (++seen > TINY_MAX) return -1;
-                const int j = q == F.qs[u] ? F.j0[u] : ldx<NC>(bcol + q);
-                int pos = n;
-                while (pos > 0 && cols[(pos - 1) * stride] > j) pos--;
-                if (pos > 0 && cols[(pos - 1) * stride] == j) continue;
-                for (int t = n; t > pos; t--) cols[t * stride] = cols[(t - 1) * stride];
-                cols[pos * stride] = j;
-                n++;
+            s[u] = p0 + u < a_hi ? __ldg(acol + p0 + u) : -1;
+            if (VALS) a[u] = p0 + u < a_hi ? __ldg(aval + p0 + u) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < TINY_BATCH; u++) {
+            const int k = s[u];
+            s[u] = e[u] = 0;
+            if (k >= 0) {
+                s[u] = __ldg(brp + k);
+                e[u] = __ldg(brp + k + 1);
             }
+        }
+#pragma unroll
+        for (int u = 0; u < TINY_BATCH; u++) {
+            const int m = min(e[u] - s[u], TINY_MAX - n);
+            for (int i = 0; i < m; i++) {
+                qs[n + i][lane] = s[u] + i;
+                if (VALS) t[n + i][lane] = a[u];
+            }
+            n += e[u] - s[u];
         }
     }
     return n;
+}
+
+// distinct columns of the lane's n <= N listed products
+template <int N>
+__device__ __forceinline__ int tiny_list_count(int n, const int *__restrict__ bcol, const int (*qs)[WARP]) {
+    unsigned key[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) key[u] = u < n ? (unsigned)__ldg(bcol + qs[u][lane_id()]) : ~0u;
+    sort_keys<N>(key);
+    int c = 0;
+#pragma unroll
+    for (int u = 0; u < N; u++) c += key[u] != ~0u && (u == 0 || key[u] != key[u - 1]);
+    return c;
+}
+
+// The lane's n <= N listed products sorted by column (stable by product), summed run by run and written,
+// at most cap entries; returns the distinct columns.
+template <int AR, int N>
+__device__ __forceinline__ int tiny_list_fill(int n, const int *__restrict__ bcol, const double *__restrict__ bval,
+                                              TinySmem<AR> &S, int cap, int *__restrict__ oc,
+                                              double *__restrict__ ov) {
+    const int lane = lane_id();
+    unsigned key[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) key[u] = u < n ? ((unsigned)__ldg(bcol + S.q[u][lane]) << 5) | (unsigned)u : ~0u;
+#pragma unroll
+    for (int u0 = 0; u0 < N; u0 += 8) {
+        double b[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) b[i] = u0 + i < n ? __ldg(bval + S.q[u0 + i][lane]) : 0.0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            if (u0 + i < n) {
+                const double a = S.t[u0 + i][lane];
+                if (AR == AR_FMA) S.a[u0 + i][lane] = a;
+                S.t[u0 + i][lane] = term<AR>(a, b[i]);
+            }
+        }
+    }
+    sort_keys<N>(key);
+    int at = -1;
+    double acc = 0.0;
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        if (key[u] != ~0u) {
+            const bool head = u == 0 || key[u] >> 5 != key[u - 1] >> 5;
+            const int o = (int)(key[u] & 31u);
+            at += head;
+            acc = add_term<AR>(head ? 0.0 : acc, AR == AR_FMA ? S.a[o][lane] : 0.0, S.t[o][lane]);
+            if ((u == N - 1 || key[u + 1 < N ? u + 1 : u] >> 5 != key[u] >> 5) && at < cap) {
+                oc[at] = (int)(key[u] >> 5);
+                ov[at] = acc;
+            }
+        }
+    }
+    return at + 1;
 }
 
 // Builds the row's sorted distinct columns and their accumulated values in

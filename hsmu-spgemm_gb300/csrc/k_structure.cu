@@ -472,9 +472,57 @@ __global__ void __launch_bounds__(SLS_THREADS, 6) k_struct_ls(int M, RowInfo ri,
 
 constexpr int TINYF_THREADS = 128;
 
-// tiny rows: one thread per row writes its sorted columns and values
+// tiny rows: one thread per row, a warp's rows by one network (hsmu_rowops.cuh)
 template <int AR>
-__global__ void __launch_bounds__(TINYF_THREADS) k_fill_tiny(int M, const int *__restrict__ arp,
+__global__ void __launch_bounds__(TINYF_THREADS, 4) k_fill_tiny(int M, const int *__restrict__ arp,
+                                                                const int *__restrict__ acol,
+                                                                const double *__restrict__ aval,
+                                                                const int *__restrict__ brp,
+                                                                const int *__restrict__ bcol,
+                                                                const double *__restrict__ bval, RowInfo ri,
+                                                                RowOut out, Ctl *ctl) {
+    extern __shared__ unsigned long long s_dyn[];
+    TinySmem<AR> &S = reinterpret_cast<TinySmem<AR> *>(s_dyn)[threadIdx.x >> 5];
+    const int *rows = ri.bins + (size_t)BIN_TINY * M;
+    int b0, b1;
+    bin_slice(rows, ctl->bin_count[BIN_TINY], out, M, b0, b1);
+    bool bad = false;
+    for (int r0 = b0 + blockIdx.x * TINYF_THREADS + (threadIdx.x & ~31); r0 < b1; r0 += gridDim.x * TINYF_THREADS) {
+        const int r = r0 + lane_id();
+        int i = r < b1 ? rows[r] : -1;
+        if (i >= 0 && skip_row(out, i)) i = -1;
+        long long c0 = 0;
+        int lim = 0, np = 0;
+        if (i >= 0) {
+            c0 = out_base(out, i);
+            lim = out_limit(out, i);
+            np = tiny_list<true>(arp[i], arp[i + 1], acol, aval, brp, S.q, S.t);
+        }
+        int got = 0;
+        if (np > TINY_MAX) {  // a row of another class
+            got = -1;
+            np = 0;
+        }
+        const int most = __reduce_max_sync(FULL, np);
+        if (most > 16) np = tiny_list_fill<AR, 32>(np, bcol, bval, S, lim, out.ccol + c0, out.cval + c0);
+        else if (most > 8) np = tiny_list_fill<AR, 16>(np, bcol, bval, S, lim, out.ccol + c0, out.cval + c0);
+        else np = tiny_list_fill<AR, 8>(np, bcol, bval, S, lim, out.ccol + c0, out.cval + c0);
+        got = got < 0 || np > lim ? -1 : np;
+        if (i < 0) continue;
+        if (out.mode == OUT_SPEC) {
+            out.cnnz[i] = got < 0 ? 0 : got;
+            out.flag[i] = got < 0 ? ROW_OVERFLOW : ROW_VALUES;
+            if (got < 0) bad = true;  // tiny rows get a capacity that always fits
+        } else if (got != lim) {
+            bad = true;
+        }
+    }
+    if (bad) set_err(&ctl->err, DERR_INTERNAL);
+}
+
+// the same by insertion lists, where a sort key does not hold a column (B.N > TINY_KEY_COLS)
+template <int AR>
+__global__ void __launch_bounds__(TINYF_THREADS) k_fill_tiny_wide(int M, const int *__restrict__ arp,
                                                              const int *__restrict__ acol,
                                                              const double *__restrict__ aval,
                                                              const int *__restrict__ brp,
@@ -508,9 +556,13 @@ __global__ void __launch_bounds__(TINYF_THREADS) k_fill_tiny(int M, const int *_
 void launch_structure_light(const DevCSR &A, const DevCSR &B, RowInfo ri, RowOut out, Ctl *ctl, int arith, int nsm,
                             cudaStream_t st, const int *class_rows) {
     if (!class_rows || class_rows[BIN_TINY] > 0) {
-        auto kt = arith == AR_IMUL ? k_fill_tiny<AR_IMUL> : arith == AR_FMA ? k_fill_tiny<AR_FMA> : k_fill_tiny<AR_RN>;
-        kt<<<grid_for(nsm * 4, class_rows ? class_rows[BIN_TINY] : A.M, TINYF_THREADS), TINYF_THREADS, 0, st>>>(
-            A.M, A.rp, A.col, A.val, B.rp, B.col, B.val, ri, out, ctl);
+        const bool keys = B.N <= TINY_KEY_COLS;
+        auto kt = arith == AR_IMUL  ? (keys ? k_fill_tiny<AR_IMUL> : k_fill_tiny_wide<AR_IMUL>)
+                  : arith == AR_FMA ? (keys ? k_fill_tiny<AR_FMA> : k_fill_tiny_wide<AR_FMA>)
+                                    : (keys ? k_fill_tiny<AR_RN> : k_fill_tiny_wide<AR_RN>);
+        const size_t smem = !keys ? 0 : arith == AR_FMA ? sizeof(TinySmem<AR_FMA>) : sizeof(TinySmem<AR_RN>);
+        kt<<<grid_for(nsm * 4, class_rows ? class_rows[BIN_TINY] : A.M, TINYF_THREADS), TINYF_THREADS,
+             TINYF_THREADS / WARP * smem, st>>>(A.M, A.rp, A.col, A.val, B.rp, B.col, B.val, ri, out, ctl);
     }
     if (class_rows ? class_rows[BIN_H] > 0 : B.N > SPAN_T * 64)
         launch_fill_scattered(A, B, ri, out, ctl, arith, nsm, st);
@@ -547,6 +599,12 @@ int configure_structure() {
                    k_struct_ds<AR_RN, true>, k_struct_ds<AR_FMA, true>, k_struct_ds<AR_IMUL, true>}) {
         const int e = (int)cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 SDS_WARPS * (int)sizeof(SdsSmem));
+        if (e) return e;
+    }
+    for (auto k : {k_fill_tiny<AR_RN>, k_fill_tiny<AR_FMA>, k_fill_tiny<AR_IMUL>}) {
+        const size_t warp = k == k_fill_tiny<AR_FMA> ? sizeof(TinySmem<AR_FMA>) : sizeof(TinySmem<AR_RN>);
+        const int e = (int)cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                TINYF_THREADS / WARP * (int)warp);
         if (e) return e;
     }
     return (int)cudaFuncSetAttribute(k_struct_l, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SlSmem));

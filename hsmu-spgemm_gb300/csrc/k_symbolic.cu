@@ -230,20 +230,33 @@ __global__ void __launch_bounds__(L_THREADS, L_BLOCK_THREADS / L_THREADS) k_coun
 
 constexpr int TINY_THREADS = 256;
 
-// tiny rows: one thread per row, distinct columns counted by sorted insertion
+// tiny rows: one thread per row, a warp's rows by one network (hsmu_rowops.cuh)
 __global__ void __launch_bounds__(TINY_THREADS) k_count_tiny(int M, const int *__restrict__ arp,
                                                              const int *__restrict__ acol,
                                                              const int *__restrict__ brp,
                                                              const int *__restrict__ bcol, RowInfo ri, Ctl *ctl) {
-    __shared__ int s_cols[TINY_MAX * TINY_THREADS];
+    __shared__ int s_q[TINY_THREADS / WARP][TINY_MAX][WARP];
+    int (*qs)[WARP] = s_q[threadIdx.x >> 5];
     const int n = ctl->bin_count[BIN_TINY];
     const int *rows = ri.bins + (size_t)BIN_TINY * M;
     bool bad = false;
-    for (int r = blockIdx.x * TINY_THREADS + threadIdx.x; r < n; r += gridDim.x * TINY_THREADS) {
-        const int i = rows[r];
-        const int c = tiny_row_count(arp[i], arp[i + 1], acol, brp, brp + 1, bcol, s_cols + threadIdx.x, TINY_THREADS);
-        if (c < 0) bad = true;
-        ri.cnnz[i] = c < 0 ? 0 : c;
+    for (int r0 = blockIdx.x * TINY_THREADS + (threadIdx.x & ~31); r0 < n; r0 += gridDim.x * TINY_THREADS) {
+        const int r = r0 + lane_id();
+        const int i = r < n ? rows[r] : -1;
+        const int np = i >= 0 ? tiny_list<false>(arp[i], arp[i + 1], acol, nullptr, brp, qs, nullptr) : 0;
+        const int most = __reduce_max_sync(FULL, np);
+        int c;
+        if (most > TINY_MAX) {  // a row of another class
+            bad = true;
+            c = 0;
+        } else if (most <= 8) {
+            c = tiny_list_count<8>(np, bcol, qs);
+        } else if (most <= 16) {
+            c = tiny_list_count<16>(np, bcol, qs);
+        } else {
+            c = tiny_list_count<32>(np, bcol, qs);
+        }
+        if (i >= 0) ri.cnnz[i] = c;
     }
     if (bad) set_err(&ctl->err, DERR_INTERNAL);
 }
