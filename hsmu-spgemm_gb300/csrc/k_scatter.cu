@@ -18,10 +18,11 @@
 // an accumulator step by step, lanes that share a slot in lane order -- the
 // oracle's order, 0.0 + p_1 + p_2 + ..., either way.
 //
-// Bound by instruction issue and shared-memory latency.  Measured on 150,001
-// rows of 12 uniform columns (144 products per row): count 167 us, fill 424 us
-// (a form that read the products again and looked every slot up: 191 and 646 us;
-// the CTA-per-row passes: count 1,889, structure 379, cursors 55, values 362 us).
+// Bound by instruction issue (1,600 warp instructions a row, 47 % of the issue slots) and latency.
+// Measured on 150,001 rows of 12 uniform columns (144 products per row): count 155 us, fill 414 us
+// (166 and 432 before a row's range and A columns were read during the row ahead of it; a form that read
+// the products again and looked every slot up: 191 and 646; the CTA-per-row passes: count 1,889,
+// structure 379, cursors 55, values 362 us).
 #include "hsmu_block.cuh"
 #include "hsmu_kernels.h"
 #include "hsmu_products.cuh"
@@ -52,14 +53,14 @@ struct HProducts {
     double p[VALS ? H_STEPS : 1];
     double av[VALS && AR == AR_FMA ? H_STEPS : 1];
 
-    __device__ __forceinline__ void load(int a_lo, int a_hi, const int *__restrict__ acol,
-                                         const double *__restrict__ aval, const int *__restrict__ brp,
-                                         const int *__restrict__ bcol, const double *__restrict__ bval) {
+    // k: the lane's A entry's column (HRows)
+    __device__ __forceinline__ void load(int a_lo, int a_hi, int k, const double *__restrict__ aval,
+                                         const int *__restrict__ brp, const int *__restrict__ bcol,
+                                         const double *__restrict__ bval) {
         const int lane = lane_id();
         int lo = 0, len = 0;
         double a = 0.0;
         if (a_lo + lane < a_hi) {
-            const int k = __ldg(acol + a_lo + lane);
             if (VALS) a = __ldg(aval + a_lo + lane);
             lo = __ldg(brp + k);
             len = __ldg(brp + k + 1) - lo;
@@ -101,14 +102,44 @@ struct HProducts {
     }
 };
 
+// A warp's rows of a class list, the next one's A range and A columns read while the current one is
+// computed: two of a row's four dependent round trips to memory.
+struct HRows {
+    const int *rows, *arp, *acol;
+    int end, stride, r;
+    int i, a_lo, a_hi, k;  // the current row (i < 0: none), its A range, the lane's A column
+
+    __device__ __forceinline__ void range() {
+        a_lo = i >= 0 ? __ldg(arp + i) : 0;
+        a_hi = i >= 0 ? __ldg(arp + i + 1) : 0;
+    }
+    __device__ __forceinline__ void column() { k = a_lo + lane_id() < a_hi ? __ldg(acol + a_lo + lane_id()) : 0; }
+    __device__ __forceinline__ void row() { i = r < end ? rows[r] : -1; }
+    __device__ __forceinline__ HRows(const int *rows, const int *arp, const int *acol, int begin, int end, int stride)
+        : rows(rows), arp(arp), acol(acol), end(end), stride(stride), r(begin) {
+        row();
+        range();
+        column();
+    }
+    // the next row's first step; range() and column() follow
+    __device__ __forceinline__ void next() {
+        r += stride;
+        row();
+    }
+};
+
 // Ranks the tiles of a row's products (first tile t0, `span` tiles): tmask by rank, and for FILL
 // each tile's id in tid and rank << 6 | column bit in every product's c.  Returns the number of
 // tiles, -1 (nothing usable) for a column outside.
-template <bool FILL, class P>
-__device__ __forceinline__ int h_order(P &R, int t0, int span, HSmem &S) {
+// `midway` runs once, between the passes.
+template <bool FILL, class P, class F>
+__device__ __forceinline__ int h_order(P &R, int t0, int span, HSmem &S, F midway) {
     const int lane = lane_id();
     const int nw = (span + 63) >> 6;
-    if (R.n < 0 || span <= 0 || nw > H_OCCW) return -1;
+    if (R.n < 0 || span <= 0 || nw > H_OCCW) {
+        midway();
+        return -1;
+    }
     for (int q = lane; q < nw; q += WARP) S.occ[q] = 0ull;
     __syncwarp();
     bool bad = false;
@@ -121,6 +152,7 @@ __device__ __forceinline__ int h_order(P &R, int t0, int span, HSmem &S) {
             else bad = true;
         }
     }
+    midway();
     if (__any_sync(FULL, bad)) return -1;  // the vote orders the warp's shared accesses as well
     __syncwarp();
     const int per = (nw + WARP - 1) / WARP;
@@ -164,12 +196,15 @@ __global__ void __launch_bounds__(HC_WARPS * 32, HC_CTAS_PER_SM)
     HSmem &S = reinterpret_cast<HSmem *>(s_dyn)[w];
     const int n = ctl->bin_count[BIN_H];
     const int *rows = ri.bins + (size_t)BIN_H * M;
-    for (int r = blockIdx.x * HC_WARPS + w; r < n; r += gridDim.x * HC_WARPS) {
-        const int i = rows[r];
-        const int t0 = ri.tmin[i];
+    HRows H(rows, arp, acol, blockIdx.x * HC_WARPS + w, n, gridDim.x * HC_WARPS);
+    while (H.i >= 0) {
+        const int i = H.i;
+        const int t0 = ri.tmin[i], t1 = ri.tmax[i];
         HProducts<AR_RN, false> R;
-        R.load(arp[i], arp[i + 1], acol, nullptr, brp, bcol, nullptr);
-        const int nt = h_order<false>(R, t0, ri.tmax[i] - t0 + 1, S);
+        R.load(H.a_lo, H.a_hi, H.k, nullptr, brp, bcol, nullptr);
+        H.next();
+        const int nt = h_order<false>(R, t0, t1 - t0 + 1, S, [&] { H.range(); });
+        H.column();
         int cnt = 0;
         for (int q = lane; q < nt; q += WARP) cnt += popc64(S.tmask[q]);
         cnt = warp_sum(cnt);
@@ -182,10 +217,11 @@ __global__ void __launch_bounds__(HC_WARPS * 32, HC_CTAS_PER_SM)
 }
 
 constexpr int HF_WARPS = 4;
-// 24 warps per SM at 80 registers; the fused multiply-add keeps every product's A value too
+// 24 warps per SM at 80 registers; the fused multiply-add keeps every product's A value too, and the
+// integer product spills at 80
 template <int AR>
 constexpr int hf_ctas() {
-    return AR == AR_FMA ? 4 : 6;
+    return AR == AR_FMA ? 4 : AR == AR_IMUL ? 5 : 6;
 }
 static_assert(hf_ctas<AR_RN>() * (HF_WARPS * sizeof(HSmem) + 1024) <= 228 * 1024, "CTAs per SM");
 
@@ -201,15 +237,23 @@ __global__ void __launch_bounds__(HF_WARPS * 32, hf_ctas<AR>())
     const int *rows = ri.bins + (size_t)BIN_H * M;
     int b0, b1;
     bin_slice(rows, ctl->bin_count[BIN_H], out, M, b0, b1);
-    for (int r = b0 + blockIdx.x * HF_WARPS + w; r < b1; r += gridDim.x * HF_WARPS) {
-        const int i = rows[r];
-        if (skip_row(out, i)) continue;
-        const int t0 = ri.tmin[i];
+    HRows H(rows, arp, acol, b0 + blockIdx.x * HF_WARPS + w, b1, gridDim.x * HF_WARPS);
+    while (H.i >= 0) {
+        const int i = H.i;
+        if (skip_row(out, i)) {
+            H.next();
+            H.range();
+            H.column();
+            continue;
+        }
+        const int t0 = ri.tmin[i], t1 = ri.tmax[i];
         const long long rowbase = out_base(out, i);
         const int limit = out_limit(out, i);
         HProducts<AR, true> R;
-        R.load(arp[i], arp[i + 1], acol, aval, brp, bcol, bval);
-        const int nt = h_order<true>(R, t0, ri.tmax[i] - t0 + 1, S);
+        R.load(H.a_lo, H.a_hi, H.k, aval, brp, bcol, bval);
+        H.next();
+        const int nt = h_order<true>(R, t0, t1 - t0 + 1, S, [&] { H.range(); });
+        H.column();
         int nnz = 0;  // first slot of every tile
         for (int q0 = 0; q0 < nt; q0 += WARP) {
             const int q = q0 + lane;
