@@ -8,12 +8,15 @@
 // the row's C tiles are ORed into a dense per-tile table indexed by
 // (tile id - first tile of the row), which needs no hashing or probing
 // because the bounds kernel already knows the row's exact tile span.
-//   BIN_DS rows (span <= SPAN_T): one warp per row, 4 KB table per warp.
+//   BIN_DS rows (span <= SPAN_T, at most DS_PROD products): one warp per row,
+//                4 KB table per warp.
 //   BIN_L  rows: one CTA per row, the span processed in chunks of DCH_COUNT
-//                tiles (64 KB); B tile ranges restricted per chunk by binary
+//                tiles (32 KB); B tile ranges restricted per chunk by binary
 //                search when the span needs more than one chunk.
 // Every B tile access is a coalesced 4+8 byte load of the flat (A entry,
 // B tile) sequence, 32 lanes busy regardless of row lengths.
+// Tiny rows are counted here too, without tiles (hsmu_rowops.cuh); scattered
+// rows have their own kernels (k_scatter.cu).
 // With a tile store, the large-row pass also writes every row's non-empty C
 // tiles (id + mask, ascending) to the store, compacted chunk by chunk with one
 // block scan, so that the structure pass can stream them (the reference
@@ -185,9 +188,9 @@ __global__ void __launch_bounds__(L_THREADS, L_BLOCK_THREADS / L_THREADS) k_coun
             __syncthreads();
             bool bad = false;
             if (one_chunk)
-                warp_or_tiles<false, true>(a_lo, a_hi, w * WARP, NWARP * WARP, acol, tptr, tcol, tmask, c0, c1 - c0, msk, bad);
+                warp_or_tiles<false, true, L_THREADS == L_WIDE>(a_lo, a_hi, w * WARP, NWARP * WARP, acol, tptr, tcol, tmask, c0, c1 - c0, msk, bad);
             else
-                warp_or_tiles<true, true>(a_lo, a_hi, w * WARP, NWARP * WARP, acol, tptr, tcol, tmask, c0, c1 - c0, msk, bad);
+                warp_or_tiles<true, true, L_THREADS == L_WIDE>(a_lo, a_hi, w * WARP, NWARP * WARP, acol, tptr, tcol, tmask, c0, c1 - c0, msk, bad);
             if (bad) set_err(&ctl->err, DERR_INTERNAL);
             __syncthreads();
             if (STORE && sbase >= 0) {
