@@ -2,17 +2,20 @@
 //
 // Pipeline for C = A * B (reference: compressed_NHC_spgemm,
 // src/compressed/compressed_NHC_spgemm.cu:22-248):
-//   1. B -> 64-column bit tiles (k_tiles count, scan, fill)      [skipped with hsmu_spgemm_tiled]
-//   2. per-row bounds + row binning (k_bounds)
-//   3. exact symbolic count (k_count_ds / k_count_l)
-//   4. exclusive scan -> C row_ptr, nnz(C); ONE host read (8 bytes + flags)
+//   1. B -> 64-column bit tiles (k_tiles count, scan, fill)      [skipped with hsmu_spgemm_tiled;
+//      for small B after 2, where the classes that read tiles may turn out empty]
+//   2. per-row bounds + row binning (k_bounds, k_bounds_long, k_bins)
+//   3. exact symbolic count: tiny and scattered rows on the handle's side stream
+//      (k_count_tiny, k_count_h), warp and large rows (k_count_ds, k_count_l)
+//   4. exclusive scan -> C row_ptr, nnz(C); ONE host read (the control block)
 //      and the output allocation
-//   5a. sorted C columns + numeric windows (k_struct_ds / k_struct_l)
-//   5b. values (k_numeric)
+//   5a. tiny and scattered rows finished on the side stream (k_fill_tiny, k_fill_h); sorted C columns
+//      + numeric windows of the others (k_struct_ds, k_struct_ls / k_struct_l)
+//   5b. values (k_win_cursors, k_numeric)
 // The reference makes ~10 blocking host round trips and several cudaMalloc
 // calls inside its timed region; this engine makes one read of a small
-// control block and allocates from a stream-ordered pool that keeps freed
-// memory cached across calls.
+// control block, takes its scratch from a block of the handle's and C from a
+// stream-ordered pool that keeps freed memory cached across calls.
 #include <cuda_runtime.h>
 
 #include <algorithm>
