@@ -1428,12 +1428,18 @@ int hsmu_handle_create(hsmu_handle *out) {
             return HSMU_ERR_CUDA;
         }
     }
+    // cleared before the handle is given out: the scans run on streams that do not wait for the
+    // default one, where a clear may be queued behind the caller's work
     for (ScanState *s : {&h->scan, &h->scan_tiles})
         if (cudaMalloc(&s->word, scan_state_bytes()) != cudaSuccess ||
-            cudaMemset(s->word, 0, scan_state_bytes()) != cudaSuccess) {
+            cudaMemsetAsync(s->word, 0, scan_state_bytes(), h->cs_tiles) != cudaSuccess) {
             hsmu_handle_destroy(h);
             return HSMU_ERR_ALLOC;
         }
+    if (cudaStreamSynchronize(h->cs_tiles) != cudaSuccess) {
+        hsmu_handle_destroy(h);
+        return HSMU_ERR_CUDA;
+    }
     // keep freed pool memory cached between calls (no re-mapping of large outputs)
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
