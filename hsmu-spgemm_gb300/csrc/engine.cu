@@ -38,8 +38,8 @@ int configure_count();
 int status_from_dev_err(int err) {
     if (!err) return HSMU_OK;
     if (err & DERR_UNSORTED) return HSMU_ERR_UNSORTED;
+    if (err & DERR_TIMEOUT) return HSMU_ERR_TIMEOUT;  // before what follows from it
     if (err & DERR_OVERFLOW) return HSMU_ERR_OVERFLOW;
-    if (err & DERR_TIMEOUT) return HSMU_ERR_TIMEOUT;
     return HSMU_ERR_INTERNAL;
 }
 int configure_structure();
@@ -264,6 +264,9 @@ struct ScratchScope {
 
 int grid_rows(const hsmu_handle_s *h) { return h->nsm * 8; }
 
+// limit of the call's look-backs (hsmu_opts.scan_polls; 0: the default)
+void set_scan_polls(hsmu_handle_s *h, int polls) { h->scan.polls = h->scan_tiles.polls = polls; }
+
 // arrays the library allocated from the stream-ordered pool and handed to the caller:
 // returned to the pool once every stream of the device is done with them (the free
 // functions take no stream; a plain cudaFree measured not to give the bytes back to
@@ -394,6 +397,7 @@ struct PlainRun {
         M = A->M;
         Ad = dev(A);
         Bd = dev(B);
+        set_scan_polls(h, o.scan_polls);
         CKR(salloc(h, &ctl, 1, st));
         CKR(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
         if (o.validate) {
@@ -1241,6 +1245,7 @@ int row_nnz_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, int32_t
     DevCSR Ad = dev(A), Bd = dev(B);
     DevTiles Btd{};
     ScratchScope scope(h, st);
+    set_scan_polls(h, 0);
     CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     rc = build_tiles(h, B, &bt, ctl, 0, st, false, false);
@@ -1530,6 +1535,7 @@ int hsmu_btiles_build(hsmu_handle h, const hsmu_csr *B, hsmu_btiles *out, void *
     Ctl hc{};
     std::memset(out, 0, sizeof(*out));
     ScratchScope scope(h, st);
+    set_scan_polls(h, 0);
     CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     launch_validate(dev(B), ctl, grid_rows(h), st);
@@ -1574,6 +1580,7 @@ int hsmu_csr_transpose(hsmu_handle h, const hsmu_csr *A, hsmu_csr *At, void *str
     long long *tot = nullptr;
     Ctl *ctl = nullptr;
     ScratchScope scope(h, st);
+    set_scan_polls(h, 0);
     CK(palloc(&trp, (size_t)A->N + 1, st));
     CK(palloc(&tcol, (size_t)n, st));
     CK(palloc(&tval, (size_t)n, st));

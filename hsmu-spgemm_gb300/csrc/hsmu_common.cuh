@@ -64,7 +64,7 @@ enum DevErr : int {
     DERR_INTERNAL = 2,
     DERR_CAPACITY = 4,
     DERR_OVERFLOW = 8,
-    DERR_TIMEOUT = 16  // a bounded wait (an asynchronous copy) ran out
+    DERR_TIMEOUT = 16  // a bounded wait (an asynchronous copy, a scan's look-back) ran out
 };
 
 struct Window {
@@ -122,6 +122,14 @@ struct Ctl {
 
 // whether any row of A reads B's tiles (after the bounds pass)
 __device__ __forceinline__ bool tiles_read(const Ctl *ctl) { return ctl->bin_count[BIN_DS] || ctl->bin_count[BIN_L]; }
+
+// A scan of the call has given up (or another wait): the bins, pointers and positions that it should
+// have written are not all there.  Kernels that index by them return at once (every thread of a
+// block asks first, and all get the same answer); the host reports the error at its next read of the
+// control block.
+__device__ __forceinline__ bool scan_failed(const Ctl *ctl) {
+    return __syncthreads_or(*(const volatile int *)&ctl->err & DERR_TIMEOUT) != 0;
+}
 
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;

@@ -88,11 +88,13 @@ constexpr int LB_STREAMS = 4;   // sums looked back over at once
 struct ScanState {
     void *word;
     unsigned epoch;
+    int polls;  // polls of an earlier tile's sum before a look-back gives up (0: the default limit)
 };
 struct LookBack {
     unsigned *ctr;             // tickets handed out, blocks done
     unsigned long long *word;  // [LB_STREAMS][LB_TILES]
     unsigned epoch;
+    int polls;
 };
 size_t scan_state_bytes();
 

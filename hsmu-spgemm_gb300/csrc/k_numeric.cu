@@ -166,6 +166,7 @@ __global__ void __launch_bounds__(256) k_win_cursors(const Window *__restrict__ 
                                                      const int *__restrict__ tcol, const int *__restrict__ toff,
                                                      const int *__restrict__ item_off, int *__restrict__ wcur,
                                                      Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     const int nwin = min(ctl->win_count, win_cap);
     const int lane = lane_id();
     const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
@@ -223,6 +224,7 @@ __global__ void __launch_bounds__(NUM_WARPS * 32, NUM_CTAS_PER_SM) k_numeric(con
                                                             const int *__restrict__ ts_tcol,
                                                             const TileEnt *__restrict__ ts_tent,
                                                             const int *__restrict__ heavy, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     extern __shared__ __align__(16) unsigned long long s_dyn[];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     NumSmem &S = reinterpret_cast<NumSmem *>(s_dyn)[w];

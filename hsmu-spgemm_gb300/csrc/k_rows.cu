@@ -177,7 +177,9 @@ __device__ __forceinline__ long long block_excl_scan(long long v, long long *s_w
 // is flag | epoch | value, so one 64-bit store publishes it; words of earlier
 // launches carry another epoch and need no clearing.  The ticket counter resets
 // itself when the last block is done.  The look-back's polls are bounded: a
-// block that gives up sets DERR_TIMEOUT and goes on with what it has.
+// block that gives up sets DERR_TIMEOUT and goes on with what it has, a prefix
+// no larger than the right one, so what it writes stays in bounds; the kernels
+// that index by the result return at once then (scan_failed).
 //
 // Small calls are launch-bound: with three launches per scan and two more for the
 // binning a Laplacian product had 18, now 10 (64^2 grid 163 -> 130 us, 256^2 210 ->
@@ -217,14 +219,15 @@ __device__ __forceinline__ unsigned long long lb_prefix(LookBack lb, int stream,
         const int t = at - lane;
         unsigned long long x = 0;
         bool ready = false;
-        for (int poll = 0; poll < LB_POLLS; poll++) {
+        for (int poll = 0; poll < lb.polls; poll++) {
             if (t >= 0 && !ready) {
                 x = w[t];
                 ready = (x >> 62) != 0 && (unsigned)((x >> LB_VALUE_BITS) & ((1u << LB_EPOCH_BITS) - 1u)) == lb.epoch;
             }
             if (__all_sync(FULL, t < 0 || ready)) break;
         }
-        if (!__all_sync(FULL, t < 0 || ready)) {
+        const bool gave_up = !__all_sync(FULL, t < 0 || ready);
+        if (gave_up) {
             if (lane == 0) set_err(&ctl->err, DERR_TIMEOUT);
             if (!ready) x = 0;
         }
@@ -232,7 +235,7 @@ __device__ __forceinline__ unsigned long long lb_prefix(LookBack lb, int stream,
         const unsigned pre = __ballot_sync(FULL, ready && (x >> 62) == 2);
         const int last = pre ? __ffs(pre) - 1 : WARP - 1;
         sum += warp_sum(t >= 0 && lane <= last ? x & LB_MAX : 0ull);
-        if (pre) break;
+        if (pre || gave_up) break;
     }
     if (lane == 0) w[tile] = lb_word(LB_PREFIX, lb.epoch, sum + mine);
     return sum;
@@ -318,7 +321,8 @@ static LookBack next_epoch(ScanState &s, cudaStream_t st) {
         s.epoch = 1;
     }
     unsigned long long *w = reinterpret_cast<unsigned long long *>(s.word);
-    return LookBack{reinterpret_cast<unsigned *>(w + (size_t)LB_STREAMS * LB_TILES), w, s.epoch};
+    return LookBack{reinterpret_cast<unsigned *>(w + (size_t)LB_STREAMS * LB_TILES), w, s.epoch,
+                    s.polls > 0 ? s.polls : LB_POLLS};
 }
 
 size_t scan_state_bytes() { return sizeof(unsigned long long) * ((size_t)LB_STREAMS * LB_TILES + 1); }

@@ -191,6 +191,7 @@ constexpr int HC_CTAS_PER_SM = 6;
 __global__ void __launch_bounds__(HC_WARPS * 32, HC_CTAS_PER_SM)
     k_count_h(int M, const int *__restrict__ arp, const int *__restrict__ acol, const int *__restrict__ brp,
               const int *__restrict__ bcol, RowInfo ri, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     HSmem &S = reinterpret_cast<HSmem *>(s_dyn)[w];
@@ -231,6 +232,7 @@ __global__ void __launch_bounds__(HF_WARPS * 32, hf_ctas<AR>())
     k_fill_h(int M, const int *__restrict__ arp, const int *__restrict__ acol, const double *__restrict__ aval,
              const int *__restrict__ brp, const int *__restrict__ bcol, const double *__restrict__ bval, RowInfo ri,
              RowOut out, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     HSmem &S = reinterpret_cast<HSmem *>(s_dyn)[w];

@@ -97,6 +97,7 @@ __global__ void __launch_bounds__(SDS_WARPS * 32, SDS_CTAS_PER_SM)
                 const int *__restrict__ tptr, const int *__restrict__ tcol,
                 const unsigned long long *__restrict__ tmask, RowInfo ri, RowOut out, Window *__restrict__ win,
                 long long win_cap, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     SdsSmem &S = reinterpret_cast<SdsSmem *>(s_dyn)[w];
@@ -266,6 +267,7 @@ __global__ void __launch_bounds__(SL_THREADS, 3) k_struct_l(int M, const int *__
                                                          RowOut out, Window *__restrict__ win, long long win_cap,
                                                          const int *__restrict__ stored, long long arena,
                                                          Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     SlSmem &S = *reinterpret_cast<SlSmem *>(s_dyn);
     // warp totals of the three block scans of a chunk (one array each: one barrier per scan)
@@ -407,6 +409,7 @@ constexpr int SLS_THREADS = 256;
 
 __global__ void __launch_bounds__(SLS_THREADS, 6) k_struct_ls(int M, RowInfo ri, TileStore ts, RowOut out,
                                                            Window *__restrict__ win, long long win_cap, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     constexpr int NT = SLS_THREADS;
     __shared__ int s_wbase, s_next;
     const int lane = lane_id(), w = threadIdx.x >> 5;
@@ -481,6 +484,7 @@ __global__ void __launch_bounds__(TINYF_THREADS, 4) k_fill_tiny(int M, const int
                                                                 const int *__restrict__ bcol,
                                                                 const double *__restrict__ bval, RowInfo ri,
                                                                 RowOut out, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     TinySmem<AR> &S = reinterpret_cast<TinySmem<AR> *>(s_dyn)[threadIdx.x >> 5];
     const int *rows = ri.bins + (size_t)BIN_TINY * M;
@@ -529,6 +533,7 @@ __global__ void __launch_bounds__(TINYF_THREADS) k_fill_tiny_wide(int M, const i
                                                              const int *__restrict__ bcol,
                                                              const double *__restrict__ bval, RowInfo ri,
                                                              RowOut out, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     __shared__ int s_cols[TINY_MAX * TINYF_THREADS];
     __shared__ double s_acc[TINY_MAX * TINYF_THREADS];
     const int *rows = ri.bins + (size_t)BIN_TINY * M;

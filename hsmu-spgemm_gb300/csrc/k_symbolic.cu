@@ -58,6 +58,7 @@ __global__ void __launch_bounds__(DS_WARPS * 32) k_count_ds(int M, const int *__
                                                             const int *__restrict__ tcol,
                                                             const unsigned long long *__restrict__ tmask,
                                                             RowInfo ri, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     __shared__ unsigned long long s_mask[DS_WARPS][SPAN_T];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     unsigned long long *msk = s_mask[w];
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(L_THREADS, L_BLOCK_THREADS / L_THREADS) k_coun
                                                        const unsigned long long *__restrict__ tmask,
                                                        RowInfo ri, TileStore ts, RowOut out, Ctl *ctl) {
     constexpr bool STORE = MODE != LM_COUNT;
+    if (scan_failed(ctl)) return;
     constexpr bool SPEC = MODE == LM_SPEC;
     extern __shared__ unsigned long long s_dyn[];
     unsigned long long *msk = s_dyn;  // DCH_COUNT entries
@@ -238,6 +240,7 @@ __global__ void __launch_bounds__(TINY_THREADS) k_count_tiny(int M, const int *_
                                                              const int *__restrict__ acol,
                                                              const int *__restrict__ brp,
                                                              const int *__restrict__ bcol, RowInfo ri, Ctl *ctl) {
+    if (scan_failed(ctl)) return;
     __shared__ int s_q[TINY_THREADS / WARP][TINY_MAX][WARP];
     int (*qs)[WARP] = s_q[threadIdx.x >> 5];
     const int n = ctl->bin_count[BIN_TINY];

@@ -76,7 +76,7 @@ class c_btiles(ctypes.Structure):
 class c_opts(ctypes.Structure):
     _fields_ = [("validate", ctypes.c_int32), ("arith", ctypes.c_int32),
                 ("window_cap", ctypes.c_int32), ("panels", ctypes.c_int32), ("wait_polls", ctypes.c_int32),
-                ("no_tile_store", ctypes.c_int32), ("learned_always", ctypes.c_int32), ("reserved", ctypes.c_int32)]
+                ("no_tile_store", ctypes.c_int32), ("learned_always", ctypes.c_int32), ("scan_polls", ctypes.c_int32)]
 
 
 class c_mlp(ctypes.Structure):

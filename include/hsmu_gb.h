@@ -104,18 +104,21 @@ typedef struct hsmu_opts {
                            * part they double from the first panel to the middle and halve
                            * towards the last.  The panels run in the order that keeps the host
                            * link busy soonest (the least compute first) */
-    int32_t wait_polls;   /* test hook, 0 in normal use.  > 0: every bounded device wait of the call
-                           * gives up after this many polls instead of its default limit (the value
-                           * pass's wait for a window's column copy polls without blocking; the batch's
-                           * grid barriers spin this many times) and the call reports
-                           * HSMU_ERR_TIMEOUT.  A wait that gives up still lets its own copy land
-                           * before the kernel returns; the handle stays usable.  For hsmu_batch_create
-                           * it applies to every launch of the batch. */
+    int32_t wait_polls;   /* test hook, 0 in normal use.  > 0: the value pass's wait for a window's
+                           * column copy (which then polls without blocking) and the batch's grid
+                           * barriers give up after this many polls instead of their default limit
+                           * (scan_polls: the scans' waits) and the call reports HSMU_ERR_TIMEOUT.
+                           * A wait that gives up still lets its own copy land before the kernel
+                           * returns; the handle stays usable.  For hsmu_batch_create it applies to
+                           * every launch of the batch. */
     int32_t no_tile_store; /* 1: the count pass keeps no C tiles of the large rows, and the structure
                            * pass repeats their OR walk over B's tiles (same output; less scratch) */
     int32_t learned_always; /* test hook, 0 in normal use.  1: hsmu_spgemm_learned never hands the
                            * product to the plain path (it uses its prediction whatever the rows) */
-    int32_t reserved;
+    int32_t scan_polls;   /* test hook, 0 in normal use.  > 0: the single-launch scans of the call (row
+                           * pointers, tiles, row classes, windows) give up after this many polls of an
+                           * earlier block's sum, and the call reports HSMU_ERR_TIMEOUT; the handle
+                           * stays usable */
 } hsmu_opts;
 
 /* Per-call statistics (filled by hsmu_spgemm when stats != NULL). */
