@@ -52,6 +52,7 @@
 #include "hsmu_gb.h"
 #include "hsmu_kernels.h"
 #include "hsmu_rowops.cuh"
+#include "hsmu_steps.cuh"
 
 namespace hsmu {
 
@@ -814,21 +815,20 @@ __device__ void phase_place(const BParams &P, const BRound &R) {
         const double *sv = R.val_pool + base + src;
         int *dc = R.out_col + base + dst;
         double *dv = R.out_val + base + dst;
-        for (int q0 = lane; q0 < n; q0 += PLACE_U * WARP) {
+        for (StepPos q0 = lane; step_in(q0, 0, n); q0 += PLACE_U * WARP) {
             int c8[PLACE_U];
             double v8[PLACE_U];
 #pragma unroll
             for (int u = 0; u < PLACE_U; u++) {
-                const int q = q0 + u * WARP;
-                c8[u] = q < n ? ldx<false>(sc + q) : 0;
-                v8[u] = q < n ? ldx<false>(sv + q) : 0.0;
+                const bool in = step_in(q0, u * WARP, n);
+                c8[u] = in ? ldx<false>(sc + q0 + u * WARP) : 0;
+                v8[u] = in ? ldx<false>(sv + q0 + u * WARP) : 0.0;
             }
 #pragma unroll
             for (int u = 0; u < PLACE_U; u++) {
-                const int q = q0 + u * WARP;
-                if (q < n) {
-                    dc[q] = c8[u];
-                    dv[q] = v8[u];
+                if (step_in(q0, u * WARP, n)) {
+                    dc[q0 + u * WARP] = c8[u];
+                    dv[q0 + u * WARP] = v8[u];
                 }
             }
         }

@@ -10,6 +10,7 @@
 // 101 -> 17 + 8 us, features 65 -> 12 + 7 us; scale 18: bounds 477 -> 68 + 47 us.
 #pragma once
 #include "hsmu_common.cuh"
+#include "hsmu_steps.cuh"
 
 namespace hsmu {
 
@@ -22,19 +23,19 @@ struct RowSums {
     int longest;     // the longest of them
     int cmin, cmax;  // first and last column (INT_MAX, -1: none)
 
-    // entries first, first + stride, ... below hi of A's columns
-    __device__ __forceinline__ void walk(int first, int hi, int stride, const int *__restrict__ acol,
+    // entries first, first + stride, ... of the len from acol on
+    __device__ __forceinline__ void walk(int first, int len, int stride, const int *__restrict__ acol,
                                          const int *__restrict__ brp, const int *__restrict__ bcol) {
         prod = 0;
         longest = 0;
         cmin = INT_MAX;
         cmax = -1;
-        for (int p = first; p < hi; p += stride * SUM_U) {
+        for (StepPos p = first; step_in(p, 0, len); p += stride * SUM_U) {
             int s[SUM_U], e[SUM_U];
 #pragma unroll
             for (int u = 0; u < SUM_U; u++) {
                 s[u] = e[u] = 0;
-                if (hi - p > u * stride) {
+                if (step_in(p, u * stride, len)) {
                     const int k = __ldg(acol + p + u * stride);
                     s[u] = __ldg(brp + k);
                     e[u] = __ldg(brp + k + 1);
@@ -83,7 +84,7 @@ __device__ __forceinline__ RowSums block_row_sums(int lo, int hi, const int *__r
     }
     __syncthreads();
     RowSums r;
-    r.walk(lo + (int)threadIdx.x, hi, SUM_THREADS, acol, brp, bcol);
+    r.walk((int)threadIdx.x, hi - lo, SUM_THREADS, acol + lo, brp, bcol);
     r.reduce<WARP>();
     if (lane_id() == 0) {
         atomicAdd(&S.prod, (unsigned long long)r.prod);

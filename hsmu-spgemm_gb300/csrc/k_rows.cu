@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(SUM_THREADS) k_bounds(int M, const int *__rest
         const int lo = i < M ? arp[i] : 0, hi = i < M ? arp[i + 1] : 0;
         const bool listed = long_list && hi - lo > SUM_LONG;
         RowSums r;
-        r.walk(lo + sub, listed ? lo : hi, G, acol, brp, bcol);
+        r.walk(sub, listed ? 0 : hi - lo, G, acol + lo, brp, bcol);
         r.reduce<G>();
         if (i < M && sub == 0) {
             if (listed) long_list[atomicAdd(&ctl->long_rows, 1)] = i;

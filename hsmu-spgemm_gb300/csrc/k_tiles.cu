@@ -13,6 +13,7 @@
 // first entry (tile_off) so the numeric phase can jump straight to it.
 #include "hsmu_common.cuh"
 #include "hsmu_kernels.h"
+#include "hsmu_steps.cuh"
 
 namespace hsmu {
 
@@ -35,19 +36,17 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
         unsigned long long pend_m = 0;
         int prev_col = -1;
         bool bad = false;
-        for (int base0 = s; base0 < e; base0 += WARP * TILE_U) {
+        for (StepPos base0 = s; step_in(base0, 0, e); base0 += WARP * TILE_U) {
             int cu[TILE_U];
 #pragma unroll
             for (int u = 0; u < TILE_U; u++) {
-                const int idx = base0 + u * WARP + lane;
-                cu[u] = idx < e ? __ldg(bcol + idx) : 0;
+                cu[u] = step_in(base0, u * WARP + lane, e) ? __ldg(bcol + base0 + u * WARP + lane) : 0;
             }
 #pragma unroll
             for (int u = 0; u < TILE_U; u++) {
-                const int base = base0 + u * WARP;
-                if (base >= e) break;
-                const int idx = base + lane;
-                const bool valid = idx < e;
+                if (!step_in(base0, u * WARP, e)) break;
+                const int base = (int)base0 + u * WARP;
+                const bool valid = step_in(base, lane, e);
                 const int c = cu[u];
                 if (validate) {
                     int cp = __shfl_up_sync(FULL, c, 1);
@@ -95,7 +94,7 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
                         const int pos = run + __popc(heads & lanemask_lt());
                         tcol[pos] = t;
                         tmask[pos] = v;
-                        toff[pos] = idx;
+                        toff[pos] = base + lane;
                     }
                     run += __popc(heads) - 1;
                     pend_t = __shfl_sync(FULL, t, last);

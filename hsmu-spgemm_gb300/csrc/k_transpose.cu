@@ -17,6 +17,7 @@
 // column).  Everything is integer and data movement: bit-exact by design.
 #include "hsmu_common.cuh"
 #include "hsmu_kernels.h"
+#include "hsmu_steps.cuh"
 
 namespace hsmu {
 
@@ -52,7 +53,7 @@ __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_hist(const int *__restrict
     __syncwarp();
     if (tile < ntiles) {
         const int lo = tile * te, hi = (int)min((long long)n, (long long)lo + te);
-        for (int e = lo + lane; e < hi; e += WARP) atomicAdd(&s_h[w][(key[e] >> shift) & (TR_RADIX - 1)], 1);
+        for (int o = lane; o < hi - lo; o += WARP) atomicAdd(&s_h[w][(key[lo + o] >> shift) & (TR_RADIX - 1)], 1);
         __syncwarp();
         for (int d = lane; d < TR_RADIX; d += WARP) hist[d * ntiles + tile] = s_h[w][d];
     }
@@ -71,19 +72,20 @@ __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_scatter(const int *__restr
     for (int d = lane; d < TR_RADIX; d += WARP) s_run[w][d] = off[d * ntiles + tile];
     __syncwarp();
     const int lo = tile * te, hi = (int)min((long long)n, (long long)lo + te);
-    for (int b = lo; b < hi; b += TR_U * WARP) {
+    for (StepPos b = lo; step_in(b, 0, hi); b += TR_U * WARP) {
         int k[TR_U], i[TR_U];
         double x[TR_U];
 #pragma unroll
         for (int u = 0; u < TR_U; u++) {
-            const int e = b + u * WARP + lane;
-            k[u] = e < hi ? key[e] : 0;
-            i[u] = e < hi ? row[e] : 0;
-            x[u] = e < hi ? val[e] : 0.0;
+            const bool v = step_in(b, u * WARP + lane, hi);
+            const StepPos e = b + u * WARP + lane;
+            k[u] = v ? key[e] : 0;
+            i[u] = v ? row[e] : 0;
+            x[u] = v ? val[e] : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < TR_U; u++) {
-            const bool v = b + u * WARP + lane < hi;
+            const bool v = step_in(b, u * WARP + lane, hi);
             const int d = v ? (k[u] >> shift) & (TR_RADIX - 1) : TR_RADIX + lane;  // invalid lanes: own group
             const unsigned grp = __match_any_sync(FULL, d);
             if (v) {
