@@ -121,8 +121,10 @@ constexpr long long HOST_PANEL_BYTES = 32ll << 20;
 constexpr int TILES_ASIDE_MIN_NNZ = 1 << 19;
 // entries of A from which the count pass takes the side stream too
 constexpr int SIDE_MIN_NNZ = 1 << 16;
-// hsmu_spgemm64: window cursors (4 bytes each) up to which all panels share one symbolic pass
-constexpr unsigned long long ONE_PASS_CURSORS = 1ull << 30;
+// hsmu_spgemm64: bytes of windows and cursors up to which all panels share one symbolic pass, and what
+// a window and a cursor take (PlainRun::alloc_output)
+constexpr unsigned long long ONE_PASS_BYTES = 4ull << 30;
+constexpr unsigned long long WINDOW_BYTES = sizeof(Window) + sizeof(long long) + 3 * sizeof(int);
 // average entries of B's rows from which repeated rows are looked for: chains of shorter rows
 // are not taken (hsmu_products.cuh), and the chain kernel's registers cost rows without chains
 // (scalar 27-point rows: 296 us with it, 169 us without)
@@ -385,6 +387,7 @@ struct PlainRun {
     long long *ts_off = nullptr;
     int *ts_cnt = nullptr, *ts_nwin = nullptr, *ts_wbase = nullptr;
     bool have_store = false;
+    bool arena_failed = false;  // tiles_bounds: no memory for a larger arena (the next call starts without one)
     // the count pass reserves the large rows' windows (one product, one panel of
     // structure + values); the row panels of the host-buffer path restart the window
     // buffer at 0 for every panel and reserve them in the structure pass instead
@@ -463,7 +466,9 @@ struct PlainRun {
         CKR(salloc(h, &ri.cls, (size_t)M, st));
         CKR(salloc(h, &ri.cnnz, (size_t)M + 1, st));
         if (store) {
-            CKR(grow_arena());
+            const cudaError_t ae = grow_arena();
+            arena_failed = ae != cudaSuccess;
+            CKR(ae);
             ri.store = 1;
             if (h->arena_cap > 0) {
                 CKR(salloc(h, &ts_off, (size_t)M, st));
@@ -1273,10 +1278,107 @@ done:
 // its place in C; B's tiles are built once for all panels.
 //
 // The panels share one symbolic pass (bounds, bins, counts and tile lists of all rows) when
-// the cursors of all windows take at most ONE_PASS_CURSORS: a panel is then a structure and a
-// value pass on its slice of the bins, with row pointers of its own.  Beyond that every panel
-// runs the plain engine on its rows, so that only one panel's windows and cursors exist at a
-// time.  A power-law graph of 49,999 vertices in four panels: 4.65 -> 3.55 ms with one pass.
+// the windows and cursors of all rows take at most ONE_PASS_BYTES: a panel is then a structure
+// and a value pass on its slice of the bins, with row pointers of its own.  Beyond that, or when
+// the memory for them or for the tile lists is not there, every panel runs the plain engine on
+// its rows, so that only one panel's lists, windows and cursors exist at a time.  A power-law
+// graph of 49,999 vertices in four panels: 4.65 -> 3.55 ms with one pass.
+struct Panels {
+    long long cap = 0;           // entries of a panel
+    std::vector<long long> hrp;  // C's row pointers
+    long long *rp = nullptr;     // the same on the device
+    int *col = nullptr;
+    double *val = nullptr;
+
+    // rows r0 .. end - 1: as many as keep the panel within the cap, at least one
+    int end(int r0) const {
+        const int r1 = (int)(std::upper_bound(hrp.begin() + r0 + 1, hrp.end(), hrp[r0] + cap) - hrp.begin()) - 1;
+        return r1 <= r0 ? r0 + 1 : r1;
+    }
+};
+
+// C's row pointers and arrays, and all of its rows when one pass holds them (done); memory: the one
+// pass ran out of it
+int spgemm64_whole(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, Panels &P, const hsmu_opts &o, bool one_pass,
+                   cudaStream_t st, bool &done, bool &memory) {
+    const int M = A->M;
+    done = memory = false;
+    ScratchScope scope(h, st);
+    PlainRun r(h, st, o);
+    CKQ(r.begin(A, B));
+    r.reserve_windows = false;  // the output is written in row panels
+    if (!P.rp) CKR(palloc(&P.rp, (size_t)M + 1, st));
+    P.hrp.resize((size_t)M + 1);
+    int rc = r.tiles_bounds(B, nullptr, false, nullptr, one_pass && o.no_tile_store == 0);
+    memory = r.arena_failed;
+    if (rc) return rc;
+    if (one_pass) {
+        CKR(cudaMemcpyAsync(h->h_ctl, r.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
+        CKR(cudaStreamSynchronize(st));
+        // (the warp class's share is a bound before the count)
+        const Ctl &b = *h->h_ctl;
+        one_pass = b.win_bound <= INT_MAX &&
+                   sizeof(int) * (b.cur_bound + b.cur_bound_ds) + WINDOW_BYTES * b.win_bound <= ONE_PASS_BYTES;
+        if (!one_pass) {  // each panel keeps its own tile lists
+            r.have_store = false;
+            r.ri.store = 0;
+        }
+    }
+    CKQ(r.count_scan64(P.rp, P.hrp.data()));
+    if (!P.col) CKR(palloc(&P.col, (size_t)P.hrp[M] + COL_PAD, st));
+    if (!P.val) CKR(palloc(&P.val, (size_t)P.hrp[M], st));
+    if (!one_pass) return HSMU_OK;
+    CKR(palloc(&r.crp, (size_t)M + 1, st));
+    r.ext_col = P.col;  // never the run's own
+    r.ext_val = P.val;
+    rc = r.alloc_output();
+    memory = rc == HSMU_ERR_ALLOC;
+    if (rc) return rc;
+    for (int r0 = 0, r1; r0 < M; r0 = r1) {
+        r1 = P.end(r0);
+        if (r0 > 0) CKQ(r.next_panel());
+        launch_panel_ptr(P.rp, r0, r1, r.crp, grid_rows(h), st);
+        r.ccol = P.col + P.hrp[r0];
+        r.cval = P.val + P.hrp[r0];
+        CKQ(r.structure(r0, r1));
+        r.values();
+    }
+    done = true;
+    return r.finish();
+}
+
+// every panel by itself
+int spgemm64_panels(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, const Panels &P, const hsmu_opts &o,
+                    cudaStream_t st) {
+    hsmu_btiles bt{};
+    Ctl *ctl = nullptr;
+    ScratchScope scope(h, st);
+    CKR(salloc(h, &ctl, 1, st));
+    CKR(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
+    CKQ(build_tiles(h, B, &bt, ctl, 0, st, true, false));
+    CKR(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
+    CKR(cudaStreamSynchronize(st));
+    if (h->h_ctl->err) return err_from_dev(h->h_ctl->err);
+    for (int r0 = 0, r1; r0 < A->M; r0 = r1) {
+        r1 = P.end(r0);
+        hsmu_csr Ap = *A;
+        Ap.M = r1 - r0;
+        Ap.row_ptr = A->row_ptr + r0;
+        ScratchScope panel(h, st);
+        PlainRun r(h, st, o);
+        r.ext_col = P.col + P.hrp[r0];
+        r.ext_val = P.val + P.hrp[r0];
+        CKQ(r.begin(&Ap, B));
+        CKQ(r.symbolic(B, &bt, false, nullptr, nullptr));
+        if (r.hc.nnz != P.hrp[r1] - P.hrp[r0]) return HSMU_ERR_INTERNAL;
+        CKQ(r.alloc_output());
+        CKQ(r.structure(0, Ap.M));
+        r.values();
+        CKQ(r.finish());
+    }
+    return HSMU_OK;
+}
+
 int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_csr64 *C, long long max_panel,
                   const hsmu_opts *opts, cudaStream_t st) {
     if (!h || !csr_ok(A) || !csr_ok(B) || !C || A->N != B->M || max_panel < 0) return HSMU_ERR_INVALID;
@@ -1284,101 +1386,31 @@ int spgemm64_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, hsmu_c
     if (opts) o = *opts;
     if (!arith_ok(o)) return HSMU_ERR_INVALID;
     std::memset(C, 0, sizeof(*C));
-    const long long cap = (max_panel == 0 || max_panel > INT_MAX) ? INT_MAX : max_panel;
-    const int M = A->M;
-    int rc = HSMU_OK;
-    int *col = nullptr;
-    long long *rp = nullptr;
-    double *val = nullptr;
-    bool one_pass = false;
-    std::vector<long long> hrp;
-    ScratchScope scope(h, st);
-    PlainRun one(h, st, o);
-    hsmu_opts po = o;
-    po.validate = 0;  // the panels are views into A: the operands are checked once, here
-    rc = one.begin(A, B);
-    if (rc) goto done;
-    one.reserve_windows = false;  // the output is written in row panels
-    CK(palloc(&rp, (size_t)M + 1, st));
-    hrp.resize((size_t)M + 1);
-    rc = one.tiles_bounds(B, nullptr, false, nullptr, o.no_tile_store == 0);
-    if (rc) goto done;
-    CK(cudaMemcpyAsync(h->h_ctl, one.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    // (the warp class's share is a bound before the count)
-    one_pass = h->h_ctl->cur_bound + h->h_ctl->cur_bound_ds <= ONE_PASS_CURSORS && h->h_ctl->win_bound <= INT_MAX;
-    if (!one_pass) {  // each panel keeps its own tile lists
-        one.have_store = false;
-        one.ri.store = 0;
+    Panels P;
+    P.cap = (max_panel == 0 || max_panel > INT_MAX) ? INT_MAX : max_panel;
+    bool done, memory;
+    int rc = spgemm64_whole(h, A, B, P, o, true, st, done, memory);
+    o.validate = 0;  // the operands are checked once (the panels are views into A)
+    if (rc == HSMU_ERR_ALLOC && memory) {
+        cudaStreamSynchronize(st);
+        rc = spgemm64_whole(h, A, B, P, o, false, st, done, memory);
     }
-    rc = one.count_scan64(rp, hrp.data());
-    if (rc) goto done;
-    CK(palloc(&col, (size_t)hrp[M] + COL_PAD, st));
-    CK(palloc(&val, (size_t)hrp[M], st));
-    if (one_pass) {
-        CK(palloc(&one.crp, (size_t)M + 1, st));
-        one.ext_col = col;  // never the run's own
-        one.ext_val = val;
-        rc = one.alloc_output();
-        if (rc) goto done;
-    } else {
-        one.release();
+    if (!rc && !done) rc = spgemm64_panels(h, A, B, P, o, st);
+    if (rc) {
+        pfree(P.rp, st);
+        pfree(P.col, st);
+        pfree(P.val, st);
+        cudaStreamSynchronize(st);
+        return rc;
     }
-    for (int r0 = 0; r0 < M;) {
-        // rows r0 .. r1-1: as many as keep the panel within the cap, at least one
-        int r1 = (int)(std::upper_bound(hrp.begin() + r0 + 1, hrp.end(), hrp[r0] + cap) - hrp.begin()) - 1;
-        if (r1 <= r0) r1 = r0 + 1;
-        if (one_pass) {
-            if (r0 > 0) rc = one.next_panel();
-            if (rc) goto done;
-            launch_panel_ptr(rp, r0, r1, one.crp, grid_rows(h), st);
-            one.ccol = col + hrp[r0];
-            one.cval = val + hrp[r0];
-            rc = one.structure(r0, r1);
-            if (rc) goto done;
-            one.values();
-            r0 = r1;
-            continue;
-        }
-        hsmu_csr Ap = *A;
-        Ap.M = r1 - r0;
-        Ap.row_ptr = A->row_ptr + r0;
-        ScratchScope panel(h, st);
-        PlainRun r(h, st, po);
-        r.ext_col = col + hrp[r0];
-        r.ext_val = val + hrp[r0];
-        rc = r.begin(&Ap, B);
-        if (!rc) rc = r.symbolic(B, &one.bt, false, nullptr, nullptr);
-        if (!rc && r.hc.nnz != hrp[r1] - hrp[r0]) rc = HSMU_ERR_INTERNAL;
-        if (!rc) rc = r.alloc_output();
-        if (!rc) {
-            rc = r.structure(0, Ap.M);
-            if (!rc) r.values();
-            if (!rc) rc = r.finish();
-        }
-        r.release();
-        if (rc) goto done;
-        r0 = r1;
-    }
-    if (one_pass) rc = one.finish();
-    if (rc) goto done;
-    C->M = M;
+    C->M = A->M;
     C->N = B->N;
-    C->nnz = hrp[M];
+    C->nnz = P.hrp[A->M];
     C->owned = 1;
-    C->row_ptr = reinterpret_cast<int64_t *>(rp);
-    C->col = col;
-    C->val = val;
-    rp = nullptr;
-    col = nullptr;
-    val = nullptr;
-done:
-    one.release();
-    pfree(rp, st);
-    pfree(col, st);
-    pfree(val, st);
-    cudaStreamSynchronize(st);
-    return rc;
+    C->row_ptr = reinterpret_cast<int64_t *>(P.rp);
+    C->col = P.col;
+    C->val = P.val;
+    return HSMU_OK;
 }
 
 }  // namespace
