@@ -366,6 +366,7 @@ struct PlainRun {
     int M = 0;
     DevCSR Ad{}, Bd{};
     hsmu_btiles bt{};
+    bool in_line = false;    // B's tiles are built on `st`, after the bounds pass
     bool side_busy = false;  // the handle's side stream has work that `st` does not wait for yet
     DevTiles Btd{};
     RowInfo ri{};
@@ -442,7 +443,8 @@ struct PlainRun {
                             h->ev_side_done));
             launches += 3;
         }
-        const bool in_line = !Bt_in && !side_busy;
+        in_line = !Bt_in && !side_busy;
+        if (ev_tiles && in_line) cudaEventRecord(h->ev[7], st);
         if (ev_tiles && !in_line) cudaEventRecord(ev_tiles, side_busy ? h->cs_tiles : st);
         if (B->M > 0 && B->nnz >= (long long)REPEAT_MIN_ROW * B->M) {
             CKR(salloc(h, &rep, (size_t)B->M, st));
@@ -482,6 +484,7 @@ struct PlainRun {
         launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), h->scan, st);
         launches += 2 + long_rows_apart(Ad);  // bounds + binning
         if (in_line) {
+            if (ev_tiles) cudaEventRecord(h->ev[6], st);
             CKQ(build_tiles(h, B, &bt, ctl, 0, st, count_tiles, false, !count_tiles));
             launches += 3;
             if (ev_tiles) cudaEventRecord(ev_tiles, st);
@@ -687,16 +690,28 @@ struct PlainRun {
     }
 };
 
+// ms_convert and ms_symbolic.  In-line tiles are built between the bounds pass and the count
+// (events 6 to 1), after what comes ahead of both (0 to 7).
+void conversion_times(const hsmu_handle_s *h, bool in_line, hsmu_stats *stats) {
+    float t, u;
+    cudaEventElapsedTime(&t, h->ev[0], h->ev[in_line ? 7 : 1]);
+    stats->ms_convert = t;
+    cudaEventElapsedTime(&t, h->ev[1], h->ev[2]);
+    stats->ms_symbolic = t;
+    if (!in_line) return;
+    cudaEventElapsedTime(&t, h->ev[6], h->ev[1]);
+    cudaEventElapsedTime(&u, h->ev[7], h->ev[6]);
+    stats->ms_convert += t;
+    stats->ms_symbolic += u;
+}
+
 void fill_stats(hsmu_handle_s *h, const PlainRun &r, const hsmu_btiles *Bt_in, hsmu_stats *stats) {
     float t;
     stats->products = r.hc.products;
     stats->nnz_c = r.hc.nnz;
     stats->ntiles_b = Bt_in ? Bt_in->ntiles : r.hc.ntiles;
     stats->windows = r.hc.win_count;
-    cudaEventElapsedTime(&t, h->ev[0], h->ev[1]);
-    stats->ms_convert = t;
-    cudaEventElapsedTime(&t, h->ev[1], h->ev[2]);
-    stats->ms_symbolic = t;
+    conversion_times(h, r.in_line, stats);
     cudaEventElapsedTime(&t, h->ev[2], h->ev[3]);
     stats->ms_alloc = t;
     cudaEventElapsedTime(&t, h->ev[3], h->ev[4]);
@@ -1214,10 +1229,7 @@ learned:
         stats->windows = hc.win_count;
         stats->spec_capacity = spec_total;
         stats->fallback_rows = hc.fallback;
-        cudaEventElapsedTime(&t, h->ev[0], h->ev[1]);
-        stats->ms_convert = t;
-        cudaEventElapsedTime(&t, h->ev[1], h->ev[2]);
-        stats->ms_symbolic = t;
+        conversion_times(h, r.in_line, stats);
         cudaEventElapsedTime(&t, h->ev[2], h->ev[3]);
         stats->ms_alloc = t;
         cudaEventElapsedTime(&t, h->ev[3], h->ev[4]);
