@@ -129,6 +129,12 @@ constexpr unsigned long long WINDOW_BYTES = sizeof(Window) + sizeof(long long) +
 // are not taken (hsmu_products.cuh), and the chain kernel's registers cost rows without chains
 // (scalar 27-point rows: 296 us with it, 169 us without)
 constexpr int REPEAT_MIN_ROW = 36;
+// ... and the chains that B's rows may form, in percent of the rows, for the chain kernel to be launched.
+// Fused row kernel with and without chains, 27-point stencils: 3 rows a node (33 %) 1,069 and 1,186 us,
+// 5 rows (40 %) 1,501 and 1,536; 2 rows (50 %) 398 and 404, 4 rows (50 %) 3,124 and 2,819; nodes of 3
+// of which four in five repeat (47 %) 754 and 700, three in five 848 and 700; no repeated rows (a band of
+// 101 entries) 3,046 and 1,059
+constexpr long long CHAINS_MAX_PCT = 45;
 constexpr long long HOST_MAX_PANELS = 8;
 constexpr double HOST_PANEL_GROWTH = 2.0;
 constexpr double HOST_PANEL_RATIO = 0.7;
@@ -448,7 +454,7 @@ struct PlainRun {
         if (ev_tiles && !in_line) cudaEventRecord(ev_tiles, side_busy ? h->cs_tiles : st);
         if (B->M > 0 && B->nnz >= (long long)REPEAT_MIN_ROW * B->M) {
             CKR(salloc(h, &rep, (size_t)B->M, st));
-            launch_row_repeat(Bd, rep, grid_rows(h), st);
+            launch_row_repeat(Bd, rep, &ctl->rep_chains, grid_rows(h), st);
             launches++;
             ri.rep = rep;
             const bool same = Ad.rp == Bd.rp && Ad.col == Bd.col && M == B->M;
@@ -456,7 +462,7 @@ struct PlainRun {
                 ri.rep_a = rep;
             } else if (Ad.nnz >= (long long)REPEAT_MIN_ROW * M && M > 0) {
                 CKR(salloc(h, &rep_a, (size_t)M, st));
-                launch_row_repeat(Ad, rep_a, grid_rows(h), st);
+                launch_row_repeat(Ad, rep_a, nullptr, grid_rows(h), st);
                 launches++;
                 ri.rep_a = rep_a;
             }
@@ -625,6 +631,14 @@ struct PlainRun {
                          (int)(hc.store_used <= h->arena_cap)};
     }
 
+    // The row information for the structure pass: with B's repeated rows where they form few enough
+    // chains (known since the last host read).
+    RowInfo chains(const Ctl &c) const {
+        RowInfo x = ri;
+        if (100ll * c.rep_chains > CHAINS_MAX_PCT * Bd.M) x.rep = nullptr;
+        return x;
+    }
+
     // sorted columns of rows lo..hi-1, values of warp-sized rows, numeric windows of the others
     int structure(int lo, int hi) {
         if (hc.nnz == 0) return HSMU_OK;
@@ -645,7 +659,7 @@ struct PlainRun {
             rows[BIN_TINY] = 0;
             if (heavy) rows[BIN_H] = 0;
         }
-        launch_structure(Ad, Bd, Btd, ri, out, win, win_cap, ctl, o.arith, h->nsm, st, rows,
+        launch_structure(Ad, Bd, Btd, chains(hc), out, win, win_cap, ctl, o.arith, h->nsm, st, rows,
                          have_store ? &tsd : nullptr);
         return apart ? join() : HSMU_OK;
     }
@@ -1124,7 +1138,7 @@ learned:
         Ctl *ctl = r.ctl;
         const DevCSR &Ad = r.Ad, &Bd = r.Bd;
         const DevTiles &Btd = r.Btd;
-        RowInfo &ri = r.ri;
+        const RowInfo ri = r.chains(hc);
         if (stats) cudaEventRecord(h->ev[2], st);
         spec_total = hc.nnz;
         win_cap = 2 * (long long)hc.win_bound;  // speculative pass + redo of overflowing rows

@@ -117,6 +117,7 @@ struct Ctl {
                                      // above FUSE_CAP entries
     long long win_listed;            // windows of the rows with a tile list (scan total)
     int long_rows;                   // rows listed by the bounds pass for its second launch
+    int rep_chains;                  // chains that B's rows form, single rows among them (k_row_repeat)
     RowCounter rows[3];              // row hand-out of the kernels that give a CTA one row at a time
 };
 

@@ -111,8 +111,9 @@ void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int 
                         bool gated = false);
 void launch_tiles_fill(const DevCSR &B, const int *tptr, int *tcol, unsigned long long *tmask, int *toff, Ctl *ctl,
                        int grid, cudaStream_t st, bool gated = false);
-// rep[k]: row k of B has the columns of row k - 1 (B.M bytes)
-void launch_row_repeat(const DevCSR &B, unsigned char *rep, int grid, cudaStream_t st);
+// rep[k]: row k of B has the columns of row k - 1 (B.M bytes); *chains (nullable) is raised by the
+// number of chains that the rows form
+void launch_row_repeat(const DevCSR &B, unsigned char *rep, int *chains, int grid, cudaStream_t st);
 void launch_validate(const DevCSR &A, Ctl *ctl, int grid, cudaStream_t st);
 
 // k_rows.cu

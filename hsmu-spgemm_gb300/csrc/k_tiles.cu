@@ -13,6 +13,7 @@
 // first entry (tile_off) so the numeric phase can jump straight to it.
 #include "hsmu_common.cuh"
 #include "hsmu_kernels.h"
+#include "hsmu_products.cuh"
 #include "hsmu_steps.cuh"
 
 namespace hsmu {
@@ -136,25 +137,40 @@ void launch_tiles_fill(const DevCSR &B, const int *tptr, int *tcol, unsigned lon
 
 // rep[k] = 1 when row k of B holds the same columns as row k - 1 (the rows of one finite-element
 // node; the fused row kernel chains their products).  One warp per row, stopped at the first
-// difference.
+// difference; a block takes 32 rows, as many as the row kernel looks at together, and counts
+// the chains that they form.
 __global__ void __launch_bounds__(256) k_row_repeat(int K, const int *__restrict__ brp, const int *__restrict__ bcol,
-                                                    unsigned char *__restrict__ rep) {
-    const int lane = lane_id();
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int k = gw; k < K; k += nw) {
-        const int s = brp[k], n = brp[k + 1] - s;
-        bool same = k > 0 && n > 0 && s - brp[k - 1] == n;
-        for (int base = 0; same && base < n; base += WARP) {
-            const int i = base + lane;
-            same = !__any_sync(FULL, i < n && __ldg(bcol + s + i) != __ldg(bcol + s - n + i));
+                                                    unsigned char *__restrict__ rep, int *chains) {
+    __shared__ unsigned s_join;  // rows of the 32 that repeat the one before them
+    const int lane = lane_id(), w = threadIdx.x >> 5;
+    int found = 0;
+    for (int k0 = blockIdx.x * WARP; k0 < K; k0 += gridDim.x * WARP) {
+        if (threadIdx.x == 0) s_join = 0;
+        __syncthreads();
+        for (int k = k0 + w; k < min(k0 + WARP, K); k += 256 / WARP) {
+            const int s = brp[k], n = brp[k + 1] - s;
+            bool same = k > 0 && n > 0 && s - brp[k - 1] == n;
+            for (int base = 0; same && base < n; base += WARP) {
+                const int i = base + lane;
+                same = !__any_sync(FULL, i < n && __ldg(bcol + s + i) != __ldg(bcol + s - n + i));
+            }
+            if (lane == 0) {
+                rep[k] = same;
+                if (same) atomicOr(&s_join, 1u << (k - k0));
+            }
         }
-        if (lane == 0) rep[k] = same;
+        __syncthreads();
+        if (w == 0) {
+            const int pos = lane - (31 - __clz(~(s_join & ~1u) & lanemask_le()));  // place in its run
+            found += __popc(__ballot_sync(FULL, k0 + lane < K && pos % REP_MAX == 0));
+        }
+        __syncthreads();
     }
+    if (threadIdx.x == 0 && chains && found) atomicAdd(chains, found);
 }
 
-void launch_row_repeat(const DevCSR &B, unsigned char *rep, int grid, cudaStream_t st) {
-    k_row_repeat<<<grid_for(grid, B.M, 256 / WARP), 256, 0, st>>>(B.M, B.rp, B.col, rep);
+void launch_row_repeat(const DevCSR &B, unsigned char *rep, int *chains, int grid, cudaStream_t st) {
+    k_row_repeat<<<grid_for(grid, B.M, WARP), 256, 0, st>>>(B.M, B.rp, B.col, rep, chains);
 }
 
 // Validation of A: sorted, unique, in-range columns (one warp per row).
