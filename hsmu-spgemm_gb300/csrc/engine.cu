@@ -124,7 +124,7 @@ constexpr int SIDE_MIN_NNZ = 1 << 16;
 // hsmu_spgemm64: bytes of windows and cursors up to which all panels share one symbolic pass, and what
 // a window and a cursor take (PlainRun::alloc_output)
 constexpr unsigned long long ONE_PASS_BYTES = 4ull << 30;
-constexpr unsigned long long WINDOW_BYTES = sizeof(Window) + sizeof(long long) + 3 * sizeof(int);
+constexpr unsigned long long WINDOW_BYTES = sizeof(Window) + sizeof(long long) + 3 * sizeof(int) + 1;
 // average entries of B's rows from which repeated rows are looked for: chains of shorter rows
 // are not taken (hsmu_products.cuh), and the chain kernel's registers cost rows without chains
 // (scalar 27-point rows: 296 us with it, 169 us without)
@@ -622,6 +622,7 @@ struct PlainRun {
         CKR(salloc(h, &wc.item_off, (size_t)nwin + 1, st));
         CKR(salloc(h, &wc.cur, (size_t)cap, st));
         CKR(salloc(h, &wc.heavy, (size_t)nwin, st));
+        CKR(salloc(h, &wc.cls, (size_t)nwin, st));
         return HSMU_OK;
     }
 
@@ -1160,6 +1161,7 @@ learned:
             CK(salloc(h, &wc.item_off, (size_t)win_cap + 1, st));
             CK(salloc(h, &wc.cur, (size_t)cur_cap, st));
             CK(salloc(h, &wc.heavy, (size_t)win_cap, st));
+            CK(salloc(h, &wc.cls, (size_t)win_cap, st));
         }
         if (stats) cudaEventRecord(h->ev[3], st);
         // structure (+ values of warp-sized rows) into the slots; exact counts found here.

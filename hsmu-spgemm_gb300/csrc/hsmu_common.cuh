@@ -100,7 +100,7 @@ struct Ctl {
     int bin_count[NBIN];
     int win_count;                   // windows emitted by the structure pass
     int win_next;                    // dynamic work counter of the numeric pass
-    int win_heavy, win_long;         // windows it hands out first (cleared together with win_next)
+    int win_heavy, win_long;         // windows it hands out first (k_win_len)
     int err;
     int ntiles;                      // B tiles (after the B conversion scan)
     int fallback;                    // learned path: rows that did not fit their slot

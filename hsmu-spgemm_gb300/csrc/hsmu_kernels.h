@@ -97,6 +97,8 @@ struct LookBack {
     int polls;
 };
 size_t scan_state_bytes();
+// the state for one launch that looks back
+LookBack next_epoch(ScanState &s, cudaStream_t st);
 
 // blocks of a grid-stride launch: `most`, or fewer when `per_block` items each are enough (a small
 // call's launches otherwise spend their time on a thousand empty blocks)
@@ -201,6 +203,7 @@ struct WinCursors {
     int *item_off;  // the cursor pass's work items per window, scanned in place
     int *cur;
     int *heavy;     // windows of rows with many A entries (win_cap entries)
+    signed char *cls;  // 0 and 1 for such windows (win_cap entries)
     long long cap;
 };
 void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const int *crp, int *ccol, double *cval,

@@ -39,6 +39,7 @@
 // compulsory bytes).  The next step's B loads are issued before the current
 // step's lookups and adds.
 #include "hsmu_kernels.h"
+#include "hsmu_lookback.cuh"
 #include "hsmu_products.cuh"
 
 namespace hsmu {
@@ -53,7 +54,9 @@ constexpr int GW = 2;  // consecutive windows per work item, handed out dynamica
 // transpose cropped to 30,011 vertices 1.49 -> 1.01 ms, scale 16 2.93 -> 2.27, scale 18
 // 19.00 -> 18.57, four row panels of a 49,999-vertex graph 2.75 -> 1.92 ms.  (One limit of 2,048
 // changed little, one of 512 gave 2.43 and one of 128 2.30 ms at scale 16; second limits of 64 and
-// first ones of 384 or 768 are within 3 % of these.)
+// first ones of 384 or 768 are within 3 % of these.)  Within a list the windows keep their order, that of
+// the rows: neighbours read the same rows of B.  27-point stencils with all windows listed, 30^3 grid x 6
+// rows a node 16.4 ms listed in any order, 14.1 in order; 32^3 x 5 10.6 and 8.5.
 constexpr int HEAVY_ROW = 512;
 constexpr int LONG_ROW = 128;
 constexpr int STAGE_LIMIT = 1 << 20;  // polls of a column copy before the kernel reports a timeout
@@ -88,26 +91,33 @@ __device__ __forceinline__ bool cur_continues(const Window *win, int w, int row,
 // here: up to the next window's first slot when that window continues the
 // same row, else up to the row's end; and its tile count likewise, up to the
 // next window's first tile or the end of the row's list.
-// Windows of rows with at least HEAVY_ROW A entries are listed (in any order) from the front of
-// `heavy`, those of rows with at least LONG_ROW from its back: the value pass hands them out first.
-__global__ void __launch_bounds__(256) k_win_len(Window *__restrict__ win, int win_cap, int M, const int *__restrict__ arp,
-                                                 const int *__restrict__ crp, const long long *__restrict__ ts_off,
-                                                 const int *__restrict__ ts_cnt, Ctl *ctl, int *__restrict__ len,
-                                                 int *__restrict__ items, int *__restrict__ heavy) {
+// Windows of rows with at least HEAVY_ROW A entries are listed from the front of `heavy`, those of rows
+// with at least LONG_ROW from its back, in order (bin_tile): the value pass hands them out first.
+// `windows` per block, in one pass over the list.
+__global__ void __launch_bounds__(BIN_T) k_win_len(Window *__restrict__ win, int win_cap, int M, const int *__restrict__ arp,
+                                                   const int *__restrict__ crp, const long long *__restrict__ ts_off,
+                                                   const int *__restrict__ ts_cnt, Ctl *ctl, int *__restrict__ len,
+                                                   int *__restrict__ items, signed char *cls, int *__restrict__ heavy,
+                                                   int windows, int ntiles, LookBack lb) {
+    __shared__ BinSmem<2> S;
+    const int tile = lb_tile(lb, &S.tile);
     const int nwin = min(ctl->win_count, win_cap);
-    for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < win_cap; w += gridDim.x * blockDim.x) {
+    const long long w_lo = (long long)tile * windows;
+    const int w_end = (int)min(w_lo + windows, (long long)win_cap);
+    for (int w = (int)w_lo + (int)threadIdx.x; w < w_end; w += BIN_T) {
         int n = 0, it = 0;
+        signed char c = -1;
         if (w < nwin) {
             const int row = win[w].row;
             if ((unsigned)row >= (unsigned)M) {  // a window left unwritten after a reported error
                 set_err(&ctl->err, DERR_INTERNAL);
                 len[w] = 0;
                 items[w] = 0;
+                cls[w] = -1;
                 continue;
             }
             n = arp[row + 1] - arp[row];
-            if (n >= HEAVY_ROW) heavy[atomicAdd(&ctl->win_heavy, 1)] = w;
-            else if (n >= LONG_ROW) heavy[win_cap - 1 - atomicAdd(&ctl->win_long, 1)] = w;
+            c = n >= HEAVY_ROW ? 0 : n >= LONG_ROW ? 1 : -1;
             // a chunk of the cursor pass starts here: one work item per 32 A entries
             if (!cur_continues(win, w, row, win[w].t0)) it = (n + WARP - 1) / WARP;
             if (win[w].cnt == 0) {
@@ -125,6 +135,14 @@ __global__ void __launch_bounds__(256) k_win_len(Window *__restrict__ win, int w
         }
         len[w] = n;
         items[w] = it;
+        cls[w] = c;
+    }
+    __syncthreads();
+    bin_tile<2>(cls, tile, windows, win_cap, ntiles, lb, ctl, S,
+                [&](int b, int at, int w) { heavy[b == 0 ? at : win_cap - 1 - at] = w; });
+    if (tile == ntiles - 1 && threadIdx.x == 0) {
+        ctl->win_heavy = S.cnt[0];
+        ctl->win_long = S.cnt[1];
     }
 }
 
@@ -473,9 +491,12 @@ void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const 
                     const long long *soff, const WinCursors &wc, Ctl *ctl, int arith, int nsm, cudaStream_t st,
                     ScanState &scan, int wait_polls, const TileStore *ts) {
     if (win_cap <= 0) return;
-    cudaMemsetAsync(&ctl->win_next, 0, 3 * sizeof(int), st);  // and win_heavy, win_long
-    k_win_len<<<nsm * 4, 256, 0, st>>>(const_cast<Window *>(win), (int)win_cap, A.M, A.rp, crp, ts ? ts->off : nullptr,
-                                       ts ? ts->cnt : nullptr, ctl, wc.len, wc.item_off, wc.heavy);
+    cudaMemsetAsync(&ctl->win_next, 0, sizeof(int), st);
+    int chunks;
+    const int ntiles = lb_tiles(win_cap, BIN_ROWS, chunks);
+    k_win_len<<<ntiles, BIN_T, 0, st>>>(const_cast<Window *>(win), (int)win_cap, A.M, A.rp, crp, ts ? ts->off : nullptr,
+                                        ts ? ts->cnt : nullptr, ctl, wc.len, wc.item_off, wc.cls, wc.heavy,
+                                        chunks * BIN_ROWS, ntiles, next_epoch(scan, st));
     launch_scan64(wc.len, wc.off, (int)win_cap, wc.total, scan, ctl, st);
     launch_scan(wc.item_off, wc.item_off, (int)win_cap, wc.total + 1, scan, ctl, st);
     k_win_cursors<<<nsm * 16, 256, 0, st>>>(win, (int)win_cap, A.M, wc.off, wc.cap, A.rp, A.col, B.rp, Bt.ptr, Bt.col,
