@@ -1290,7 +1290,7 @@ int row_nnz_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, int32_t
     CK(salloc(h, &ri.bins, (size_t)M * NBIN, st));
     CK(salloc(h, &ri.cls, (size_t)M, st));
     ri.cnnz = nnz_out;
-    launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), h->scan, st);
+    launch_bounds(Ad, Bd, ri, ctl, grid_rows(h), h->scan, st, true);
     launch_count(Ad, Bd, Btd, ri, ctl, h->nsm, st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(h->h_ctl, ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));

@@ -22,13 +22,23 @@ constexpr unsigned FULL = 0xffffffffu;
 // A C row whose tile span is at most SPAN_T tiles is handled by one warp
 // with a dense per-tile table in shared memory (symbolic / structure).
 constexpr int SPAN_T = 512;
-// ... unless it has more products than this: then a CTA takes it (BIN_L), with a tile list.  One warp
-// took 1 ms over a hub row of a power-law graph within 512 tiles, in the count pass and again in the
-// structure pass: A*A^T of 30,011 vertices 4.18 ms without the limit, 2.44 at 32,768 products, 2.37 at
-// 24,576, 2.29 at 16,384, 2.25 at 12,288.  The line is kept where the learned scheduler still has its
-// saving, the warp class's count pass (R-MAT scale 15: 2.13 ms against 2.18 at 24,576; at 16,384 the
-// two are within 1.3 %).
-constexpr long long DS_PROD = 24576;
+// ... unless it stands out by the tiles of B that it reads (counted per A entry as the smaller of the B
+// row's entries and the tiles from its first to its last column) or by its products: then a CTA takes it
+// (BIN_L), with a tile list.  One warp took 1 ms over a hub row of a power-law graph within 512 tiles, in
+// the count pass and again in the structure pass.  A row stands out when it has more than DS_TILES and more
+// than an average warp's share of the pass (launch_bounds), for the products DS_PROD and that share.
+//
+// DS_TILES: A*A^T of 30,011 vertices 4.18 ms without a line, 2.33 at 16,384, 2.24 at 14,336, 2.17 at 12,288;
+// R-MAT scale 15 plain 2.23, 2.19 and 2.09, by the learned scheduler 2.13, 2.10 and 2.06.  It is kept where
+// that still has its saving, the warp class's count pass.
+// The share: rows alike leave no tail, and a CTA per row costs more than it gives.  27-point stencils of
+// 30^3 nodes x 6 rows 17.8 ms (19.9 with a line of 24,576 products in place of all this), 20^3 x 6 5.15
+// (5.64), 16^3 x 7 4.13 (4.85); bands of 201 entries 3.85 (4.41), their count alone 0.23 (0.57); rows of 200
+// random entries within 16,000 columns lose by it: 12.0 (10.7).
+// DS_PROD: rows of many products in few tiles (a band of 401 entries: 160,801 products, 2,900 tiles) are no
+// more work for the count, 0.23 ms against 0.49.
+constexpr int DS_TILES = 14336;
+constexpr long long DS_PROD = 196608;
 // Numeric windows: consecutive tiles of one C row with
 //   < WIN_CAP slots (cut where the tile's first slot crosses a multiple of WIN_CUT),
 //   <= WIN_TCAP tiles (cut where the tile's rank in the row crosses a multiple of WIN_TCAP),

@@ -119,7 +119,9 @@ void launch_row_repeat(const DevCSR &B, unsigned char *rep, int *chains, int gri
 void launch_validate(const DevCSR &A, Ctl *ctl, int grid, cudaStream_t st);
 
 // k_rows.cu
-void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, ScanState &scan, cudaStream_t st);
+// counts_only: the call ends with the count pass (lines for its warps, none by products)
+void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, ScanState &scan, cudaStream_t st,
+                   bool counts_only = false);
 // whether rows of many entries are taken in a launch of their own (hsmu_rowsums.cuh): it costs about
 // 3 us where there are none (a 5-point Laplacian of 65,536 rows: 9 + 3 us) and takes 30 us off a
 // power-law graph of 430,000 entries, so small or short-rowed matrices go without

@@ -1,6 +1,6 @@
-// Sums over the B rows that a row of A references: products, longest row,
-// first and last column -- what the bounds pass (k_rows.cu) and the learned
-// scheduler's features (learned.cu) are made of.
+// Sums over the B rows that a row of A references: products, tiles (bounds
+// pass), longest row, first and last column -- what the bounds pass (k_rows.cu)
+// and the learned scheduler's features (learned.cu) are made of.
 //
 // Bound by L2 latency: three dependent gathers per entry.  A group of G lanes
 // takes a row, SUM_U entries per lane in flight; rows of more than SUM_LONG
@@ -18,8 +18,11 @@ constexpr int SUM_THREADS = 256;
 constexpr int SUM_LONG = 256;
 constexpr int SUM_U = 4;
 
+template <bool TILES>
 struct RowSums {
     long long prod;  // sum of the B rows' lengths
+    float tiles;     // TILES: of the smaller of length and tiles from first to last column (for a dividing
+                     // line: single precision will do)
     int longest;     // the longest of them
     int cmin, cmax;  // first and last column (INT_MAX, -1: none)
 
@@ -27,6 +30,7 @@ struct RowSums {
     __device__ __forceinline__ void walk(int first, int len, int stride, const int *__restrict__ acol,
                                          const int *__restrict__ brp, const int *__restrict__ bcol) {
         prod = 0;
+        tiles = 0.f;
         longest = 0;
         cmin = INT_MAX;
         cmax = -1;
@@ -46,8 +50,10 @@ struct RowSums {
                 prod += e[u] - s[u];
                 longest = max(longest, e[u] - s[u]);
                 if (e[u] > s[u]) {
-                    cmin = min(cmin, __ldg(bcol + s[u]));
-                    cmax = max(cmax, __ldg(bcol + e[u] - 1));
+                    const int c0 = __ldg(bcol + s[u]), c1 = __ldg(bcol + e[u] - 1);
+                    cmin = min(cmin, c0);
+                    cmax = max(cmax, c1);
+                    if (TILES) tiles += (float)min(e[u] - s[u], (c1 >> 6) - (c0 >> 6) + 1);
                 }
             }
         }
@@ -59,6 +65,7 @@ struct RowSums {
 #pragma unroll
         for (int d = W / 2; d > 0; d >>= 1) {
             prod += __shfl_xor_sync(FULL, prod, d, W);
+            if (TILES) tiles += __shfl_xor_sync(FULL, tiles, d, W);
             longest = max(longest, __shfl_xor_sync(FULL, longest, d, W));
             cmin = min(cmin, __shfl_xor_sync(FULL, cmin, d, W));
             cmax = max(cmax, __shfl_xor_sync(FULL, cmax, d, W));
@@ -68,32 +75,37 @@ struct RowSums {
 
 struct SumSmem {
     unsigned long long prod;
+    float tiles;
     int longest, cmin, cmax;
 };
 
 // one long row by the whole block (SUM_THREADS threads, all of them call it); valid on every thread
-__device__ __forceinline__ RowSums block_row_sums(int lo, int hi, const int *__restrict__ acol,
+template <bool TILES>
+__device__ __forceinline__ RowSums<TILES> block_row_sums(int lo, int hi, const int *__restrict__ acol,
                                                   const int *__restrict__ brp, const int *__restrict__ bcol,
                                                   SumSmem &S) {
     __syncthreads();  // the previous row's sums have been read
     if (threadIdx.x == 0) {
         S.prod = 0;
+        S.tiles = 0.f;
         S.longest = 0;
         S.cmin = INT_MAX;
         S.cmax = -1;
     }
     __syncthreads();
-    RowSums r;
+    RowSums<TILES> r;
     r.walk((int)threadIdx.x, hi - lo, SUM_THREADS, acol + lo, brp, bcol);
-    r.reduce<WARP>();
+    r.template reduce<WARP>();
     if (lane_id() == 0) {
         atomicAdd(&S.prod, (unsigned long long)r.prod);
+        if (TILES) atomicAdd(&S.tiles, r.tiles);
         atomicMax(&S.longest, r.longest);
         atomicMin(&S.cmin, r.cmin);
         atomicMax(&S.cmax, r.cmax);
     }
     __syncthreads();
     r.prod = (long long)S.prod;
+    r.tiles = S.tiles;
     r.longest = S.longest;
     r.cmin = S.cmin;
     r.cmax = S.cmax;

@@ -26,6 +26,12 @@
 
 namespace hsmu {
 
+// the most tiles and products of a warp row
+struct ClassLine {
+    float tiles;
+    long long products;
+};
+
 // What a block adds up over its rows for the control block: one thread per sum sends it there.
 enum BoundsSum { BS_PROD, BS_WB, BS_CB, BS_CBD, BS_WDP, BS_SPAN, BS_BIN, BS_N = BS_BIN + NBIN };
 struct BoundsSmem {
@@ -38,7 +44,8 @@ struct BoundsSums {
     int cnt[NBIN] = {};
 
     // one row's products, tile span and class
-    __device__ __forceinline__ void row(int i, int len, const RowSums &sums, int N, const RowInfo &ri) {
+    __device__ __forceinline__ void row(int i, int len, const RowSums<true> &sums, int N, const RowInfo &ri,
+                                        ClassLine line) {
         const long long prod = sums.prod;
         const int tmin = sums.cmin == INT_MAX ? INT_MAX : sums.cmin >> 6, tmax = sums.cmax >> 6;
         ri.prod[i] = prod;
@@ -50,7 +57,8 @@ struct BoundsSums {
         } else {
             const int span = tmax - tmin + 1;
             const bool scattered = prod <= H_MAX && span <= H_SPAN && len <= H_ROW;
-            bin = prod <= TINY_MAX ? BIN_TINY : span <= SPAN_T && prod <= DS_PROD ? BIN_DS : scattered ? BIN_H : BIN_L;
+            const bool narrow = span <= SPAN_T && sums.tiles <= line.tiles && prod <= line.products;
+            bin = prod <= TINY_MAX ? BIN_TINY : narrow ? BIN_DS : scattered ? BIN_H : BIN_L;
             t_prod += (unsigned long long)prod;
             const long long cap = prod < (long long)N ? prod : (long long)N;
             // windows per row <= slot cuts + tile-rank cuts + span cuts + 1
@@ -110,7 +118,7 @@ template <int G>
 __global__ void __launch_bounds__(SUM_THREADS) k_bounds(int M, const int *__restrict__ arp,
                                                         const int *__restrict__ acol, const int *__restrict__ brp,
                                                         const int *__restrict__ bcol, int N, RowInfo ri,
-                                                        int *__restrict__ long_list, Ctl *ctl) {
+                                                        int *__restrict__ long_list, ClassLine line, Ctl *ctl) {
     constexpr int RPB = SUM_THREADS / G;  // rows per block iteration
     __shared__ BoundsSmem s_tot;
     const int sub = threadIdx.x & (G - 1);
@@ -119,12 +127,12 @@ __global__ void __launch_bounds__(SUM_THREADS) k_bounds(int M, const int *__rest
         const int i = rb + (int)threadIdx.x / G;
         const int lo = i < M ? arp[i] : 0, hi = i < M ? arp[i + 1] : 0;
         const bool listed = long_list && hi - lo > SUM_LONG;
-        RowSums r;
+        RowSums<true> r;
         r.walk(sub, listed ? 0 : hi - lo, G, acol + lo, brp, bcol);
-        r.reduce<G>();
+        r.template reduce<G>();
         if (i < M && sub == 0) {
             if (listed) long_list[atomicAdd(&ctl->long_rows, 1)] = i;
-            else mine.row(i, hi - lo, r, N, ri);
+            else mine.row(i, hi - lo, r, N, ri, line);
         }
     }
     mine.flush(s_tot, ctl);
@@ -133,7 +141,7 @@ __global__ void __launch_bounds__(SUM_THREADS) k_bounds(int M, const int *__rest
 __global__ void __launch_bounds__(SUM_THREADS) k_bounds_long(const int *__restrict__ arp, const int *__restrict__ acol,
                                                              const int *__restrict__ brp, const int *__restrict__ bcol,
                                                              int N, RowInfo ri, const int *__restrict__ long_list,
-                                                             Ctl *ctl) {
+                                                             ClassLine line, Ctl *ctl) {
     __shared__ SumSmem s_sum;
     __shared__ BoundsSmem s_tot;
     BoundsSums mine;
@@ -141,8 +149,8 @@ __global__ void __launch_bounds__(SUM_THREADS) k_bounds_long(const int *__restri
     for (int e = blockIdx.x; e < n; e += gridDim.x) {
         const int i = long_list[e];
         const int lo = arp[i], hi = arp[i + 1];
-        const RowSums r = block_row_sums(lo, hi, acol, brp, bcol, s_sum);
-        if (threadIdx.x == 0) mine.row(i, hi - lo, r, N, ri);
+        const RowSums<true> r = block_row_sums<true>(lo, hi, acol, brp, bcol, s_sum);
+        if (threadIdx.x == 0) mine.row(i, hi - lo, r, N, ri, line);
     }
     mine.flush(s_tot, ctl);
 }
@@ -281,15 +289,20 @@ static void launch_bins(int M, const RowInfo &ri, ScanState &scan, Ctl *ctl, cud
     k_bins<<<nt, BIN_T, 0, st>>>(M, ri.cls, chunks * BIN_ROWS, nt, ri.bins, next_epoch(scan, st), ctl);
 }
 
-void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, ScanState &scan, cudaStream_t st) {
+void launch_bounds(const DevCSR &A, const DevCSR &B, RowInfo ri, Ctl *ctl, int grid, ScanState &scan, cudaStream_t st,
+                   bool counts_only) {
+    // an average warp's share of the products, by the averages of A's and B's rows: 24 warps per SM in the
+    // fused row kernel, 48 in the count pass
+    const float share = B.M ? (float)((double)A.nnz * (double)B.nnz / B.M / (grid * (counts_only ? 6.0 : 3.0))) : 0.f;
+    const ClassLine line{fmaxf((float)DS_TILES, share), counts_only ? LLONG_MAX : max(DS_PROD, (long long)share)};
     const double avg = A.M ? (double)A.nnz / A.M : 0.0;
     // the bins are written after this pass: until then their space holds the long rows
     int *list = long_rows_apart(A) ? ri.bins : nullptr;
     const int lanes = avg <= 6 ? 4 : avg <= 12 ? 8 : avg <= 24 ? 16 : 32;
     auto k = avg <= 6 ? k_bounds<4> : avg <= 12 ? k_bounds<8> : avg <= 24 ? k_bounds<16> : k_bounds<32>;
     k<<<grid_for(grid, A.M, SUM_THREADS / lanes), SUM_THREADS, 0, st>>>(A.M, A.rp, A.col, B.rp, B.col, B.N, ri, list,
-                                                                        ctl);
-    if (list) k_bounds_long<<<grid / 2, SUM_THREADS, 0, st>>>(A.rp, A.col, B.rp, B.col, B.N, ri, list, ctl);
+                                                                        line, ctl);
+    if (list) k_bounds_long<<<grid / 2, SUM_THREADS, 0, st>>>(A.rp, A.col, B.rp, B.col, B.N, ri, list, line, ctl);
     launch_bins(A.M, ri, scan, ctl, st);
 }
 

@@ -8,7 +8,7 @@
 // the row's C tiles are ORed into a dense per-tile table indexed by
 // (tile id - first tile of the row), which needs no hashing or probing
 // because the bounds kernel already knows the row's exact tile span.
-//   BIN_DS rows (span <= SPAN_T, at most DS_PROD products): one warp per row,
+//   BIN_DS rows (span <= SPAN_T, without the rows that stand out): one warp per row,
 //                4 KB table per warp.
 //   BIN_L  rows: one CTA per row, the span processed in chunks of DCH_COUNT
 //                tiles (32 KB); B tile ranges restricted per chunk by binary

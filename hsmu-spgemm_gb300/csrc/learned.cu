@@ -48,7 +48,7 @@ constexpr int OFF_MU = MLP_NPARAM, OFF_SD = OFF_MU + NF, OFF_YMU = OFF_SD + NF, 
 static_assert(MLP_NTOTAL == HSMU_MLP_FLOATS, "parameter layout and the C ABI disagree");
 
 // ---------------------------------------------------------------- features
-__device__ __forceinline__ void store_features(int i, int len, const RowSums &r, float4 *__restrict__ feat,
+__device__ __forceinline__ void store_features(int i, int len, const RowSums<false> &r, float4 *__restrict__ feat,
                                                long long *__restrict__ prod_out) {
     const float span = r.cmax >= r.cmin ? (float)(r.cmax - r.cmin) : 0.f;
     feat[i] = make_float4(log2f(1.f + (float)len), log2f(1.f + (float)r.prod), log2f(1.f + (float)r.longest),
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(SUM_THREADS) k_features(int M, const int *__re
         const int i = rb + (int)threadIdx.x / G, sub = threadIdx.x & (G - 1);
         const int lo = i < M ? arp[i] : 0, hi = i < M ? arp[i + 1] : 0;
         const bool listed = long_list && hi - lo > SUM_LONG;
-        RowSums r;
+        RowSums<false> r;
         r.walk(sub, listed ? 0 : hi - lo, G, acol + lo, brp, bcol);
         r.reduce<G>();
         if (i < M && sub == 0) {
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(SUM_THREADS) k_features_long(const int *__rest
     for (int e = blockIdx.x; e < n; e += gridDim.x) {
         const int i = long_list[1 + e];
         const int lo = arp[i], hi = arp[i + 1];
-        const RowSums r = block_row_sums(lo, hi, acol, brp, bcol, s_sum);
+        const RowSums<false> r = block_row_sums<false>(lo, hi, acol, brp, bcol, s_sum);
         if (threadIdx.x == 0) store_features(i, hi - lo, r, feat, prod_out);
     }
 }
