@@ -640,6 +640,12 @@ struct PlainRun {
         return x;
     }
 
+    // The warp class's kernel has a block for every slot of the device, with a fixed share of the rows each:
+    // where light rows' blocks hold slots when it starts, its last blocks start late and are its tail
+    // (400,000 one-entry rows over rows of 30 to 60 entries: 1.44 ms behind 30,000 tiny rows, 0.86 ahead of
+    // them).  With fewer rows than two rounds of its warps that is no matter, and the light rows go first.
+    bool warp_rows_first(int rows) const { return rows >= h->nsm * 48; }
+
     // sorted columns of rows lo..hi-1, values of warp-sized rows, numeric windows of the others
     int structure(int lo, int hi) {
         if (hc.nnz == 0) return HSMU_OK;
@@ -653,15 +659,18 @@ struct PlainRun {
         // tiny and scattered rows beside the warp and large classes, or beside each other
         const bool heavy = rows[BIN_DS] > 0 || rows[BIN_L] > 0;
         const bool apart = rows[BIN_TINY] > 0 ? heavy || rows[BIN_H] > 0 : heavy && rows[BIN_H] > 0;
+        const bool light_first = !warp_rows_first(rows[BIN_DS]);
+        int side[NBIN] = {0, 0, rows[BIN_TINY], heavy ? rows[BIN_H] : 0};
         if (apart) {
             CKQ(fork());
-            int side[NBIN] = {0, 0, rows[BIN_TINY], heavy ? rows[BIN_H] : 0};
-            launch_structure_light(Ad, Bd, ri, out, ctl, o.arith, h->nsm, h->cs_tiles, side);
+            if (light_first) launch_structure_light(Ad, Bd, ri, out, ctl, o.arith, h->nsm, h->cs_tiles, side);
             rows[BIN_TINY] = 0;
             if (heavy) rows[BIN_H] = 0;
         }
         launch_structure(Ad, Bd, Btd, chains(hc), out, win, win_cap, ctl, o.arith, h->nsm, st, rows,
                          have_store ? &tsd : nullptr);
+        if (apart && !light_first)
+            launch_structure_light(Ad, Bd, ri, out, ctl, o.arith, h->nsm, h->cs_tiles, side);
         return apart ? join() : HSMU_OK;
     }
 
@@ -1180,8 +1189,11 @@ learned:
             rc = r.fork();
             if (rc) goto done;
         }
-        launch_structure_light(Ad, Bd, ri, spec, ctl, o.arith, h->nsm, apart ? h->cs_tiles : st, light_rows);
+        const bool light_first = !apart || !r.warp_rows_first(hc.bin_count[BIN_DS]);
+        if (light_first)
+            launch_structure_light(Ad, Bd, ri, spec, ctl, o.arith, h->nsm, apart ? h->cs_tiles : st, light_rows);
         launch_structure(Ad, Bd, Btd, ri, spec, win, win_cap, ctl, o.arith, h->nsm, st, warp_rows);
+        if (!light_first) launch_structure_light(Ad, Bd, ri, spec, ctl, o.arith, h->nsm, h->cs_tiles, light_rows);
         if (hc.bin_count[BIN_L] > 0)
             launch_structure(Ad, Bd, Btd, ri, spec, win, win_cap, ctl, o.arith, h->nsm, st, large_rows,
                              r.have_store ? &tsd : nullptr);
