@@ -496,19 +496,28 @@ __global__ void __launch_bounds__(TINYF_THREADS, 4) k_fill_tiny(int M, const int
         int i = r < b1 ? rows[r] : -1;
         if (i >= 0 && skip_row(out, i)) i = -1;
         long long c0 = 0;
-        int lim = 0, np = 0;
+        int lim = 0, np = 0, a_lo = 0, a_hi = 0;
         if (i >= 0) {
             c0 = out_base(out, i);
             lim = out_limit(out, i);
-            np = tiny_list<true>(arp[i], arp[i + 1], acol, aval, brp, S.q, S.t);
+            a_lo = arp[i];
+            a_hi = arp[i + 1];
         }
         int got = 0;
+        const bool copies = __all_sync(FULL, a_hi - a_lo <= 1);
+        if (!copies) np = tiny_list<true>(a_lo, a_hi, acol, aval, brp, S.q, S.t);
         if (np > TINY_MAX) {  // a row of another class
             got = -1;
             np = 0;
         }
         const int most = __reduce_max_sync(FULL, np);
-        if (most > 16) np = tiny_list_fill<AR, 32>(np, bcol, bval, S, lim, out.ccol + c0, out.cval + c0);
+        if (copies) {
+            if (a_lo < a_hi) {
+                const int k = __ldg(acol + a_lo);
+                np = tiny_copy_fill<AR>(__ldg(brp + k), __ldg(brp + k + 1), __ldg(aval + a_lo), bcol, bval, lim,
+                                        out.ccol + c0, out.cval + c0);
+            }
+        } else if (most > 16) np = tiny_list_fill<AR, 32>(np, bcol, bval, S, lim, out.ccol + c0, out.cval + c0);
         else if (most > 8) np = tiny_list_fill<AR, 16>(np, bcol, bval, S, lim, out.ccol + c0, out.cval + c0);
         else np = tiny_list_fill<AR, 8>(np, bcol, bval, S, lim, out.ccol + c0, out.cval + c0);
         got = got < 0 || np > lim ? -1 : np;

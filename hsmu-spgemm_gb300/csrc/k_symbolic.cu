@@ -249,7 +249,14 @@ __global__ void __launch_bounds__(TINY_THREADS) k_count_tiny(int M, const int *_
     for (int r0 = blockIdx.x * TINY_THREADS + (threadIdx.x & ~31); r0 < n; r0 += gridDim.x * TINY_THREADS) {
         const int r = r0 + lane_id();
         const int i = r < n ? rows[r] : -1;
-        const int np = i >= 0 ? tiny_list<false>(arp[i], arp[i + 1], acol, nullptr, brp, qs, nullptr) : 0;
+        const int a_lo = i >= 0 ? arp[i] : 0, a_hi = i >= 0 ? arp[i + 1] : 0;
+        if (__all_sync(FULL, a_hi - a_lo <= 1)) {  // one entry of A each: its B row
+            if (i < 0) continue;
+            const int k = a_lo < a_hi ? __ldg(acol + a_lo) : -1;
+            ri.cnnz[i] = k >= 0 ? __ldg(brp + k + 1) - __ldg(brp + k) : 0;
+            continue;
+        }
+        const int np = tiny_list<false>(a_lo, a_hi, acol, nullptr, brp, qs, nullptr);
         const int most = __reduce_max_sync(FULL, np);
         int c;
         if (most > TINY_MAX) {  // a row of another class
