@@ -52,15 +52,19 @@ using namespace hsmu;
 // Scratch of a handle's calls: one block, handed out from its start and taken back when the
 // call ends (every call waits for its work before it returns, so nothing still reads it then,
 // whatever stream the next call uses).  What does not fit comes from a memory pool of the
-// handle's own, and the block then grows to the call's need, up to SCRATCH_BLOCK_MAX.  C's arrays
-// stay in the device's default pool: with the scratch carved from the block a freed C had left
-// there, the pool re-mapped memory for every second C (1 ms for 2 GB, 7 ms for 15 GB).
+// handle's own, and the next call then starts with a block of what this one needed, up to
+// SCRATCH_BLOCK_MAX.  C's arrays stay in the device's default pool: with the scratch carved from
+// the block a freed C had left there, the pool re-mapped memory for every second C (1 ms for 2 GB,
+// 7 ms for 15 GB).  A handle's first call takes its scratch from the default pool too, and the
+// handle's pool is made by the second: programs that make a handle for one product do not pay for
+// what only further calls use (handle, product of a 64^2 Laplacian and release: 475 us, 195 so).
 struct Scratch {
     char *base = nullptr;
     size_t cap = 0, used = 0;    // the block
     size_t need = 0, peak = 0;   // bytes handed out, in the block or not; the most in a call
+    size_t want = 0;             // the most that a call needed
     int depth = 0;               // nested scopes
-    cudaMemPool_t pool = nullptr;
+    cudaMemPool_t pool = nullptr;  // null: the device's default pool
     std::vector<void *> extra;   // allocations outside the block
 };
 
@@ -83,6 +87,7 @@ struct hsmu_handle_s {
     size_t h_prod_cap;
     // look-back state of the scans on the caller's stream, and of those on cs_tiles
     ScanState scan, scan_tiles;
+    bool scan_kept;  // beyond the call (else they are scratch)
     // side stream: B's tile conversion beside the bounds pass, light row classes beside the others
     cudaStream_t cs_tiles;
     cudaEvent_t ev_side_start, ev_side_done;
@@ -217,7 +222,7 @@ cudaError_t salloc(hsmu_handle_s *h, T **p, size_t n, cudaStream_t st) {
         s.used += bytes;
     } else {
         void *q = nullptr;
-        const cudaError_t e = cudaMallocFromPoolAsync(&q, bytes, s.pool, st);
+        const cudaError_t e = s.pool ? cudaMallocFromPoolAsync(&q, bytes, s.pool, st) : cudaMallocAsync(&q, bytes, st);
         if (e != cudaSuccess) {
             (void)cudaGetLastError();
             return e;
@@ -235,15 +240,47 @@ cudaError_t salloc(hsmu_handle_s *h, T **p, size_t n, cudaStream_t st) {
     return cudaSuccess;
 }
 
-// gives back, at its end, what was taken since its start; the outermost one (a public call's)
-// then sizes the block for what the call needed.  `st` has finished every use by then.
+// the handle's pool and a block of what its calls have needed (for the call on `st` that starts, and,
+// as every call is waited for, for later ones on any stream); without the memory for it calls do as before
+void grow_block(hsmu_handle_s *h, cudaStream_t st) {
+    Scratch &s = h->scratch;
+    if (!s.pool) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = h->device;
+        unsigned long long keep = SCRATCH_POOL_KEEP;
+        if (cudaMemPoolCreate(&s.pool, &props) != cudaSuccess) {
+            (void)cudaGetLastError();
+            s.pool = nullptr;
+            return;
+        }
+        cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    if (s.base) cudaFreeAsync(s.base, st);
+    s.base = nullptr;
+    s.cap = 0;
+    const size_t size = std::min(SCRATCH_BLOCK_MAX, s.want + s.want / 4 + (1 << 20));
+    void *q = nullptr;
+    if (cudaMallocFromPoolAsync(&q, size, s.pool, st) == cudaSuccess) {
+        s.base = static_cast<char *>(q);
+        s.cap = size;
+    } else {
+        (void)cudaGetLastError();
+    }
+}
+
+// gives back, at its end, what was taken since its start.  `st` has finished every use by then.
 struct ScratchScope {
     hsmu_handle_s *h;
     cudaStream_t st;
     size_t used, need, extra;
     ScratchScope(hsmu_handle_s *h_, cudaStream_t st_)
         : h(h_), st(st_), used(h_->scratch.used), need(h_->scratch.need), extra(h_->scratch.extra.size()) {
-        if (h->scratch.depth++ == 0) h->scratch.peak = 0;
+        Scratch &s = h->scratch;
+        if (s.depth++ > 0) return;
+        s.peak = 0;  // a public call's scope
+        if (s.want > s.cap && s.cap < SCRATCH_BLOCK_MAX) grow_block(h, st);
     }
     ScratchScope(const ScratchScope &) = delete;
     ~ScratchScope() {
@@ -254,26 +291,37 @@ struct ScratchScope {
         }
         s.used = used;
         s.need = need;
-        if (--s.depth > 0 || s.peak <= s.cap || s.cap >= SCRATCH_BLOCK_MAX) return;
-        if (s.base) cudaFreeAsync(s.base, st);
-        s.base = nullptr;
-        s.cap = 0;
-        const size_t want = std::min(SCRATCH_BLOCK_MAX, s.peak + s.peak / 4 + (1 << 20));
-        void *q = nullptr;
-        // the block must be there for a later call on any stream
-        if (cudaMallocFromPoolAsync(&q, want, s.pool, st) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess) {
-            s.base = static_cast<char *>(q);
-            s.cap = want;
-        } else {
-            (void)cudaGetLastError();
-        }
+        if (--s.depth > 0) return;
+        s.want = std::max(s.want, s.peak);
+        if (!h->scan_kept) h->scan.word = h->scan_tiles.word = nullptr;
     }
 };
 
 int grid_rows(const hsmu_handle_s *h) { return h->nsm * 8; }
 
-// limit of the call's look-backs (hsmu_opts.scan_polls; 0: the default)
-void set_scan_polls(hsmu_handle_s *h, int polls) { h->scan.polls = h->scan_tiles.polls = polls; }
+// Before a call's first scan: the limit of its look-backs (hsmu_opts.scan_polls; 0: the default), and the
+// scan states, cleared on `st` (the side stream's scans come after an event of `st`): the call's own
+// scratch on the handle's first call, kept from the second on.
+cudaError_t prepare_scans(hsmu_handle_s *h, int polls, cudaStream_t st) {
+    const size_t bytes = 2 * scan_state_bytes();
+    h->scan.polls = h->scan_tiles.polls = polls;
+    if (h->scan.word) return cudaSuccess;
+    char *w = nullptr;
+    void *kept = nullptr;
+    if (h->scratch.pool && cudaMallocFromPoolAsync(&kept, bytes, h->scratch.pool, st) == cudaSuccess)
+        w = static_cast<char *>(kept);
+    cudaError_t e = w ? cudaSuccess : salloc(h, &w, bytes, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(w, 0, bytes, st);
+    if (e != cudaSuccess) {
+        if (kept) cudaFreeAsync(kept, st);
+        (void)cudaGetLastError();
+        return e;
+    }
+    h->scan.word = w;
+    h->scan_tiles.word = w + scan_state_bytes();
+    h->scan_kept = kept != nullptr;
+    return cudaSuccess;
+}
 
 // arrays the library allocated from the stream-ordered pool and handed to the caller:
 // returned to the pool once every stream of the device is done with them (the free
@@ -407,7 +455,7 @@ struct PlainRun {
         M = A->M;
         Ad = dev(A);
         Bd = dev(B);
-        set_scan_polls(h, o.scan_polls);
+        CKR(prepare_scans(h, o.scan_polls, st));
         CKR(salloc(h, &ctl, 1, st));
         CKR(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
         if (o.validate) {
@@ -1290,7 +1338,7 @@ int row_nnz_impl(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, int32_t
     DevCSR Ad = dev(A), Bd = dev(B);
     DevTiles Btd{};
     ScratchScope scope(h, st);
-    set_scan_polls(h, 0);
+    CK(prepare_scans(h, 0, st));
     CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     rc = build_tiles(h, B, &bt, ctl, 0, st, false, false);
@@ -1393,6 +1441,7 @@ int spgemm64_panels(hsmu_handle_s *h, const hsmu_csr *A, const hsmu_csr *B, cons
     hsmu_btiles bt{};
     Ctl *ctl = nullptr;
     ScratchScope scope(h, st);
+    CKR(prepare_scans(h, o.scan_polls, st));
     CKR(salloc(h, &ctl, 1, st));
     CKR(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     CKQ(build_tiles(h, B, &bt, ctl, 0, st, true, false));
@@ -1493,30 +1542,6 @@ int hsmu_handle_create(hsmu_handle *out) {
         hsmu_handle_destroy(h);
         return HSMU_ERR_CUDA;
     }
-    {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        unsigned long long keep = SCRATCH_POOL_KEEP;
-        if (cudaMemPoolCreate(&h->scratch.pool, &props) != cudaSuccess ||
-            cudaMemPoolSetAttribute(h->scratch.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            hsmu_handle_destroy(h);
-            return HSMU_ERR_CUDA;
-        }
-    }
-    // cleared before the handle is given out: the scans run on streams that do not wait for the
-    // default one, where a clear may be queued behind the caller's work
-    for (ScanState *s : {&h->scan, &h->scan_tiles})
-        if (cudaMalloc(&s->word, scan_state_bytes()) != cudaSuccess ||
-            cudaMemsetAsync(s->word, 0, scan_state_bytes(), h->cs_tiles) != cudaSuccess) {
-            hsmu_handle_destroy(h);
-            return HSMU_ERR_ALLOC;
-        }
-    if (cudaStreamSynchronize(h->cs_tiles) != cudaSuccess) {
-        hsmu_handle_destroy(h);
-        return HSMU_ERR_CUDA;
-    }
     // keep freed pool memory cached between calls (no re-mapping of large outputs)
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
@@ -1549,12 +1574,9 @@ int hsmu_handle_destroy(hsmu_handle h) {
     }
     for (cudaStream_t s : {h->cs_in, h->cs_out, h->cs_tiles})
         if (s) cudaStreamDestroy(s);
-    if (h->scratch.base) {
-        cudaFreeAsync(h->scratch.base, 0);  // every call of the handle has finished
-        cudaStreamSynchronize(0);
-    }
-    for (const ScanState *s : {&h->scan, &h->scan_tiles})
-        if (s->word) cudaFree(s->word);
+    for (void *p : {(void *)h->scratch.base, h->scan.word})  // one allocation holds both scan states
+        if (p) cudaFreeAsync(p, 0);  // every call of the handle has finished
+    if (h->scratch.pool) cudaStreamSynchronize(0);
     if (h->scratch.pool) cudaMemPoolDestroy(h->scratch.pool);
     if (h->h_ctl) cudaFreeHost(h->h_ctl);
     if (h->h_prod) cudaFreeHost(h->h_prod);
@@ -1607,7 +1629,7 @@ int hsmu_btiles_build(hsmu_handle h, const hsmu_csr *B, hsmu_btiles *out, void *
     Ctl hc{};
     std::memset(out, 0, sizeof(*out));
     ScratchScope scope(h, st);
-    set_scan_polls(h, 0);
+    CK(prepare_scans(h, 0, st));
     CK(salloc(h, &ctl, 1, st));
     CK(cudaMemsetAsync(ctl, 0, sizeof(Ctl), st));
     launch_validate(dev(B), ctl, grid_rows(h), st);
@@ -1652,7 +1674,7 @@ int hsmu_csr_transpose(hsmu_handle h, const hsmu_csr *A, hsmu_csr *At, void *str
     long long *tot = nullptr;
     Ctl *ctl = nullptr;
     ScratchScope scope(h, st);
-    set_scan_polls(h, 0);
+    CK(prepare_scans(h, 0, st));
     CK(palloc(&trp, (size_t)A->N + 1, st));
     CK(palloc(&tcol, (size_t)n, st));
     CK(palloc(&tval, (size_t)n, st));

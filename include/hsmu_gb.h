@@ -145,7 +145,14 @@ const char *hsmu_strerror(int status);
 int hsmu_abi_version(void);
 
 /* Library context for the current device: scratch pool, events, cached
- * device properties.  One handle per host thread (not reentrant). */
+ * device properties.  One handle per host thread (not reentrant).
+ * Device memory that a handle holds between calls, until it is destroyed
+ * (each handle its own): from its second call on, a scratch block of what its
+ * calls have needed, at most 1 GB, and a pool that keeps at most 8 GB of freed
+ * scratch beyond it; and the tile lists of the widest product so far, at most
+ * 16 GB.  The device's default pool, where outputs come from, keeps what is
+ * freed.  The driver takes back what a pool merely keeps when another
+ * allocation needs it. */
 int hsmu_handle_create(hsmu_handle *out);
 int hsmu_handle_destroy(hsmu_handle h);
 
