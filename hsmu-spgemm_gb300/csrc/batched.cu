@@ -518,7 +518,7 @@ struct ShortSmem {
 };
 static_assert(sizeof(ShortSmem) <= sizeof(BWarpSmem), "short tiles use the warp's shared memory");
 
-// One tile, a row per lane; as select_tile, but each lane writes its own row (take gives the pointers of
+// One tile, a row per lane; as in k_batch_select, but each lane writes its own row (take gives the pointers of
 // the tile's block).
 template <int AR, bool NC, class Take>
 __device__ __forceinline__ int short_tile(int a_lo, int a_hi, const BOp &A, const BOp &B, ShortSmem &S, Take take) {
@@ -622,7 +622,8 @@ __device__ void phase_tiles(const BParams &P, int r, BWarpSmem &S) {
             oc = fits ? R.col_pool + base + (off - before) : nullptr;
             ov = R.val_pool + base + (off - before);
         };
-        if (P.tiny >= SHORT_P && p != no_short && B.N <= SHORT_COLS) {
+        // (rows of one entry of A are in order as they are: the lists append them)
+        if (P.tiny >= SHORT_P && p != no_short && B.N <= SHORT_COLS && !__all_sync(FULL, a_hi - a_lo <= 1)) {
             if (short_tile<AR, NC>(a_lo, a_hi, A, B, reinterpret_cast<ShortSmem &>(S), take) >= 0) continue;
             no_short = p;
         }
