@@ -1,5 +1,5 @@
 """Which tiles of a batch take which way: rows of one entry keep the insertion lists (a row of B is in order
-already)."""
+already), and the selecting tiles' launch is left out where too few tiles could be selecting ones."""
 import numpy as np
 import pytest
 
@@ -49,6 +49,31 @@ def test_rows_of_one_entry(engine, arith):
     batch = batch_of(engine, prods, arith=arith)
     batch.execute()
     check(batch, prods, arith)
+    batch.close()
+
+
+def kernels_of(fn):
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    for _ in range(2):  # the process's first session may see no kernels
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            fn()
+            torch.cuda.synchronize()
+    return [e.name for e in prof.events() if "k_batch" in e.name]
+
+
+# 5,000 rows, 157 tiles; rows of nine entries (not selecting): none, as many as half of the tiles, one more
+@pytest.mark.parametrize("nine,selects", [(0, True), (78, True), (79, False), (2500, False)])
+def test_selecting_launch(engine, nine, selects):
+    lens = np.full(5000, 6)
+    lens[np.random.default_rng(3).choice(5000, nine, replace=False)] = 9
+    prods = [(rows_of(lens, 700, 6), rows_of(np.ones(700), 200, 7))]
+    batch = batch_of(engine, prods)
+    names = kernels_of(batch.execute)
+    check(batch, prods, 0)
+    assert any("k_batch_select" in n for n in names) == selects, names
+    assert len(names) == 1 + selects, names
     batch.close()
 
 
