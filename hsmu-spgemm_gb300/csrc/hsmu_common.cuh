@@ -135,11 +135,15 @@ struct Ctl {
 __device__ __forceinline__ bool tiles_read(const Ctl *ctl) { return ctl->bin_count[BIN_DS] || ctl->bin_count[BIN_L]; }
 
 // A scan of the call has given up (or another wait): the bins, pointers and positions that it should
-// have written are not all there.  Kernels that index by them return at once (every thread of a
-// block asks first, and all get the same answer); the host reports the error at its next read of the
-// control block.
+// have written are not all there.  Kernels that index by them take no row then, and the host reports the
+// error at its next read of the control block.  The bit is read beside the count that a kernel starts with
+// (asked first, past L1 and by the whole block it cost up to 1.5 us per launch).
+__device__ __forceinline__ int unless_failed(const Ctl *ctl, int n) {
+    return __shfl_sync(FULL, ctl->err & DERR_TIMEOUT ? 0 : n, 0);  // one answer per warp
+}
+// the same for kernels whose rows take the whole block: one answer per block
 __device__ __forceinline__ bool scan_failed(const Ctl *ctl) {
-    return __syncthreads_or(*(const volatile int *)&ctl->err & DERR_TIMEOUT) != 0;
+    return __syncthreads_or(ctl->err & DERR_TIMEOUT) != 0;
 }
 
 __device__ __forceinline__ unsigned lanemask_lt() {

@@ -9,7 +9,7 @@
 // itself when the last block is done.  The look-back's polls are bounded: a
 // block that gives up sets DERR_TIMEOUT and goes on with what it has, a prefix
 // no larger than the right one, so what it writes stays in bounds; the kernels
-// that index by the result return at once then (scan_failed).
+// that index by the result take no row then (unless_failed, scan_failed).
 //
 // Small calls are launch-bound: with three launches per scan and two more for the
 // binning a Laplacian product had 18, now 10 (64^2 grid 163 -> 130 us, 256^2 210 ->

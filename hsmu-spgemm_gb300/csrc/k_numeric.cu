@@ -184,8 +184,8 @@ __global__ void __launch_bounds__(256) k_win_cursors(const Window *__restrict__ 
                                                      const int *__restrict__ tcol, const int *__restrict__ toff,
                                                      const int *__restrict__ item_off, int *__restrict__ wcur,
                                                      Ctl *ctl) {
-    if (scan_failed(ctl)) return;
-    const int nwin = min(ctl->win_count, win_cap);
+    const int nwin = unless_failed(ctl, min(ctl->win_count, win_cap));
+    if (nwin == 0) return;
     const int lane = lane_id();
     const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;

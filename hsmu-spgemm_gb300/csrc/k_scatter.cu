@@ -191,11 +191,10 @@ constexpr int HC_CTAS_PER_SM = 6;
 __global__ void __launch_bounds__(HC_WARPS * 32, HC_CTAS_PER_SM)
     k_count_h(int M, const int *__restrict__ arp, const int *__restrict__ acol, const int *__restrict__ brp,
               const int *__restrict__ bcol, RowInfo ri, Ctl *ctl) {
-    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     HSmem &S = reinterpret_cast<HSmem *>(s_dyn)[w];
-    const int n = ctl->bin_count[BIN_H];
+    const int n = unless_failed(ctl, ctl->bin_count[BIN_H]);
     const int *rows = ri.bins + (size_t)BIN_H * M;
     HRows H(rows, arp, acol, blockIdx.x * HC_WARPS + w, n, gridDim.x * HC_WARPS);
     while (H.i >= 0) {
@@ -232,13 +231,12 @@ __global__ void __launch_bounds__(HF_WARPS * 32, hf_ctas<AR>())
     k_fill_h(int M, const int *__restrict__ arp, const int *__restrict__ acol, const double *__restrict__ aval,
              const int *__restrict__ brp, const int *__restrict__ bcol, const double *__restrict__ bval, RowInfo ri,
              RowOut out, Ctl *ctl) {
-    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     HSmem &S = reinterpret_cast<HSmem *>(s_dyn)[w];
     const int *rows = ri.bins + (size_t)BIN_H * M;
     int b0, b1;
-    bin_slice(rows, ctl->bin_count[BIN_H], out, M, b0, b1);
+    bin_slice(rows, unless_failed(ctl, ctl->bin_count[BIN_H]), out, M, b0, b1);
     HRows H(rows, arp, acol, b0 + blockIdx.x * HF_WARPS + w, b1, gridDim.x * HF_WARPS);
     while (H.i >= 0) {
         const int i = H.i;

@@ -97,13 +97,12 @@ __global__ void __launch_bounds__(SDS_WARPS * 32, SDS_CTAS_PER_SM)
                 const int *__restrict__ tptr, const int *__restrict__ tcol,
                 const unsigned long long *__restrict__ tmask, RowInfo ri, RowOut out, Window *__restrict__ win,
                 long long win_cap, Ctl *ctl) {
-    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     SdsSmem &S = reinterpret_cast<SdsSmem *>(s_dyn)[w];
     const int *rows = ri.bins + (size_t)BIN_DS * M;
     int b0, b1;
-    bin_slice(rows, ctl->bin_count[BIN_DS], out, M, b0, b1);
+    bin_slice(rows, unless_failed(ctl, ctl->bin_count[BIN_DS]), out, M, b0, b1);
     int *__restrict__ ccol = out.ccol;
     double *__restrict__ cval = out.cval;
     for (int r = b0 + blockIdx.x * SDS_WARPS + w; r < b1; r += gridDim.x * SDS_WARPS) {
@@ -484,12 +483,11 @@ __global__ void __launch_bounds__(TINYF_THREADS, 4) k_fill_tiny(int M, const int
                                                                 const int *__restrict__ bcol,
                                                                 const double *__restrict__ bval, RowInfo ri,
                                                                 RowOut out, Ctl *ctl) {
-    if (scan_failed(ctl)) return;
     extern __shared__ unsigned long long s_dyn[];
     TinySmem<AR> &S = reinterpret_cast<TinySmem<AR> *>(s_dyn)[threadIdx.x >> 5];
     const int *rows = ri.bins + (size_t)BIN_TINY * M;
     int b0, b1;
-    bin_slice(rows, ctl->bin_count[BIN_TINY], out, M, b0, b1);
+    bin_slice(rows, unless_failed(ctl, ctl->bin_count[BIN_TINY]), out, M, b0, b1);
     bool bad = false;
     for (int r0 = b0 + blockIdx.x * TINYF_THREADS + (threadIdx.x & ~31); r0 < b1; r0 += gridDim.x * TINYF_THREADS) {
         const int r = r0 + lane_id();
@@ -542,12 +540,11 @@ __global__ void __launch_bounds__(TINYF_THREADS) k_fill_tiny_wide(int M, const i
                                                              const int *__restrict__ bcol,
                                                              const double *__restrict__ bval, RowInfo ri,
                                                              RowOut out, Ctl *ctl) {
-    if (scan_failed(ctl)) return;
     __shared__ int s_cols[TINY_MAX * TINYF_THREADS];
     __shared__ double s_acc[TINY_MAX * TINYF_THREADS];
     const int *rows = ri.bins + (size_t)BIN_TINY * M;
     int b0, b1;
-    bin_slice(rows, ctl->bin_count[BIN_TINY], out, M, b0, b1);
+    bin_slice(rows, unless_failed(ctl, ctl->bin_count[BIN_TINY]), out, M, b0, b1);
     bool bad = false;
     for (int r = b0 + blockIdx.x * TINYF_THREADS + threadIdx.x; r < b1; r += gridDim.x * TINYF_THREADS) {
         const int i = rows[r];

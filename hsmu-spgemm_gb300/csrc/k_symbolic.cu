@@ -58,11 +58,10 @@ __global__ void __launch_bounds__(DS_WARPS * 32) k_count_ds(int M, const int *__
                                                             const int *__restrict__ tcol,
                                                             const unsigned long long *__restrict__ tmask,
                                                             RowInfo ri, Ctl *ctl) {
-    if (scan_failed(ctl)) return;
     __shared__ unsigned long long s_mask[DS_WARPS][SPAN_T];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     unsigned long long *msk = s_mask[w];
-    const int n = ctl->bin_count[BIN_DS];
+    const int n = unless_failed(ctl, ctl->bin_count[BIN_DS]);
     const int *rows = ri.bins + (size_t)BIN_DS * M;
     const int nwarps = gridDim.x * DS_WARPS, gw = blockIdx.x * DS_WARPS + w;
     for (int turn = 0; (long long)turn * nwarps < n; turn++) {
@@ -240,10 +239,9 @@ __global__ void __launch_bounds__(TINY_THREADS) k_count_tiny(int M, const int *_
                                                              const int *__restrict__ acol,
                                                              const int *__restrict__ brp,
                                                              const int *__restrict__ bcol, RowInfo ri, Ctl *ctl) {
-    if (scan_failed(ctl)) return;
     __shared__ int s_q[TINY_THREADS / WARP][TINY_MAX][WARP];
     int (*qs)[WARP] = s_q[threadIdx.x >> 5];
-    const int n = ctl->bin_count[BIN_TINY];
+    const int n = unless_failed(ctl, ctl->bin_count[BIN_TINY]);
     const int *rows = ri.bins + (size_t)BIN_TINY * M;
     bool bad = false;
     for (int r0 = blockIdx.x * TINY_THREADS + (threadIdx.x & ~31); r0 < n; r0 += gridDim.x * TINY_THREADS) {

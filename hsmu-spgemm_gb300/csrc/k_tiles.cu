@@ -25,7 +25,6 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
                                                unsigned long long *__restrict__ tmask, int *__restrict__ toff,
                                                int validate, Ctl *ctl, bool gated) {
     if (gated && !tiles_read(ctl)) return;
-    if (FILL && scan_failed(ctl)) return;
     const int lane = lane_id();
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;

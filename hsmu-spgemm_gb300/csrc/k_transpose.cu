@@ -44,8 +44,7 @@ __global__ void __launch_bounds__(256) k_tr_rows(int M, const int *__restrict__ 
 inline int tr_tile(long long n) { return n <= TR_SMALL ? TR_TILE_SMALL : TR_TILE; }
 
 __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_hist(const int *__restrict__ key, int n, int te, int shift,
-                                                           int ntiles, int *__restrict__ hist, const Ctl *ctl) {
-    if (scan_failed(ctl)) return;
+                                                           int ntiles, int *__restrict__ hist) {
     __shared__ int s_h[TR_WARPS][TR_RADIX];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     const int tile = blockIdx.x * TR_WARPS + w;
@@ -59,12 +58,13 @@ __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_hist(const int *__restrict
     }
 }
 
+// (A scan that gave up leaves offsets no larger than the right ones, so the positions stay below n whatever
+// keys an earlier pass has left; the row pointers are not made then.)
 __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_scatter(const int *__restrict__ key, const int *__restrict__ row,
                                                               const double *__restrict__ val, int n, int te, int shift,
                                                               int ntiles, const int *__restrict__ off,
                                                               int *__restrict__ okey, int *__restrict__ orow,
-                                                              double *__restrict__ oval, const Ctl *ctl) {
-    if (scan_failed(ctl)) return;
+                                                              double *__restrict__ oval) {
     __shared__ int s_run[TR_WARPS][TR_RADIX];
     const int lane = lane_id(), w = threadIdx.x >> 5;
     const int tile = blockIdx.x * TR_WARPS + w;
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(TR_WARPS * 32) k_tr_scatter(const int *__restr
 // row pointers of B = A^T from the sorted column ids: rp[c] = first position of column c
 __global__ void __launch_bounds__(256) k_tr_rowptr(const int *__restrict__ key, int n, int N, int *__restrict__ rp,
                                                    const Ctl *ctl) {
-    if (scan_failed(ctl)) return;
+    if (unless_failed(ctl, 1) == 0) return;  // the keys are not in order, or not there
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e <= n; e += (long long)gridDim.x * blockDim.x) {
         const int prev = e == 0 ? -1 : min(key[e - 1], N);
         const int cur = e == n ? N : min(key[e], N);
@@ -135,10 +135,10 @@ int launch_transpose(const DevCSR &A, int *trp, int *tcol, double *tval, int *sc
         int *dkey = (p % 2 == 0) ? key1 : key0;
         int *drow = last ? tcol : ((p % 2 == 0) ? row1 : row0);
         double *dval = last ? tval : ((p % 2 == 0) ? val1 : val0);
-        k_tr_hist<<<blocks, TR_WARPS * 32, 0, st>>>(skey, n, te, 8 * p, ntiles, hist, ctl);
+        k_tr_hist<<<blocks, TR_WARPS * 32, 0, st>>>(skey, n, te, 8 * p, ntiles, hist);
         launch_scan(hist, hist + (size_t)TR_RADIX * ntiles + 1, TR_RADIX * ntiles, total64, scan, ctl, st);
         k_tr_scatter<<<blocks, TR_WARPS * 32, 0, st>>>(skey, srow, sval, n, te, 8 * p, ntiles,
-                                                      hist + (size_t)TR_RADIX * ntiles + 1, dkey, drow, dval, ctl);
+                                                      hist + (size_t)TR_RADIX * ntiles + 1, dkey, drow, dval);
         skey = dkey;
         srow = drow;
         sval = dval;
