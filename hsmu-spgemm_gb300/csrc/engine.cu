@@ -129,7 +129,7 @@ constexpr int SIDE_MIN_NNZ = 1 << 16;
 // hsmu_spgemm64: bytes of windows and cursors up to which all panels share one symbolic pass, and what
 // a window and a cursor take (PlainRun::alloc_output)
 constexpr unsigned long long ONE_PASS_BYTES = 4ull << 30;
-constexpr unsigned long long WINDOW_BYTES = sizeof(Window) + sizeof(long long) + 3 * sizeof(int) + 1;
+constexpr unsigned long long WINDOW_BYTES = sizeof(Window) + sizeof(long long) + 2 * sizeof(int);
 // average entries of B's rows from which repeated rows are looked for: chains of shorter rows
 // are not taken (hsmu_products.cuh), and the chain kernel's registers cost rows without chains
 // (scalar 27-point rows: 296 us with it, 169 us without)
@@ -664,13 +664,10 @@ struct PlainRun {
     int alloc_cursors(long long nwin, long long cap) {
         if (nwin == 0) return HSMU_OK;
         wc.cap = cap;
-        CKR(salloc(h, &wc.len, (size_t)nwin, st));
         CKR(salloc(h, &wc.off, (size_t)nwin + 1, st));
-        CKR(salloc(h, &wc.total, 2, st));
         CKR(salloc(h, &wc.item_off, (size_t)nwin + 1, st));
         CKR(salloc(h, &wc.cur, (size_t)cap, st));
         CKR(salloc(h, &wc.heavy, (size_t)nwin, st));
-        CKR(salloc(h, &wc.cls, (size_t)nwin, st));
         return HSMU_OK;
     }
 
@@ -729,7 +726,7 @@ struct PlainRun {
         const TileStore tsd = store_view();
         launch_numeric(Ad, Bd, Btd, crp, ccol, cval, win, win_cap, nullptr, nullptr, nullptr, wc, ctl, o.arith, h->nsm,
                        st, h->scan, o.wait_polls, have_store ? &tsd : nullptr);
-        launches += 5;  // window lengths, two scans, cursors, values
+        launches += 3;  // window lengths, cursors, values
     }
 
     // start a new panel: its windows reuse the window buffer from slot 0
@@ -1212,13 +1209,10 @@ learned:
         cur_cap = 2 * (long long)(hc.cur_bound + hc.cur_bound_ds);
         if (win_cap > 0) {
             wc.cap = cur_cap;
-            CK(salloc(h, &wc.len, (size_t)win_cap, st));
             CK(salloc(h, &wc.off, (size_t)win_cap + 1, st));
-            CK(salloc(h, &wc.total, 2, st));
             CK(salloc(h, &wc.item_off, (size_t)win_cap + 1, st));
             CK(salloc(h, &wc.cur, (size_t)cur_cap, st));
             CK(salloc(h, &wc.heavy, (size_t)win_cap, st));
-            CK(salloc(h, &wc.cls, (size_t)win_cap, st));
         }
         if (stats) cudaEventRecord(h->ev[3], st);
         // structure (+ values of warp-sized rows) into the slots; exact counts found here.
@@ -1315,8 +1309,8 @@ learned:
         cudaEventElapsedTime(&t, h->ev[0], h->ev[5]);
         stats->ms_total = t;
         // tiles 3, bounds + binning 2, features 1, capacity 1, scan 1, structure 3, scan 1, compact 1, redo 3,
-        // window lengths 1, their two scans 2, cursors 1, numeric 1
-        stats->launches = (o.validate ? 2 : 0) + (win_cap > 0 ? 21 : 16);
+        // window lengths 1, cursors 1, numeric 1
+        stats->launches = (o.validate ? 2 : 0) + (win_cap > 0 ? 19 : 16);
     }
 done:
     pfree(crp, st);

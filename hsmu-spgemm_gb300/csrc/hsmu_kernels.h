@@ -196,16 +196,13 @@ void launch_structure_light(const DevCSR &A, const DevCSR &B, RowInfo ri, RowOut
 // flag (nullable): speculative-pass windows of rows flagged ROW_OVERFLOW are skipped;
 // scol/soff (nullable): speculative slots holding the columns of speculative-pass
 // windows, which the kernel copies to ccol
-// per-window cursors into the B rows (k_win_cursors): len/off/item_off sized
-// for win_cap windows (+1), total for 2 entries, cur for cap entries (Ctl::cur_bound)
+// per-window cursors into the B rows (k_win_cursors): off/item_off sized
+// for win_cap windows + 1, cur for cap entries (Ctl::cur_bound)
 struct WinCursors {
-    int *len;
     long long *off;
-    long long *total;
-    int *item_off;  // the cursor pass's work items per window, scanned in place
+    int *item_off;  // the cursor pass's work items per window, scanned
     int *cur;
     int *heavy;     // windows of rows with many A entries (win_cap entries)
-    signed char *cls;  // 0 and 1 for such windows (win_cap entries)
     long long cap;
 };
 void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const int *crp, int *ccol, double *cval,

@@ -84,65 +84,130 @@ __device__ __forceinline__ bool cur_continues(const Window *win, int w, int row,
     return w % CUR_CHUNK != 0 && win[w - 1].row == row && win[w - 1].t0 < t0;
 }
 
-// A entries of each window's row (0 past the emitted windows), scanned into
-// the windows' offsets in the cursor array, and the cursor pass's work items
-// (CUR_CHUNK).  A window written with a slot
-// count of 0 (the large rows built from their stored tiles) gets its count
-// here: up to the next window's first slot when that window continues the
-// same row, else up to the row's end; and its tile count likewise, up to the
-// next window's first tile or the end of the row's list.
-// Windows of rows with at least HEAVY_ROW A entries are listed from the front of `heavy`, those of rows
-// with at least LONG_ROW from its back, in order (bin_tile): the value pass hands them out first.
-// `windows` per block, in one pass over the list.
-__global__ void __launch_bounds__(BIN_T) k_win_len(Window *__restrict__ win, int win_cap, int M, const int *__restrict__ arp,
-                                                   const int *__restrict__ crp, const long long *__restrict__ ts_off,
-                                                   const int *__restrict__ ts_cnt, Ctl *ctl, int *__restrict__ len,
-                                                   int *__restrict__ items, signed char *cls, int *__restrict__ heavy,
-                                                   int windows, int ntiles, LookBack lb) {
-    __shared__ BinSmem<2> S;
-    const int tile = lb_tile(lb, &S.tile);
-    const int nwin = min(ctl->win_count, win_cap);
-    const long long w_lo = (long long)tile * windows;
-    const int w_end = (int)min(w_lo + windows, (long long)win_cap);
-    for (int w = (int)w_lo + (int)threadIdx.x; w < w_end; w += BIN_T) {
-        int n = 0, it = 0;
-        signed char c = -1;
-        if (w < nwin) {
-            const int row = win[w].row;
-            if ((unsigned)row >= (unsigned)M) {  // a window left unwritten after a reported error
-                set_err(&ctl->err, DERR_INTERNAL);
-                len[w] = 0;
-                items[w] = 0;
-                cls[w] = -1;
-                continue;
-            }
-            n = arp[row + 1] - arp[row];
-            c = n >= HEAVY_ROW ? 0 : n >= LONG_ROW ? 1 : -1;
-            // a chunk of the cursor pass starts here: one work item per 32 A entries
-            if (!cur_continues(win, w, row, win[w].t0)) it = (n + WARP - 1) / WARP;
-            if (win[w].cnt == 0) {
-                const int s0 = win[w].s0, li = win[w].li;
-                int e = crp[row + 1] - crp[row];
-                long long le = (li >= 0 && ts_off) ? ts_off[row] + ts_cnt[row] : -1;
-                if (w + 1 < nwin && win[w + 1].row == row && win[w + 1].s0 > s0) {
-                    e = win[w + 1].s0;
-                    if (win[w + 1].li > li) le = win[w + 1].li;
-                }
-                win[w].cnt = e - s0;
-                // the tile path of the value pass needs 1..WIN_TCAP tiles; else the columns are used
-                win[w].nt = (li >= 0 && le > li && le - li <= WIN_TCAP) ? (int)(le - li) : 0;
-            }
+// What the window length pass knows of a window: its row's A entries, the cursor pass's work items
+// that start at it (CUR_CHUNK), its list (0: heavy, 1: long, -1: none); all 0 past the emitted windows.
+struct WinItem {
+    int n = 0, items = 0, list = -1;
+
+    __device__ __forceinline__ void read(const Window *win, int w, int nwin, int M, const int *__restrict__ arp, Ctl *ctl) {
+        n = items = 0;
+        list = -1;
+        if (w >= nwin) return;
+        const int row = win[w].row;
+        if ((unsigned)row >= (unsigned)M) {  // a window left unwritten after a reported error
+            set_err(&ctl->err, DERR_INTERNAL);
+            return;
         }
-        len[w] = n;
-        items[w] = it;
-        cls[w] = c;
+        n = arp[row + 1] - arp[row];
+        list = n >= HEAVY_ROW ? 0 : n >= LONG_ROW ? 1 : -1;
+        // a chunk of the cursor pass starts here: one work item per 32 A entries
+        if (!cur_continues(win, w, row, win[w].t0)) items = (n + WARP - 1) / WARP;
+    }
+};
+
+// A window written with a slot count of 0 (the large rows built from their stored tiles) gets its count
+// here: up to the next window's first slot when that window continues the same row, else up to the row's
+// end; and its tile count likewise, up to the next window's first tile or the end of the row's list.
+__device__ __forceinline__ void close_window(Window *win, int w, int nwin, int M, const int *__restrict__ crp,
+                                             const long long *__restrict__ ts_off, const int *__restrict__ ts_cnt) {
+    const int row = win[w].row;
+    if (win[w].cnt != 0 || (unsigned)row >= (unsigned)M) return;
+    const int s0 = win[w].s0, li = win[w].li;
+    int e = crp[row + 1] - crp[row];
+    long long le = (li >= 0 && ts_off) ? ts_off[row] + ts_cnt[row] : -1;
+    if (w + 1 < nwin && win[w + 1].row == row && win[w + 1].s0 > s0) {
+        e = win[w + 1].s0;
+        if (win[w + 1].li > li) le = win[w + 1].li;
+    }
+    win[w].cnt = e - s0;
+    // the tile path of the value pass needs 1..WIN_TCAP tiles; else the columns are used
+    win[w].nt = (li >= 0 && le > li && le - li <= WIN_TCAP) ? (int)(le - li) : 0;
+}
+
+// Window length pass, one launch over the windows with four look-backs side by side (hsmu_lookback.cuh):
+// the A entries of each window's row, scanned into the windows' offsets in the cursor array (off); the
+// cursor pass's work items, scanned (item_off); and the windows of rows with at least HEAVY_ROW A entries
+// listed from the front of `heavy`, those of rows with at least LONG_ROW from its back, in order: the value
+// pass hands them out first.  A thread has WL_IPT windows next to each other; a tile of several pieces of
+// WL_ITEMS reads its windows twice.  (In three launches, lengths and lists, then two scans: 13.8 + 10.4 us for
+// A*A^T of 30,011 vertices, 13.9 us so; four row panels of 49,999 vertices 55.6 + 47.8 us, 65.6 us so.)
+constexpr int WL_T = 256, WL_IPT = 4, WL_ITEMS = WL_T * WL_IPT;
+
+__global__ void __launch_bounds__(WL_T) k_win_len(Window *__restrict__ win, int win_cap, int M, const int *__restrict__ arp,
+                                                  const int *__restrict__ crp, const long long *__restrict__ ts_off,
+                                                  const int *__restrict__ ts_cnt, Ctl *ctl, long long *__restrict__ off,
+                                                  int *__restrict__ item_off, int *__restrict__ heavy, int chunks,
+                                                  int ntiles, LookBack lb) {
+    __shared__ long long s_n[WL_T / WARP], s_i[WL_T / WARP], s_c[WL_T / WARP], s_before[4];
+    __shared__ int s_tile;
+    const int tile = lb_tile(lb, &s_tile);
+    const int lane = lane_id(), wid = threadIdx.x >> 5;
+    const int nwin = min(ctl->win_count, win_cap);
+    const long long first = (long long)tile * chunks * WL_ITEMS + (long long)threadIdx.x * WL_IPT;
+    WinItem x[WL_IPT];
+    long long tn = 0, ti = 0, tc = 0;  // the thread's sums; tc: heavy windows << 32 | long ones
+    auto read = [&](long long base) {
+#pragma unroll
+        for (int j = 0; j < WL_IPT; j++) {
+            x[j].read(win, (int)min(base + j, (long long)INT_MAX), nwin, M, arp, ctl);
+            tn += x[j].n;
+            ti += x[j].items;
+            tc += x[j].list == 0 ? 1ll << 32 : x[j].list == 1 ? 1ll : 0ll;
+        }
+    };
+    for (int c = 0; c < chunks; c++) {
+        const long long base = first + (long long)c * WL_ITEMS;
+        read(base);
+#pragma unroll
+        for (int j = 0; j < WL_IPT; j++)
+            if (base + j < nwin) close_window(win, (int)(base + j), nwin, M, crp, ts_off, ts_cnt);
+    }
+    long long sn, si, sc;  // the tile's sums
+    long long en = block_excl_sum1<WL_T>(tn, s_n, sn), ei = block_excl_sum1<WL_T>(ti, s_i, si);
+    long long ec = block_excl_sum1<WL_T>(tc, s_c, sc);
+    if (wid < 4) {
+        const long long mine = wid == 0 ? sn : wid == 1 ? si : wid == 2 ? sc >> 32 : sc & 0xffffffffll;
+        const unsigned long long p = lb_prefix(lb, wid, tile, (unsigned long long)mine, ctl);
+        if (lane == 0) s_before[wid] = (long long)p;
     }
     __syncthreads();
-    bin_tile<2>(cls, tile, windows, win_cap, ntiles, lb, ctl, S,
-                [&](int b, int at, int w) { heavy[b == 0 ? at : win_cap - 1 - at] = w; });
+    if (threadIdx.x == 0) lb_done(lb, ntiles);
+    long long rn = s_before[0], ri = s_before[1], r0 = s_before[2], r1 = s_before[3];
     if (tile == ntiles - 1 && threadIdx.x == 0) {
-        ctl->win_heavy = S.cnt[0];
-        ctl->win_long = S.cnt[1];
+        off[win_cap] = rn + sn;
+        item_off[win_cap] = (int)min(ri + si, (long long)INT_MAX);
+        if (ri + si > INT_MAX) set_err(&ctl->err, DERR_OVERFLOW);
+        ctl->win_heavy = (int)(r0 + (sc >> 32));
+        ctl->win_long = (int)(r1 + (sc & 0xffffffffll));
+    }
+    for (int c = 0; c < chunks; c++) {
+        const long long base = first + (long long)c * WL_ITEMS;
+        if (chunks > 1) {  // again, a piece at a time
+            tn = ti = tc = 0;
+            read(base);
+            __syncthreads();  // the piece before has read the warps' sums
+            en = block_excl_sum1<WL_T>(tn, s_n, sn);
+            ei = block_excl_sum1<WL_T>(ti, s_i, si);
+            ec = block_excl_sum1<WL_T>(tc, s_c, sc);
+        }
+        long long an = rn + en, ai = ri + ei;
+        int a0 = (int)(r0 + (ec >> 32)), a1 = (int)(r1 + (ec & 0xffffffffll));
+#pragma unroll
+        for (int j = 0; j < WL_IPT; j++) {
+            if (base + j < win_cap) {
+                const int w = (int)(base + j);
+                off[w] = an;
+                item_off[w] = (int)min(ai, (long long)INT_MAX);
+                if (x[j].list == 0) heavy[a0++] = w;
+                else if (x[j].list == 1) heavy[win_cap - 1 - a1++] = w;
+            }
+            an += x[j].n;
+            ai += x[j].items;
+        }
+        rn += sn;
+        ri += si;
+        r0 += sc >> 32;
+        r1 += sc & 0xffffffffll;
     }
 }
 
@@ -493,12 +558,10 @@ void launch_numeric(const DevCSR &A, const DevCSR &B, const DevTiles &Bt, const 
     if (win_cap <= 0) return;
     cudaMemsetAsync(&ctl->win_next, 0, sizeof(int), st);
     int chunks;
-    const int ntiles = lb_tiles(win_cap, BIN_ROWS, chunks);
-    k_win_len<<<ntiles, BIN_T, 0, st>>>(const_cast<Window *>(win), (int)win_cap, A.M, A.rp, crp, ts ? ts->off : nullptr,
-                                        ts ? ts->cnt : nullptr, ctl, wc.len, wc.item_off, wc.cls, wc.heavy,
-                                        chunks * BIN_ROWS, ntiles, next_epoch(scan, st));
-    launch_scan64(wc.len, wc.off, (int)win_cap, wc.total, scan, ctl, st);
-    launch_scan(wc.item_off, wc.item_off, (int)win_cap, wc.total + 1, scan, ctl, st);
+    const int ntiles = lb_tiles(win_cap, WL_ITEMS, chunks);
+    k_win_len<<<ntiles, WL_T, 0, st>>>(const_cast<Window *>(win), (int)win_cap, A.M, A.rp, crp, ts ? ts->off : nullptr,
+                                       ts ? ts->cnt : nullptr, ctl, wc.off, wc.item_off, wc.heavy, chunks, ntiles,
+                                       next_epoch(scan, st));
     k_win_cursors<<<nsm * 16, 256, 0, st>>>(win, (int)win_cap, A.M, wc.off, wc.cap, A.rp, A.col, B.rp, Bt.ptr, Bt.col,
                                             Bt.off, wc.item_off, wc.cur, ctl);
     auto k = arith == AR_IMUL ? k_numeric<AR_IMUL> : arith == AR_FMA ? k_numeric<AR_FMA> : k_numeric<AR_RN>;

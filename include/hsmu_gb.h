@@ -215,7 +215,7 @@ typedef struct hsmu_csr64 {
  * in panels whose entries fit int32 (at most max_panel_nnz each, 0 = INT32_MAX;
  * a row with more entries than the cap is a panel of its own), each written
  * straight into its place in C.  B's tiles are built once for all panels, and
- * so is the symbolic pass while the windows (49 bytes each) and cursors (4) of
+ * so is the symbolic pass while the windows (44 bytes each) and cursors (4) of
  * all rows take at most 4 GB and there is memory for them; else each panel has
  * its own, and only one panel's exist at a time.
  * Synchronizes `stream` before returning. */
