@@ -18,8 +18,32 @@
 
 namespace hsmu {
 
-// TILE_U: steps of 32 entries whose loads are in flight (launch_tiles_*)
-template <bool FILL, int TILE_U>
+// Steps of 32 entries whose loads are in flight.  A hub row of a power-law graph is a chain of hundreds of
+// steps, and with one step's load in flight it was the pass's tail: R-MAT scale 18 count 207 -> 120 us, fill
+// 385 -> 310 us, scale 15 30 -> 16 and 71 -> 56 us with four.  Rows of one step are taken apart, whole tiles
+// straight to their places (count / fill, against the four-step loop for all rows: 150,001 rows of 12 entries
+// 16.5 / 33.5 -> 10.4 / 24.5 us, 27-point rows of a 64^3 grid 27.5 / 57.4 -> 19 / 40.2; against a loop of one
+// step, by the average of the rows: R-MAT scale 17 of 7.6 entries 57.8 / 130 -> 30 / 85.4, a 5-point Laplacian
+// of 4.2 million rows 340 / 880 -> 327 / 791).
+constexpr int TILE_U = 4;
+
+// the 32 lanes' column bits, ORed over each run of lanes from a lane to seg_end
+__device__ __forceinline__ unsigned long long tile_or(unsigned long long v, int seg_end) {
+#pragma unroll
+    for (int d = 1; d < WARP; d <<= 1) {
+        const unsigned long long o = __shfl_down_sync(FULL, v, d);
+        if (lane_id() + d <= seg_end) v |= o;
+    }
+    return v;
+}
+// the last lane of the tile that a lane's column lies in, of nvalid lanes
+__device__ __forceinline__ int tile_end(unsigned heads, int nvalid) {
+    const int lane = lane_id();
+    const unsigned above = lane == 31 ? 0u : heads & ~((2u << lane) - 1u);
+    return above ? __ffs(above) - 2 : nvalid - 1;
+}
+
+template <bool FILL>
 __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ brp, const int *__restrict__ bcol,
                                                int N, int *__restrict__ tcnt_or_ptr, int *__restrict__ tcol,
                                                unsigned long long *__restrict__ tmask, int *__restrict__ toff,
@@ -31,6 +55,27 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
     for (int k = gw; k < K; k += nw) {
         const int s = brp[k], e = brp[k + 1];
         int run = FILL ? tcnt_or_ptr[k] : 0;  // output position (FILL) / count
+        if (e - s <= WARP) {  // one step, every tile whole
+            const bool valid = lane < e - s;
+            const int c = valid ? __ldg(bcol + s + lane) : 0;
+            const int cp = __shfl_up_sync(FULL, c, 1);
+            const bool head = valid && (lane == 0 || c >> 6 != cp >> 6);
+            const unsigned heads = __ballot_sync(FULL, head);
+            if (FILL) {
+                const unsigned long long v = tile_or(valid ? 1ull << (c & 63) : 0ull, tile_end(heads, e - s));
+                if (head) {
+                    const int pos = run + __popc(heads & lanemask_lt());
+                    tcol[pos] = c >> 6;
+                    tmask[pos] = v;
+                    toff[pos] = s + lane;
+                }
+            } else if (lane == 0) {
+                tcnt_or_ptr[k] = __popc(heads);
+            }
+            if (validate && __any_sync(FULL, valid && (c < 0 || c >= N || (lane > 0 && c <= cp))) && lane == 0)
+                set_err(&ctl->err, DERR_UNSORTED);
+            continue;
+        }
         bool have_pend = false;
         int pend_t = -1, pend_off = 0;
         unsigned long long pend_m = 0;
@@ -66,15 +111,7 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
                     have_pend = true;
                     continue;
                 }
-                unsigned above = heads & ~((2u << lane) - 1u);
-                if (lane == 31) above = 0;
-                const int seg_end = above ? (__ffs(above) - 2) : (nvalid - 1);
-                unsigned long long v = valid ? (1ull << (c & 63)) : 0ull;
-#pragma unroll
-                for (int d = 1; d < WARP; d <<= 1) {
-                    unsigned long long o = __shfl_down_sync(FULL, v, d);
-                    if (lane + d <= seg_end) v |= o;
-                }
+                const unsigned long long v = tile_or(valid ? 1ull << (c & 63) : 0ull, tile_end(heads, nvalid));
                 const unsigned long long lane0_or = __shfl_sync(FULL, v, 0);
                 if (have_pend) {
                     if (!(heads & 1u)) pend_m |= lane0_or;  // lane 0 continues the pending tile
@@ -117,21 +154,17 @@ __global__ void __launch_bounds__(256) k_tiles(int K, const int *__restrict__ br
     }
 }
 
-// A hub row of a power-law graph is a chain of hundreds of steps, and with one step's load in flight
-// it was the pass's tail: R-MAT scale 18 count 207 -> 120 us, fill 385 -> 310 us, scale 15 30 -> 16 and
-// 71 -> 56 us with four.  Rows that fit one step only pay for the wider loop (5-point Laplacian of
-// 65,536 rows: 5.7 -> 8.2 and 13.7 -> 15.7 us).
-static bool tiles_short(const DevCSR &B) { return B.nnz <= 8ll * B.M; }
-
 void launch_tiles_count(const DevCSR &B, int *tcnt, int validate, Ctl *ctl, int grid, cudaStream_t st, bool gated) {
-    grid = grid_for(grid, B.M, 256 / WARP);
-    (tiles_short(B) ? k_tiles<false, 1> : k_tiles<false, 4>)<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, tcnt, nullptr, nullptr, nullptr, validate, ctl, gated);
+    k_tiles<false><<<grid_for(grid, B.M, 256 / WARP), 256, 0, st>>>(B.M, B.rp, B.col, B.N, tcnt, nullptr, nullptr,
+                                                                    nullptr, validate, ctl, gated);
 }
 
 void launch_tiles_fill(const DevCSR &B, const int *tptr, int *tcol, unsigned long long *tmask, int *toff, Ctl *ctl,
                        int grid, cudaStream_t st, bool gated) {
-    grid = grid_for(grid, B.M, 256 / WARP);
-    (tiles_short(B) ? k_tiles<true, 1> : k_tiles<true, 4>)<<<grid, 256, 0, st>>>(B.M, B.rp, B.col, B.N, const_cast<int *>(tptr), tcol, tmask, toff, 0, ctl, gated);
+    // five blocks fit an SM: a grid of eight leaves a second wave of three (4.2 million rows 935 us, 791 so); but
+    // a gated launch may have nothing to do, and four thousand empty blocks take 4 us
+    k_tiles<true><<<grid_for(gated ? grid : 4 * grid, B.M, 256 / WARP), 256, 0, st>>>(B.M, B.rp, B.col, B.N, const_cast<int *>(tptr), tcol,
+                                                                   tmask, toff, 0, ctl, gated);
 }
 
 // rep[k] = 1 when row k of B holds the same columns as row k - 1 (the rows of one finite-element
