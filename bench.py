@@ -86,10 +86,8 @@ TRAFFIC = {
     # profiles/k_numeric_rmat16_AA.md: 1.828 GB on R-MAT scale 16, scaled by the algorithmic
     # bytes (x7.765) to scale 18
     "rmat18_AA": 14.19e9,
-    # profiles/k_batch_amg32_galerkin.md: 3.12 GB per launch of the 32-product batch (tuned
-    # launch); the 512-product batch scaled by its algorithmic bytes (x11.82)
-    "amg32_galerkin": 3.12e9,
-    "amg512_galerkin": 36.9e9,
+    # none for the Galerkin batches: profiles/k_batch_amg32_galerkin.md captured them as one
+    # kernel (3.12 GB per launch of the 32-product batch), they now run as two
 }
 
 WORKLOADS = {

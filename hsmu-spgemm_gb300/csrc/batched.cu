@@ -1,13 +1,14 @@
 // Batched persistent engine: many independent SpGEMMs (C_p = A_p * B_p) or
-// AMG Galerkin triple products (C_p = Pt_p * (A_p * P_p)) in ONE launch.
+// AMG Galerkin triple products (C_p = Pt_p * (A_p * P_p)) in one graph launch
+// of one kernel, or of two.
 //
 // The reference runs each product separately, with ~10 blocking host round
 // trips and several cudaMalloc calls per product
 // (src/compressed/compressed_NHC_spgemm.cu:22-248); for hundreds of small
 // products that overhead, not the arithmetic, sets the time.  Here all rows of
 // all products form one flattened row space, cut into tiles of 32 rows that
-// never span two products, and a single cooperative, persistent kernel takes
-// every row in ONE pass:
+// never span two products, and a cooperative, persistent kernel takes every
+// row in one pass:
 //   * a warp computes its tile's rows (thread per row with a sorted list in
 //     shared memory; warp per row with a dense tile table for rows with more
 //     products), so the tile's entry count is known;
@@ -946,7 +947,7 @@ struct hsmu_batch_s {
     std::vector<void *> allocs;
     std::vector<long long> row0[2], rpo[2], reg[2];
     std::vector<int> ncol[2];
-    void *reset;          // zeroed before every launch: barrier, error word, wide-row counters, tile status
+    void *reset;          // zeroed before every launch: barrier, error word, wide-row counters, tiles left, allocation counters
     size_t reset_bytes;
     cudaGraph_t graph;
     cudaGraphExec_t gexec;

@@ -1,6 +1,9 @@
 // Single-pass scans: a look-back over the earlier tiles' sums, and stable
 // binning by it (k_rows.cu, k_numeric.cu).
 //
+// The method is the single-pass prefix scan with decoupled look-back (D. Merrill and
+// M. Garland, 2016), with a word layout and bounded waits of this file's own.
+//
 // One launch instead of three: a block takes the next tile of the input (a
 // ticket, so every earlier tile has been started), publishes the tile's sum,
 // and looks back over its predecessors' words until one holds a prefix.  A word

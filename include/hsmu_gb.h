@@ -162,8 +162,8 @@ int hsmu_handle_destroy(hsmu_handle h);
  * are sorted ascending; entries whose products cancel to 0.0 are kept.
  * Values: each product a_ik*b_kj is rounded to double, then added to the
  * entry in the order of A(i,:)'s storage (bit-identical run to run).
- * Stream-ordered on `stream`; returns after one host read of nnz(C) and
- * leaves the remaining kernels queued on `stream`. */
+ * Stream-ordered on `stream`; the host reads nnz(C) in the middle, and the
+ * product is complete when the call returns. */
 int hsmu_spgemm(hsmu_handle h, const hsmu_csr *A, const hsmu_csr *B, hsmu_csr *C,
                 const hsmu_opts *opts, void *stream, hsmu_stats *stats);
 
